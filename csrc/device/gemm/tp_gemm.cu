@@ -129,18 +129,36 @@ bool tailWorkspace(int device, cudaStream_t s, TailWs* out) {
   return true;
 }
 
-int* errFlagFor(int device) {
+// What every launch asks of the device, asked once.
+struct DeviceInfo { int sms; };
+const DeviceInfo& deviceInfo(int device) {
+  static DeviceInfo info[64];
+  static std::once_flag once[64];
+  device &= 63;
+  std::call_once(once[device], [&] {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    info[device].sms = sms;
+  });
+  return info[device];
+}
+
+// The word a kernel records an error in: mapped host memory, allocated once per device.
+struct ErrFlag { int* host = nullptr; int* dev = nullptr; };
+ErrFlag errFlagFor(int device) {
   static std::mutex mu;
-  static int* flags[64] = {nullptr};
+  static ErrFlag flags[64];
   std::lock_guard<std::mutex> lk(mu);
-  if (device < 0 || device >= 64) return nullptr;
-  if (flags[device] == nullptr) {
-    int* host = nullptr;
-    if (cudaHostAlloc((void**)&host, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (device < 0 || device >= 64) return ErrFlag{};
+  ErrFlag& f = flags[device];
+  if (f.host == nullptr) {
+    int *host = nullptr, *dev = nullptr;
+    if (cudaHostAlloc((void**)&host, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return ErrFlag{}; }
+    if (cudaHostGetDevicePointer((void**)&dev, host, 0) != cudaSuccess) { cudaGetLastError(); cudaFreeHost(host); return ErrFlag{}; }
     *host = 0;
-    flags[device] = host;
+    f.host = host; f.dev = dev;
   }
-  return flags[device];
+  return f;
 }
 
 template <int MODE>
@@ -168,10 +186,9 @@ mcclResult_t launchMode(const GemmArgs& a, int bn, int grid, cudaStream_t s) {
 }
 
 int smCount() {
-  int dev = 0, sms = 148;
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
+  return deviceInfo(dev).sms;
 }
 
 // ---- two-SM kernel: clusters of two CTAs ------------------------------------------------------------------------
@@ -219,7 +236,15 @@ void pairConfig(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int pairs, i
 }
 
 mcclResult_t pairPrepare(const void* fn, int smem) {
+  // Once per kernel and device: the attribute stays with the function.
+  static std::mutex mu;
+  static std::vector<std::pair<const void*, int>> done;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  for (auto& d : done) if (d.first == fn && d.second == dev) return mcclSuccess;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return mcclSystemError; }
+  done.push_back({fn, dev});
   return mcclSuccess;
 }
 
@@ -267,7 +292,7 @@ extern "C" {
 int mcclTpGemmLastError(void) {
   int dev = 0;
   cudaGetDevice(&dev);
-  int* f = errFlagFor(dev);
+  volatile int* f = errFlagFor(dev).host;
   if (f == nullptr) return -1;
   const int v = *f;
   *f = 0;
@@ -305,8 +330,8 @@ mcclResult_t mcclTpGemm(const void* A, const void* B, void* C, int M, int N, int
   a.epilogue = epilogue;
   int dev = 0;
   cudaGetDevice(&dev);
-  int* hostFlag = errFlagFor(dev);
-  if (hostFlag == nullptr || cudaHostGetDevicePointer((void**)&a.errFlag, hostFlag, 0) != cudaSuccess) return mcclSystemError;
+  a.errFlag = errFlagFor(dev).dev;
+  if (a.errFlag == nullptr) return mcclSystemError;
   a.budgetNs = 2000000000ull;
   a.panel = pickPanel(M / BM);
   const int tiles = (M / BM) * (N / bn);
@@ -338,8 +363,8 @@ mcclResult_t mcclTpGemm2(const void* A, const void* B, void* C, int M, int N, in
   a.epilogue = epilogue;
   int dev = 0;
   cudaGetDevice(&dev);
-  int* hostFlag = errFlagFor(dev);
-  if (hostFlag == nullptr || cudaHostGetDevicePointer((void**)&a.errFlag, hostFlag, 0) != cudaSuccess) return mcclSystemError;
+  a.errFlag = errFlagFor(dev).dev;
+  if (a.errFlag == nullptr) return mcclSystemError;
   a.budgetNs = 2000000000ull;
   a.debug = (int)envInt("MCCL_GEMM_DEBUG", 0);
   MCCLCHECK(makeMap(&a.mapC, C, M, N, 32));
@@ -408,8 +433,8 @@ mcclResult_t mcclTpAllGatherGemm(mcclComm_t comm, const void* xShard, void* xFul
     if (a.tailTiles > 0 && a.tailTiles <= 80 && tailWorkspace(comm->device, s, &w)) { a.tailWs = w.ws; a.tailCount = w.count; }
     else a.tailTiles = a.tailSlices = 0;
   }
-  int* hostFlag = errFlagFor(comm->device);
-  if (hostFlag == nullptr || cudaHostGetDevicePointer((void**)&a.errFlag, hostFlag, 0) != cudaSuccess) return mcclSystemError;
+  a.errFlag = errFlagFor(comm->device).dev;
+  if (a.errFlag == nullptr) return mcclSystemError;
   a.peers = comm->cu->peers;
   a.budgetNs = 2 * a.peers.timeoutNs;
   a.callIndex = 1;
@@ -479,8 +504,8 @@ mcclResult_t mcclTpGemmReduceScatter(mcclComm_t comm, const void* H, const void*
   a.C = static_cast<__nv_bfloat16*>(partial);
   a.epilogue = EPI_NONE;
   if (two) { MCCLCHECK(makeMap(&a.mapC, partial, M, N, 32)); a.tmaStore = 1; }
-  int* hostFlag = errFlagFor(comm->device);
-  if (hostFlag == nullptr || cudaHostGetDevicePointer((void**)&a.errFlag, hostFlag, 0) != cudaSuccess) return mcclSystemError;
+  a.errFlag = errFlagFor(comm->device).dev;
+  if (a.errFlag == nullptr) return mcclSystemError;
   a.peers = comm->cu->peers;
   a.budgetNs = 2 * a.peers.timeoutNs;
   a.callIndex = callIndex;

@@ -1,5 +1,5 @@
 // Fused softmax cross-entropy over bf16 logits for the language-model head.
-//   forward : one CTA per row, one pass (online max / sum-of-exponentials in fp32) -> per-row loss and
+//   forward : one CTA per row (several when rows are few), one pass (online max / sum-of-exponentials in fp32) -> per-row loss and
 //             log-sum-exp; the 8192 x 50304 logits are read once and never widened to an fp32 tensor.
 //   backward: dlogits = (exp(logit - lse) - [j == target]) * grad / rows, written in bf16 over the logits
 //             (they are not needed afterwards); padding columns beyond the vocabulary get zero.
@@ -9,39 +9,82 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "col_reduce.cuh"
 #include "mccl.h"
 #include "mccl_ops.h"
 
 namespace {
 
-constexpr int kCeThreads = 256;
+using namespace mccl;
 
-struct MaxSum { float m, s; };
+constexpr int kCeThreads = 512;
+constexpr int kCeUnroll = 4;                   // 16-byte pieces in flight per thread: with one, the row's loads wait for each other
+constexpr float kLog2e = 1.4426950408889634f;
+
+struct MaxSum { float m, s; };                 // running maximum and sum of exp(x - m)
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ MaxSum combine(MaxSum a, MaxSum b) {
   const float m = fmaxf(a.m, b.m);
   if (m == -INFINITY) return MaxSum{m, 0.f};
-  return MaxSum{m, a.s * __expf(a.m - m) + b.s * __expf(b.m - m)};
+  return MaxSum{m, a.s * ex2((a.m - m) * kLog2e) + b.s * ex2((b.m - m) * kLog2e)};
 }
-__device__ __forceinline__ void push(MaxSum& a, float x) {
-  if (x > a.m) { a.s = a.s * __expf(a.m - x) + 1.f; a.m = x; }
-  else a.s += __expf(x - a.m);
+__device__ __forceinline__ void unpack(const uint4& q, float* f) {
+  const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { const float2 t = __bfloat1622float2(e[k]); f[2 * k] = t.x; f[2 * k + 1] = t.y; }
+}
+// Eight values at once: one comparison with the running maximum and, in the common case that it stands, eight fused
+// multiply-adds and exponentials with no branch between them.  (One value at a time, every value waits for a branch: the
+// forward pass took 217 us on 8192 x 50257, 3.8 TB/s; this form takes 163 us, 5.0 TB/s.)
+__device__ __forceinline__ void push8(MaxSum& a, const uint4& q) {
+  float f[8];
+  unpack(q, f);
+  const float mx = fmaxf(fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])), fmaxf(fmaxf(f[4], f[5]), fmaxf(f[6], f[7])));
+  if (mx > a.m) { a.s *= ex2((a.m - mx) * kLog2e); a.m = mx; }
+  const float off = a.m == -INFINITY ? 0.f : -a.m * kLog2e;
+  float t[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) t[k] = ex2(fmaf(f[k], kLog2e, off));
+  a.s += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+}
+__device__ __forceinline__ void push1(MaxSum& a, float x) {
+  if (x > a.m) { a.s *= ex2((a.m - x) * kLog2e); a.m = x; }
+  if (x != -INFINITY) a.s += ex2((x - a.m) * kLog2e);
 }
 
+// The part of a row between its first and last 16-byte boundary: [head, head + 8 * vecs) of n elements.
+struct Span { int head, vecs; };
+__device__ __forceinline__ Span spanOf(const __nv_bfloat16* x, int n) {
+  int head = (int)((16u - (uint32_t)(reinterpret_cast<uintptr_t>(x) & 15u)) & 15u) / 2;
+  if (head > n) head = n;
+  return Span{head, (n - head) / 8};
+}
+
+// A cluster of CTAs per row (one CTA each when there are enough rows to fill the GPU): CTA r takes every
+// clusterSize-th tile of the row, and the per-CTA (maximum, sum) pairs meet in CTA 0's shared memory.
 __global__ void __launch_bounds__(kCeThreads) ceForwardKernel(const __nv_bfloat16* logits, int64_t ld, int vocab,
                                                               const int64_t* targets, float* loss, float* lse) {
   __shared__ MaxSum warpAcc[kCeThreads / 32];
-  const int64_t row = blockIdx.x;
+  __shared__ MaxSum ctaAcc;
+  const uint32_t R = colred::clusterSize(), r = colred::clusterRank();
+  const int64_t row = blockIdx.x / R;
   const __nv_bfloat16* x = logits + row * ld;
   MaxSum acc{-INFINITY, 0.f};
-  const bool vec = ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
-  const int nVec = vec ? vocab / 8 : 0;
-  for (int i = threadIdx.x; i < nVec; i += kCeThreads) {
-    const uint4 q = reinterpret_cast<const uint4*>(x)[i];
-    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
+  const Span sp = spanOf(x, vocab);
+  const uint4* v = reinterpret_cast<const uint4*>(x + sp.head);
+  const int stride = (int)R * kCeThreads;
+  for (int i = (int)r * kCeThreads + threadIdx.x; i < sp.vecs; i += kCeUnroll * stride) {
+    uint4 q[kCeUnroll];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) push(acc, __bfloat162float(e[k]));
+    for (int u = 0; u < kCeUnroll; ++u) if (i + u * stride < sp.vecs) q[u] = v[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < kCeUnroll; ++u) if (i + u * stride < sp.vecs) push8(acc, q[u]);
   }
-  for (int i = nVec * 8 + threadIdx.x; i < vocab; i += kCeThreads) push(acc, __bfloat162float(x[i]));
+  if (r == 0) {
+    const int tail = sp.head + sp.vecs * 8;
+    if ((int)threadIdx.x < sp.head) push1(acc, __bfloat162float(x[threadIdx.x]));
+    if (tail + (int)threadIdx.x < vocab) push1(acc, __bfloat162float(x[tail + threadIdx.x]));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     MaxSum other{__shfl_xor_sync(0xffffffffu, acc.m, o), __shfl_xor_sync(0xffffffffu, acc.s, o)};
@@ -52,41 +95,97 @@ __global__ void __launch_bounds__(kCeThreads) ceForwardKernel(const __nv_bfloat1
   if (threadIdx.x == 0) {
     MaxSum t = warpAcc[0];
     for (int w = 1; w < kCeThreads / 32; ++w) t = combine(t, warpAcc[w]);
+    ctaAcc = t;
+  }
+  if (R > 1) colred::clusterSync();
+  if (r == 0 && threadIdx.x == 0) {
+    MaxSum t = ctaAcc;
+    for (uint32_t p = 1; p < R; ++p) t = combine(t, MaxSum{colred::ldPeerShared(&ctaAcc.m, p), colred::ldPeerShared(&ctaAcc.s, p)});
     const float l = t.m + logf(t.s);
     const int64_t tgt = targets[row];
     lse[row] = l;
     loss[row] = (tgt >= 0 && tgt < vocab) ? l - __bfloat162float(x[tgt]) : 0.f;     // out-of-range target: ignored row
   }
+  if (R > 1) colred::clusterSync();
 }
 
+// mean over the rows' losses, in a fixed order.
+__global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, float* out) {
+  __shared__ float acc[32];
+  float t = 0.f;
+  for (int64_t i = threadIdx.x; i < n; i += 8 * 1024) {
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = i + u * 1024 < n ? v[i + u * 1024] : 0.f;
+    t += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) acc[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  t = acc[threadIdx.x];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) *out = t / (float)n;
+}
+
+// Reads and writes every logit once: 301 us on 8192 x 50304 with one piece in flight, 288 us (5.7 TB/s) with four.
+// blockIdx.y: which slice of the row (one unless there are few rows).  The last rows come first: they are what the forward
+// pass, or the projection, left in L2.
 __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* logits, int64_t ld, int vocab, int width,
                                                                const int64_t* targets, const float* lse, const float* gradOut,
                                                                float invRows) {
-  const int64_t row = blockIdx.x;
+  const int64_t row = (int64_t)gridDim.x - 1 - blockIdx.x;
   __nv_bfloat16* x = logits + row * ld;
   const float l = lse[row];
-  const int64_t tgt = targets[row];
-  const bool live = tgt >= 0 && tgt < vocab;
+  const int64_t tgt64 = targets[row];
+  const bool live = tgt64 >= 0 && tgt64 < vocab;
+  const int tgt = live ? (int)tgt64 : -1;
   const float scale = live ? (*gradOut) * invRows : 0.f;
-  const bool vec = ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
-  const int nVec = vec ? width / 8 : 0;
-  for (int i = threadIdx.x; i < nVec; i += kCeThreads) {
-    uint4 q = reinterpret_cast<const uint4*>(x)[i];
-    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&q);
+  const float off = -l * kLog2e;
+  auto one = [&](int j, float xj) -> float {
+    if (j >= vocab) return 0.f;
+    return (ex2(fmaf(xj, kLog2e, off)) - (j == tgt ? 1.f : 0.f)) * scale;
+  };
+  const Span sp = spanOf(x, width);
+  uint4* v = reinterpret_cast<uint4*>(x + sp.head);
+  const int stride = (int)gridDim.y * kCeThreads;
+  for (int i = (int)blockIdx.y * kCeThreads + threadIdx.x; i < sp.vecs; i += kCeUnroll * stride) {
+    uint4 q[kCeUnroll];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int j = i * 8 + k;
-      float g = 0.f;
-      if (j < vocab) g = (__expf(__bfloat162float(e[k]) - l) - (j == tgt ? 1.f : 0.f)) * scale;
-      e[k] = __float2bfloat16_rn(g);
+    for (int u = 0; u < kCeUnroll; ++u) if (i + u * stride < sp.vecs) q[u] = v[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < kCeUnroll; ++u) {
+      if (i + u * stride >= sp.vecs) continue;
+      const int j0 = sp.head + (i + u * stride) * 8;
+      float f[8];
+      unpack(q[u], f);
+      if (j0 + 8 <= vocab && (unsigned)(tgt - j0) >= 8u) {       // neither the target nor padding in these eight
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = ex2(fmaf(f[k], kLog2e, off)) * scale;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = one(j0 + k, f[k]);
+      }
+      __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&q[u]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) e[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+      v[i + u * stride] = q[u];
     }
-    reinterpret_cast<uint4*>(x)[i] = q;
   }
-  for (int j = nVec * 8 + threadIdx.x; j < width; j += kCeThreads) {
-    float g = 0.f;
-    if (j < vocab) g = (__expf(__bfloat162float(x[j]) - l) - (j == tgt ? 1.f : 0.f)) * scale;
-    x[j] = __float2bfloat16_rn(g);
+  if (blockIdx.y == 0) {
+    const int tail = sp.head + sp.vecs * 8, h = threadIdx.x, t = tail + (int)threadIdx.x;
+    if (h < sp.head) x[h] = __float2bfloat16_rn(one(h, __bfloat162float(x[h])));
+    if (t < width) x[t] = __float2bfloat16_rn(one(t, __bfloat162float(x[t])));
   }
+}
+
+// CTAs per row: with fewer rows than SMs a row is shared by up to eight, as long as each keeps a tile of it.
+int ceSplit(int64_t rows, int n) {
+  int r = 1;
+  while (r < 8 && rows * r * 2 <= 148 && n / (r * 2) >= kCeThreads * 8) r *= 2;
+  return r;
 }
 
 }  // namespace
@@ -97,8 +196,18 @@ extern "C" mcclResult_t mcclCrossEntropyForward(const void* logits, int64_t rows
   if (logits == nullptr || targets == nullptr || loss == nullptr || lse == nullptr || rows < 0 || vocab <= 0 || ld < vocab)
     return mcclInvalidArgument;
   if (rows == 0) return mcclSuccess;
-  ceForwardKernel<<<(unsigned)rows, kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(logits), ld, vocab, targets, loss, lse);
+  const int split = ceSplit(rows, vocab);
+  return colred::launch(ceForwardKernel, (int)rows * split, split, kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream),
+                        static_cast<const __nv_bfloat16*>(logits), ld, vocab, targets, loss, lse) == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
+
+// The same followed by the mean of the rows' losses in *mean.
+extern "C" mcclResult_t mcclCrossEntropyMean(const void* logits, int64_t rows, int64_t ld, int vocab, const int64_t* targets, float* loss,
+                                             float* lse, float* mean, mcclStream_t stream) {
+  if (mean == nullptr) return mcclInvalidArgument;
+  const mcclResult_t rc = mcclCrossEntropyForward(logits, rows, ld, vocab, targets, loss, lse, stream);
+  if (rc != mcclSuccess) return rc;
+  meanKernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(loss, rows, mean);     // no rows: 0 / 0, as a mean over none
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 
@@ -109,7 +218,7 @@ extern "C" mcclResult_t mcclCrossEntropyBackward(void* logits, int64_t rows, int
   if (logits == nullptr || targets == nullptr || lse == nullptr || gradOut == nullptr || rows < 0 || vocab <= 0 || width < vocab ||
       ld < width) return mcclInvalidArgument;
   if (rows == 0) return mcclSuccess;
-  ceBackwardKernel<<<(unsigned)rows, kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  ceBackwardKernel<<<dim3((unsigned)rows, (unsigned)ceSplit(rows, width)), kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       static_cast<__nv_bfloat16*>(logits), ld, vocab, width, targets, lse, gradOut, 1.0f / (float)rows);
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }

@@ -1,23 +1,29 @@
-// LayerNorm forward and backward for bf16 activations with rows of 256, 512 or 1024 elements (wider rows
-// would spill the per-lane column sums out of registers; callers fall back to the framework's kernel).
-// One warp per row, each lane holding VPL 16-byte vectors of the row in registers.
-//   forward : mean / rstd by warp shuffles, y = (x - mean) * rstd * gamma + beta, mean and rstd saved in fp32.
-//   backward: dx per row from two warp reductions; every lane also accumulates dgamma / dbeta of its columns
-//             over the rows its warp walks, the CTA folds its warps through shared memory and writes one
-//             partial per CTA; a second small kernel adds the partials.  One pass over x and dy instead of
-//             the separate (and slow) column-reduction kernel of an unfused backward.
+// LayerNorm and RMSNorm forward and backward for bf16 activations, rows of up to 4096 elements (a multiple of 8).
+// A group of W warps owns a row, every lane holding VPL 16-byte vectors of it in registers, so a row is read once.
+//   forward : mean / rstd by warp shuffles, y = (x - mean) * rstd * gamma + beta, mean and rstd saved in fp32.  With
+//             `delta` the row is x + delta, rounded to bf16 and written out too: the residual add of a pre-norm block and
+//             the norm behind it in one pass over memory.
+//   backward: dx per row from two reductions; every lane also accumulates dgamma / dbeta of its columns over the rows its
+//             group walks (col_reduce.cuh adds them up).  With `dres` the gradient that reaches the row past the norm (the
+//             residual branch) is added, and the column sums of the total can be had as well: the bias gradient of the
+//             projection that produced `delta`.
+// Both are bound by memory: forward 4 bytes an element (8 with delta), backward 6 (8 with dres).
 // No counterpart in the reference (it has no model code).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "col_reduce.cuh"
 #include "mccl.h"
 #include "mccl_ops.h"
 
 namespace {
 
-constexpr int kLnWarps = 4;
+using namespace mccl;
+
+constexpr int kLnWarps = 8;
 constexpr int kLnThreads = kLnWarps * 32;
+constexpr int kLnMaxD = 4096;
 
 __device__ __forceinline__ float warpSum(float v) {
 #pragma unroll
@@ -25,176 +31,344 @@ __device__ __forceinline__ float warpSum(float v) {
   return v;
 }
 
-template <int VPL>
-__global__ void __launch_bounds__(kLnThreads) lnForwardKernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma,
-                                                              const __nv_bfloat16* beta, __nv_bfloat16* y, float* mean,
-                                                              float* rstd, int64_t rows, float eps) {
-  constexpr int D = VPL * 256;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float g[VPL * 8], b[VPL * 8];
+// Sum of (a, b) over the W warps of a row's group.  `slot`: shared memory of two floats a warp, alternating between two
+// copies from call to call, which makes one barrier per call enough.
+template <int W>
+__device__ __forceinline__ float2 groupSum(float a, float b, float2* slot, int group, int warpInGroup) {
+  a = warpSum(a); b = warpSum(b);
+  if (W == 1) return make_float2(a, b);
+  if ((threadIdx.x & 31) == 0) slot[group * W + warpInGroup] = make_float2(a, b);
+  asm volatile("bar.sync %0, %1;" :: "r"(1 + group), "n"(W * 32) : "memory");
+  float2 t = slot[group * W];
 #pragma unroll
-  for (int j = 0; j < VPL; ++j) {
-    const uint4 gq = reinterpret_cast<const uint4*>(gamma)[lane + 32 * j], bq = reinterpret_cast<const uint4*>(beta)[lane + 32 * j];
-    const __nv_bfloat16* ge = reinterpret_cast<const __nv_bfloat16*>(&gq);
-    const __nv_bfloat16* be = reinterpret_cast<const __nv_bfloat16*>(&bq);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { g[j * 8 + k] = __bfloat162float(ge[k]); b[j * 8 + k] = __bfloat162float(be[k]); }
-  }
-  for (int64_t row = (int64_t)blockIdx.x * kLnWarps + warp; row < rows; row += (int64_t)gridDim.x * kLnWarps) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * D);
-    float v[VPL * 8];
-    float s = 0.f;
-#pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-      const uint4 q = xr[lane + 32 * j];
-      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { v[j * 8 + k] = __bfloat162float(e[k]); s += v[j * 8 + k]; }
-    }
-    const float mu = warpSum(s) * (1.0f / D);
-    float sq = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPL * 8; ++i) { const float d = v[i] - mu; sq += d * d; }
-    const float rs = rsqrtf(warpSum(sq) * (1.0f / D) + eps);
-    uint4* yr = reinterpret_cast<uint4*>(y + row * D);
-#pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-      uint4 q;
-      __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&q);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) e[k] = __float2bfloat16_rn((v[j * 8 + k] - mu) * rs * g[j * 8 + k] + b[j * 8 + k]);
-      yr[lane + 32 * j] = q;
-    }
-    if (lane == 0) { mean[row] = mu; rstd[row] = rs; }
-  }
+  for (int w = 1; w < W; ++w) { const float2 u = slot[group * W + w]; t.x += u.x; t.y += u.y; }
+  return t;
 }
 
-template <int VPL>
-__global__ void __launch_bounds__(kLnThreads) lnBackwardKernel(const __nv_bfloat16* x, const __nv_bfloat16* dy,
-                                                               const __nv_bfloat16* gamma, const float* mean, const float* rstd,
-                                                               __nv_bfloat16* dx, float* partial, int64_t rows) {
-  constexpr int D = VPL * 256;
-  __shared__ float red[kLnWarps][D];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float g[VPL * 8], dg[VPL * 8], db[VPL * 8];
+__device__ __forceinline__ void unpack(const uint4& q, float* f) {
+  const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { const float2 t = __bfloat1622float2(e[k]); f[2 * k] = t.x; f[2 * k + 1] = t.y; }
+}
+__device__ __forceinline__ uint4 pack(const float* f) {
+  uint4 q;
+  __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) e[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+  return q;
+}
+
+struct LnFwdArgs {
+  const uint4 *x, *delta, *gamma, *beta;       // delta, beta: may be null
+  uint4 *sum, *y;                              // sum: x + delta, written when delta is given
+  float *mean, *rstd;                          // mean: null for RMSNorm
+  int64_t rows;
+  int D;
+  float eps;
+};
+
+// One row per group and no loop: every load of a row is issued before the first wait, and 64 warps a SM keep up to 128 KB
+// in flight.  Gamma and beta come from L1 after a CTA's first row.
+template <int W, int VPL, bool RMS>
+__global__ void __launch_bounds__(kLnThreads) lnForwardKernel(const __grid_constant__ LnFwdArgs a) {
+  constexpr int G = kLnWarps / W, T = W * 32;
+  __shared__ float2 slots[2][kLnWarps];
+  const int group = threadIdx.x / T, t = threadIdx.x % T, vecs = a.D / 8;
+  const int64_t row = (int64_t)blockIdx.x * G + group;
+  if (row >= a.rows) return;
+  const uint4* xr = a.x + row * vecs;
+  const uint4* dr = a.delta + row * vecs;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 xq[VPL], dq[VPL], gq[VPL], bq[VPL];
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
-    const uint4 gq = reinterpret_cast<const uint4*>(gamma)[lane + 32 * j];
-    const __nv_bfloat16* ge = reinterpret_cast<const __nv_bfloat16*>(&gq);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { g[j * 8 + k] = __bfloat162float(ge[k]); dg[j * 8 + k] = 0.f; db[j * 8 + k] = 0.f; }
+    const int i = t + T * j;
+    const bool in = i < vecs;
+    xq[j] = in ? xr[i] : zero;
+    dq[j] = in && a.delta != nullptr ? dr[i] : zero;
+    gq[j] = in ? a.gamma[i] : zero;
+    bq[j] = in && !RMS ? a.beta[i] : zero;
   }
-  for (int64_t row = (int64_t)blockIdx.x * kLnWarps + warp; row < rows; row += (int64_t)gridDim.x * kLnWarps) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * D);
-    const uint4* dr = reinterpret_cast<const uint4*>(dy + row * D);
-    uint4 xq[VPL], dq[VPL];
+  float v[VPL * 8];
+  float s = 0.f, ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) { xq[j] = xr[lane + 32 * j]; dq[j] = dr[lane + 32 * j]; }
-    const float mu = mean[row], rs = rstd[row];
+  for (int j = 0; j < VPL; ++j) {
+    unpack(xq[j], v + 8 * j);
+    if (a.delta != nullptr) {
+      float d[8];
+      unpack(dq[j], d);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[8 * j + k] += d[k];
+      const uint4 q = pack(v + 8 * j);
+      unpack(q, v + 8 * j);                    // the norm reads what a separate add would have stored
+      if (t + T * j < vecs) a.sum[row * vecs + t + T * j] = q;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { s += v[8 * j + k]; if (RMS) ss += v[8 * j + k] * v[8 * j + k]; }
+  }
+  const float invD = 1.0f / (float)a.D;
+  float mu = 0.f, rs;
+  if (RMS) {
+    rs = rsqrtf(groupSum<W>(0.f, ss, slots[0], group, t >> 5).y * invD + a.eps);
+  } else {
+    mu = groupSum<W>(s, 0.f, slots[0], group, t >> 5).x * invD;
+    float sq = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j)
+      if (t + T * j < vecs)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { const float d = v[8 * j + k] - mu; sq += d * d; }
+    rs = rsqrtf(groupSum<W>(sq, 0.f, slots[1], group, t >> 5).x * invD + a.eps);
+  }
+#pragma unroll
+  for (int j = 0; j < VPL; ++j) {
+    if (t + T * j >= vecs) continue;
+    float g[8], b[8], y[8];
+    unpack(gq[j], g);
+    unpack(bq[j], b);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (RMS) y[k] = __bfloat162float(__float2bfloat16_rn(v[8 * j + k] * rs)) * g[k];     // normalised, rounded, then scaled
+      else y[k] = (v[8 * j + k] - mu) * rs * g[k] + b[k];
+    }
+    a.y[row * vecs + t + T * j] = pack(y);
+  }
+  if (t == 0) { if (!RMS) a.mean[row] = mu; a.rstd[row] = rs; }
+}
+
+struct LnBwdArgs {
+  const uint4 *x, *dy, *dres, *gamma;          // dres: may be null
+  const float *mean, *rstd;
+  uint4* dx;
+  float* partial;
+  int64_t rows;
+  int D;
+  colred::Out out;                             // dgamma, dbeta, column sums of dx
+};
+
+// Rows are walked by a fixed number of CTAs (two per SM) so that a lane can keep its columns' sums in registers; the
+// vectors of the next row are loaded before the current one is worked on.  Two vectors per lane bound the registers: 16
+// columns x (three sums + gamma) + two rows of x, dy and dres.
+template <int W, int VPL, bool RMS, bool RES>
+__global__ void __launch_bounds__(kLnThreads, VPL == 1 ? 3 : 2) lnBackwardKernel(const __grid_constant__ LnBwdArgs a) {
+  constexpr int G = kLnWarps / W, T = W * 32;
+  extern __shared__ float cols[];
+  __shared__ float2 slots[2][kLnWarps];
+  const int group = threadIdx.x / T, t = threadIdx.x % T, vecs = a.D / 8;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const bool third = RES && !RMS && a.out.segments == 3;
+  float g[VPL * 8], dg[VPL * 8], db[VPL * 8], dc[VPL * 8];
+#pragma unroll
+  for (int j = 0; j < VPL; ++j) {
+    unpack(t + T * j < vecs ? a.gamma[t + T * j] : zero, g + 8 * j);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) dg[8 * j + k] = db[8 * j + k] = dc[8 * j + k] = 0.f;
+  }
+  const float invD = 1.0f / (float)a.D;
+  const int64_t step = (int64_t)gridDim.x * G;
+  int64_t row = (int64_t)blockIdx.x * G + group;
+  uint4 xq[VPL], dq[VPL], rq[VPL];
+  float mu = 0.f, rs = 0.f;
+  auto load = [&](int64_t r) {
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      const int i = t + T * j;
+      const bool in = r < a.rows && i < vecs;
+      xq[j] = in ? a.x[r * vecs + i] : zero;
+      dq[j] = in ? a.dy[r * vecs + i] : zero;
+      if (RES) rq[j] = in ? a.dres[r * vecs + i] : zero;
+    }
+    if (r < a.rows) { if (!RMS) mu = a.mean[r]; rs = a.rstd[r]; }
+  };
+  load(row);
+  for (int par = 0; row < a.rows; row += step, par ^= 1) {
+    uint4 xc[VPL], dc4[VPL], rc[VPL];
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) { xc[j] = xq[j]; dc4[j] = dq[j]; if (RES) rc[j] = rq[j]; }
+    const float m = mu, r = rs;
+    load(row + step);
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
-      const __nv_bfloat16* xe = reinterpret_cast<const __nv_bfloat16*>(&xq[j]);
-      const __nv_bfloat16* de = reinterpret_cast<const __nv_bfloat16*>(&dq[j]);
+      float xf[8], df[8];
+      unpack(xc[j], xf);
+      unpack(dc4[j], df);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float xh = (__bfloat162float(xe[k]) - mu) * rs, d = __bfloat162float(de[k]), gd = d * g[j * 8 + k];
+        const float xh = (xf[k] - m) * r, gd = df[k] * g[8 * j + k];
         s1 += gd; s2 += gd * xh;
-        dg[j * 8 + k] += d * xh; db[j * 8 + k] += d;
+        dg[8 * j + k] += df[k] * (RMS ? __bfloat162float(__float2bfloat16_rn(xh)) : xh);
+        if (!RMS) db[8 * j + k] += df[k];
       }
     }
-    s1 = warpSum(s1) * (1.0f / D);
-    s2 = warpSum(s2) * (1.0f / D);
-    uint4* outr = reinterpret_cast<uint4*>(dx + row * D);
+    float2 sums = groupSum<W>(s1, s2, slots[par], group, t >> 5);
+    s1 = RMS ? 0.f : sums.x * invD;
+    s2 = sums.y * invD;
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
-      const __nv_bfloat16* xe = reinterpret_cast<const __nv_bfloat16*>(&xq[j]);
-      const __nv_bfloat16* de = reinterpret_cast<const __nv_bfloat16*>(&dq[j]);
-      uint4 q;
-      __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&q);
+      if (t + T * j >= vecs) continue;
+      float xf[8], df[8], o[8];
+      unpack(xc[j], xf);
+      unpack(dc4[j], df);
+      if (RES) unpack(rc[j], o);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float xh = (__bfloat162float(xe[k]) - mu) * rs, gd = __bfloat162float(de[k]) * g[j * 8 + k];
-        e[k] = __float2bfloat16_rn(rs * (gd - s1 - xh * s2));
+        const float xh = (xf[k] - m) * r, gd = df[k] * g[8 * j + k];
+        o[k] = r * (gd - s1 - xh * s2) + (RES ? o[k] : 0.f);
       }
-      outr[lane + 32 * j] = q;
+      const uint4 q = pack(o);
+      if (third) {
+        unpack(q, o);                          // the sum over what is stored, as a separate reduction would read it
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dc[8 * j + k] += o[k];
+      }
+      a.dx[row * vecs + t + T * j] = q;
     }
   }
-  // Fold the four warps' column sums, dgamma first, then dbeta, through shared memory.
-  float* out = partial + (int64_t)blockIdx.x * 2 * D;
-  for (int pass = 0; pass < 2; ++pass) {
-    __syncthreads();
+  const int C = a.out.segments * a.D;
+  float* mine = cols + group * C;
 #pragma unroll
-    for (int j = 0; j < VPL; ++j)
+  for (int j = 0; j < VPL; ++j) {
+    if (t + T * j >= vecs) continue;
+    const int c = (t + T * j) * 8;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) red[warp][(lane + 32 * j) * 8 + k] = pass == 0 ? dg[j * 8 + k] : db[j * 8 + k];
-    __syncthreads();
-    for (int c = threadIdx.x; c < D; c += kLnThreads) {
-      float t = 0.f;
-#pragma unroll
-      for (int w = 0; w < kLnWarps; ++w) t += red[w][c];
-      out[pass * D + c] = t;
+    for (int k = 0; k < 8; ++k) {
+      mine[c + k] = dg[8 * j + k];
+      if (a.out.segments > 1) mine[a.D + c + k] = db[8 * j + k];
+      if (third) mine[2 * a.D + c + k] = dc[8 * j + k];
     }
   }
-}
-
-__global__ void lnReducePartialsKernel(const float* partial, int nPartials, int D, __nv_bfloat16* dgamma, __nv_bfloat16* dbeta) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= 2 * D) return;
-  float t = 0.f;
-  for (int p = 0; p < nPartials; ++p) t += partial[(int64_t)p * 2 * D + c];
-  if (c < D) dgamma[c] = __float2bfloat16_rn(t); else dbeta[c - D] = __float2bfloat16_rn(t);
-}
-
-int lnGrid(int64_t rows) {
-  int64_t ctas = (rows + kLnWarps * 8 - 1) / (kLnWarps * 8);     // about eight rows per warp
-  if (ctas > 148 * 4) ctas = 148 * 4;
-  return ctas < 1 ? 1 : (int)ctas;
+  colred::finish(cols, G, C, a.partial, a.out);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+template <int W, int VPL, bool RMS>
+cudaError_t fwd(const LnFwdArgs& a, cudaStream_t s) {
+  constexpr int G = kLnWarps / W;
+  lnForwardKernel<W, VPL, RMS><<<(unsigned)((a.rows + G - 1) / G), kLnThreads, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+// Up to 1024 columns one warp holds a row (no barrier); wider rows are spread over four warps.
+template <bool RMS>
+cudaError_t fwdAny(const LnFwdArgs& a, cudaStream_t s) {
+  if (a.D <= 256) return fwd<1, 1, RMS>(a, s);
+  if (a.D <= 512) return fwd<1, 2, RMS>(a, s);
+  if (a.D <= 768) return fwd<1, 3, RMS>(a, s);
+  if (a.D <= 1024) return fwd<1, 4, RMS>(a, s);
+  if (a.D <= 2048) return fwd<4, 2, RMS>(a, s);
+  return fwd<4, 4, RMS>(a, s);
+}
+
+template <int W, int VPL, bool RMS, bool RES>
+cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
+  constexpr int G = kLnWarps / W;
+  static bool opted[64] = {false};             // 48 KB of column sums and the row slots: past the default limit
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!opted[dev & 63]) {
+    const cudaError_t e = cudaFuncSetAttribute(lnBackwardKernel<W, VPL, RMS, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
+    if (e != cudaSuccess) return e;
+    opted[dev & 63] = true;
+  }
+  int cluster;
+  const int grid = colred::grid((a.rows + G * 4 - 1) / (G * 4), VPL == 1 ? 3 : 2, &cluster);      // four rows per group before more CTAs pay
+  const int C = a.out.segments * a.D;
+  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
+  return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, C, a.out, s);
+}
+
+// A lane's columns cost four registers each (three sums and gamma) beside two rows of x, dy and dres: two vectors a lane
+// fit 128 registers without dres and spill with it (8192 x 1024: 26 us, with one vector a lane 19 us).
+template <bool RMS>
+cudaError_t bwdAny(const LnBwdArgs& a, cudaStream_t s) {
+  if (a.dres) {
+    if (a.D <= 256) return bwdLaunch<1, 1, RMS, true>(a, s);
+    if (a.D <= 512) return bwdLaunch<2, 1, RMS, true>(a, s);
+    if (a.D <= 1024) return bwdLaunch<4, 1, RMS, true>(a, s);
+    if (a.D <= 2048) return bwdLaunch<8, 1, RMS, true>(a, s);
+    return bwdLaunch<8, 2, RMS, true>(a, s);
+  }
+  if (a.D <= 256) return bwdLaunch<1, 1, RMS, false>(a, s);
+  if (a.D <= 512) return bwdLaunch<1, 2, RMS, false>(a, s);
+  if (a.D <= 1024) return bwdLaunch<2, 2, RMS, false>(a, s);
+  if (a.D <= 2048) return bwdLaunch<4, 2, RMS, false>(a, s);
+  return bwdLaunch<8, 2, RMS, false>(a, s);
+}
+
+mcclResult_t forward(const void* x, const void* delta, const void* gamma, const void* beta, void* sum, void* y, float* mean, float* rstd,
+                     int64_t rows, int D, float eps, bool rms, mcclStream_t stream) {
+  if (!x || !gamma || !y || !rstd || rows < 0 || (!rms && (!beta || !mean)) || (delta && !sum)) return mcclInvalidArgument;
+  if (D <= 0 || D % 8 || D > kLnMaxD) return mcclInvalidArgument;
+  if (!aligned16(x) || !aligned16(delta) || !aligned16(gamma) || !aligned16(beta) || !aligned16(sum) || !aligned16(y)) return mcclInvalidArgument;
+  if (rows == 0) return mcclSuccess;
+  LnFwdArgs a;
+  a.x = static_cast<const uint4*>(x); a.delta = static_cast<const uint4*>(delta);
+  a.gamma = static_cast<const uint4*>(gamma); a.beta = static_cast<const uint4*>(beta);
+  a.sum = static_cast<uint4*>(sum); a.y = static_cast<uint4*>(y);
+  a.mean = mean; a.rstd = rstd; a.rows = rows; a.D = D; a.eps = eps;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return (rms ? fwdAny<true>(a, s) : fwdAny<false>(a, s)) == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
+
+mcclResult_t backward(const void* x, const void* dy, const void* dres, const void* gamma, const float* mean, const float* rstd, void* dx,
+                      void* dgamma, void* dbeta, void* dcol, int accumulate, float* partial, int64_t rows, int D, bool rms,
+                      mcclStream_t stream) {
+  if (!x || !dy || !gamma || !rstd || !dx || !dgamma || !partial || rows <= 0 || (!rms && (!mean || !dbeta)) || (dcol && !dres)) return mcclInvalidArgument;
+  if (D <= 0 || D % 8 || D > kLnMaxD) return mcclInvalidArgument;
+  if (!aligned16(x) || !aligned16(dy) || !aligned16(dres) || !aligned16(gamma) || !aligned16(dx)) return mcclInvalidArgument;
+  LnBwdArgs a;
+  a.x = static_cast<const uint4*>(x); a.dy = static_cast<const uint4*>(dy); a.dres = static_cast<const uint4*>(dres);
+  a.gamma = static_cast<const uint4*>(gamma); a.mean = mean; a.rstd = rstd;
+  a.dx = static_cast<uint4*>(dx); a.partial = partial; a.rows = rows; a.D = D;
+  a.out = colred::Out{};
+  a.out.seg[0] = static_cast<__nv_bfloat16*>(dgamma); a.out.seg[1] = static_cast<__nv_bfloat16*>(dbeta);
+  a.out.seg[2] = static_cast<__nv_bfloat16*>(dcol);
+  a.out.segments = dcol && dres ? 3 : dbeta ? 2 : 1; a.out.width = D; a.out.accumulate = accumulate;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return (rms ? bwdAny<true>(a, s) : bwdAny<false>(a, s)) == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
+
 }  // namespace
 
-// Number of CTAs the backward pass uses for `rows` rows = number of fp32 partials of 2*D floats it writes.
-extern "C" int mcclLayerNormPartials(int64_t rows) { return lnGrid(rows); }
+// Partial sums the backward pass may write for `rows` rows (fp32, up to 3 x D each).
+extern "C" int mcclLayerNormPartials(int64_t rows) { return rows <= 0 ? 1 : colred::kMaxPartials; }
 
 extern "C" mcclResult_t mcclLayerNormForward(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                                              int64_t rows, int D, float eps, mcclStream_t stream) {
-  if (!x || !gamma || !beta || !y || !mean || !rstd || rows < 0) return mcclInvalidArgument;
-  if (!aligned16(x) || !aligned16(gamma) || !aligned16(beta) || !aligned16(y)) return mcclInvalidArgument;
-  if (rows == 0) return mcclSuccess;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  auto* X = static_cast<const __nv_bfloat16*>(x); auto* G = static_cast<const __nv_bfloat16*>(gamma);
-  auto* B = static_cast<const __nv_bfloat16*>(beta); auto* Y = static_cast<__nv_bfloat16*>(y);
-  const int grid = lnGrid(rows);
-  switch (D) {
-    case 256:  lnForwardKernel<1><<<grid, kLnThreads, 0, s>>>(X, G, B, Y, mean, rstd, rows, eps); break;
-    case 512:  lnForwardKernel<2><<<grid, kLnThreads, 0, s>>>(X, G, B, Y, mean, rstd, rows, eps); break;
-    case 1024: lnForwardKernel<4><<<grid, kLnThreads, 0, s>>>(X, G, B, Y, mean, rstd, rows, eps); break;
-    default: return mcclInvalidArgument;
-  }
-  return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
+  return forward(x, nullptr, gamma, beta, nullptr, y, mean, rstd, rows, D, eps, false, stream);
+}
+
+// sum = x + delta (rounded to bf16), y = LayerNorm(sum).
+extern "C" mcclResult_t mcclAddLayerNormForward(const void* x, const void* delta, const void* gamma, const void* beta, void* sum, void* y,
+                                                float* mean, float* rstd, int64_t rows, int D, float eps, mcclStream_t stream) {
+  if (!delta) return mcclInvalidArgument;
+  return forward(x, delta, gamma, beta, sum, y, mean, rstd, rows, D, eps, false, stream);
 }
 
 // partial: fp32 work memory of mcclLayerNormPartials(rows) * 2 * D floats.
 extern "C" mcclResult_t mcclLayerNormBackward(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                                               void* dx, void* dgamma, void* dbeta, float* partial, int64_t rows, int D,
                                               mcclStream_t stream) {
-  if (!x || !dy || !gamma || !mean || !rstd || !dx || !dgamma || !dbeta || !partial || rows <= 0) return mcclInvalidArgument;
-  if (!aligned16(x) || !aligned16(dy) || !aligned16(gamma) || !aligned16(dx)) return mcclInvalidArgument;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  auto* X = static_cast<const __nv_bfloat16*>(x); auto* DY = static_cast<const __nv_bfloat16*>(dy);
-  auto* G = static_cast<const __nv_bfloat16*>(gamma); auto* DX = static_cast<__nv_bfloat16*>(dx);
-  const int grid = lnGrid(rows);
-  switch (D) {
-    case 256:  lnBackwardKernel<1><<<grid, kLnThreads, 0, s>>>(X, DY, G, mean, rstd, DX, partial, rows); break;
-    case 512:  lnBackwardKernel<2><<<grid, kLnThreads, 0, s>>>(X, DY, G, mean, rstd, DX, partial, rows); break;
-    case 1024: lnBackwardKernel<4><<<grid, kLnThreads, 0, s>>>(X, DY, G, mean, rstd, DX, partial, rows); break;
-    default: return mcclInvalidArgument;
-  }
-  if (cudaGetLastError() != cudaSuccess) return mcclSystemError;
-  lnReducePartialsKernel<<<(2 * D + 255) / 256, 256, 0, s>>>(partial, grid, D, static_cast<__nv_bfloat16*>(dgamma),
-                                                             static_cast<__nv_bfloat16*>(dbeta));
-  return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
+  return backward(x, dy, nullptr, gamma, mean, rstd, dx, dgamma, dbeta, nullptr, 0, partial, rows, D, false, stream);
+}
+
+// The same with dx += dres and, when dcol is given, dcol = column sums of dx (needs dres); `accumulate`: add dgamma, dbeta and dcol to what
+// is there.  partial: mcclLayerNormPartials(rows) * 3 * D floats.
+extern "C" mcclResult_t mcclAddLayerNormBackward(const void* x, const void* dy, const void* dres, const void* gamma, const float* mean,
+                                                 const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate,
+                                                 float* partial, int64_t rows, int D, mcclStream_t stream) {
+  return backward(x, dy, dres, gamma, mean, rstd, dx, dgamma, dbeta, dcol, accumulate, partial, rows, D, false, stream);
+}
+
+// RMSNorm: y = bf16(x * rstd) * gamma; delta / sum as in mcclAddLayerNormForward (both may be null).
+extern "C" mcclResult_t mcclRmsNormForward(const void* x, const void* delta, const void* gamma, void* sum, void* y, float* rstd,
+                                           int64_t rows, int D, float eps, mcclStream_t stream) {
+  return forward(x, delta, gamma, nullptr, sum, y, nullptr, rstd, rows, D, eps, true, stream);
+}
+
+extern "C" mcclResult_t mcclRmsNormBackward(const void* x, const void* dy, const void* dres, const void* gamma, const float* rstd, void* dx,
+                                            void* dgamma, int accumulate, float* partial, int64_t rows, int D, mcclStream_t stream) {
+  return backward(x, dy, dres, gamma, nullptr, rstd, dx, dgamma, nullptr, nullptr, accumulate, partial, rows, D, true, stream);
 }

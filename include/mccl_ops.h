@@ -58,15 +58,30 @@ mcclResult_t mcclSumSquaresBf16(const void* x, uint64_t n, float* scratch, uint6
 /* Cross-entropy over bf16 logits [rows, ld] (vocab <= ld): per-row loss and log-sum-exp; backward in place. */
 mcclResult_t mcclCrossEntropyForward(const void* logits, int64_t rows, int64_t ld, int vocab, const int64_t* targets, float* loss,
                                      float* lse, mcclStream_t stream);
+/* The same with the mean of the rows' losses in *mean. */
+mcclResult_t mcclCrossEntropyMean(const void* logits, int64_t rows, int64_t ld, int vocab, const int64_t* targets, float* loss, float* lse,
+                                  float* mean, mcclStream_t stream);
 mcclResult_t mcclCrossEntropyBackward(void* logits, int64_t rows, int64_t ld, int vocab, int width, const int64_t* targets,
                                       const float* lse, const float* gradOut, mcclStream_t stream);
-/* LayerNorm over bf16 rows of D in {256, 512, 1024}. */
+/* LayerNorm over bf16 rows of D elements, D % 8 == 0 and D <= 4096.  The backward passes need partial:
+ * mcclLayerNormPartials(rows) x 2 x D (3 x D for the Add form) floats of work memory. */
 int          mcclLayerNormPartials(int64_t rows);
 mcclResult_t mcclLayerNormForward(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int64_t rows,
                                   int D, float eps, mcclStream_t stream);
-/* partial: mcclLayerNormPartials(rows) x 2 x D floats of work memory. */
 mcclResult_t mcclLayerNormBackward(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx,
                                    void* dgamma, void* dbeta, float* partial, int64_t rows, int D, mcclStream_t stream);
+/* With the residual add of a pre-norm block: sum = x + delta, y = LayerNorm(sum).  Backward (x: the sum): dx = d sum of the norm +
+ * dres; dcol (nullable, needs dres) = column sums of dx; accumulate: dgamma, dbeta and dcol are added to what is there. */
+mcclResult_t mcclAddLayerNormForward(const void* x, const void* delta, const void* gamma, const void* beta, void* sum, void* y, float* mean,
+                                     float* rstd, int64_t rows, int D, float eps, mcclStream_t stream);
+mcclResult_t mcclAddLayerNormBackward(const void* x, const void* dy, const void* dres, const void* gamma, const float* mean,
+                                      const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate, float* partial,
+                                      int64_t rows, int D, mcclStream_t stream);
+/* RMSNorm, y = bf16(x * rstd) * gamma; delta and sum (nullable) as above; dres nullable. */
+mcclResult_t mcclRmsNormForward(const void* x, const void* delta, const void* gamma, void* sum, void* y, float* rstd, int64_t rows, int D,
+                                float eps, mcclStream_t stream);
+mcclResult_t mcclRmsNormBackward(const void* x, const void* dy, const void* dres, const void* gamma, const float* rstd, void* dx,
+                                 void* dgamma, int accumulate, float* partial, int64_t rows, int D, mcclStream_t stream);
 
 #ifdef __cplusplus
 }

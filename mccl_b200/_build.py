@@ -1,8 +1,8 @@
-"""In-tree build of libmccl.so (host C++ with g++, device code with nvcc for sm_100a).
+"""In-tree build of libmccl.so (host C++ with g++, device code with nvcc for sm_100a) and of the torch binding.
 
-`python -m mccl_b200._build` compiles every file under csrc/ that is newer than its object and links
-mccl_b200/lib/libmccl.so.  Objects live in build/ (ignored by git); the shared library stays inside the
-package so that it travels with the source tree.
+`python -m mccl_b200._build` compiles every file under csrc/ that changed since its object was made, or whose headers did, and links
+mccl_b200/lib/libmccl.so, and mccl_torch.so from csrc/torch.  Objects live in build/ (ignored by git); the shared libraries stay inside the
+package so that they travel with the source tree.
 """
 from __future__ import annotations
 
@@ -16,7 +16,9 @@ from pathlib import Path
 ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "csrc"
 OBJ = ROOT / "build" / "obj"
+TORCH_SRC = CSRC / "torch"                       # the torch binding: a library of its own, so that libmccl needs no torch
 LIB = ROOT / "mccl_b200" / "lib" / "libmccl.so"
+EXT = LIB.with_name("mccl_torch.so")
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 
@@ -27,20 +29,25 @@ NVCCFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,co
              "--expt-relaxed-constexpr", "-Xptxas", "-v"]
 
 
-def _headers_mtime() -> float:
-    newest = 0.0
-    for pat in ("*.h", "*.cuh"):
-        for h in list(CSRC.rglob(pat)) + list((ROOT / "include").rglob(pat)):
-            newest = max(newest, h.stat().st_mtime)
-    return newest
+def _stale(src: Path, obj: Path) -> bool:
+    """Whether `src` or a file it included when `obj` was made is newer than `obj`."""
+    dep = obj.with_suffix(".d")
+    if not obj.exists() or not dep.exists():
+        return True
+    made = obj.stat().st_mtime
+    for name in dep.read_text().replace("\\\n", " ").split(":", 1)[1].split():
+        f = Path(name)
+        if not f.exists() or f.stat().st_mtime > made:
+            return True
+    return False
 
 
-def _compile(src: Path, obj: Path, verbose: bool) -> tuple[Path, str]:
+def _compile(src: Path, obj: Path, extra: list[str]) -> tuple[Path, str]:
     obj.parent.mkdir(parents=True, exist_ok=True)
     if src.suffix == ".cu":
-        cmd = [NVCC, *NVCCFLAGS, "-c", str(src), "-o", str(obj)]
+        cmd = [NVCC, *NVCCFLAGS, "-MMD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)]
     else:
-        cmd = ["g++", *CXXFLAGS, "-c", str(src), "-o", str(obj)]
+        cmd = ["g++", *CXXFLAGS, *extra, "-MMD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)]
     p = subprocess.run(cmd, capture_output=True, text=True)
     if p.returncode != 0:
         raise RuntimeError(f"compile failed: {' '.join(cmd)}\n{p.stdout}\n{p.stderr}")
@@ -50,38 +57,64 @@ def _compile(src: Path, obj: Path, verbose: bool) -> tuple[Path, str]:
     return src, log
 
 
+def _torch_flags() -> tuple[list[str], list[str]] | None:
+    """Compile and link flags of the torch binding; None where torch is not installed (the tcp transport works without)."""
+    import sysconfig
+    try:
+        import torch
+    except ImportError:
+        return None
+    inc = Path(torch.__file__).parent / "include"
+    lib = Path(torch.__file__).parent / "lib"
+    cflags = [f"-isystem{inc}", f"-isystem{inc / 'torch/csrc/api/include'}", f"-isystem{sysconfig.get_paths()['include']}",
+              "-DTORCH_EXTENSION_NAME=mccl_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-fvisibility=hidden"]
+    lflags = [f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", f"-L{LIB.parent}", "-lmccl",
+              "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{lib}"]
+    return cflags, lflags
+
+
+def _link(cmd: list[str], target: Path) -> None:
+    # Linked beside the target and renamed into place: whoever copies or loads the tree never sees half a library.
+    target.parent.mkdir(parents=True, exist_ok=True)
+    tmp = target.with_name(f".{target.name}.{os.getpid()}.tmp")
+    p = subprocess.run([*cmd, "-o", str(tmp)], capture_output=True, text=True)
+    if p.returncode != 0:
+        tmp.unlink(missing_ok=True)
+        raise RuntimeError(f"link failed: {' '.join(cmd)}\n{p.stdout}\n{p.stderr}")
+    os.replace(tmp, target)
+
+
 def build(verbose: bool = False, force: bool = False) -> Path:
     if shutil.which(NVCC) is None and not Path(NVCC).exists():
         raise RuntimeError(f"nvcc not found at {NVCC}")
     srcs = sorted(list(CSRC.rglob("*.cc")) + list(CSRC.rglob("*.cu")))
-    hdr = _headers_mtime()
-    jobs = []
-    objs = []
+    torch_flags = _torch_flags()
+    jobs, objs, ext_objs = [], [], []
     for s in srcs:
+        in_ext = TORCH_SRC in s.parents
+        if in_ext and torch_flags is None:
+            continue
         o = OBJ / s.relative_to(CSRC).with_suffix(s.suffix + ".o")
-        objs.append(o)
-        if force or not o.exists() or o.stat().st_mtime < max(s.stat().st_mtime, hdr):
-            jobs.append((s, o))
+        (ext_objs if in_ext else objs).append(o)
+        if force or _stale(s, o):
+            jobs.append((s, o, torch_flags[0] if in_ext else []))
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
-            for src, log in ex.map(lambda so: _compile(so[0], so[1], verbose), jobs):
+            for src, log in ex.map(lambda job: _compile(*job), jobs):
                 if verbose:
                     print(f"[mccl build] {src.relative_to(ROOT)}")
                     if log:
                         print(log)
     if jobs or not LIB.exists():
-        LIB.parent.mkdir(parents=True, exist_ok=True)
-        # Linked beside the target and renamed into place: whoever copies or loads the tree never sees half a library.
-        tmp = LIB.with_name(f".{LIB.name}.{os.getpid()}.tmp")
-        cmd = [NVCC, "-shared", "-o", str(tmp), *map(str, objs), "-cudart", "static",
-               "-gencode", "arch=compute_100a,code=sm_100a", "-Xlinker", "--no-undefined", "-lpthread", "-ldl", "-lrt"]
-        p = subprocess.run(cmd, capture_output=True, text=True)
-        if p.returncode != 0:
-            tmp.unlink(missing_ok=True)
-            raise RuntimeError(f"link failed: {' '.join(cmd)}\n{p.stdout}\n{p.stderr}")
-        os.replace(tmp, LIB)
+        _link([NVCC, "-shared", *map(str, objs), "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a",
+               "-Xlinker", "--no-undefined", "-lpthread", "-ldl", "-lrt"], LIB)
         if verbose:
             print(f"[mccl build] linked {LIB.relative_to(ROOT)}")
+    if ext_objs and (jobs or not EXT.exists()):
+        _link(["g++", "-shared", *map(str, ext_objs), *torch_flags[1]], EXT)
+        if verbose:
+            print(f"[mccl build] linked {EXT.relative_to(ROOT)}")
     return LIB
 
 

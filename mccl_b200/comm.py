@@ -80,6 +80,17 @@ def _stream_of(buf, stream):
     return C.c_void_p(0)
 
 
+def _fast_calls():
+    if torch is None:
+        return None
+    from . import _ext
+    return _ext.load()
+
+
+def _fast_stream(stream) -> Optional[int]:
+    return stream if stream is None or isinstance(stream, int) else stream.cuda_stream
+
+
 def get_unique_id() -> bytes:
     """mcclGetUniqueId: 128 bytes to create on one rank and hand to the others (it names a listener of this process)."""
     uid = L.UniqueId()
@@ -151,6 +162,8 @@ class Communicator:
             L.check(self._lib.mcclCommInitRankConfig(C.byref(self._h), n_ranks, uid, rank, C.byref(cfg)),
                     "mcclCommInitRankConfig")
         self._sym = {}
+        # The calls on torch tensors in C++ (None without torch); they answer -1 for whatever needs the general path here.
+        self._fast = _fast_calls()
         _live.add(self)
 
     # ---- queries
@@ -280,6 +293,12 @@ class Communicator:
     def all_reduce(self, send, recv=None, op: str = "sum", dtype: Optional[int] = None, stream=None) -> None:
         """recv (default: in place) = op over the ranks' `send`; torch tensors, numpy arrays, or raw pointers with `dtype`."""
         recv = send if recv is None else recv
+        if dtype is None and self._fast is not None:
+            rc = self._fast.all_reduce(self._h.value or 0, send, recv, L.OPS[op], _fast_stream(stream))
+            if rc >= 0:
+                if rc:
+                    L.check(rc, "mcclAllReduce")
+                return
         _check_pair("all_reduce", send, recv)
         sp, cnt, dt, _ = _describe(send, dtype)
         rp, _, _, _ = _describe(recv, dtype)
@@ -287,6 +306,12 @@ class Communicator:
 
     def all_gather(self, send, recv, dtype: Optional[int] = None, stream=None) -> None:
         """recv = the ranks' `send` concatenated in rank order (`send` may be this rank's slot of `recv`)."""
+        if dtype is None and self._fast is not None:
+            rc = self._fast.all_gather(self._h.value or 0, send, recv, _fast_stream(stream))
+            if rc >= 0:
+                if rc:
+                    L.check(rc, "mcclAllGather")
+                return
         _check_pair("all_gather", send, recv, self.size)
         sp, cnt, dt, _ = _describe(send, dtype)
         rp, _, _, _ = _describe(recv, dtype)
@@ -294,6 +319,12 @@ class Communicator:
 
     def reduce_scatter(self, send, recv, op: str = "sum", dtype: Optional[int] = None, stream=None) -> None:
         """recv = block `rank` of op over the ranks' `send` (n blocks of recv's size)."""
+        if dtype is None and self._fast is not None:
+            rc = self._fast.reduce_scatter(self._h.value or 0, send, recv, L.OPS[op], _fast_stream(stream))
+            if rc >= 0:
+                if rc:
+                    L.check(rc, "mcclReduceScatter")
+                return
         _check_pair("reduce_scatter", recv, send, self.size)      # send holds one block of recv's size per rank
         sp, _, dt, _ = _describe(send, dtype)
         rp, cnt, _, _ = _describe(recv, dtype)
@@ -302,6 +333,12 @@ class Communicator:
 
     def broadcast(self, send, recv, root: int = 0, dtype: Optional[int] = None, stream=None) -> None:
         """recv on every rank = the root's `send` (may be None elsewhere)."""
+        if dtype is None and self._fast is not None:
+            rc = self._fast.broadcast(self._h.value or 0, send, recv, root, _fast_stream(stream))
+            if rc >= 0:
+                if rc:
+                    L.check(rc, "mcclBroadcast")
+                return
         _check_pair("broadcast", recv, send)                      # the root sends as many elements as everyone receives
         rp, cnt, dt, _ = _describe(recv, dtype)
         sp = _describe(send, dtype)[0] if send is not None else None
@@ -316,6 +353,12 @@ class Communicator:
 
     def all_to_all(self, send, recv, dtype: Optional[int] = None, stream=None) -> None:
         """Block j of `send` goes to rank j; block i of `recv` came from rank i (equal blocks)."""
+        if dtype is None and self._fast is not None:
+            rc = self._fast.all_to_all(self._h.value or 0, send, recv, _fast_stream(stream))
+            if rc >= 0:
+                if rc:
+                    L.check(rc, "mcclAllToAll")
+                return
         _check_pair("all_to_all", send, recv)
         if _describe(send, dtype)[1] % self.size:
             raise ValueError(f"all_to_all: {_describe(send, dtype)[1]} elements do not split into {self.size} equal blocks")

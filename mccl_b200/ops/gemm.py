@@ -6,6 +6,7 @@ import ctypes as C
 
 import torch
 
+from .. import _ext
 from .. import _lib as L
 
 _counter = {"launches": 0}
@@ -13,7 +14,7 @@ EPI = {"none": 0, "silu": 1}
 
 
 def launches() -> int:
-    return _counter["launches"]
+    return _counter["launches"] + _ext.load().launches("gemm")
 
 
 def _lib():
@@ -47,25 +48,22 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, epil
     """out[M, N] = act(x[M, K] @ w[N, K].T) in bf16 with fp32 accumulation, by the library's own tcgen05 kernel.
     `two_sm` selects the form in which pairs of SMs share a 256-row tile (needs M % 256 == 0); by default it is
     used whenever the shape allows it."""
-    if not x.is_cuda:
+    if x.is_cuda:
+        y = _ext.load().gemm(x, w, out, EPI[epilogue], max_ctas, stream.cuda_stream if stream is not None else None, two_sm)
+        if isinstance(y, torch.Tensor):
+            return y
+    else:
         raise RuntimeError("mccl gemm runs on CUDA (sm_100a) only")
+    # Not taken by the kernels: say why.
     assert x.dtype == w.dtype == torch.bfloat16 and x.is_contiguous() and w.is_contiguous()
     M, K = x.shape
     N = w.shape[0]
     assert w.shape[1] == K
     if not supported(M, N, K):
         raise ValueError(f"unsupported GEMM shape {M}x{N}x{K}: M % 128, N % 64 and K % 64 must be 0")
-    if out is None:
-        out = torch.empty(M, N, device=x.device, dtype=torch.bfloat16)
-    if two_sm is None:
-        two_sm = M % 256 == 0
     if two_sm and M % 256:
         raise ValueError(f"the two-SM GEMM needs M % 256 == 0 (got {M})")
-    fn = _lib().mcclTpGemm2 if two_sm else _lib().mcclTpGemm
-    L.check(fn(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, EPI[epilogue], max_ctas, _stream(x, stream)),
-            "mcclTpGemm2" if two_sm else "mcclTpGemm")
-    _counter["launches"] += 1
-    return out
+    L.check(L.INVALID_ARGUMENT if y is None else y, "mcclTpGemm2" if (M % 256 == 0 if two_sm is None else two_sm) else "mcclTpGemm")
 
 
 def last_error() -> int:

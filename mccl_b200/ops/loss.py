@@ -3,56 +3,13 @@ forward pass, the gradient written in bf16 over the logits in the backward pass,
 rows x vocab matrix."""
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
-from .. import _lib as L
-
-_counter = {"launches": 0}
+from .. import _ext
 
 
 def launches() -> int:
-    return _counter["launches"]
-
-
-def _lib():
-    lib = L.load()
-    if not getattr(lib, "_ce_declared", False):
-        vp, i64, i = C.c_void_p, C.c_int64, C.c_int
-        lib.mcclCrossEntropyForward.restype = i
-        lib.mcclCrossEntropyForward.argtypes = [vp, i64, i64, i, vp, vp, vp, vp]
-        lib.mcclCrossEntropyBackward.restype = i
-        lib.mcclCrossEntropyBackward.argtypes = [vp, i64, i64, i, i, vp, vp, vp, vp]
-        lib._ce_declared = True
-    return lib
-
-
-class _FusedCrossEntropy(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, logits: torch.Tensor, targets: torch.Tensor, vocab: int):
-        rows, width = logits.shape
-        loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
-        lse = torch.empty_like(loss)
-        s = C.c_void_p(torch.cuda.current_stream(logits.device).cuda_stream)
-        L.check(_lib().mcclCrossEntropyForward(logits.data_ptr(), rows, logits.stride(0), vocab, targets.data_ptr(),
-                                               loss.data_ptr(), lse.data_ptr(), s), "mcclCrossEntropyForward")
-        _counter["launches"] += 1
-        ctx.save_for_backward(logits, targets, lse)
-        ctx.vocab = vocab
-        return loss.mean()
-
-    @staticmethod
-    def backward(ctx, grad_out: torch.Tensor):
-        logits, targets, lse = ctx.saved_tensors
-        rows, width = logits.shape
-        g = grad_out.to(torch.float32).contiguous()
-        s = C.c_void_p(torch.cuda.current_stream(logits.device).cuda_stream)
-        # The gradient overwrites the logits: nothing downstream of the output projection reads them again.
-        L.check(_lib().mcclCrossEntropyBackward(logits.data_ptr(), rows, logits.stride(0), ctx.vocab, width, targets.data_ptr(),
-                                                lse.data_ptr(), g.data_ptr(), s), "mcclCrossEntropyBackward")
-        _counter["launches"] += 1
-        return logits, None, None
+    return _ext.load().launches("loss")
 
 
 def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, vocab: int | None = None) -> torch.Tensor:
@@ -62,4 +19,7 @@ def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, vocab: int 
         raise RuntimeError("fused_cross_entropy runs on CUDA (sm_100a) only")
     assert logits.dim() == 2 and logits.dtype == torch.bfloat16 and logits.stride(1) == 1
     assert targets.dtype == torch.int64 and targets.is_contiguous() and targets.numel() == logits.shape[0]
-    return _FusedCrossEntropy.apply(logits, targets, vocab if vocab is not None else logits.shape[1])
+    loss = _ext.load().cross_entropy(logits, targets, vocab)
+    if loss is None:
+        raise ValueError("fused_cross_entropy: logits and targets do not fit together")
+    return loss
