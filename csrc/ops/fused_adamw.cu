@@ -28,7 +28,30 @@ struct AdamArgs {
                              // launch recorded in a CUDA graph follows the schedule when it is replayed
 };
 
-__global__ void __launch_bounds__(256) adamwKernel(AdamArgs a) {
+// Eight floats with one access: a lane's 32 bytes are a whole sector, where two 16-byte stores leave the L2 with two
+// partial writes of it.  WIDE needs 32-byte aligned arrays.
+template <bool WIDE> __device__ __forceinline__ void ld8(const float* p, float* f) {
+  if (WIDE) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]),
+                 "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p) : "memory");
+  } else {
+    const float4 x = reinterpret_cast<const float4*>(p)[0], y = reinterpret_cast<const float4*>(p)[1];
+    f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
+  }
+}
+template <bool WIDE> __device__ __forceinline__ void st8(float* p, const float* f) {
+  if (WIDE) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" :: "l"(p), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]), "f"(f[4]),
+                 "f"(f[5]), "f"(f[6]), "f"(f[7]) : "memory");
+  } else {
+    reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
+  }
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(256) adamwKernel(const __grid_constant__ AdamArgs arg) {
+  AdamArgs a = arg;
   if (a.hyper != nullptr) { a.lr = a.hyper[0]; a.biasCorr1 = a.hyper[1]; a.biasCorr2Sqrt = a.hyper[2]; }
   if (a.normSq != nullptr) {   // global-norm clipping: scale = min(1, maxNorm / ||g||), read on the device (no host sync)
     const float norm = sqrtf(*a.normSq) * a.gradScale;
@@ -39,13 +62,10 @@ __global__ void __launch_bounds__(256) adamwKernel(AdamArgs a) {
   for (uint64_t i = tid; i < nVec; i += nth) {
     uint4 gq = reinterpret_cast<const uint4*>(a.grad)[i];
     const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&gq);
-    float4 w[2], m[2], v[2];
-    w[0] = reinterpret_cast<float4*>(a.master)[2 * i]; w[1] = reinterpret_cast<float4*>(a.master)[2 * i + 1];
-    m[0] = reinterpret_cast<float4*>(a.expAvg)[2 * i]; m[1] = reinterpret_cast<float4*>(a.expAvg)[2 * i + 1];
-    v[0] = reinterpret_cast<float4*>(a.expAvgSq)[2 * i]; v[1] = reinterpret_cast<float4*>(a.expAvgSq)[2 * i + 1];
-    float* wf = reinterpret_cast<float*>(w);
-    float* mf = reinterpret_cast<float*>(m);
-    float* vf = reinterpret_cast<float*>(v);
+    float wf[8], mf[8], vf[8];
+    ld8<WIDE>(a.master + 8 * i, wf);
+    ld8<WIDE>(a.expAvg + 8 * i, mf);
+    ld8<WIDE>(a.expAvgSq + 8 * i, vf);
     uint4 pq;
     __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(&pq);
 #pragma unroll
@@ -57,9 +77,9 @@ __global__ void __launch_bounds__(256) adamwKernel(AdamArgs a) {
       wf[k] = wf[k] * (1.f - a.lr * a.weightDecay) - (a.lr / a.biasCorr1) * (mf[k] / denom);
       p[k] = __float2bfloat16_rn(wf[k]);
     }
-    reinterpret_cast<float4*>(a.master)[2 * i] = w[0]; reinterpret_cast<float4*>(a.master)[2 * i + 1] = w[1];
-    reinterpret_cast<float4*>(a.expAvg)[2 * i] = m[0]; reinterpret_cast<float4*>(a.expAvg)[2 * i + 1] = m[1];
-    reinterpret_cast<float4*>(a.expAvgSq)[2 * i] = v[0]; reinterpret_cast<float4*>(a.expAvgSq)[2 * i + 1] = v[1];
+    st8<WIDE>(a.master + 8 * i, wf);
+    st8<WIDE>(a.expAvg + 8 * i, mf);
+    st8<WIDE>(a.expAvgSq + 8 * i, vf);
     reinterpret_cast<uint4*>(a.param)[i] = pq;
     if (a.zeroGrad) reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(a.grad))[i] = make_uint4(0, 0, 0, 0);
   }
@@ -101,10 +121,13 @@ static mcclResult_t adamwLaunch(void* param, float* master, float* expAvg, float
   a.maxNorm = maxNorm;
   a.hyper = hyper;
   const uint64_t vec = (n + 7) / 8;
-  int blocks = (int)((vec + 255) / 256);
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  if (blocks < 1) blocks = 1;
-  adamwKernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+  // One vector of eight elements per thread and no loop: with eight blocks per SM walking the array the last turn of the
+  // walk leaves most of them idle (25 MB bucket: 63.7 us, 64 Mi elements: 314 us; without the walk 58.0 and 275 us).
+  const uint64_t want = (vec + 255) / 256;
+  const unsigned blocks = (unsigned)(want < (1u << 30) ? want : (1u << 30));
+  const bool wide = (((uintptr_t)master | (uintptr_t)expAvg | (uintptr_t)expAvgSq) & 31u) == 0;
+  auto* kernel = wide ? adamwKernel<true> : adamwKernel<false>;
+  kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 

@@ -58,6 +58,6 @@ extern "C" mcclResult_t mcclSumSquaresBf16NoAlloc(const void* x, uint64_t n, flo
   // The array keeps whatever the previous call left.  Only the ticket counter has to start at zero (every
   // partial that is read is written first); clear it here in case an earlier launch never finished.
   if (cudaMemsetAsync(scratch, 0, sizeof(unsigned), s) != cudaSuccess) return mcclSystemError;
-  sumSquaresKernel<<<(unsigned)normBlocks(n), kNormThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(x), n, scratch, out, accumulate);
+  sumSquaresKernel<<<(unsigned)normBlocks(n), kNormThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(x), n, scratch, out, accumulate, normTile(n));
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
