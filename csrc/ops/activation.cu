@@ -1,0 +1,266 @@
+// Activations and their gradients over flat bf16 arrays: SiLU, SwiGLU and tanh-GELU, each one pass over memory with the
+// arithmetic in fp32, and the GELU gradient together with its column sums (the bias gradient of the layer in front).
+// Bound by memory: two to five 2-byte accesses an element.  Four 16-byte pieces of every operand are in flight per thread,
+// which is what 6 TB/s takes at this occupancy; with one, the passes ran at half of that.
+// No counterpart in the reference (it has no model code).
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <initializer_list>
+
+#include "col_reduce.cuh"
+#include "mccl.h"
+#include "mccl_ops.h"
+
+namespace {
+
+using namespace mccl;
+
+constexpr int kActThreads = 256;
+
+__device__ __forceinline__ void unpack(const uint4& q, float* f) {
+  const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { const float2 t = __bfloat1622float2(e[k]); f[2 * k] = t.x; f[2 * k + 1] = t.y; }
+}
+__device__ __forceinline__ uint4 pack(const float* f) {
+  uint4 q;
+  __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) e[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+  return q;
+}
+__device__ __forceinline__ float rounded(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+
+// tanh by its exponential form: relative error of a few 2^-22, far below the bf16 rounding of the result.
+__device__ __forceinline__ float tanhOf(float x) {
+  const float e = __expf(-2.f * fabsf(x));
+  return copysignf(__fdividef(1.f - e, 1.f + e), x);
+}
+constexpr float kGeluC = 0.7978845608028654f;      // sqrt(2 / pi)
+constexpr float kGeluA = 0.044715f;
+__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + tanhOf(kGeluC * (x + kGeluA * x * x * x))); }
+__device__ __forceinline__ float geluGrad(float x) {
+  const float t = tanhOf(kGeluC * (x + kGeluA * x * x * x));
+  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * kGeluC * (1.f + 3.f * kGeluA * x * x);
+}
+
+// An operation maps IN input values to OUT output values.
+struct SiluFwd { static constexpr int IN = 1, OUT = 1; __device__ static void f(const float* i, float* o) { o[0] = i[0] * sigmoid(i[0]); } };
+struct SiluBwd {                                   // (pre-activation, gradient) -> gradient of the pre-activation
+  static constexpr int IN = 2, OUT = 1;
+  __device__ static void f(const float* i, float* o) { const float s = sigmoid(i[0]); o[0] = i[1] * (s * (1.f + i[0] * (1.f - s))); }
+};
+struct SiluBoth {                                  // (pre-activation, gradient) -> activation, gradient of the pre-activation
+  static constexpr int IN = 2, OUT = 2;
+  __device__ static void f(const float* i, float* o) {
+    const float s = sigmoid(i[0]);
+    o[0] = i[0] * s;
+    o[1] = i[1] * (s * (1.f + i[0] * (1.f - s)));
+  }
+};
+struct SwigluFwd {                                 // (gate, up) -> silu(gate) * up, the activation rounded before the product
+  static constexpr int IN = 2, OUT = 1;
+  __device__ static void f(const float* i, float* o) { o[0] = rounded(i[0] * sigmoid(i[0])) * i[1]; }
+};
+struct SwigluBwd {                                 // (gate, up, gradient) -> product (for the weight gradient behind), d gate, d up
+  static constexpr int IN = 3, OUT = 3;
+  __device__ static void f(const float* i, float* o) {
+    const float s = sigmoid(i[0]), act = rounded(i[0] * s);
+    o[0] = act * i[1];
+    o[1] = i[2] * i[1] * (s * (1.f + i[0] * (1.f - s)));
+    o[2] = i[2] * act;
+  }
+};
+struct GeluFwd { static constexpr int IN = 1, OUT = 1; __device__ static void f(const float* i, float* o) { o[0] = gelu(i[0]); } };
+
+template <class Op> struct ActArgs { const uint4* in[Op::IN]; uint4* out[Op::OUT]; int64_t n; };
+
+template <class Op>
+__global__ void __launch_bounds__(kActThreads) actKernel(const __grid_constant__ ActArgs<Op> a) {
+  constexpr int U = Op::IN + Op::OUT >= 5 ? 2 : 4;
+  const int64_t vecs = a.n / 8;
+  const int64_t i0 = (int64_t)blockIdx.x * (kActThreads * U) + threadIdx.x;
+  uint4 q[Op::IN][U];
+#pragma unroll
+  for (int k = 0; k < Op::IN; ++k)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * kActThreads < vecs) q[k][u] = a.in[k][i0 + u * kActThreads];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (i0 + u * kActThreads >= vecs) continue;
+    float x[Op::IN][8], y[Op::OUT][8];
+#pragma unroll
+    for (int k = 0; k < Op::IN; ++k) unpack(q[k][u], x[k]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float in[Op::IN], out[Op::OUT];
+#pragma unroll
+      for (int k = 0; k < Op::IN; ++k) in[k] = x[k][e];
+      Op::f(in, out);
+#pragma unroll
+      for (int k = 0; k < Op::OUT; ++k) y[k][e] = out[k];
+    }
+#pragma unroll
+    for (int k = 0; k < Op::OUT; ++k) a.out[k][i0 + u * kActThreads] = pack(y[k]);
+  }
+  if (blockIdx.x == 0 && threadIdx.x < (unsigned)(a.n % 8)) {        // the last few elements
+    const int64_t i = vecs * 8 + threadIdx.x;
+    float in[Op::IN], out[Op::OUT];
+#pragma unroll
+    for (int k = 0; k < Op::IN; ++k) in[k] = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.in[k])[i]);
+    Op::f(in, out);
+#pragma unroll
+    for (int k = 0; k < Op::OUT; ++k) reinterpret_cast<__nv_bfloat16*>(a.out[k])[i] = __float2bfloat16_rn(out[k]);
+  }
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+template <class Op>
+mcclResult_t act(std::initializer_list<const void*> in, std::initializer_list<void*> out, int64_t n, mcclStream_t stream) {
+  ActArgs<Op> a;
+  int k = 0;
+  for (const void* p : in) { if (p == nullptr || !aligned16(p)) return mcclInvalidArgument; a.in[k++] = static_cast<const uint4*>(p); }
+  k = 0;
+  for (void* p : out) { if (p == nullptr || !aligned16(p)) return mcclInvalidArgument; a.out[k++] = static_cast<uint4*>(p); }
+  if (n < 0) return mcclInvalidArgument;
+  if (n == 0) return mcclSuccess;
+  a.n = n;
+  constexpr int U = Op::IN + Op::OUT >= 5 ? 2 : 4;
+  const int64_t per = (int64_t)kActThreads * U, blocks = (n / 8 + per - 1) / per;
+  actKernel<Op><<<(unsigned)(blocks < 1 ? 1 : blocks), kActThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+  return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
+
+// ---- column sums ------------------------------------------------------------------------------------------------------
+// A CTA takes a strip of 64 x 8 columns (one vector per lane of two warps' width) and walks rows; four groups of 64 threads
+// take every fourth row.  Up to three matrices of the same shape in one launch (blockIdx.z).  With GELU the matrix is the
+// gradient of the activation, replaced by the gradient of the pre-activation on the way.
+constexpr int kStripVecs = 64, kStripCols = kStripVecs * 8, kRowGroups = kActThreads / kStripVecs;
+
+struct ColArgs {
+  const uint4* x[colred::kMaxSegments];       // [rows, D] each, row stride `ld` vectors
+  const uint4* pre;                           // GELU: pre-activation
+  uint4* dx;                                  // GELU: where the gradient goes
+  float* partial;                             // [gridDim.y][segments * D]
+  int64_t rows, ld;
+  int D;
+  colred::Out out;
+};
+
+template <bool GELU>
+__global__ void __launch_bounds__(kActThreads, 3) colSumKernel(const __grid_constant__ ColArgs a) {
+  __shared__ float red[kRowGroups][kStripCols];
+  const int tv = threadIdx.x % kStripVecs, g = threadIdx.x / kStripVecs, vecs = a.D / 8;
+  const int v = blockIdx.x * kStripVecs + tv, seg = blockIdx.z;
+  constexpr int U = 4;                         // rows in flight per thread
+  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (v < vecs) {
+    const uint4* x = a.x[seg];
+    const int64_t step = (int64_t)gridDim.y * kRowGroups;
+    for (int64_t r0 = (int64_t)blockIdx.y * kRowGroups + g; r0 < a.rows; r0 += U * step) {
+      uint4 q[U], p[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t r = r0 + u * step;
+        if (r < a.rows) { q[u] = x[r * a.ld + v]; if (GELU) p[u] = a.pre[r * a.ld + v]; }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t r = r0 + u * step;
+        if (r >= a.rows) continue;
+        float f[8];
+        unpack(q[u], f);
+        if (GELU) {
+          float z[8];
+          unpack(p[u], z);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] *= geluGrad(z[k]);
+          const uint4 o = pack(f);
+          a.dx[r * a.ld + v] = o;
+          unpack(o, f);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum[k] += f[k];
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) red[g][tv + kStripVecs * k] = sum[k];      // transposed: no bank conflicts
+  __syncthreads();
+  for (int c = threadIdx.x; c < kStripCols; c += kActThreads) {
+    float t = red[0][c];
+#pragma unroll
+    for (int i = 1; i < kRowGroups; ++i) t += red[i][c];
+    const int col = (blockIdx.x * kStripVecs + c % kStripVecs) * 8 + c / kStripVecs;
+    if (col >= a.D) continue;
+    if (gridDim.y == 1) colred::put(a.out, seg * a.D + col, t);
+    else a.partial[((int64_t)blockIdx.y * gridDim.z + seg) * a.D + col] = t;
+  }
+}
+
+// Row slices: enough CTAs for three per SM, at least 16 rows a slice (four rows in flight for each of the four row groups).
+int colSlices(int64_t rows, int D, int segments) {
+  const int64_t strips = (int64_t)((D / 8 + kStripVecs - 1) / kStripVecs) * segments;
+  int64_t s = 148 * 3 / strips;
+  const int64_t most = (rows + 15) / 16;
+  if (s > most) s = most;
+  if (s > colred::kMaxPartials) s = colred::kMaxPartials;
+  return s < 1 ? 1 : (int)s;
+}
+
+template <bool GELU>
+mcclResult_t colSums(const ColArgs& a, cudaStream_t s) {
+  const int strips = (a.D / 8 + kStripVecs - 1) / kStripVecs, slices = colSlices(a.rows, a.D, a.out.segments);
+  colSumKernel<GELU><<<dim3(strips, slices, a.out.segments), kActThreads, 0, s>>>(a);
+  if (cudaGetLastError() != cudaSuccess) return mcclSystemError;
+  return colred::addPartials(a.partial, slices, 1, a.out.segments * a.D, a.out, s) == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
+
+}  // namespace
+
+extern "C" mcclResult_t mcclSiluForward(const void* x, void* y, int64_t n, mcclStream_t s) { return act<SiluFwd>({x}, {y}, n, s); }
+extern "C" mcclResult_t mcclSiluBackward(const void* x, const void* dy, void* dx, int64_t n, mcclStream_t s) { return act<SiluBwd>({x, dy}, {dx}, n, s); }
+extern "C" mcclResult_t mcclSiluForwardBackward(const void* x, const void* dy, void* y, void* dx, int64_t n, mcclStream_t s) {
+  return act<SiluBoth>({x, dy}, {y, dx}, n, s);
+}
+extern "C" mcclResult_t mcclSwigluForward(const void* gate, const void* up, void* y, int64_t n, mcclStream_t s) { return act<SwigluFwd>({gate, up}, {y}, n, s); }
+extern "C" mcclResult_t mcclSwigluBackward(const void* gate, const void* up, const void* dy, void* y, void* dgate, void* dup, int64_t n, mcclStream_t s) {
+  return act<SwigluBwd>({gate, up, dy}, {y, dgate, dup}, n, s);
+}
+extern "C" mcclResult_t mcclGeluForward(const void* x, void* y, int64_t n, mcclStream_t s) { return act<GeluFwd>({x}, {y}, n, s); }
+
+// Floats of work memory the two functions below need.
+extern "C" int64_t mcclColumnSumScratch(int64_t rows, int D, int segments) {
+  return rows <= 0 || D <= 0 || segments <= 0 ? 0 : (int64_t)colSlices(rows, D, segments) * segments * D;
+}
+
+// dx = dy * gelu'(x) for [rows, D] matrices, dbias (nullable) = [+] column sums of dx.
+extern "C" mcclResult_t mcclGeluBackward(const void* x, const void* dy, void* dx, void* dbias, int accumulate, float* scratch, int64_t rows,
+                                         int D, mcclStream_t stream) {
+  if (!x || !dy || !dx || !scratch || rows <= 0 || D <= 0 || D % 8 || !aligned16(x) || !aligned16(dy) || !aligned16(dx)) return mcclInvalidArgument;
+  ColArgs a = {};
+  a.x[0] = static_cast<const uint4*>(dy); a.pre = static_cast<const uint4*>(x); a.dx = static_cast<uint4*>(dx);
+  a.partial = scratch; a.rows = rows; a.ld = D / 8; a.D = D;
+  a.out.seg[0] = static_cast<__nv_bfloat16*>(dbias); a.out.segments = 1; a.out.width = D; a.out.accumulate = accumulate;
+  return colSums<true>(a, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// out[i] = [+] column sums of x[i], up to three [rows, D] matrices with rows `ld` elements apart.
+extern "C" mcclResult_t mcclColumnSums(const void* const* x, void* const* out, int n, int accumulate, float* scratch, int64_t rows, int D,
+                                       int64_t ld, mcclStream_t stream) {
+  if (!x || !out || !scratch || n < 1 || n > colred::kMaxSegments || rows <= 0 || D <= 0 || D % 8 || ld < D || ld % 8) return mcclInvalidArgument;
+  ColArgs a = {};
+  for (int i = 0; i < n; ++i) {
+    if (!x[i] || !out[i] || !aligned16(x[i])) return mcclInvalidArgument;
+    a.x[i] = static_cast<const uint4*>(x[i]);
+    a.out.seg[i] = static_cast<__nv_bfloat16*>(out[i]);
+  }
+  a.partial = scratch; a.rows = rows; a.ld = ld / 8; a.D = D;
+  a.out.segments = n; a.out.width = D; a.out.accumulate = accumulate;
+  return colSums<false>(a, reinterpret_cast<cudaStream_t>(stream));
+}

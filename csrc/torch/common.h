@@ -40,5 +40,6 @@ inline bool bf16Cuda(const Tensor& t) { return t.is_cuda() && t.scalar_type() ==
 // One module's functions each, defined in the files of the same names.
 void bindOps(pybind11::module_& m);
 void bindComm(pybind11::module_& m);
+void bindMoe(pybind11::module_& m);
 
 }  // namespace mccl_torch

@@ -166,4 +166,5 @@ void bindOps(py::module_& m) {
 PYBIND11_MODULE(mccl_torch, m) {
   mccl_torch::bindOps(m);
   mccl_torch::bindComm(m);
+  mccl_torch::bindMoe(m);
 }

@@ -41,6 +41,43 @@ mcclResult_t mcclMoeScatter(mcclComm_t comm, const void* tokens, const int32_t* 
 mcclResult_t mcclMoeGather(mcclComm_t comm, const void* exchange, const int32_t* flat, const float* scale, void* out,
                            int nTokens, int rowBytes, int expertsPerRank, int capacity, mcclDataType_t dt, mcclStream_t stream);
 
+/* ---- routing and token movement with all experts on this GPU (bf16 rows of d elements, d % 8 == 0) ------------------- */
+/* Top-1 routing from logits [tokens, experts]: gate (fp32, rounded to bf16), log-sum-exp, flat[t] = expert * capacity + slot in
+ * token order or -1; inverse[expert * capacity + slot] = t and kept[expert] (both nullable).  At most mcclMoeRouteMaxExperts()
+ * experts; scratch: mcclMoeRouteScratch() ints. */
+int          mcclMoeRouteMaxExperts(void);
+int64_t      mcclMoeRouteScratch(int tokens, int experts);
+mcclResult_t mcclMoeRoute(const void* logits, int tokens, int experts, int capacity, float* gate, float* lse, int32_t* flat,
+                          int32_t* inverse, int32_t* kept, int32_t* scratch, mcclStream_t stream);
+/* slots[s] = rows[inverse[s]], zero where empty. */
+mcclResult_t mcclMoeFillSlots(const void* rows, const int32_t* inverse, const int32_t* kept, void* slots, int experts, int capacity,
+                              int d, mcclStream_t stream);
+/* out[t] = gate[t] * slots[flat[t]], zero for a dropped token. */
+mcclResult_t mcclMoeCombine(const void* slots, const int32_t* flat, const float* gate, void* out, int tokens, int d, mcclStream_t stream);
+mcclResult_t mcclMoeCombineBackward(const void* dy, const void* slots, const int32_t* inverse, const int32_t* kept, const float* gate,
+                                    void* dslots, float* dgate, int experts, int capacity, int d, mcclStream_t stream);
+/* dlogits through the softmax of the gate and dx = dslots[flat] + dlogits router (router null: without the second term; d = 0:
+ * dlogits only). */
+mcclResult_t mcclMoeTokenBackward(const void* dslots, const int32_t* flat, const float* dgate, const void* logits, const float* lse,
+                                  const void* router, void* dlogits, void* dx, int tokens, int experts, int capacity, int d,
+                                  mcclStream_t stream);
+
+/* ---- activations over n bf16 values (16-byte aligned) ---------------------------------------------------------------- */
+mcclResult_t mcclSiluForward(const void* x, void* y, int64_t n, mcclStream_t stream);
+mcclResult_t mcclSiluBackward(const void* x, const void* dy, void* dx, int64_t n, mcclStream_t stream);
+mcclResult_t mcclSiluForwardBackward(const void* x, const void* dy, void* y, void* dx, int64_t n, mcclStream_t stream);
+mcclResult_t mcclSwigluForward(const void* gate, const void* up, void* y, int64_t n, mcclStream_t stream);
+mcclResult_t mcclSwigluBackward(const void* gate, const void* up, const void* dy, void* y, void* dgate, void* dup, int64_t n,
+                                mcclStream_t stream);
+mcclResult_t mcclGeluForward(const void* x, void* y, int64_t n, mcclStream_t stream);
+/* dx = dy * gelu'(x) over [rows, D] and dbias (nullable) = [+] its column sums; scratch: mcclColumnSumScratch(rows, D, 1) floats. */
+mcclResult_t mcclGeluBackward(const void* x, const void* dy, void* dx, void* dbias, int accumulate, float* scratch, int64_t rows, int D,
+                              mcclStream_t stream);
+/* out[i] = [+] column sums of x[i], n <= 3 matrices [rows, D] with rows ld elements apart. */
+int64_t      mcclColumnSumScratch(int64_t rows, int D, int segments);
+mcclResult_t mcclColumnSums(const void* const* x, void* const* out, int n, int accumulate, float* scratch, int64_t rows, int D, int64_t ld,
+                            mcclStream_t stream);
+
 /* ---- training-step kernels (bf16 parameters and gradients, fp32 state) --------------------------------------------- */
 /* AdamW on n elements; normSq / maxNorm (nullable / 0): clip by the global gradient norm held on the device. */
 mcclResult_t mcclFusedAdamW(void* param, float* master, float* expAvg, float* expAvgSq, const void* grad, uint64_t n, float lr,

@@ -24,7 +24,8 @@ _DT = {torch.float32: L.FLOAT32, torch.bfloat16: L.BFLOAT16, torch.float16: L.FL
 
 
 def launches() -> int:
-    return _counter["launches"]
+    from .. import _ext
+    return _counter["launches"] + _ext.load().launches("moe")
 
 
 def _lib():

@@ -176,20 +176,31 @@ class ExpertParallelMoE(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         n, e, c, d = self.comm.size, self.local, self.capacity, self.hidden
-        expert, gate, slot, keep = self.route(x)
-        flat = expert * c + slot                                               # slot in the [experts, capacity] grid
         if self.fused and x.is_cuda:
+            from .. import _ext
             from ..ops import moe as M
+            if n == 1:                                                         # nothing to exchange: the whole layer is one node
+                y = _ext.load().moe_layer(x, self.router.weight, self.w_in, self.w_out, c)
+                if y is not None:
+                    return y
             if self._buf is None:                                              # collective allocations, first call
                 self._buf = M.ExchangeBuffer(self.comm, e, c, d, x.dtype)
                 self._grad_buf = M.ExchangeBuffer(self.comm, e, c, d, x.dtype)
-            flat32 = torch.where(keep, flat, torch.full_like(flat, -1)).to(torch.int32)
+            routed = _ext.load().moe_route(self.router(x), c)                  # None where the kernels do not cover the case
+            if routed is not None:
+                gate, flat32 = routed
+            else:
+                expert, gate, slot, keep = self.route(x)
+                flat = expert * c + slot
+                flat32 = torch.where(keep, flat, torch.full_like(flat, -1)).to(torch.int32)
             recv = M.dispatch(x, flat32, self._buf, self._grad_buf)            # [n (source), e, c, d]
             tokens = recv.transpose(0, 1).reshape(e, n * c, d)
             hidden = F.silu(torch.einsum("etd,efd->etf", tokens, self.w_in))
             out = torch.einsum("etf,edf->etd", hidden, self.w_out)
             back = out.view(e, n, c, d).transpose(0, 1).contiguous()
             return M.combine(back, flat32, gate, self._buf, self._grad_buf)
+        expert, gate, slot, keep = self.route(x)
+        flat = expert * c + slot                                               # slot in the [experts, capacity] grid
         send = x.new_zeros(self.experts * c, d)
         send = send.index_put((flat[keep],), x[keep])
         recv = PF.all_to_all_rows(send, self.comm)                             # [n (source), e, c, d]
