@@ -41,5 +41,6 @@ inline bool bf16Cuda(const Tensor& t) { return t.is_cuda() && t.scalar_type() ==
 void bindOps(pybind11::module_& m);
 void bindComm(pybind11::module_& m);
 void bindMoe(pybind11::module_& m);
+void bindGpt2(pybind11::module_& m);
 
 }  // namespace mccl_torch

@@ -167,4 +167,5 @@ PYBIND11_MODULE(mccl_torch, m) {
   mccl_torch::bindOps(m);
   mccl_torch::bindComm(m);
   mccl_torch::bindMoe(m);
+  mccl_torch::bindGpt2(m);
 }

@@ -78,6 +78,14 @@ int64_t      mcclColumnSumScratch(int64_t rows, int D, int segments);
 mcclResult_t mcclColumnSums(const void* const* x, void* const* out, int n, int accumulate, float* scratch, int64_t rows, int D, int64_t ld,
                             mcclStream_t stream);
 
+/* ---- embedding: out[t] = table[idx[t]] + pos[t % seq]; the backward pass adds into both gradients ---------------------- */
+mcclResult_t mcclEmbeddingForward(const int64_t* idx, const void* table, const void* pos, void* out, int64_t tokens, int seq, int64_t vocab,
+                                  int D, mcclStream_t stream);
+/* tokens <= mcclEmbeddingMaxTokens(), D <= 4096; count: vocab ints of work memory. */
+int          mcclEmbeddingMaxTokens(void);
+mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, int32_t* count, int64_t tokens, int seq,
+                                   int64_t vocab, int D, mcclStream_t stream);
+
 /* ---- training-step kernels (bf16 parameters and gradients, fp32 state) --------------------------------------------- */
 /* AdamW on n elements; normSq / maxNorm (nullable / 0): clip by the global gradient norm held on the device. */
 mcclResult_t mcclFusedAdamW(void* param, float* master, float* expAvg, float* expAvgSq, const void* grad, uint64_t n, float lr,

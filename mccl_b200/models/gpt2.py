@@ -1,9 +1,11 @@
 """GPT-2 style decoder used as the data-parallel workload (24 layers, d_model 1024, 16 heads, FFN 4096,
 vocab 50257, sequence 1024 for the "medium" shape, ~355M parameters).
 
-The model is plain PyTorch in bf16: attention goes through scaled_dot_product_attention, the linear layers
-through cuBLAS.  What this library adds around it is the communication (gradient buckets in symmetric
-memory, all-reduced by the library's own kernels while backward still runs) and the fused optimizer step.
+Attention goes through scaled_dot_product_attention, the linear layers through cuBLAS.  On CUDA in bf16 everything
+between them runs in this library's kernels, two autograd nodes per block (csrc/torch/gpt2.cc): a block hands on its
+residual stream and its MLP output un-added, because the norm behind them adds them anyway.  Elsewhere the model is
+plain PyTorch.  What the library adds around it is the communication (gradient buckets in symmetric memory,
+all-reduced by the library's own kernels while backward still runs) and the fused optimizer step.
 The token embedding is padded to a multiple of 64 rows so the tied output projection is tensor-core
 friendly; the padding rows never receive probability mass (their logits are cut before the loss).
 """
@@ -16,6 +18,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _ext
 from ..ops.norm import FusedLayerNorm
 
 
@@ -42,7 +45,17 @@ class GPT2Config:
         return GPT2Config(n_layer=2, d_model=128, n_head=4, d_ff=512, vocab_size=1000, seq_len=64)
 
 
+def _added(x: torch.Tensor, pending, pending_bias) -> torch.Tensor:
+    """x + pending in plain PyTorch, where the fused node that would have added them cannot run; the bias that is already
+    part of `pending` gets its gradient here (its value is added and subtracted)."""
+    if pending is None:
+        return x
+    return x + pending if pending_bias is None else x + pending + (pending_bias - pending_bias.detach())
+
+
 class Block(nn.Module):
+    grad_sink = 0          # set by a data-parallel wrapper: how the fused nodes hand over weight gradients (csrc/torch/gradsink.h)
+
     def __init__(self, cfg: GPT2Config, fused: bool = True):
         super().__init__()
         norm = FusedLayerNorm if fused else nn.LayerNorm
@@ -62,8 +75,35 @@ class Block(nn.Module):
         self.ln2 = norm(cfg.d_model)
         self.fc = nn.Linear(cfg.d_model, cfg.d_ff)
         self.out = nn.Linear(cfg.d_ff, cfg.d_model)
+        # Where the parameters live, in the order the fused nodes take them (a look-up per parameter and call otherwise).
+        self._slots = [(m._parameters, n) for m in (self.ln1, self.q, self.k, self.v, self.proj, self.ln2, self.fc, self.out)
+                       for n in ("weight", "bias")] if fused else None
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def fused(self, x: torch.Tensor, pending, pending_bias, shape, bias_here: bool):
+        """The block on x + pending ([tokens, d_model]) as two tensors still to be added, or None where it has to run as plain
+        PyTorch.  `bias_here`: whether the gradient of the last bias is taken here or by whoever adds the two."""
+        if self._slots is None or not x.is_cuda or torch.is_autocast_enabled("cuda"):
+            return None
+        b, s = shape
+        return _ext.load().gpt2_block(x, pending, pending_bias, [d[n] for d, n in self._slots], b, s, self.n_head, bias_here,
+                                      self.ln1.eps, self.grad_sink)
+
+    def forward(self, x: torch.Tensor, pending=None, pending_bias=None, shape=None):
+        """x [batch, seq, d_model] -> the same.  With `shape` = (batch, seq), as GPT2 calls it: x and `pending` are
+        [batch * seq, d_model], the input is their sum, and the result is a pair whose sum is the output."""
+        if shape is not None:
+            pair = self.fused(x, pending, pending_bias, shape, False)
+            if pair is not None:
+                return pair
+            x = _added(x, pending, pending_bias)
+            return self._plain(x.view(*shape, -1)).view(x.shape), None
+        if self._slots is not None and x.is_cuda and x.dim() == 3 and x.is_contiguous():
+            pair = self.fused(x.view(-1, x.shape[-1]), None, None, x.shape[:2], True)
+            if pair is not None:
+                return (pair[0] + pair[1]).view(x.shape)
+        return self._plain(x)
+
+    def _plain(self, x: torch.Tensor) -> torch.Tensor:
         b, s, d = x.shape
         h = self.ln1(x)
         if self.split_qkv:
@@ -79,6 +119,8 @@ class Block(nn.Module):
 class GPT2(nn.Module):
     """Decoder-only transformer with learned positions, pre-LayerNorm blocks and a tied output projection;
     forward(idx, targets) returns the mean cross-entropy, forward(idx) the logits."""
+
+    grad_sink = 0          # see Block
 
     def __init__(self, cfg: GPT2Config, fused_loss: bool = True):
         super().__init__()
@@ -105,12 +147,28 @@ class GPT2(nn.Module):
 
     def forward(self, idx: torch.Tensor, targets: torch.Tensor | None = None):
         b, s = idx.shape
-        pos = torch.arange(s, device=idx.device)
-        x = self.wte(idx) + self.wpe(pos)
-        for blk in self.blocks:
-            x = blk(x)
-        x = self.ln_f(x)
-        logits = F.linear(x, self.wte.weight)            # tied output projection, padded vocab
+        w = self.wte.weight
+        x = None
+        if self.fused_loss and w.is_cuda and w.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
+            x = _ext.load().gpt2_embed(idx, w, self.wpe.weight, self.grad_sink)      # None where the kernels do not cover the case
+        if x is not None:
+            pending = bias = None
+            for blk in self.blocks:
+                x, pending = blk(x, pending, bias, (b, s))
+                # a block that ran as plain PyTorch has added everything and taken its bias gradient itself
+                bias = blk.out.bias if pending is not None else None
+            x = self._final_norm(x, pending, bias)
+        else:
+            pos = torch.arange(s, device=idx.device)
+            x = self.wte(idx) + self.wpe(pos)
+            for blk in self.blocks:
+                x = blk(x)
+            x = self.ln_f(x)
+        if targets is not None and self.fused_loss and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
+            loss = _ext.load().gpt2_head_loss(x.view(b * s, -1), w, targets, self.cfg.vocab_size, self.grad_sink)
+            if loss is not None:
+                return loss
+        logits = F.linear(x, w).view(b, s, -1)           # tied output projection, padded vocab
         if targets is None:
             return logits[..., : self.cfg.vocab_size]
         flat = logits.view(b * s, -1)
@@ -118,3 +176,10 @@ class GPT2(nn.Module):
             from ..ops.loss import fused_cross_entropy
             return fused_cross_entropy(flat, targets.reshape(-1).contiguous(), self.cfg.vocab_size)
         return F.cross_entropy(flat[:, : self.cfg.vocab_size].float(), targets.reshape(-1))
+
+    def _final_norm(self, x: torch.Tensor, pending, bias) -> torch.Tensor:
+        n = self.ln_f
+        if pending is None:
+            return n(x)
+        h = _ext.load().gpt2_final_norm(x, pending, bias, n.weight, n.bias, n.eps, self.grad_sink)
+        return h if h is not None else n(_added(x, pending, bias))

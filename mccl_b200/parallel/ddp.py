@@ -23,6 +23,7 @@ docs/perf-scaling.png, README.md:55-57); the wrapper itself has no counterpart t
 from __future__ import annotations
 
 import os
+import weakref
 from contextlib import contextmanager
 from typing import List, Optional
 
@@ -121,9 +122,31 @@ class DistributedDataParallel(nn.Module):
             self.comm_stream = torch.cuda.Stream(device=self.device, priority=-1) if self.device.type == "cuda" else None
             for p in params:
                 p.register_post_accumulate_grad_hook(self._on_grad)
+        self._attach_sink(module)
         self._reset()
 
     # ---- construction helpers
+    def _attach_sink(self, module: nn.Module) -> None:
+        """Modules with fused nodes (an attribute `grad_sink`) add their weight gradients to the bucket views themselves and,
+        with several ranks, report every finished parameter as the gradient hooks do."""
+        if self.device.type != "cuda":
+            return
+        sink = -1
+        if self.world > 1:
+            from .. import _ext
+            me = weakref.ref(self)
+
+            def finished(p):
+                ddp = me()
+                if ddp is not None:
+                    ddp._on_grad(p)
+
+            sink = _ext.load().register_sink(finished)
+            weakref.finalize(self, _ext.load().drop_sink, sink)
+        for m in module.modules():
+            if hasattr(m, "grad_sink"):
+                m.grad_sink = sink
+
     def _sync_initial_state(self, module: nn.Module) -> None:
         """Every replica starts from rank 0's parameters and buffers, whatever each rank was seeded with (only
         gradients are averaged afterwards, so replicas that start apart stay apart)."""
@@ -371,6 +394,7 @@ class _GraphedStep:
                 loss = ddp(*self.inputs)
                 loss.backward()
                 ddp.step(lr=lr, max_grad_norm=max_grad_norm, _hyper=self.hyper)
+                loss = None                       # its autograd graph belongs to this stream, which the recording must not touch
         cur.wait_stream(side)
         torch.cuda.synchronize(ddp.device)
         from ..ops import loss as loss_ops
