@@ -109,16 +109,25 @@ __global__ void __launch_bounds__(kCeThreads) ceForwardKernel(const __nv_bfloat1
   if (R > 1) colred::clusterSync();
 }
 
-// mean over the rows' losses, in a fixed order.
-__global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, float* out) {
+// Mean over the rows' losses, in a fixed order: over all rows or, with `targets`, over those whose target is a column
+// (`inverse`: one over their number, for the backward pass).
+__global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, const int64_t* targets, int vocab, float* out, float* inverse) {
   __shared__ float acc[32];
+  __shared__ int used;
+  if (threadIdx.x == 0) used = 0;
+  __syncthreads();
   float t = 0.f;
+  int c = 0;
   for (int64_t i = threadIdx.x; i < n; i += 8 * 1024) {
     float x[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) x[u] = i + u * 1024 < n ? v[i + u * 1024] : 0.f;
+    if (targets != nullptr)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) c += i + u * 1024 < n && targets[i + u * 1024] >= 0 && targets[i + u * 1024] < vocab;
     t += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
   }
+  if (targets != nullptr) atomicAdd(&used, c);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   if ((threadIdx.x & 31) == 0) acc[threadIdx.x >> 5] = t;
@@ -127,7 +136,10 @@ __global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, fl
   t = acc[threadIdx.x];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (threadIdx.x == 0) *out = t / (float)n;
+  if (threadIdx.x != 0) return;
+  const float rows = targets != nullptr ? (float)used : (float)n;
+  *out = t / rows;
+  if (inverse != nullptr) *inverse = 1.f / rows;
 }
 
 // Reads and writes every logit once: 301 us on 8192 x 50304 with one piece in flight, 288 us (5.7 TB/s) with four.
@@ -135,14 +147,14 @@ __global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, fl
 // pass, or the projection, left in L2.
 __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* logits, int64_t ld, int vocab, int width,
                                                                const int64_t* targets, const float* lse, const float* gradOut,
-                                                               float invRows) {
+                                                               const float* inverse, float invRows) {
   const int64_t row = (int64_t)gridDim.x - 1 - blockIdx.x;
   __nv_bfloat16* x = logits + row * ld;
   const float l = lse[row];
   const int64_t tgt64 = targets[row];
   const bool live = tgt64 >= 0 && tgt64 < vocab;
   const int tgt = live ? (int)tgt64 : -1;
-  const float scale = live ? (*gradOut) * invRows : 0.f;
+  const float scale = live ? (*gradOut) * (inverse != nullptr ? *inverse : invRows) : 0.f;
   const float off = -l * kLog2e;
   auto one = [&](int j, float xj) -> float {
     if (j >= vocab) return 0.f;
@@ -201,24 +213,31 @@ extern "C" mcclResult_t mcclCrossEntropyForward(const void* logits, int64_t rows
                         static_cast<const __nv_bfloat16*>(logits), ld, vocab, targets, loss, lse) == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 
-// The same followed by the mean of the rows' losses in *mean.
+// The same followed by the mean of the rows' losses in *mean: over all rows, or with `inverse` over the rows whose target is
+// a column, one over whose number goes there.
 extern "C" mcclResult_t mcclCrossEntropyMean(const void* logits, int64_t rows, int64_t ld, int vocab, const int64_t* targets, float* loss,
-                                             float* lse, float* mean, mcclStream_t stream) {
+                                             float* lse, float* mean, float* inverse, mcclStream_t stream) {
   if (mean == nullptr) return mcclInvalidArgument;
   const mcclResult_t rc = mcclCrossEntropyForward(logits, rows, ld, vocab, targets, loss, lse, stream);
   if (rc != mcclSuccess) return rc;
-  meanKernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(loss, rows, mean);     // no rows: 0 / 0, as a mean over none
+  meanKernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(loss, rows, inverse != nullptr ? targets : nullptr, vocab,
+                                                                         mean, inverse);     // no rows: 0 / 0, as a mean over none
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 
-// In place: logits[row, j] <- d(mean loss)/d(logit) * gradOut for j < vocab, 0 for vocab <= j < width.
-extern "C" mcclResult_t mcclCrossEntropyBackward(void* logits, int64_t rows, int64_t ld, int vocab, int width,
-                                                 const int64_t* targets, const float* lse, const float* gradOut,
-                                                 mcclStream_t stream) {
+// In place: logits[row, j] <- d(mean loss)/d(logit) * gradOut for j < vocab, 0 for vocab <= j < width.  inverse: what
+// mcclCrossEntropyMean stored there, or null where the mean was over all rows.
+extern "C" mcclResult_t mcclCrossEntropyMeanBackward(void* logits, int64_t rows, int64_t ld, int vocab, int width, const int64_t* targets,
+                                                     const float* lse, const float* gradOut, const float* inverse, mcclStream_t stream) {
   if (logits == nullptr || targets == nullptr || lse == nullptr || gradOut == nullptr || rows < 0 || vocab <= 0 || width < vocab ||
       ld < width) return mcclInvalidArgument;
   if (rows == 0) return mcclSuccess;
   ceBackwardKernel<<<dim3((unsigned)rows, (unsigned)ceSplit(rows, width)), kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(logits), ld, vocab, width, targets, lse, gradOut, 1.0f / (float)rows);
+      static_cast<__nv_bfloat16*>(logits), ld, vocab, width, targets, lse, gradOut, inverse, 1.0f / (float)rows);
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
+
+extern "C" mcclResult_t mcclCrossEntropyBackward(void* logits, int64_t rows, int64_t ld, int vocab, int width, const int64_t* targets,
+                                                 const float* lse, const float* gradOut, mcclStream_t stream) {
+  return mcclCrossEntropyMeanBackward(logits, rows, ld, vocab, width, targets, lse, gradOut, nullptr, stream);
 }

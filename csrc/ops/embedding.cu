@@ -27,7 +27,7 @@ __device__ __forceinline__ uint4 pack(const float* f) {
   return q;
 }
 
-// out[t] = table[idx[t]] + pos[t % seq]; NaN for an index outside the table.
+// out[t] = table[idx[t]] + pos[t % seq] (pos may be null); NaN for an index outside the table.
 __global__ void __launch_bounds__(256) embedKernel(const int64_t* idx, const uint4* table, const uint4* pos, int64_t n, int seq,
                                                    int64_t vocab, int vecs, uint4* out) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(256) embedKernel(const int64_t* idx, const uin
   const int v = (int)(i - t * vecs);
   const int64_t id = idx[t];
   float a[8], b[8];
-  unpack(pos[(t % seq) * vecs + v], b);
+  unpack(pos != nullptr ? pos[(t % seq) * vecs + v] : make_uint4(0, 0, 0, 0), b);
   if (id >= 0 && id < vocab) {
     unpack(table[id * vecs + v], a);
 #pragma unroll
@@ -152,7 +152,7 @@ extern "C" {
 
 mcclResult_t mcclEmbeddingForward(const int64_t* idx, const void* table, const void* pos, void* out, int64_t tokens, int seq, int64_t vocab,
                                   int D, mcclStream_t stream) {
-  if (!idx || !table || !pos || !out || tokens <= 0 || seq <= 0 || D <= 0 || D % 8 || !aligned16(table) || !aligned16(pos) || !aligned16(out))
+  if (!idx || !table || !out || tokens <= 0 || seq <= 0 || D <= 0 || D % 8 || !aligned16(table) || !aligned16(pos) || !aligned16(out))
     return mcclInvalidArgument;
   embedKernel<<<(unsigned)((tokens * (D / 8) + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       idx, static_cast<const uint4*>(table), static_cast<const uint4*>(pos), tokens, seq, vocab, D / 8, static_cast<uint4*>(out));
@@ -161,10 +161,10 @@ mcclResult_t mcclEmbeddingForward(const int64_t* idx, const void* table, const v
 
 int mcclEmbeddingMaxTokens(void) { return kMaxTokens; }
 
-// tableGrad rows += the rows of dy with their index; posGrad += dy summed over the batch.  count: vocab ints of work memory.
+// tableGrad rows += the rows of dy with their index; posGrad (may be null) += dy summed over the batch.  count: vocab ints of work memory.
 mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, int32_t* count, int64_t tokens, int seq,
                                    int64_t vocab, int D, mcclStream_t stream) {
-  if (!idx || !dy || !tableGrad || !posGrad || !count || tokens <= 0 || tokens > kMaxTokens || seq <= 0 || tokens % seq || D <= 0 || D % 8 ||
+  if (!idx || !dy || !tableGrad || !count || tokens <= 0 || tokens > kMaxTokens || seq <= 0 || tokens % seq || D <= 0 || D % 8 ||
       D / 8 > kMaxVecs || !aligned16(dy) || !aligned16(tableGrad) || !aligned16(posGrad)) return mcclInvalidArgument;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int n = (int)tokens, vecs = D / 8;
@@ -176,7 +176,7 @@ mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tab
   else if (vecs <= 2 * kEmbThreads) tableGradKernel<2><<<n, kEmbThreads, 0, s>>>(idx, g, count, n, vocab, vecs, tg);
   else tableGradKernel<4><<<n, kEmbThreads, 0, s>>>(idx, g, count, n, vocab, vecs, tg);
   const int64_t perSeq = (int64_t)seq * vecs;
-  posGradKernel<<<(unsigned)((perSeq + 255) / 256), 256, 0, s>>>(g, n / seq, perSeq, static_cast<uint4*>(posGrad));
+  if (posGrad != nullptr) posGradKernel<<<(unsigned)((perSeq + 255) / 256), 256, 0, s>>>(g, n / seq, perSeq, static_cast<uint4*>(posGrad));
   return launchedOk();
 }
 

@@ -42,5 +42,6 @@ void bindOps(pybind11::module_& m);
 void bindComm(pybind11::module_& m);
 void bindMoe(pybind11::module_& m);
 void bindGpt2(pybind11::module_& m);
+void bindLlama(pybind11::module_& m);
 
 }  // namespace mccl_torch

@@ -7,12 +7,10 @@
 //     kernel for the projections that feed a residual add, the GELU's for the up projection;
 //   * weight gradients are accumulated by the matrix product itself (gradsink.h).
 // The bias of a projection whose output is added by the NEXT node gets its gradient there; it is passed along for that.
-#include "gradsink.h"
+#include "nodes.h"
 
 namespace mccl_torch {
 namespace {
-
-using OptTensor = std::optional<Tensor>;
 
 std::mutex sinkMutex;
 std::vector<py::object>& sinkTable() { static auto* t = new std::vector<py::object>(1); return *t; }
@@ -28,22 +26,6 @@ void dropSink(int64_t id) {
   std::lock_guard<std::mutex> lk(sinkMutex);
   if (id > 0 && id < (int64_t)sinkTable().size()) sinkTable()[id] = py::object();
 }
-
-struct Norm { Tensor stats; float* mean() const { return stats.data_ptr<float>(); } float* rstd(int64_t rows) const { return mean() + rows; } };
-
-Norm normStats(const Tensor& x, int64_t rows) { return Norm{at::empty({2, rows}, x.options().dtype(at::kFloat))}; }
-
-Tensor columnScratch(const Tensor& like, int64_t rows, int64_t d, int n) {
-  return at::empty({mcclColumnSumScratch(rows, (int)d, n)}, like.options().dtype(at::kFloat));
-}
-
-Tensor rows2d(const Tensor& g, int64_t T, int64_t d) {
-  Tensor r = g.reshape({T, d});
-  return r.is_contiguous() && aligned16(r) ? r : r.clone(at::MemoryFormat::Contiguous);
-}
-
-// [b, h, s, hd] (any layout) -> [b s, h hd]; no copy when the memory is laid out that way.
-Tensor fromHeads(const Tensor& a, int64_t T, int64_t d) { return rows2d(a.transpose(1, 2), T, d); }
 
 // Three adjacent matrices (or vectors) of one storage as one, in memory order; undefined where they are not adjacent.
 Tensor adjacent(const Tensor& a, const Tensor& b, const Tensor& c) {
@@ -293,13 +275,14 @@ struct FinalNormFn : torch::autograd::Function<FinalNormFn> {
 
 // ---- embedding ----------------------------------------------------------------------------------------------------------
 struct EmbedFn : torch::autograd::Function<EmbedFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& idx, const Tensor& table, const Tensor& pos, int64_t sink) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& idx, const Tensor& table, const OptTensor& pos, int64_t sink) {
     at::AutoDispatchBelowADInplaceOrView below;
     const int64_t T = idx.numel(), d = table.size(1), seq = idx.size(-1);
     Tensor i = idx.contiguous(), out = at::empty({T, d}, table.options());
-    check(mcclEmbeddingForward(i.data_ptr<int64_t>(), table.data_ptr(), pos.data_ptr(), out.data_ptr(), T, (int)seq, table.size(0), (int)d,
+    check(mcclEmbeddingForward(i.data_ptr<int64_t>(), table.data_ptr(), pos ? pos->data_ptr() : nullptr, out.data_ptr(), T, (int)seq,
+                               table.size(0), (int)d,
                                streamOf(out)), "mcclEmbeddingForward");
-    ctx->save_for_backward({i, table, pos});
+    ctx->save_for_backward({i, table, pos ? *pos : Tensor()});
     ctx->saved_data["sink"] = sink;
     return out;
   }
@@ -313,43 +296,49 @@ struct EmbedFn : torch::autograd::Function<EmbedFn> {
     Tensor dy = rows2d(g[0], T, d);
     variable_list ret(4);
     const bool here = T <= mcclEmbeddingMaxTokens();
-    Tensor dt = here ? sink.buffer(table) : Tensor(), dp = here ? sink.buffer(pos) : Tensor();
-    const bool direct = dt.defined() && dp.defined();
+    const bool withPos = pos.defined();
+    Tensor dt = here ? sink.buffer(table) : Tensor(), dp = here && withPos ? sink.buffer(pos) : Tensor();
+    const bool direct = dt.defined() && (dp.defined() || !withPos);
     if (!direct) {
       if (here) {
         ret[1] = dt = at::zeros(table.sizes(), table.options());
-        ret[2] = dp = at::zeros(pos.sizes(), pos.options());
+        if (withPos) ret[2] = dp = at::zeros(pos.sizes(), pos.options());
       } else {
         // Too many tokens for the kernel's scan: the sorting form of the tensor library.
         ret[1] = at::embedding_dense_backward(dy, idx.view({T}), V, -1, false);
-        ret[2] = at::zeros(pos.sizes(), pos.options());
-        ret[2].narrow(0, 0, seq).copy_(dy.view({T / seq, seq, d}).sum(0));
+        if (withPos) {
+          ret[2] = at::zeros(pos.sizes(), pos.options());
+          ret[2].narrow(0, 0, seq).copy_(dy.view({T / seq, seq, d}).sum(0));
+        }
         return ret;
       }
     }
     Tensor count = at::empty({V}, idx.options().dtype(at::kInt));
-    check(mcclEmbeddingBackward(idx.data_ptr<int64_t>(), dy.data_ptr(), dt.data_ptr(), dp.data_ptr(), count.data_ptr<int32_t>(), T, (int)seq, V,
+    check(mcclEmbeddingBackward(idx.data_ptr<int64_t>(), dy.data_ptr(), dt.data_ptr(), withPos ? dp.data_ptr() : nullptr, count.data_ptr<int32_t>(), T, (int)seq, V,
                                 (int)d, streamOf(dy)), "mcclEmbeddingBackward");
-    if (direct) { sink.done(table); sink.done(pos); }
+    if (direct) { sink.done(table); if (withPos) sink.done(pos); }
     sink.flush();
     return ret;
   }
 };
 
-// ---- head: tied projection and cross-entropy ----------------------------------------------------------------------------
+// ---- head: projection and cross-entropy ----------------------------------------------------------------------------
 struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, int64_t sink) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, bool tied, bool meanOfUsed,
+                        int64_t sink) {
     at::AutoDispatchBelowADInplaceOrView below;
     const int64_t T = h.size(0);
     Tensor logits = at::linear(h, w);
     Tensor t = targets.contiguous();
-    Tensor perRow = at::empty({2, T}, h.options().dtype(at::kFloat)), mean = at::empty({}, perRow.options());
+    Tensor perRow = at::empty({2 * T + 1}, h.options().dtype(at::kFloat)), mean = at::empty({}, perRow.options());
     float* loss = perRow.data_ptr<float>();
     check(mcclCrossEntropyMean(logits.data_ptr(), T, logits.stride(0), (int)vocab, t.data_ptr<int64_t>(), loss, loss + T, mean.data_ptr<float>(),
-                               streamOf(h)), "mcclCrossEntropyForward");
+                               meanOfUsed ? loss + 2 * T : nullptr, streamOf(h)), "mcclCrossEntropyForward");
     counters().loss++;
     ctx->save_for_backward({h, w, t, logits, perRow});
     ctx->saved_data["vocab"] = vocab;
+    ctx->saved_data["tied"] = tied;
+    ctx->saved_data["used"] = meanOfUsed;
     ctx->saved_data["sink"] = sink;
     return mean;
   }
@@ -362,29 +351,21 @@ struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
     GradSink sink(ctx->saved_data["sink"].toInt());
     const int64_t T = h.size(0);
     Tensor go = g[0].scalar_type() == at::kFloat ? g[0] : g[0].to(at::kFloat);
-    check(mcclCrossEntropyBackward(logits.data_ptr(), T, logits.stride(0), (int)ctx->saved_data["vocab"].toInt(), (int)logits.size(1),
-                                   t.data_ptr<int64_t>(), perRow.data_ptr<float>() + T, go.data_ptr<float>(), streamOf(h)),
+    float* rows = perRow.data_ptr<float>();
+    check(mcclCrossEntropyMeanBackward(logits.data_ptr(), T, logits.stride(0), (int)ctx->saved_data["vocab"].toInt(), (int)logits.size(1),
+                                       t.data_ptr<int64_t>(), rows + T, go.data_ptr<float>(),
+                                       ctx->saved_data["used"].toBool() ? rows + 2 * T : nullptr, streamOf(h)),
           "mcclCrossEntropyBackward");
     counters().loss++;
-    variable_list ret(5);
+    variable_list ret(7);
     ret[0] = at::mm(logits, w);
-    weightGrad(sink, w, logits, h, &ret[1], /*last=*/false);       // the tied weight gets the embedding's share later
+    weightGrad(sink, w, logits, h, &ret[1], !ctx->saved_data["tied"].toBool());      // a tied weight gets the embedding's share later
+    sink.flush();
     return ret;
   }
 };
 
 // ---- entry points ---------------------------------------------------------------------------------------------------------
-bool plainBf16(const Tensor& t, const Tensor& like) {
-  return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.device() == like.device() && t.is_contiguous() &&
-         !t.unsafeGetTensorImpl()->is_python_dispatch() && aligned16(t);
-}
-
-bool usable(const Tensor& x, const std::vector<Tensor>& params) {
-  if (!plainBf16(x, x) || x.size(-1) % 8 || x.size(-1) > 4096 || x.numel() == 0) return false;
-  for (const Tensor& p : params) if (!plainBf16(p, x)) return false;
-  return true;
-}
-
 // One block on x + pending (both [T, d]; pending may be missing).  params: ln1 w b, q w b, k w b, v w b, proj w b, ln2 w b,
 // fc w b, out w b.  Returns (residual, MLP output), whose sum is the block's output, or None where the kernels do not cover
 // the case.
@@ -401,8 +382,10 @@ py::object block(const Tensor& x, const OptTensor& pending, const OptTensor& pen
   return py::make_tuple(out[0], out[1]);
 }
 
-py::object embed(const Tensor& idx, const Tensor& table, const Tensor& pos, int64_t sink) {
-  if (!idx.is_cuda() || idx.scalar_type() != at::kLong || idx.numel() == 0 || idx.size(-1) > pos.size(0) || !usable(table, {table, pos})) return py::none();
+// table[idx] + pos (pos may be missing) as [tokens, d].
+py::object embed(const Tensor& idx, const Tensor& table, const OptTensor& pos, int64_t sink) {
+  if (!idx.is_cuda() || idx.scalar_type() != at::kLong || idx.numel() == 0 || !usable(table, {table})) return py::none();
+  if (pos && (idx.size(-1) > pos->size(0) || !usable(*pos, {}))) return py::none();
   c10::cuda::CUDAGuard guard(table.device());
   return py::cast(EmbedFn::apply(idx, table, pos, sink));
 }
@@ -413,10 +396,12 @@ py::object finalNorm(const Tensor& x, const Tensor& pending, const OptTensor& pe
   return py::cast(FinalNormFn::apply(x, pending, pendingBias, w, b, eps, sink, !at::GradMode::is_enabled()));
 }
 
-py::object headLoss(const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, int64_t sink) {
+// Mean cross-entropy of h w^T: over all rows, or over those whose target is a column (`meanOfUsed`).  tied: w is the embedding
+// table too.
+py::object headLoss(const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, bool tied, bool meanOfUsed, int64_t sink) {
   if (!usable(h, {w}) || !targets.is_cuda() || targets.scalar_type() != at::kLong || targets.numel() != h.size(0) || w.size(0) < vocab) return py::none();
   c10::cuda::CUDAGuard guard(h.device());
-  return py::cast(HeadLossFn::apply(h, w, targets.reshape({-1}), vocab, sink));
+  return py::cast(HeadLossFn::apply(h, w, targets.reshape({-1}), vocab, tied, meanOfUsed, sink));
 }
 
 }  // namespace
@@ -435,9 +420,9 @@ void GradSink::flush() {
 
 void bindGpt2(py::module_& m) {
   m.def("gpt2_block", &block);
-  m.def("gpt2_embed", &embed);
+  m.def("decoder_embed", &embed);
   m.def("gpt2_final_norm", &finalNorm);
-  m.def("gpt2_head_loss", &headLoss);
+  m.def("decoder_head_loss", &headLoss);
   m.def("register_sink", &registerSink);
   m.def("drop_sink", &dropSink);
 }

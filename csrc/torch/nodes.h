@@ -1,0 +1,37 @@
+// Helpers of the decoders' nodes.
+#pragma once
+
+#include "gradsink.h"
+
+namespace mccl_torch {
+
+using OptTensor = std::optional<Tensor>;
+
+struct Norm { Tensor stats; float* mean() const { return stats.data_ptr<float>(); } float* rstd(int64_t rows) const { return mean() + rows; } };
+
+inline Norm normStats(const Tensor& x, int64_t rows) { return Norm{at::empty({2, rows}, x.options().dtype(at::kFloat))}; }
+
+inline Tensor columnScratch(const Tensor& like, int64_t rows, int64_t d, int n) {
+  return at::empty({mcclColumnSumScratch(rows, (int)d, n)}, like.options().dtype(at::kFloat));
+}
+
+inline Tensor rows2d(const Tensor& g, int64_t T, int64_t d) {
+  Tensor r = g.reshape({T, d});
+  return r.is_contiguous() && aligned16(r) ? r : r.clone(at::MemoryFormat::Contiguous);
+}
+
+// [b, h, s, hd] (any layout) -> [b s, h hd]; no copy when the memory is laid out that way.
+inline Tensor fromHeads(const Tensor& a, int64_t T, int64_t d) { return rows2d(a.transpose(1, 2), T, d); }
+
+inline bool plainBf16(const Tensor& t, const Tensor& like) {
+  return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.device() == like.device() && t.is_contiguous() &&
+         !t.unsafeGetTensorImpl()->is_python_dispatch() && aligned16(t);
+}
+
+inline bool usable(const Tensor& x, const std::vector<Tensor>& params) {
+  if (!plainBf16(x, x) || x.size(-1) % 8 || x.size(-1) > 4096 || x.numel() == 0) return false;
+  for (const Tensor& p : params) if (!plainBf16(p, x)) return false;
+  return true;
+}
+
+}  // namespace mccl_torch

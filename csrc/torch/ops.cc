@@ -59,7 +59,7 @@ struct CrossEntropyFn : torch::autograd::Function<CrossEntropyFn> {
     float* loss = perRow.data_ptr<float>();
     c10::cuda::CUDAGuard guard(logits.device());
     check(mcclCrossEntropyMean(logits.data_ptr(), rows, logits.stride(0), (int)vocab, targets.data_ptr<int64_t>(), loss, loss + rows,
-                               mean.data_ptr<float>(), streamOf(logits)), "mcclCrossEntropyForward");
+                               mean.data_ptr<float>(), nullptr, streamOf(logits)), "mcclCrossEntropyForward");
     counters().loss++;
     ctx->save_for_backward({logits, targets, perRow});
     ctx->saved_data["vocab"] = vocab;
@@ -168,4 +168,5 @@ PYBIND11_MODULE(mccl_torch, m) {
   mccl_torch::bindComm(m);
   mccl_torch::bindMoe(m);
   mccl_torch::bindGpt2(m);
+  mccl_torch::bindLlama(m);
 }

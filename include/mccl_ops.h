@@ -78,13 +78,19 @@ int64_t      mcclColumnSumScratch(int64_t rows, int D, int segments);
 mcclResult_t mcclColumnSums(const void* const* x, void* const* out, int n, int accumulate, float* scratch, int64_t rows, int D, int64_t ld,
                             mcclStream_t stream);
 
-/* ---- embedding: out[t] = table[idx[t]] + pos[t % seq]; the backward pass adds into both gradients ---------------------- */
+/* ---- embedding: out[t] = table[idx[t]] + pos[t % seq] (pos nullable); the backward pass adds into the gradients ---------- */
 mcclResult_t mcclEmbeddingForward(const int64_t* idx, const void* table, const void* pos, void* out, int64_t tokens, int seq, int64_t vocab,
                                   int D, mcclStream_t stream);
 /* tokens <= mcclEmbeddingMaxTokens(), D <= 4096; count: vocab ints of work memory. */
 int          mcclEmbeddingMaxTokens(void);
 mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, int32_t* count, int64_t tokens, int seq,
                                    int64_t vocab, int D, mcclStream_t stream);
+
+/* ---- rotary position embedding: pairs (i, i + hd/2) of every head turned by position x theta^(-i / (hd/2)) ---------------- */
+/* src: [batch, seq, heads, hd] at element strides sb, ss, sh (last one 1); dst: contiguous [batch, seq, heads, hd], may be src where
+ * that is contiguous too; inverse: turn back (the backward pass).  Two arrays in one launch (the second may be null). */
+mcclResult_t mcclRope(const void* src0, const void* src1, void* dst0, void* dst1, int batch, int seq, int heads, int hd, int64_t sb,
+                      int64_t ss, int64_t sh, float theta, int inverse, mcclStream_t stream);
 
 /* ---- training-step kernels (bf16 parameters and gradients, fp32 state) --------------------------------------------- */
 /* AdamW on n elements; normSq / maxNorm (nullable / 0): clip by the global gradient norm held on the device. */
@@ -103,9 +109,12 @@ mcclResult_t mcclSumSquaresBf16(const void* x, uint64_t n, float* scratch, uint6
 /* Cross-entropy over bf16 logits [rows, ld] (vocab <= ld): per-row loss and log-sum-exp; backward in place. */
 mcclResult_t mcclCrossEntropyForward(const void* logits, int64_t rows, int64_t ld, int vocab, const int64_t* targets, float* loss,
                                      float* lse, mcclStream_t stream);
-/* The same with the mean of the rows' losses in *mean. */
+/* The same with the mean of the rows' losses in *mean: over all rows, or, with inverse (nullable), over those whose target is a
+ * column; one over their number goes to *inverse, which the backward pass takes. */
 mcclResult_t mcclCrossEntropyMean(const void* logits, int64_t rows, int64_t ld, int vocab, const int64_t* targets, float* loss, float* lse,
-                                  float* mean, mcclStream_t stream);
+                                  float* mean, float* inverse, mcclStream_t stream);
+mcclResult_t mcclCrossEntropyMeanBackward(void* logits, int64_t rows, int64_t ld, int vocab, int width, const int64_t* targets,
+                                          const float* lse, const float* gradOut, const float* inverse, mcclStream_t stream);
 mcclResult_t mcclCrossEntropyBackward(void* logits, int64_t rows, int64_t ld, int vocab, int width, const int64_t* targets,
                                       const float* lse, const float* gradOut, mcclStream_t stream);
 /* LayerNorm over bf16 rows of D elements, D % 8 == 0 and D <= 4096.  The backward passes need partial:

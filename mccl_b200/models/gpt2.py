@@ -150,7 +150,7 @@ class GPT2(nn.Module):
         w = self.wte.weight
         x = None
         if self.fused_loss and w.is_cuda and w.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
-            x = _ext.load().gpt2_embed(idx, w, self.wpe.weight, self.grad_sink)      # None where the kernels do not cover the case
+            x = _ext.load().decoder_embed(idx, w, self.wpe.weight, self.grad_sink)      # None where the kernels do not cover the case
         if x is not None:
             pending = bias = None
             for blk in self.blocks:
@@ -165,7 +165,7 @@ class GPT2(nn.Module):
                 x = blk(x)
             x = self.ln_f(x)
         if targets is not None and self.fused_loss and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
-            loss = _ext.load().gpt2_head_loss(x.view(b * s, -1), w, targets, self.cfg.vocab_size, self.grad_sink)
+            loss = _ext.load().decoder_head_loss(x.view(b * s, -1), w, targets, self.cfg.vocab_size, True, False, self.grad_sink)
             if loss is not None:
                 return loss
         logits = F.linear(x, w).view(b, s, -1)           # tied output projection, padded vocab

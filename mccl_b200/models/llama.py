@@ -23,6 +23,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _ext
 from ..comm import Communicator
 from ..parallel import functional as PF
 from ..parallel.layers import ColumnParallelLinear, RowParallelLinear
@@ -69,7 +70,10 @@ def rope(x: torch.Tensor, theta: float) -> torch.Tensor:
 
 
 class Block(nn.Module):
-    """Pre-norm attention + SwiGLU block holding 1/n of every projection."""
+    """Pre-norm attention + SwiGLU block holding 1/n of every projection.  With one rank, on CUDA in bf16, it runs as two fused
+    autograd nodes around attention (csrc/torch/llama.cc)."""
+
+    grad_sink = 0          # set by a data-parallel wrapper: how the fused nodes hand over weight gradients (csrc/torch/gradsink.h)
 
     def __init__(self, cfg: LlamaConfig, comm: Communicator, sp: bool):
         super().__init__()
@@ -88,12 +92,30 @@ class Block(nn.Module):
         self.gate = ColumnParallelLinear(comm, d, f, bias=False, sequence_parallel=sp)
         self.up = ColumnParallelLinear(comm, d, f, bias=False)
         self.down = RowParallelLinear(comm, f, d, bias=False, sequence_parallel=sp)
+        self._slots = [m._parameters for m in (self.norm1, self.q, self.k, self.v, self.o, self.norm2, self.gate, self.up, self.down)] \
+            if n == 1 else None
 
     def _enter(self, x: torch.Tensor) -> torch.Tensor:
         """[batch*seq (/ n), d] -> the full token set every rank's weight shards are applied to."""
         return PF.all_gather_rows(x, self.comm) if self.sp else PF.copy_to_ranks(x, self.comm)
 
-    def forward(self, x: torch.Tensor, batch: int, seq: int) -> torch.Tensor:
+    def fused(self, x: torch.Tensor, pending, batch: int, seq: int):
+        """The block on x + pending as two tensors still to be added, or None where it has to run as separate operations."""
+        if self._slots is None or not x.is_cuda or torch.is_autocast_enabled("cuda"):
+            return None
+        return _ext.load().llama_block(x, pending, [d["weight"] for d in self._slots], batch, seq, self.heads_local, self.cfg.rope_theta,
+                                       self.cfg.eps, self.grad_sink)
+
+    def forward(self, x: torch.Tensor, batch: int, seq: int, pending=None, pair: bool = False):
+        """x [batch * seq (/ n), d] -> the same.  With `pair`, as Llama calls it, the input is x + pending and the result two
+        tensors whose sum is the output (the second one may be None)."""
+        two = self.fused(x, pending, batch, seq)
+        if two is not None:
+            return two if pair else two[0] + two[1]
+        y = self._plain(x if pending is None else x + pending, batch, seq)
+        return (y, None) if pair else y
+
+    def _plain(self, x: torch.Tensor, batch: int, seq: int) -> torch.Tensor:
         h = self._enter(self.norm1(x))
         q, k, v = (F.linear(h, m.weight).view(batch, seq, self.heads_local, self.head_dim) for m in (self.q, self.k, self.v))
         q, k = rope(q, self.cfg.rope_theta), rope(k, self.cfg.rope_theta)
@@ -107,6 +129,8 @@ class Llama(nn.Module):
     """Tensor-parallel Llama-style decoder on `comm`; forward(idx, targets) returns the mean cross-entropy over all
     tokens (the same value on every rank), forward(idx) the logits of this rank's tokens."""
 
+    grad_sink = 0          # see Block
+
     def __init__(self, cfg: LlamaConfig, comm: Communicator, sequence_parallel: bool = False):
         super().__init__()
         self.cfg, self.comm, self.sp = cfg, comm, sequence_parallel and comm.size > 1
@@ -118,6 +142,8 @@ class Llama(nn.Module):
     def forward(self, idx: torch.Tensor, targets: Optional[torch.Tensor] = None) -> torch.Tensor:
         b, s = idx.shape
         n, r = self.comm.size, self.comm.rank
+        if n == 1 and idx.is_cuda and not torch.is_autocast_enabled("cuda"):
+            return self._forward_one_rank(idx, targets)
         x = self.embed(idx).view(b * s, -1)
         if self.sp:                                       # this rank's rows of the flattened (batch, seq) tokens
             rows = b * s // n
@@ -133,6 +159,25 @@ class Llama(nn.Module):
             # mean over ALL tokens: every rank contributes the sum over its rows
             return PF.all_reduce_sum(F.cross_entropy(logits.float(), t, reduction="sum"), self.comm) / (b * s)
         return F.cross_entropy(logits.float(), t)
+
+    def _forward_one_rank(self, idx: torch.Tensor, targets: Optional[torch.Tensor]) -> torch.Tensor:
+        """Every piece in a fused node where the kernels cover it (they answer None elsewhere) and as separate operations where not."""
+        ext, (b, s) = _ext.load(), idx.shape
+        x = ext.decoder_embed(idx, self.embed.weight, None, self.grad_sink)
+        if x is None:
+            x = self.embed(idx).view(b * s, -1)
+        pending = None
+        for blk in self.blocks:
+            x, pending = blk(x, b, s, pending, True)
+        h = ext.llama_final_norm(x, pending, self.norm.weight, self.norm.eps, self.grad_sink) if pending is not None else None
+        if h is None:
+            h = self.norm(x if pending is None else x + pending)
+        if targets is not None:
+            loss = ext.decoder_head_loss(h, self.head.weight, targets, self.head.weight.shape[0], False, True, self.grad_sink)
+            if loss is not None:
+                return loss
+        logits = self.head(h)
+        return logits if targets is None else F.cross_entropy(logits.float(), targets.reshape(-1))
 
     # ---- weights
     @torch.no_grad()
