@@ -68,6 +68,8 @@ struct GemmArgs {
   unsigned int* tailCount;
   CUtensorMap mapC;            // two-SM kernel: C as [M, N] bf16, box 64 x 32, for the epilogue's TMA stores
   int tmaStore;                // 1: mapC is valid
+  __nv_bfloat16* pre;          // optional [M, N]: the sums before the activation (for a backward pass), and its map as mapC
+  CUtensorMap mapPre;
   int debug;                   // tuning aid of the two-SM kernel (MCCL_GEMM_DEBUG): bit 0 = skip the loads after the
                                // first ring fill, bit 1 = skip the epilogue's global stores (results are then meaningless), bit 2 = per-thread
                                // 16-byte stores instead of the TMA store
@@ -81,6 +83,23 @@ template <int BN> struct Smem {
 };
 
 __device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+
+// 32 accumulator columns of a row, through the activation, as bf16. 
+template <bool SILU>
+__device__ __forceinline__ void storeRow32(const uint32_t* v, __nv_bfloat16* to) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint4 q;
+    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float x0 = __uint_as_float(v[8 * j + 2 * e]), x1 = __uint_as_float(v[8 * j + 2 * e + 1]);
+      if (SILU) { x0 = silu(x0); x1 = silu(x1); }
+      o2[e] = __floats2bfloat162_rn(x0, x1);
+    }
+    reinterpret_cast<uint4*>(to)[j] = q;
+  }
+}
 
 __device__ __forceinline__ uint64_t ldAcquireGpu(const uint64_t* p) {
   uint64_t v;
@@ -313,17 +332,8 @@ __global__ void __launch_bounds__(kThreadsGemm, 1) tpGemmKernel(const __grid_con
         uint32_t v[32];
         umma::tmemLoad32x32(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * 256u + (uint32_t)c * 32u, v);
         umma::tmemLoadWait();
-        uint4 outv[4];
-        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(outv);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          float x0 = __uint_as_float(v[2 * j]), x1 = __uint_as_float(v[2 * j + 1]);
-          if (a.epilogue == EPI_SILU) { x0 = silu(x0); x1 = silu(x1); }
-          o2[j] = __floats2bfloat162_rn(x0, x1);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(dstRow + c * 32);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dst[j] = outv[j];
+        if (a.pre != nullptr) storeRow32<false>(v, a.pre + (dstRow - a.C) + c * 32);
+        if (a.epilogue == EPI_SILU) storeRow32<true>(v, dstRow + c * 32); else storeRow32<false>(v, dstRow + c * 32);
       }
       umma::tcFenceBefore();
       __syncwarp();

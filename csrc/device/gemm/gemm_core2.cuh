@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(MODE == MODE_PLAIN ? kThreadsGemm2 : kThreadsG
     umma::prefetchTensorMap(&a.mapA);
     umma::prefetchTensorMap(&a.mapB);
     if (a.tmaStore) umma::prefetchTensorMap(&a.mapC);
+    if (MODE != MODE_RS && a.pre != nullptr) umma::prefetchTensorMap(&a.mapPre);
   }
   if (warp == 2) { umma2::tmemAlloc(tmemSlot, kTmemCols); umma2::tmemRelinquish(); }
   umma::tcFenceBefore();
@@ -280,32 +281,37 @@ __global__ void __launch_bounds__(MODE == MODE_PLAIN ? kThreadsGemm2 : kThreadsG
         uint8_t* myEpi = sEpi + q * 8192;
 #pragma unroll 1
         for (int c64 = 0; c64 < BN / 64; ++c64) {
-          uint8_t* buf = myEpi + (epiCount++ & 1) * 4096;
           uint32_t v[64];
           const uint32_t taddr = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * 256u + (uint32_t)c64 * 64u;
           umma::tmemLoad32x32(taddr, v);
           umma::tmemLoad32x32(taddr + 32u, v + 32);
-          if (lane == 0) umma::tmaStoreWaitRead<1>();          // the store that read this buffer two chunks ago is done with it
           umma::tmemLoadWait();
-          __syncwarp();
+          // The sums as they are, where they are wanted, and then through the activation: two chunks of the same columns.
+          const bool withPre = MODE != MODE_RS && a.pre != nullptr;
+          for (int pass = withPre ? 0 : 1; pass < 2; ++pass) {
+            uint8_t* buf = myEpi + (epiCount++ & 1) * 4096;
+            if (lane == 0) umma::tmaStoreWaitRead<1>();        // the store that read this buffer two chunks ago is done with it
+            __syncwarp();
+            const bool act = pass == 1 && a.epilogue == EPI_SILU;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            uint4 o;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+            for (int j = 0; j < 8; ++j) {
+              uint4 o;
+              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float x0 = __uint_as_float(v[8 * j + 2 * e]), x1 = __uint_as_float(v[8 * j + 2 * e + 1]);
-              if (a.epilogue == EPI_SILU) { x0 = silu(x0); x1 = silu(x1); }
-              o2[e] = __floats2bfloat162_rn(x0, x1);
+              for (int e = 0; e < 4; ++e) {
+                float x0 = __uint_as_float(v[8 * j + 2 * e]), x1 = __uint_as_float(v[8 * j + 2 * e + 1]);
+                if (act) { x0 = silu(x0); x1 = silu(x1); }
+                o2[e] = __floats2bfloat162_rn(x0, x1);
+              }
+              // 128-byte swizzle: 16-byte chunk j of row r sits at chunk j ^ (r % 8)
+              *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = o;
             }
-            // 128-byte swizzle: 16-byte chunk j of row r sits at chunk j ^ (r % 8)
-            *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = o;
-          }
-          umma::fenceProxyAsyncShared();
-          __syncwarp();
-          if (lane == 0 && !(a.debug & 2)) {
-            umma::tmaStore2d(&a.mapC, buf, nt * BN + c64 * 64, stripe128 * BM + q * 32);
-            umma::tmaStoreCommit();
+            umma::fenceProxyAsyncShared();
+            __syncwarp();
+            if (lane == 0 && !(a.debug & 2)) {
+              umma::tmaStore2d(pass == 0 ? &a.mapPre : &a.mapC, buf, nt * BN + c64 * 64, stripe128 * BM + q * 32);
+              umma::tmaStoreCommit();
+            }
           }
         }
         cDone = (BN / 64) * 2;
@@ -315,18 +321,9 @@ __global__ void __launch_bounds__(MODE == MODE_PLAIN ? kThreadsGemm2 : kThreadsG
         uint32_t v[32];
         umma::tmemLoad32x32(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * 256u + (uint32_t)c * 32u, v);
         umma::tmemLoadWait();
-        uint4 outv[4];
-        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(outv);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          float x0 = __uint_as_float(v[2 * j]), x1 = __uint_as_float(v[2 * j + 1]);
-          if (a.epilogue == EPI_SILU) { x0 = silu(x0); x1 = silu(x1); }
-          o2[j] = __floats2bfloat162_rn(x0, x1);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(dstRow + c * 32);
         if (a.debug & 2) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dst[j] = outv[j];
+        if (MODE != MODE_RS && a.pre != nullptr) storeRow32<false>(v, a.pre + (dstRow - a.C) + c * 32);
+        if (a.epilogue == EPI_SILU) storeRow32<true>(v, dstRow + c * 32); else storeRow32<false>(v, dstRow + c * 32);
       }
       umma::tcFenceBefore();
       __syncwarp();
@@ -391,16 +388,20 @@ __global__ void __launch_bounds__(MODE == MODE_PLAIN ? kThreadsGemm2 : kThreadsG
             for (int u = 0; u < 8; ++u) __stcg(sum4 + (size_t)(c16 * 4 + u) * BM, make_float4(0.f, 0.f, 0.f, 0.f));
 #pragma unroll
             for (int h = 0; h < 4; ++h) {                     // two quads = 8 columns = one 16-byte store
-              uint32_t o[4];
+              auto put = [&](__nv_bfloat16* to, bool act) {
+                uint32_t o[4];
 #pragma unroll
-              for (int k = 0; k < 2; ++k) {
-                float4 y = x[h * 2 + k];
-                if (a.epilogue == EPI_SILU) { y.x = silu(y.x); y.y = silu(y.y); y.z = silu(y.z); y.w = silu(y.w); }
-                __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
-                o[k * 2] = *reinterpret_cast<uint32_t*>(&lo);
-                o[k * 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
-              }
-              *reinterpret_cast<uint4*>(cRow + c16 * 16 + h * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+                for (int k = 0; k < 2; ++k) {
+                  float4 y = x[h * 2 + k];
+                  if (act) { y.x = silu(y.x); y.y = silu(y.y); y.z = silu(y.z); y.w = silu(y.w); }
+                  __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+                  o[k * 2] = *reinterpret_cast<uint32_t*>(&lo);
+                  o[k * 2 + 1] = *reinterpret_cast<uint32_t*>(&hi);
+                }
+                *reinterpret_cast<uint4*>(to + c16 * 16 + h * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+              };
+              if (a.pre != nullptr) put(a.pre + (cRow - a.C), false);
+              put(cRow, a.epilogue == EPI_SILU);
             }
           }
           if (row == 0) a.tailCount[tailIdx * 2 + (int)ctaRank] = 0u;

@@ -284,6 +284,75 @@ int pickPanel(int stripesPerBlock) {
   return 1;
 }
 
+// ---- plain products -------------------------------------------------------------------------------------------------
+mcclResult_t oneSmGemm(const void* A, const void* B, void* C, void* pre, int M, int N, int K, int epilogue, int maxCtas, mcclStream_t stream) {
+  if (A == nullptr || B == nullptr || C == nullptr) return mcclInvalidArgument;
+  MCCLCHECK(checkShapes(M, N, K, 1));
+  const int sms = maxCtas > 0 ? maxCtas : smCount();
+  const int bn = pickBN(M, N, sms);
+  if (bn == 0) return mcclInvalidArgument;
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  MCCLCHECK(makeMap(&a.mapA, A, M, K, BM));
+  MCCLCHECK(makeMap(&a.mapB, B, N, K, bn));
+  a.M = M; a.N = N; a.K = K;
+  a.C = static_cast<__nv_bfloat16*>(C);
+  a.pre = static_cast<__nv_bfloat16*>(pre);
+  a.epilogue = epilogue;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  a.errFlag = errFlagFor(dev).dev;
+  if (a.errFlag == nullptr) return mcclSystemError;
+  a.budgetNs = 2000000000ull;
+  a.panel = pickPanel(M / BM);
+  const int tiles = (M / BM) * (N / bn);
+  return launchMode<MODE_PLAIN>(a, bn, tiles < sms ? tiles : sms, reinterpret_cast<cudaStream_t>(stream));
+}
+
+mcclResult_t twoSmGemm(const void* A, const void* B, void* C, void* pre, int M, int N, int K, int epilogue, int maxCtas, mcclStream_t stream) {
+  if (A == nullptr || B == nullptr || C == nullptr) return mcclInvalidArgument;
+  MCCLCHECK(checkShapes(M, N, K, 1));
+  if (M % BM2) {
+    MCCL_WARN("the two-SM GEMM needs M %% %d == 0 (got %d)", BM2, M);
+    return mcclInvalidArgument;
+  }
+  const int pairsMax = std::max(1, (maxCtas > 0 ? maxCtas : smCount()) / 2);
+  int bn = pickBN2(M / BM2, N, pairsMax, K / BK, true);
+  const int forcedBn = (int)envInt("MCCL_GEMM_BN", 0);          // tuning aid: a tile width that divides N
+  if (forcedBn > 0 && N % forcedBn == 0) bn = forcedBn;
+  const void* fn = nullptr;
+  int smem = 0;
+  if (bn == 0 || !pairKernel<MODE_PLAIN>(bn, &fn, &smem)) return mcclInvalidArgument;
+  MCCLCHECK(pairPrepare(fn, smem));
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  MCCLCHECK(makeMap(&a.mapA, A, M, K, BM));
+  MCCLCHECK(makeMap(&a.mapB, B, N, K, bn / 2));
+  a.M = M; a.N = N; a.K = K;
+  a.C = static_cast<__nv_bfloat16*>(C);
+  a.pre = static_cast<__nv_bfloat16*>(pre);
+  a.epilogue = epilogue;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  a.errFlag = errFlagFor(dev).dev;
+  if (a.errFlag == nullptr) return mcclSystemError;
+  a.budgetNs = 2000000000ull;
+  a.debug = (int)envInt("MCCL_GEMM_DEBUG", 0);
+  MCCLCHECK(makeMap(&a.mapC, C, M, N, 32));
+  if (pre != nullptr) MCCLCHECK(makeMap(&a.mapPre, pre, M, N, 32));
+  a.tmaStore = 1;
+  {
+    TailWs w;
+    tailSplit((long)(M / BM2) * (N / bn), pairsMax, K / BK, true, &a.tailTiles, &a.tailSlices);
+    if (a.tailTiles > 0 && a.tailTiles <= 80 && tailWorkspace(dev, reinterpret_cast<cudaStream_t>(stream), &w)) { a.tailWs = w.ws; a.tailCount = w.count; }
+    else a.tailTiles = a.tailSlices = 0;
+  }
+  a.panel = pickPanel(M / BM2);
+  if (envInt("MCCL_GEMM_PANEL", 0) > 0) a.panel = (int)envInt("MCCL_GEMM_PANEL", 0);
+  const int tiles = (M / BM2) * (N / bn);
+  return launchPairs(fn, kThreadsGemm2, smem, tiles < pairsMax ? tiles : pairsMax, a, reinterpret_cast<cudaStream_t>(stream));
+}
+
 }  // namespace
 
 extern "C" {
@@ -316,69 +385,17 @@ int mcclDbgGemmTile(int mode, int M, int N, int nRanks, int rank, int sms, int t
 
 // C[M,N] = act(A[M,K] * B[N,K]^T), bf16 in and out, on the current device.
 mcclResult_t mcclTpGemm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int maxCtas, mcclStream_t stream) {
-  if (A == nullptr || B == nullptr || C == nullptr) return mcclInvalidArgument;
-  MCCLCHECK(checkShapes(M, N, K, 1));
-  const int sms = maxCtas > 0 ? maxCtas : smCount();
-  const int bn = pickBN(M, N, sms);
-  if (bn == 0) return mcclInvalidArgument;
-  GemmArgs a;
-  memset(&a, 0, sizeof(a));
-  MCCLCHECK(makeMap(&a.mapA, A, M, K, BM));
-  MCCLCHECK(makeMap(&a.mapB, B, N, K, bn));
-  a.M = M; a.N = N; a.K = K;
-  a.C = static_cast<__nv_bfloat16*>(C);
-  a.epilogue = epilogue;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  a.errFlag = errFlagFor(dev).dev;
-  if (a.errFlag == nullptr) return mcclSystemError;
-  a.budgetNs = 2000000000ull;
-  a.panel = pickPanel(M / BM);
-  const int tiles = (M / BM) * (N / bn);
-  return launchMode<MODE_PLAIN>(a, bn, tiles < sms ? tiles : sms, reinterpret_cast<cudaStream_t>(stream));
+  return oneSmGemm(A, B, C, nullptr, M, N, K, epilogue, maxCtas, stream);
 }
 
 // The same product computed by pairs of SMs (tcgen05.mma.cta_group::2 on 256-row tiles); needs M % 256 == 0.
 mcclResult_t mcclTpGemm2(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int maxCtas, mcclStream_t stream) {
-  if (A == nullptr || B == nullptr || C == nullptr) return mcclInvalidArgument;
-  MCCLCHECK(checkShapes(M, N, K, 1));
-  if (M % BM2) {
-    MCCL_WARN("the two-SM GEMM needs M %% %d == 0 (got %d)", BM2, M);
-    return mcclInvalidArgument;
-  }
-  const int pairsMax = std::max(1, (maxCtas > 0 ? maxCtas : smCount()) / 2);
-  int bn = pickBN2(M / BM2, N, pairsMax, K / BK, true);
-  const int forcedBn = (int)envInt("MCCL_GEMM_BN", 0);          // tuning aid: a tile width that divides N
-  if (forcedBn > 0 && N % forcedBn == 0) bn = forcedBn;
-  const void* fn = nullptr;
-  int smem = 0;
-  if (bn == 0 || !pairKernel<MODE_PLAIN>(bn, &fn, &smem)) return mcclInvalidArgument;
-  MCCLCHECK(pairPrepare(fn, smem));
-  GemmArgs a;
-  memset(&a, 0, sizeof(a));
-  MCCLCHECK(makeMap(&a.mapA, A, M, K, BM));
-  MCCLCHECK(makeMap(&a.mapB, B, N, K, bn / 2));
-  a.M = M; a.N = N; a.K = K;
-  a.C = static_cast<__nv_bfloat16*>(C);
-  a.epilogue = epilogue;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  a.errFlag = errFlagFor(dev).dev;
-  if (a.errFlag == nullptr) return mcclSystemError;
-  a.budgetNs = 2000000000ull;
-  a.debug = (int)envInt("MCCL_GEMM_DEBUG", 0);
-  MCCLCHECK(makeMap(&a.mapC, C, M, N, 32));
-  a.tmaStore = 1;
-  {
-    TailWs w;
-    tailSplit((long)(M / BM2) * (N / bn), pairsMax, K / BK, true, &a.tailTiles, &a.tailSlices);
-    if (a.tailTiles > 0 && a.tailTiles <= 80 && tailWorkspace(dev, reinterpret_cast<cudaStream_t>(stream), &w)) { a.tailWs = w.ws; a.tailCount = w.count; }
-    else a.tailTiles = a.tailSlices = 0;
-  }
-  a.panel = pickPanel(M / BM2);
-  if (envInt("MCCL_GEMM_PANEL", 0) > 0) a.panel = (int)envInt("MCCL_GEMM_PANEL", 0);
-  const int tiles = (M / BM2) * (N / bn);
-  return launchPairs(fn, kThreadsGemm2, smem, tiles < pairsMax ? tiles : pairsMax, a, reinterpret_cast<cudaStream_t>(stream));
+  return twoSmGemm(A, B, C, nullptr, M, N, K, epilogue, maxCtas, stream);
+}
+
+// The same by whichever form the shape allows, with the sums before the activation stored to `pre` (may be null) as well.
+mcclResult_t mcclTpGemmKeepPre(const void* A, const void* B, void* C, void* pre, int M, int N, int K, int epilogue, mcclStream_t stream) {
+  return M > 0 && M % BM2 == 0 ? twoSmGemm(A, B, C, pre, M, N, K, epilogue, 0, stream) : oneSmGemm(A, B, C, pre, M, N, K, epilogue, 0, stream);
 }
 
 // Fused all-gather -> GEMM -> activation.  xShard: this rank's [M/n, K] activations in symmetric memory;

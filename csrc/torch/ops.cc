@@ -143,6 +143,58 @@ py::object gemm(const Tensor& x, const Tensor& w, const std::optional<Tensor>& o
   return py::cast(y);
 }
 
+// ---- SiLU MLP on one rank ---------------------------------------------------------------------------------------------
+// y = silu(x w_up^T) w_down^T.  The up product stores its sums beside the activation, so the backward pass is four products
+// and one elementwise pass; without gradients they are not kept.
+struct MlpFn : torch::autograd::Function<MlpFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& xIn, const Tensor& wUp, const Tensor& wDown, bool keep) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::CUDAGuard guard(xIn.device());
+    Tensor x = xIn.contiguous();
+    const int T = (int)x.size(0), h = (int)x.size(1), f = (int)wUp.size(0);
+    Tensor act = at::empty({T, f}, x.options()), pre = keep ? at::empty({T, f}, x.options()) : Tensor(), y = at::empty({T, h}, x.options());
+    check(mcclTpGemmKeepPre(x.data_ptr(), wUp.data_ptr(), act.data_ptr(), keep ? pre.data_ptr() : nullptr, T, f, h, MCCL_EPILOGUE_SILU, streamOf(x)),
+          "mcclTpGemmKeepPre");
+    check(mcclTpGemmKeepPre(act.data_ptr(), wDown.data_ptr(), y.data_ptr(), nullptr, T, h, f, MCCL_EPILOGUE_NONE, streamOf(x)), "mcclTpGemmKeepPre");
+    counters().gemm += 2;
+    if (keep) ctx->save_for_backward({x, wUp, wDown, act, pre});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto v = ctx->get_saved_variables();
+    const Tensor &x = v[0], &wUp = v[1], &wDown = v[2], &act = v[3], &pre = v[4];
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor dy = g[0].contiguous();
+    variable_list ret(4);
+    if (ctx->needs_input_grad(2)) ret[2] = at::mm(dy.t(), act);
+    Tensor du = at::mm(dy, wDown);
+    check(mcclSiluBackward(pre.data_ptr(), du.data_ptr(), du.data_ptr(), du.numel(), streamOf(x)), "mcclSiluBackward");
+    if (ctx->needs_input_grad(1)) ret[1] = at::mm(du.t(), x);
+    if (ctx->needs_input_grad(0)) ret[0] = at::mm(du, wUp);
+    return ret;
+  }
+};
+
+// None where the kernels do not cover the case.
+py::object mlp(const Tensor& x, const Tensor& wUp, const Tensor& wDown) {
+  for (const Tensor* t : {&x, &wUp, &wDown})
+    if (!bf16Cuda(*t) || t->dim() != 2 || !aligned16(*t)) return py::none();
+  const int64_t T = x.size(0), h = x.size(1), f = wUp.size(0);
+  if (!wUp.is_contiguous() || !wDown.is_contiguous() || wUp.size(1) != h || wDown.size(0) != h || wDown.size(1) != f || T <= 0 || T % 128 || h % 64 ||
+      f % 64) return py::none();
+  const bool keep = at::GradMode::is_enabled() && (x.requires_grad() || wUp.requires_grad() || wDown.requires_grad());
+  return py::cast(MlpFn::apply(x, wUp, wDown, keep));
+}
+
+// (silu(u), du) from the pre-activation and the gradient of the activation.
+std::pair<Tensor, Tensor> siluBoth(const Tensor& u, const Tensor& dh) {
+  TORCH_CHECK(bf16Cuda(u) && bf16Cuda(dh) && u.is_contiguous() && dh.is_contiguous() && u.numel() == dh.numel(), "silu_both: bf16 cuda tensors");
+  Tensor h = at::empty_like(u), du = at::empty_like(u);
+  check(mcclSiluForwardBackward(u.data_ptr(), dh.data_ptr(), h.data_ptr(), du.data_ptr(), u.numel(), streamOf(u)), "mcclSiluForwardBackward");
+  return {h, du};
+}
+
 }  // namespace
 
 void bindOps(py::module_& m) {
@@ -151,6 +203,8 @@ void bindOps(py::module_& m) {
   m.def("adamw", &adamw);
   m.def("sum_squares", &sumSquares);
   m.def("gemm", &gemm);
+  m.def("mlp", &mlp);
+  m.def("silu_both", &siluBoth);
   m.def("launches", [](const std::string& what) -> int64_t {
     Counters& c = counters();
     if (what == "norm") return c.norm;

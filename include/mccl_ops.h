@@ -21,6 +21,8 @@ extern "C" {
 mcclResult_t mcclTpGemm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int maxCtas, mcclStream_t stream);
 /* The same product by pairs of SMs on 256-row tiles (M % 256 == 0). */
 mcclResult_t mcclTpGemm2(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int maxCtas, mcclStream_t stream);
+/* The same by the form the shape allows; pre (nullable, [M, N]): the sums before the activation. */
+mcclResult_t mcclTpGemmKeepPre(const void* A, const void* B, void* C, void* pre, int M, int N, int K, int epilogue, mcclStream_t stream);
 /* Error code the last GEMM kernel on the current device recorded (0 = none); reading clears it. */
 int mcclTpGemmLastError(void);
 

@@ -14,6 +14,7 @@ import ctypes as C
 
 import torch
 
+from .. import _ext
 from .. import _lib as L
 from ..comm import Communicator
 from ..ops import gemm as G
@@ -77,8 +78,8 @@ class TensorParallelFFN:
 
 
 class _FusedMLPFunction(torch.autograd.Function):
-    """Forward through the two fused kernels; backward with the collectives and plain matrix products.  The
-    pre-activation is not kept: the backward pass recomputes it from the gathered input (one extra GEMM) instead of
+    """Forward through the two fused kernels; backward with the collectives, plain matrix products and one pass for the
+    activation and its gradient.  The pre-activation is not kept: the backward pass recomputes it from the gathered input (one extra GEMM) instead of
     storing a [tokens, ffn / n] tensor per layer."""
 
     @staticmethod
@@ -93,12 +94,8 @@ class _FusedMLPFunction(torch.autograd.Function):
         x_full, w_up, w_down = ctx.saved_tensors
         comm = ctx.layer.comm
         dy_full = PF._ag(comm, dy.contiguous())                    # [tokens, hidden]
-        u = (x_full @ w_up.t()).float()
-        sig = torch.sigmoid(u)
-        h = (u * sig).to(x_full.dtype)
+        h, du = _ext.load().silu_both(x_full @ w_up.t(), dy_full @ w_down)
         d_w_down = dy_full.t() @ h
-        dh = (dy_full @ w_down).float()
-        du = (dh * (sig * (1.0 + u * (1.0 - sig)))).to(x_full.dtype)
         d_w_up = du.t() @ x_full
         dx = PF._rs(comm, du @ w_up)                               # this rank's rows of the input gradient
         return dx, d_w_up, d_w_down, None
@@ -118,6 +115,10 @@ class FusedTensorParallelMLP(torch.nn.Module):
         self.layer = TensorParallelFFN(comm, tokens, hidden, ffn, self.w_up.data, self.w_down.data)
 
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
+        if self.layer.comm.size == 1:                             # nothing to gather or scatter: the two products are one node
+            y = _ext.load().mlp(x_shard, self.w_up, self.w_down)
+            if y is not None:
+                return y
         # the kernels read the parameters' current storage (an optimizer may have re-pointed .data)
         self.layer.w_up, self.layer.w_down = self.w_up.data, self.w_down.data
         return _FusedMLPFunction.apply(x_shard, self.w_up, self.w_down, self.layer)
