@@ -19,6 +19,7 @@ using namespace mccl;
 
 constexpr int kCeThreads = 512;
 constexpr int kCeUnroll = 4;                   // 16-byte pieces in flight per thread: with one, the row's loads wait for each other
+constexpr int64_t kIgnored = -100;             // the target value torch's cross-entropy leaves out
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct MaxSum { float m, s; };                 // running maximum and sum of exp(x - m)
@@ -110,7 +111,8 @@ __global__ void __launch_bounds__(kCeThreads) ceForwardKernel(const __nv_bfloat1
 }
 
 // Mean over the rows' losses, in a fixed order: over all rows or, with `targets`, over those whose target is a column
-// (`inverse`: one over their number, for the backward pass).
+// (`inverse`: one over their number, for the backward pass); there a target that is neither a column nor kIgnored makes the
+// mean NaN.
 __global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, const int64_t* targets, int vocab, float* out, float* inverse) {
   __shared__ float acc[32];
   __shared__ int used;
@@ -124,7 +126,12 @@ __global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, co
     for (int u = 0; u < 8; ++u) x[u] = i + u * 1024 < n ? v[i + u * 1024] : 0.f;
     if (targets != nullptr)
 #pragma unroll
-      for (int u = 0; u < 8; ++u) c += i + u * 1024 < n && targets[i + u * 1024] >= 0 && targets[i + u * 1024] < vocab;
+      for (int u = 0; u < 8; ++u) {
+        if (i + u * 1024 >= n) continue;
+        const int64_t k = targets[i + u * 1024];
+        if (k >= 0 && k < vocab) ++c;
+        else if (k != kIgnored) x[u] = __int_as_float(0x7fffffff);
+      }
     t += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
   }
   if (targets != nullptr) atomicAdd(&used, c);

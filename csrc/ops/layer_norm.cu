@@ -5,7 +5,8 @@
 //             the norm behind it in one pass over memory.
 //   backward: dx per row from two reductions; every lane also accumulates dgamma / dbeta of its columns over the rows its
 //             group walks (col_reduce.cuh adds them up).  With `dres` the gradient that reaches the row past the norm (the
-//             residual branch) is added, and the column sums of the total can be had as well: the bias gradient of the
+//             residual branch) is added (to the norm's gradient as a separate norm would have stored it), and the gradient
+//             of y may come in up to three parts (one per projection that read y), added up here.  The column sums of the total can be had as well: the bias gradient of the
 //             projection that produced `delta`.
 // Both are bound by memory: forward 4 bytes an element (8 with delta), backward 6 (8 with dres).
 // No counterpart in the reference (it has no model code).
@@ -56,6 +57,16 @@ __device__ __forceinline__ uint4 pack(const float* f) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) e[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
   return q;
+}
+
+// Sums of eight pairs, rounded as an addition of tensors rounds.
+__device__ __forceinline__ uint4 add8(const uint4& a, const uint4& b) {
+  float x[8], y[8];
+  unpack(a, x);
+  unpack(b, y);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) x[k] += y[k];
+  return pack(x);
 }
 
 struct LnFwdArgs {
@@ -138,6 +149,7 @@ __global__ void __launch_bounds__(kLnThreads) lnForwardKernel(const __grid_const
 
 struct LnBwdArgs {
   const uint4 *x, *dy, *dres, *gamma;          // dres: may be null
+  const uint4 *dy2, *dy3;                      // more parts of dy, with PARTS == 3 (may be null there)
   const float *mean, *rstd;
   uint4* dx;
   float* partial;
@@ -149,8 +161,8 @@ struct LnBwdArgs {
 // Rows are walked by a fixed number of CTAs (two per SM) so that a lane can keep its columns' sums in registers; the
 // vectors of the next row are loaded before the current one is worked on.  Two vectors per lane bound the registers: 16
 // columns x (three sums + gamma) + two rows of x, dy and dres.
-template <int W, int VPL, bool RMS, bool RES>
-__global__ void __launch_bounds__(kLnThreads, VPL == 1 ? 3 : 2) lnBackwardKernel(const __grid_constant__ LnBwdArgs a) {
+template <int W, int VPL, bool RMS, bool RES, int PARTS>
+__global__ void __launch_bounds__(kLnThreads, VPL == 1 && PARTS == 1 ? 3 : 2) lnBackwardKernel(const __grid_constant__ LnBwdArgs a) {
   constexpr int G = kLnWarps / W, T = W * 32;
   extern __shared__ float cols[];
   __shared__ float2 slots[2][kLnWarps];
@@ -167,7 +179,7 @@ __global__ void __launch_bounds__(kLnThreads, VPL == 1 ? 3 : 2) lnBackwardKernel
   const float invD = 1.0f / (float)a.D;
   const int64_t step = (int64_t)gridDim.x * G;
   int64_t row = (int64_t)blockIdx.x * G + group;
-  uint4 xq[VPL], dq[VPL], rq[VPL];
+  uint4 xq[VPL], dq[VPL], rq[VPL], d2[VPL], d3[VPL];
   float mu = 0.f, rs = 0.f;
   auto load = [&](int64_t r) {
 #pragma unroll
@@ -177,6 +189,10 @@ __global__ void __launch_bounds__(kLnThreads, VPL == 1 ? 3 : 2) lnBackwardKernel
       xq[j] = in ? a.x[r * vecs + i] : zero;
       dq[j] = in ? a.dy[r * vecs + i] : zero;
       if (RES) rq[j] = in ? a.dres[r * vecs + i] : zero;
+      if (PARTS == 3) {
+        d2[j] = in && a.dy2 != nullptr ? a.dy2[r * vecs + i] : zero;
+        d3[j] = in && a.dy3 != nullptr ? a.dy3[r * vecs + i] : zero;
+      }
     }
     if (r < a.rows) { if (!RMS) mu = a.mean[r]; rs = a.rstd[r]; }
   };
@@ -184,7 +200,7 @@ __global__ void __launch_bounds__(kLnThreads, VPL == 1 ? 3 : 2) lnBackwardKernel
   for (int par = 0; row < a.rows; row += step, par ^= 1) {
     uint4 xc[VPL], dc4[VPL], rc[VPL];
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) { xc[j] = xq[j]; dc4[j] = dq[j]; if (RES) rc[j] = rq[j]; }
+    for (int j = 0; j < VPL; ++j) { xc[j] = xq[j]; dc4[j] = PARTS == 3 ? add8(add8(dq[j], d2[j]), d3[j]) : dq[j]; if (RES) rc[j] = rq[j]; }
     const float m = mu, r = rs;
     load(row + step);
     float s1 = 0.f, s2 = 0.f;
@@ -214,7 +230,8 @@ __global__ void __launch_bounds__(kLnThreads, VPL == 1 ? 3 : 2) lnBackwardKernel
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const float xh = (xf[k] - m) * r, gd = df[k] * g[8 * j + k];
-        o[k] = r * (gd - s1 - xh * s2) + (RES ? o[k] : 0.f);
+        const float dn = r * (gd - s1 - xh * s2);
+        o[k] = RES ? __bfloat162float(__float2bfloat16_rn(dn)) + o[k] : dn;
       }
       const uint4 q = pack(o);
       if (third) {
@@ -261,35 +278,37 @@ cudaError_t fwdAny(const LnFwdArgs& a, cudaStream_t s) {
   return fwd<4, 4, RMS>(a, s);
 }
 
-template <int W, int VPL, bool RMS, bool RES>
+template <int W, int VPL, bool RMS, bool RES, int PARTS = 1>
 cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
   constexpr int G = kLnWarps / W;
   static bool opted[64] = {false};             // 48 KB of column sums and the row slots: past the default limit
   int dev = 0;
   cudaGetDevice(&dev);
   if (!opted[dev & 63]) {
-    const cudaError_t e = cudaFuncSetAttribute(lnBackwardKernel<W, VPL, RMS, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
+    const cudaError_t e = cudaFuncSetAttribute(lnBackwardKernel<W, VPL, RMS, RES, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
     if (e != cudaSuccess) return e;
     opted[dev & 63] = true;
   }
   int cluster;
-  const int grid = colred::grid((a.rows + G * 4 - 1) / (G * 4), VPL == 1 ? 3 : 2, &cluster);      // four rows per group before more CTAs pay
+  const int grid = colred::grid((a.rows + G * 4 - 1) / (G * 4), VPL == 1 && PARTS == 1 ? 3 : 2, &cluster);      // four rows per group before more CTAs pay
   const int C = a.out.segments * a.D;
-  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
+  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES, PARTS>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
   return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, C, a.out, s);
 }
 
 // A lane's columns cost four registers each (three sums and gamma) beside two rows of x, dy and dres: two vectors a lane
 // fit 128 registers without dres and spill with it (8192 x 1024: 26 us, with one vector a lane 19 us).
+template <bool RMS, int PARTS>
+cudaError_t bwdRes(const LnBwdArgs& a, cudaStream_t s) {
+  if (a.D <= 256) return bwdLaunch<1, 1, RMS, true, PARTS>(a, s);
+  if (a.D <= 512) return bwdLaunch<2, 1, RMS, true, PARTS>(a, s);
+  if (a.D <= 1024) return bwdLaunch<4, 1, RMS, true, PARTS>(a, s);
+  if (a.D <= 2048) return bwdLaunch<8, 1, RMS, true, PARTS>(a, s);
+  return bwdLaunch<8, 2, RMS, true, PARTS>(a, s);
+}
 template <bool RMS>
 cudaError_t bwdAny(const LnBwdArgs& a, cudaStream_t s) {
-  if (a.dres) {
-    if (a.D <= 256) return bwdLaunch<1, 1, RMS, true>(a, s);
-    if (a.D <= 512) return bwdLaunch<2, 1, RMS, true>(a, s);
-    if (a.D <= 1024) return bwdLaunch<4, 1, RMS, true>(a, s);
-    if (a.D <= 2048) return bwdLaunch<8, 1, RMS, true>(a, s);
-    return bwdLaunch<8, 2, RMS, true>(a, s);
-  }
+  if (a.dres) return a.dy2 ? bwdRes<RMS, 3>(a, s) : bwdRes<RMS, 1>(a, s);
   if (a.D <= 256) return bwdLaunch<1, 1, RMS, false>(a, s);
   if (a.D <= 512) return bwdLaunch<1, 2, RMS, false>(a, s);
   if (a.D <= 1024) return bwdLaunch<2, 2, RMS, false>(a, s);
@@ -312,13 +331,14 @@ mcclResult_t forward(const void* x, const void* delta, const void* gamma, const 
   return (rms ? fwdAny<true>(a, s) : fwdAny<false>(a, s)) == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 
-mcclResult_t backward(const void* x, const void* dy, const void* dres, const void* gamma, const float* mean, const float* rstd, void* dx,
+mcclResult_t backward(const void* x, const void* dy, const void* dy2, const void* dy3, const void* dres, const void* gamma, const float* mean, const float* rstd, void* dx,
                       void* dgamma, void* dbeta, void* dcol, int accumulate, float* partial, int64_t rows, int D, bool rms,
                       mcclStream_t stream) {
-  if (!x || !dy || !gamma || !rstd || !dx || !dgamma || !partial || rows <= 0 || (!rms && (!mean || !dbeta)) || (dcol && !dres)) return mcclInvalidArgument;
+  if (!x || !dy || !gamma || !rstd || !dx || !dgamma || !partial || rows <= 0 || (!rms && (!mean || !dbeta)) || (dcol && !dres) || (dy2 && !dres) || (dy3 && !dy2)) return mcclInvalidArgument;
   if (D <= 0 || D % 8 || D > kLnMaxD) return mcclInvalidArgument;
-  if (!aligned16(x) || !aligned16(dy) || !aligned16(dres) || !aligned16(gamma) || !aligned16(dx)) return mcclInvalidArgument;
+  if (!aligned16(x) || !aligned16(dy) || !aligned16(dres) || !aligned16(gamma) || !aligned16(dx) || !aligned16(dy2) || !aligned16(dy3)) return mcclInvalidArgument;
   LnBwdArgs a;
+  a.dy2 = static_cast<const uint4*>(dy2); a.dy3 = static_cast<const uint4*>(dy3);
   a.x = static_cast<const uint4*>(x); a.dy = static_cast<const uint4*>(dy); a.dres = static_cast<const uint4*>(dres);
   a.gamma = static_cast<const uint4*>(gamma); a.mean = mean; a.rstd = rstd;
   a.dx = static_cast<uint4*>(dx); a.partial = partial; a.rows = rows; a.D = D;
@@ -351,15 +371,15 @@ extern "C" mcclResult_t mcclAddLayerNormForward(const void* x, const void* delta
 extern "C" mcclResult_t mcclLayerNormBackward(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                                               void* dx, void* dgamma, void* dbeta, float* partial, int64_t rows, int D,
                                               mcclStream_t stream) {
-  return backward(x, dy, nullptr, gamma, mean, rstd, dx, dgamma, dbeta, nullptr, 0, partial, rows, D, false, stream);
+  return backward(x, dy, nullptr, nullptr, nullptr, gamma, mean, rstd, dx, dgamma, dbeta, nullptr, 0, partial, rows, D, false, stream);
 }
 
 // The same with dx += dres and, when dcol is given, dcol = column sums of dx (needs dres); `accumulate`: add dgamma, dbeta and dcol to what
-// is there.  partial: mcclLayerNormPartials(rows) * 3 * D floats.
-extern "C" mcclResult_t mcclAddLayerNormBackward(const void* x, const void* dy, const void* dres, const void* gamma, const float* mean,
-                                                 const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate,
+// is there.  dy2, dy3 (may be null, need dres): further parts of dy.  partial: mcclLayerNormPartials(rows) * 3 * D floats.
+extern "C" mcclResult_t mcclAddLayerNormBackward(const void* x, const void* dy, const void* dy2, const void* dy3, const void* dres,
+                                                 const void* gamma, const float* mean, const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate,
                                                  float* partial, int64_t rows, int D, mcclStream_t stream) {
-  return backward(x, dy, dres, gamma, mean, rstd, dx, dgamma, dbeta, dcol, accumulate, partial, rows, D, false, stream);
+  return backward(x, dy, dy2, dy3, dres, gamma, mean, rstd, dx, dgamma, dbeta, dcol, accumulate, partial, rows, D, false, stream);
 }
 
 // RMSNorm: y = bf16(x * rstd) * gamma; delta / sum as in mcclAddLayerNormForward (both may be null).
@@ -368,7 +388,7 @@ extern "C" mcclResult_t mcclRmsNormForward(const void* x, const void* delta, con
   return forward(x, delta, gamma, nullptr, sum, y, nullptr, rstd, rows, D, eps, true, stream);
 }
 
-extern "C" mcclResult_t mcclRmsNormBackward(const void* x, const void* dy, const void* dres, const void* gamma, const float* rstd, void* dx,
-                                            void* dgamma, int accumulate, float* partial, int64_t rows, int D, mcclStream_t stream) {
-  return backward(x, dy, dres, gamma, nullptr, rstd, dx, dgamma, nullptr, nullptr, accumulate, partial, rows, D, true, stream);
+extern "C" mcclResult_t mcclRmsNormBackward(const void* x, const void* dy, const void* dy2, const void* dy3, const void* dres, const void* gamma,
+                                            const float* rstd, void* dx, void* dgamma, int accumulate, float* partial, int64_t rows, int D, mcclStream_t stream) {
+  return backward(x, dy, dy2, dy3, dres, gamma, nullptr, rstd, dx, dgamma, nullptr, nullptr, accumulate, partial, rows, D, true, stream);
 }

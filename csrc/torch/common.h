@@ -13,6 +13,10 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+
 #include <atomic>
 
 #include "mccl.h"
@@ -36,6 +40,31 @@ inline void check(mcclResult_t rc, const char* what) {
 }
 inline bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
 inline bool bf16Cuda(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; }
+
+// Whether a kernel may be launched on t's memory in place of tensor operations: not for the wrappers of torch.func, of tensor
+// subclasses and of tracing, nor for a tensor with a forward-mode tangent; what sees them has to see operators.
+inline bool ordinary(const Tensor& t) {
+  constexpr c10::DispatchKeySet wrapped({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                         c10::DispatchKey::Functionalize});
+  return t.defined() && t.has_storage() && !t.key_set().has_any(wrapped) && !t._fw_grad(0).defined();
+}
+// A trace or a dispatch mode records operators: the nodes stand aside for it.
+inline bool recorded() { return torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set(); }
+
+// For the inside of a node: operators record no gradient and keep the types they are given, whatever autocast says.
+struct Below {
+  at::AutoDispatchBelowADInplaceOrView noGrad;
+  c10::impl::ExcludeDispatchKeyGuard noCast{c10::autocast_dispatch_keyset};
+};
+
+// Gradients that have no graph of their own: differentiating them (backward(create_graph=True)) raises instead of counting
+// them as constants.
+inline variable_list once(variable_list&& grads) {
+  if (!at::GradMode::is_enabled()) return std::move(grads);
+  auto raise = std::make_shared<torch::autograd::DelayedError>("mccl: the gradient of a fused node cannot be differentiated again", (int64_t)grads.size());
+  for (Tensor& g : grads) if (g.defined()) g = g.detach().requires_grad_(true);
+  return raise->apply(std::move(grads));
+}
 
 // One module's functions each, defined in the files of the same names.
 void bindOps(pybind11::module_& m);

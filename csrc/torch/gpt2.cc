@@ -12,21 +12,6 @@
 namespace mccl_torch {
 namespace {
 
-std::mutex sinkMutex;
-std::vector<py::object>& sinkTable() { static auto* t = new std::vector<py::object>(1); return *t; }
-
-int64_t registerSink(py::object fn) {
-  std::lock_guard<std::mutex> lk(sinkMutex);
-  auto& t = sinkTable();
-  for (size_t i = 1; i < t.size(); ++i) if (!t[i]) { t[i] = std::move(fn); return (int64_t)i; }
-  t.push_back(std::move(fn));
-  return (int64_t)t.size() - 1;
-}
-void dropSink(int64_t id) {
-  std::lock_guard<std::mutex> lk(sinkMutex);
-  if (id > 0 && id < (int64_t)sinkTable().size()) sinkTable()[id] = py::object();
-}
-
 // Three adjacent matrices (or vectors) of one storage as one, in memory order; undefined where they are not adjacent.
 Tensor adjacent(const Tensor& a, const Tensor& b, const Tensor& c) {
   const char *pa = (const char*)a.data_ptr(), *pb = (const char*)b.data_ptr(), *pc = (const char*)c.data_ptr();
@@ -67,8 +52,8 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
   // Outputs: residual [T, d], q, k, v [b, h, s, hd].
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& pending, const OptTensor& pendingBias, const Tensor& lw,
                                const Tensor& lb, const Tensor& wq, const Tensor& bq, const Tensor& wk, const Tensor& bk, const Tensor& wv,
-                               const Tensor& bv, int64_t b, int64_t s, int64_t heads, double eps, int64_t sink, bool exact) {
-    at::AutoDispatchBelowADInplaceOrView below;
+                               const Tensor& bv, int64_t b, int64_t s, int64_t heads, double eps, bool sink, bool exact) {
+    Below below;
     const int64_t T = x.size(0), d = x.size(1), hd = d / heads;
     Tensor sum, h, stats;
     addNorm(x, pending ? &*pending : nullptr, lw, lb, eps, exact, &sum, &h, &stats);
@@ -87,7 +72,8 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
       k = split(at::linear(h, wk, bk), d, 0);
       v = split(at::linear(h, wv, bv), d, 0);
     }
-    ctx->save_for_backward({sum, h, stats, lw, lb, wq, bq, wk, bk, wv, bv, pendingBias ? *pendingBias : Tensor()});
+    // Without a pending term the sum is the input: saved as such, so that a change made to it in place is noticed.
+    ctx->save_for_backward({pending ? sum : x, h, stats, lw, lb, wq, bq, wk, bk, wv, bv, pendingBias ? *pendingBias : Tensor()});
     ctx->saved_data["sink"] = sink;
     ctx->saved_data["pending"] = pending.has_value();
     return {sum, q, k, v};
@@ -96,9 +82,9 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     auto saved = ctx->get_saved_variables();
     const Tensor &sum = saved[0], &h = saved[1], &stats = saved[2], &lw = saved[3], &lb = saved[4], &wq = saved[5], &bq = saved[6],
                  &wk = saved[7], &bk = saved[8], &wv = saved[9], &bv = saved[10], &pb = saved[11];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(h.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const bool pending = ctx->saved_data["pending"].toBool();
     const int64_t T = h.size(0), d = h.size(1);
     mcclStream_t s = streamOf(h);
@@ -113,9 +99,7 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
       void* out[3] = {db.t[0].data_ptr(), db.t[1].data_ptr(), db.t[2].data_ptr()};
       check(mcclColumnSums(in, out, 3, db.direct, scratch.data_ptr<float>(), T, (int)d, d, s), "mcclColumnSums");
     }
-    Tensor dh = at::mm(dv, wv);
-    at::addmm_out(dh, dh, dk, wk);
-    at::addmm_out(dh, dh, dq, wq);
+    Tensor dhv = at::mm(dv, wv), dhk = at::mm(dk, wk), dhq = at::mm(dq, wq);      // the norm's backward kernel adds them up
     weightGrad(sink, wv, dv, h, &dwv);
     weightGrad(sink, wk, dk, h, &dwk);
     weightGrad(sink, wq, dq, h, &dwq);
@@ -127,13 +111,13 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
       Tensor dres = rows2d(g[0], T, d);
       if (pb.defined()) {
         VectorGrads dn(sink, {&lw, &lb, &pb});
-        check(mcclAddLayerNormBackward(sum.data_ptr(), dh.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
+        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), dhk.data_ptr(), dhq.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
                                        dn.t[0].data_ptr(), dn.t[1].data_ptr(), dn.t[2].data_ptr(), dn.direct, partial.data_ptr<float>(), T,
                                        (int)d, s), "mcclAddLayerNormBackward");
         ret[3] = dn.ret(0); ret[4] = dn.ret(1); ret[2] = dn.ret(2);
       } else {
         VectorGrads dn(sink, {&lw, &lb});
-        check(mcclAddLayerNormBackward(sum.data_ptr(), dh.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
+        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), dhk.data_ptr(), dhq.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
                                        dn.t[0].data_ptr(), dn.t[1].data_ptr(), nullptr, dn.direct, partial.data_ptr<float>(), T, (int)d, s),
               "mcclAddLayerNormBackward");
         ret[3] = dn.ret(0); ret[4] = dn.ret(1);
@@ -141,16 +125,16 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     } else {                                       // nobody uses the residual: the plain norm, and the bias on its own
       ret[3] = at::empty(lw.sizes(), lw.options());
       ret[4] = at::empty(lb.sizes(), lb.options());
+      Tensor dh = dhv.add_(dhk).add_(dhq);
       check(mcclLayerNormBackward(sum.data_ptr(), dh.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(), ret[3].data_ptr(),
                                   ret[4].data_ptr(), partial.data_ptr<float>(), T, (int)d, s), "mcclLayerNormBackward");
       if (pb.defined()) ret[2] = dx.sum(0);
     }
     counters().norm += 2;
-    sink.flush();
     ret[0] = dx;
     if (pending) ret[1] = dx;
     ret[5] = dwq; ret[6] = db.ret(0); ret[7] = dwk; ret[8] = db.ret(1); ret[9] = dwv; ret[10] = db.ret(2);
-    return ret;
+    return once(std::move(ret));
   }
 };
 
@@ -160,8 +144,8 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
   // projection is taken by this node and not by the one that adds its output.
   static variable_list forward(AutogradContext* ctx, const Tensor& a, const Tensor& res, const Tensor& wo, const Tensor& bo, const Tensor& lw,
                                const Tensor& lb, const Tensor& wf, const Tensor& bf, const Tensor& wd, const Tensor& bd, bool outBiasHere,
-                               double eps, int64_t sink, bool exact) {
-    at::AutoDispatchBelowADInplaceOrView below;
+                               double eps, bool sink, bool exact) {
+    Below below;
     const int64_t T = res.size(0), d = res.size(1);
     mcclStream_t s = streamOf(res);
     Tensor a2 = fromHeads(a, T, d);
@@ -183,9 +167,9 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     auto saved = ctx->get_saved_variables();
     const Tensor &a2 = saved[0], &x1 = saved[1], &h = saved[2], &stats = saved[3], &u = saved[4], &act = saved[5], &wo = saved[6],
                  &bo = saved[7], &lw = saved[8], &lb = saved[9], &wf = saved[10], &bf = saved[11], &wd = saved[12], &bd = saved[13];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(h.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0), d = h.size(1), f = u.size(1), b = ctx->saved_data["b"].toInt(), heads = ctx->saved_data["h"].toInt();
     mcclStream_t s = streamOf(h);
     variable_list ret(14);
@@ -215,7 +199,7 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
       VectorGrads dn(sink, {&lw, &lb, &bo});
       Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * 3 * d}, stats.options());
       const float* mean = stats.data_ptr<float>();
-      check(mcclAddLayerNormBackward(x1.data_ptr(), dh.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
+      check(mcclAddLayerNormBackward(x1.data_ptr(), dh.data_ptr(), nullptr, nullptr, dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
                                      dn.t[0].data_ptr(), dn.t[1].data_ptr(), dn.t[2].data_ptr(), dn.direct, partial.data_ptr<float>(), T, (int)d,
                                      s), "mcclAddLayerNormBackward");
       counters().norm += 2;
@@ -223,18 +207,17 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     }
     Tensor da = at::mm(dx, wo);
     weightGrad(sink, wo, dx, a2, &ret[2]);
-    sink.flush();
     ret[0] = da.view({b, T / b, heads, d / heads}).transpose(1, 2);
     ret[1] = dx;
-    return ret;
+    return once(std::move(ret));
   }
 };
 
 // ---- final norm of (residual, pending) --------------------------------------------------------------------------------
 struct FinalNormFn : torch::autograd::Function<FinalNormFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& pending, const OptTensor& pendingBias, const Tensor& lw,
-                        const Tensor& lb, double eps, int64_t sink, bool exact) {
-    at::AutoDispatchBelowADInplaceOrView below;
+                        const Tensor& lb, double eps, bool sink, bool exact) {
+    Below below;
     Tensor sum, h, stats;
     addNorm(x, &pending, lw, lb, eps, exact, &sum, &h, &stats);
     ctx->save_for_backward({sum, stats, lw, lb, pendingBias ? *pendingBias : Tensor()});
@@ -244,9 +227,9 @@ struct FinalNormFn : torch::autograd::Function<FinalNormFn> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
     const Tensor &sum = saved[0], &stats = saved[1], &lw = saved[2], &lb = saved[3], &pb = saved[4];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(sum.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = sum.size(0), d = sum.size(1);
     mcclStream_t s = streamOf(sum);
     Tensor dh = rows2d(g[0], T, d), dx = at::empty({T, d}, sum.options());
@@ -254,7 +237,7 @@ struct FinalNormFn : torch::autograd::Function<FinalNormFn> {
     const float* mean = stats.data_ptr<float>();
     variable_list ret(8);
     VectorGrads dn(sink, {&lw, &lb});
-    check(mcclAddLayerNormBackward(sum.data_ptr(), dh.data_ptr(), nullptr, lw.data_ptr(), mean, mean + T, dx.data_ptr(), dn.t[0].data_ptr(),
+    check(mcclAddLayerNormBackward(sum.data_ptr(), dh.data_ptr(), nullptr, nullptr, nullptr, lw.data_ptr(), mean, mean + T, dx.data_ptr(), dn.t[0].data_ptr(),
                                    dn.t[1].data_ptr(), nullptr, dn.direct, partial.data_ptr<float>(), T, (int)d, s), "mcclAddLayerNormBackward");
     counters().norm += 2;
     ret[3] = dn.ret(0); ret[4] = dn.ret(1);
@@ -266,17 +249,16 @@ struct FinalNormFn : torch::autograd::Function<FinalNormFn> {
       check(mcclColumnSums(in, out, 1, db.direct, scratch.data_ptr<float>(), T, (int)d, d, s), "mcclColumnSums");
       ret[2] = db.ret(0);
     }
-    sink.flush();
     ret[0] = dx;
     ret[1] = dx;
-    return ret;
+    return once(std::move(ret));
   }
 };
 
 // ---- embedding ----------------------------------------------------------------------------------------------------------
 struct EmbedFn : torch::autograd::Function<EmbedFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& idx, const Tensor& table, const OptTensor& pos, int64_t sink) {
-    at::AutoDispatchBelowADInplaceOrView below;
+  static Tensor forward(AutogradContext* ctx, const Tensor& idx, const Tensor& table, const OptTensor& pos, bool sink) {
+    Below below;
     const int64_t T = idx.numel(), d = table.size(1), seq = idx.size(-1);
     Tensor i = idx.contiguous(), out = at::empty({T, d}, table.options());
     check(mcclEmbeddingForward(i.data_ptr<int64_t>(), table.data_ptr(), pos ? pos->data_ptr() : nullptr, out.data_ptr(), T, (int)seq,
@@ -289,9 +271,9 @@ struct EmbedFn : torch::autograd::Function<EmbedFn> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
     const Tensor &idx = saved[0], &table = saved[1], &pos = saved[2];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(table.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = idx.numel(), d = table.size(1), seq = idx.size(-1), V = table.size(0);
     Tensor dy = rows2d(g[0], T, d);
     variable_list ret(4);
@@ -310,23 +292,21 @@ struct EmbedFn : torch::autograd::Function<EmbedFn> {
           ret[2] = at::zeros(pos.sizes(), pos.options());
           ret[2].narrow(0, 0, seq).copy_(dy.view({T / seq, seq, d}).sum(0));
         }
-        return ret;
+        return once(std::move(ret));
       }
     }
     Tensor count = at::empty({V}, idx.options().dtype(at::kInt));
     check(mcclEmbeddingBackward(idx.data_ptr<int64_t>(), dy.data_ptr(), dt.data_ptr(), withPos ? dp.data_ptr() : nullptr, count.data_ptr<int32_t>(), T, (int)seq, V,
                                 (int)d, streamOf(dy)), "mcclEmbeddingBackward");
-    if (direct) { sink.done(table); if (withPos) sink.done(pos); }
-    sink.flush();
-    return ret;
+    return once(std::move(ret));
   }
 };
 
 // ---- head: projection and cross-entropy ----------------------------------------------------------------------------
 struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, bool tied, bool meanOfUsed,
-                        int64_t sink) {
-    at::AutoDispatchBelowADInplaceOrView below;
+  static Tensor forward(AutogradContext* ctx, const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, bool meanOfUsed,
+                        bool sink) {
+    Below below;
     const int64_t T = h.size(0);
     Tensor logits = at::linear(h, w);
     Tensor t = targets.contiguous();
@@ -337,7 +317,6 @@ struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
     counters().loss++;
     ctx->save_for_backward({h, w, t, logits, perRow});
     ctx->saved_data["vocab"] = vocab;
-    ctx->saved_data["tied"] = tied;
     ctx->saved_data["used"] = meanOfUsed;
     ctx->saved_data["sink"] = sink;
     return mean;
@@ -346,9 +325,9 @@ struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
     auto saved = ctx->get_saved_variables();
     const Tensor &h = saved[0], &w = saved[1], &t = saved[2], &perRow = saved[4];
     Tensor logits = saved[3];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(h.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0);
     Tensor go = g[0].scalar_type() == at::kFloat ? g[0] : g[0].to(at::kFloat);
     float* rows = perRow.data_ptr<float>();
@@ -357,11 +336,10 @@ struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
                                        ctx->saved_data["used"].toBool() ? rows + 2 * T : nullptr, streamOf(h)),
           "mcclCrossEntropyBackward");
     counters().loss++;
-    variable_list ret(7);
+    variable_list ret(6);
     ret[0] = at::mm(logits, w);
-    weightGrad(sink, w, logits, h, &ret[1], !ctx->saved_data["tied"].toBool());      // a tied weight gets the embedding's share later
-    sink.flush();
-    return ret;
+    weightGrad(sink, w, logits, h, &ret[1]);
+    return once(std::move(ret));
   }
 };
 
@@ -370,10 +348,15 @@ struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
 // fc w b, out w b.  Returns (residual, MLP output), whose sum is the block's output, or None where the kernels do not cover
 // the case.
 py::object block(const Tensor& x, const OptTensor& pending, const OptTensor& pendingBias, const std::vector<Tensor>& p, int64_t b, int64_t s,
-                 int64_t heads, bool outBiasHere, double eps, int64_t sink) {
-  if (p.size() != 16 || x.dim() != 2 || !usable(x, p) || (pending && !plainBf16(*pending, x))) return py::none();
-  const int64_t d = x.size(1);
-  if (d % heads || (d / heads) % 8 || p[12].size(0) % 8) return py::none();
+                 int64_t heads, bool outBiasHere, double eps, bool sink) {
+  if (p.size() != 16 || x.dim() != 2 || !usable(x, p) || !attentionOnce()) return py::none();
+  const int64_t d = x.size(1), f = p[12].size(0);
+  if (heads <= 0 || d % heads || (d / heads) % 8 || f % 8 || x.size(0) != b * s) return py::none();
+  if (pending && (!plainBf16(*pending, x) || !shaped(*pending, x.sizes()))) return py::none();
+  if (pendingBias && (!plainBf16(*pendingBias, x) || !shaped(*pendingBias, {d}))) return py::none();
+  for (int i : {0, 1, 3, 5, 7, 9, 10, 11, 15}) if (!shaped(p[i], {d})) return py::none();
+  for (int i : {2, 4, 6, 8}) if (!shaped(p[i], {d, d})) return py::none();
+  if (!shaped(p[12], {f, d}) || !shaped(p[13], {f}) || !shaped(p[14], {d, f})) return py::none();
   c10::cuda::CUDAGuard guard(x.device());
   const bool exact = !at::GradMode::is_enabled();
   variable_list in = BlockInFn::apply(x, pending, pendingBias, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], b, s, heads, eps, sink, exact);
@@ -383,48 +366,36 @@ py::object block(const Tensor& x, const OptTensor& pending, const OptTensor& pen
 }
 
 // table[idx] + pos (pos may be missing) as [tokens, d].
-py::object embed(const Tensor& idx, const Tensor& table, const OptTensor& pos, int64_t sink) {
-  if (!idx.is_cuda() || idx.scalar_type() != at::kLong || idx.numel() == 0 || !usable(table, {table})) return py::none();
-  if (pos && (idx.size(-1) > pos->size(0) || !usable(*pos, {}))) return py::none();
+py::object embed(const Tensor& idx, const Tensor& table, const OptTensor& pos, bool sink) {
+  if (!ordinary(idx) || idx.device() != table.device() || idx.dim() == 0 || idx.scalar_type() != at::kLong || idx.numel() == 0 ||
+      !usable(table, {table}) || table.dim() != 2) return py::none();
+  if (pos && (!plainBf16(*pos, table) || pos->dim() != 2 || pos->size(1) != table.size(1) || idx.size(-1) > pos->size(0))) return py::none();
   c10::cuda::CUDAGuard guard(table.device());
   return py::cast(EmbedFn::apply(idx, table, pos, sink));
 }
 
-py::object finalNorm(const Tensor& x, const Tensor& pending, const OptTensor& pendingBias, const Tensor& w, const Tensor& b, double eps, int64_t sink) {
-  if (!usable(x, {pending, w, b})) return py::none();
+py::object finalNorm(const Tensor& x, const Tensor& pending, const OptTensor& pendingBias, const Tensor& w, const Tensor& b, double eps, bool sink) {
+  if (!usable(x, {pending, w, b}) || x.dim() != 2 || !shaped(pending, x.sizes()) || !shaped(w, {x.size(1)}) || !shaped(b, {x.size(1)}))
+    return py::none();
+  if (pendingBias && (!plainBf16(*pendingBias, x) || !shaped(*pendingBias, {x.size(1)}))) return py::none();
   c10::cuda::CUDAGuard guard(x.device());
   return py::cast(FinalNormFn::apply(x, pending, pendingBias, w, b, eps, sink, !at::GradMode::is_enabled()));
 }
 
-// Mean cross-entropy of h w^T: over all rows, or over those whose target is a column (`meanOfUsed`).  tied: w is the embedding
-// table too.
-py::object headLoss(const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, bool tied, bool meanOfUsed, int64_t sink) {
-  if (!usable(h, {w}) || !targets.is_cuda() || targets.scalar_type() != at::kLong || targets.numel() != h.size(0) || w.size(0) < vocab) return py::none();
+// Mean cross-entropy of h w^T: over all rows, or over those whose target is a column (`meanOfUsed`).
+py::object headLoss(const Tensor& h, const Tensor& w, const Tensor& targets, int64_t vocab, bool meanOfUsed, bool sink) {
+  if (!usable(h, {w}) || h.dim() != 2 || w.dim() != 2 || w.size(1) != h.size(1) || !ordinary(targets) || targets.device() != h.device() || targets.scalar_type() != at::kLong || targets.numel() != h.size(0) || w.size(0) < vocab) return py::none();
   c10::cuda::CUDAGuard guard(h.device());
-  return py::cast(HeadLossFn::apply(h, w, targets.reshape({-1}), vocab, tied, meanOfUsed, sink));
+  return py::cast(HeadLossFn::apply(h, w, targets.reshape({-1}), vocab, meanOfUsed, sink));
 }
 
 }  // namespace
-
-void GradSink::flush() {
-  if (done_.empty()) return;
-  py::gil_scoped_acquire gil;
-  py::object fn;
-  {
-    std::lock_guard<std::mutex> lk(sinkMutex);
-    if (id_ < (int64_t)sinkTable().size()) fn = sinkTable()[id_];
-  }
-  if (fn) for (const Tensor& p : done_) fn(p);
-  done_.clear();
-}
 
 void bindGpt2(py::module_& m) {
   m.def("gpt2_block", &block);
   m.def("decoder_embed", &embed);
   m.def("gpt2_final_norm", &finalNorm);
   m.def("decoder_head_loss", &headLoss);
-  m.def("register_sink", &registerSink);
-  m.def("drop_sink", &dropSink);
 }
 
 }  // namespace mccl_torch

@@ -20,13 +20,20 @@ void addRms(const Tensor& x, const Tensor* pending, const Tensor& w, double eps,
 }
 
 // Gradient of the sum from those of h and, where defined, of the residual stream.
-Tensor addRmsBackward(const Tensor& sum, const Tensor& dh, const Tensor& dres, const Tensor& w, const Tensor& rstd, GradSink& sink, Tensor* dw) {
+// dh: up to three parts, added up on the way.
+Tensor addRmsBackward(const Tensor& sum, std::initializer_list<Tensor> parts, const Tensor& dres, const Tensor& w, const Tensor& rstd, GradSink& sink, Tensor* dw) {
   const int64_t T = sum.size(0), d = sum.size(1);
   Tensor dx = at::empty({T, d}, sum.options());
   Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * d}, rstd.options());
   Tensor res = dres.defined() ? rows2d(dres, T, d) : Tensor();
+  const void* dh[3] = {};
+  int n = 0;
+  for (const Tensor& p : parts) {
+    if (n > 0 && !res.defined()) parts.begin()->add_(p);          // nobody uses the residual: the plain norm
+    else dh[n++] = p.data_ptr();
+  }
   VectorGrads g(sink, {&w});
-  check(mcclRmsNormBackward(sum.data_ptr(), dh.data_ptr(), res.defined() ? res.data_ptr() : nullptr, w.data_ptr(), rstd.data_ptr<float>(),
+  check(mcclRmsNormBackward(sum.data_ptr(), dh[0], dh[1], dh[2], res.defined() ? res.data_ptr() : nullptr, w.data_ptr(), rstd.data_ptr<float>(),
                             dx.data_ptr(), g.t[0].data_ptr(), g.direct, partial.data_ptr<float>(), T, (int)d, streamOf(sum)), "mcclRmsNormBackward");
   counters().norm += 2;
   *dw = g.ret(0);
@@ -52,8 +59,8 @@ void unrotate(const Tensor& dq, const Tensor& dk, int64_t T, int64_t d, double t
 struct LlamaInFn : torch::autograd::Function<LlamaInFn> {
   // Outputs: residual [T, d], q and k (rotated) and v as [b, h, s, hd].
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& pending, const Tensor& nw, const Tensor& wq, const Tensor& wk,
-                               const Tensor& wv, int64_t b, int64_t s, int64_t heads, double theta, double eps, int64_t sink) {
-    at::AutoDispatchBelowADInplaceOrView below;
+                               const Tensor& wv, int64_t b, int64_t s, int64_t heads, double theta, double eps, bool sink) {
+    Below below;
     const int64_t T = x.size(0), d = x.size(1), hd = d / heads;
     Tensor sum, h, rstd;
     addRms(x, pending ? &*pending : nullptr, nw, eps, &sum, &h, &rstd);
@@ -61,7 +68,7 @@ struct LlamaInFn : torch::autograd::Function<LlamaInFn> {
     check(mcclRope(q.data_ptr(), k.data_ptr(), q.data_ptr(), k.data_ptr(), (int)b, (int)s, (int)heads, (int)hd, s * d, d, hd, (float)theta, 0,
                    streamOf(x)), "mcclRope");
     auto split = [&](const Tensor& t) { return t.as_strided({b, heads, s, hd}, {s * d, hd, d, 1}); };
-    ctx->save_for_backward({sum, h, rstd, nw, wq, wk, wv});
+    ctx->save_for_backward({pending ? sum : x, h, rstd, nw, wq, wk, wv});      // the input itself: a change in place is noticed
     ctx->saved_data["sink"] = sink;
     ctx->saved_data["theta"] = theta;
     ctx->saved_data["pending"] = pending.has_value();
@@ -70,33 +77,30 @@ struct LlamaInFn : torch::autograd::Function<LlamaInFn> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
     const Tensor &sum = saved[0], &h = saved[1], &rstd = saved[2], &nw = saved[3], &wq = saved[4], &wk = saved[5], &wv = saved[6];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(h.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0), d = h.size(1);
     TORCH_CHECK(g[1].defined() && g[2].defined() && g[3].defined(), "attention returns all three gradients");
     variable_list ret(12);
     Tensor dq, dk, dv = fromHeads(g[3], T, d);
     unrotate(g[1], g[2], T, d, ctx->saved_data["theta"].toDouble(), &dq, &dk);
-    Tensor dh = at::mm(dv, wv);
-    at::addmm_out(dh, dh, dk, wk);
-    at::addmm_out(dh, dh, dq, wq);
+    Tensor dhv = at::mm(dv, wv), dhk = at::mm(dk, wk), dhq = at::mm(dq, wq);
     weightGrad(sink, wv, dv, h, &ret[5]);
     weightGrad(sink, wk, dk, h, &ret[4]);
     weightGrad(sink, wq, dq, h, &ret[3]);
-    Tensor dx = addRmsBackward(sum, dh, g[0], nw, rstd, sink, &ret[2]);
-    sink.flush();
+    Tensor dx = addRmsBackward(sum, {dhv, dhk, dhq}, g[0], nw, rstd, sink, &ret[2]);
     ret[0] = dx;
     if (ctx->saved_data["pending"].toBool()) ret[1] = dx;
-    return ret;
+    return once(std::move(ret));
   }
 };
 
 struct LlamaOutFn : torch::autograd::Function<LlamaOutFn> {
   // Outputs: residual after attention, MLP output, both [T, d].
   static variable_list forward(AutogradContext* ctx, const Tensor& a, const Tensor& res, const Tensor& wo, const Tensor& nw, const Tensor& wg,
-                               const Tensor& wu, const Tensor& wd, double eps, int64_t sink) {
-    at::AutoDispatchBelowADInplaceOrView below;
+                               const Tensor& wu, const Tensor& wd, double eps, bool sink) {
+    Below below;
     const int64_t T = res.size(0), d = res.size(1);
     Tensor a2 = fromHeads(a, T, d), p = at::linear(a2, wo), x1, h, rstd;
     addRms(res, &p, nw, eps, &x1, &h, &rstd);
@@ -113,9 +117,9 @@ struct LlamaOutFn : torch::autograd::Function<LlamaOutFn> {
     auto saved = ctx->get_saved_variables();
     const Tensor &a2 = saved[0], &x1 = saved[1], &h = saved[2], &rstd = saved[3], &gate = saved[4], &up = saved[5], &wo = saved[6], &nw = saved[7],
                  &wg = saved[8], &wu = saved[9], &wd = saved[10];
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(h.device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0), d = h.size(1), b = ctx->saved_data["b"].toInt(), heads = ctx->saved_data["h"].toInt();
     variable_list ret(9);
     Tensor dy = g[1].defined() ? rows2d(g[1], T, d) : at::zeros({T, d}, h.options());
@@ -126,23 +130,21 @@ struct LlamaOutFn : torch::autograd::Function<LlamaOutFn> {
     check(mcclSwigluBackward(gate.data_ptr(), up.data_ptr(), dact.data_ptr(), act.data_ptr(), dgate.data_ptr(), dup.data_ptr(), act.numel(),
                              streamOf(act)), "mcclSwigluBackward");
     weightGrad(sink, wd, dy, act, &ret[6]);
-    Tensor dh = at::mm(dgate, wg);
-    at::addmm_out(dh, dh, dup, wu);
+    Tensor dhu = at::mm(dup, wu), dhg = at::mm(dgate, wg);
     weightGrad(sink, wg, dgate, h, &ret[4]);
     weightGrad(sink, wu, dup, h, &ret[5]);
-    Tensor dx = addRmsBackward(x1, dh, g[0], nw, rstd, sink, &ret[3]);
+    Tensor dx = addRmsBackward(x1, {dhu, dhg}, g[0], nw, rstd, sink, &ret[3]);
     Tensor da = at::mm(dx, wo);
     weightGrad(sink, wo, dx, a2, &ret[2]);
-    sink.flush();
     ret[0] = da.view({b, T / b, heads, d / heads}).transpose(1, 2);
     ret[1] = dx;
-    return ret;
+    return once(std::move(ret));
   }
 };
 
 struct FinalRmsFn : torch::autograd::Function<FinalRmsFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& pending, const Tensor& w, double eps, int64_t sink) {
-    at::AutoDispatchBelowADInplaceOrView below;
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& pending, const Tensor& w, double eps, bool sink) {
+    Below below;
     Tensor sum, h, rstd;
     addRms(x, &pending, w, eps, &sum, &h, &rstd);
     ctx->save_for_backward({sum, rstd, w});
@@ -151,25 +153,27 @@ struct FinalRmsFn : torch::autograd::Function<FinalRmsFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(saved[0].device());
-    GradSink sink(ctx->saved_data["sink"].toInt());
+    GradSink sink(ctx->saved_data["sink"].toBool());
     variable_list ret(5);
-    Tensor dx = addRmsBackward(saved[0], rows2d(g[0], saved[0].size(0), saved[0].size(1)), Tensor(), saved[2], saved[1], sink, &ret[2]);
-    sink.flush();
+    Tensor dx = addRmsBackward(saved[0], {rows2d(g[0], saved[0].size(0), saved[0].size(1))}, Tensor(), saved[2], saved[1], sink, &ret[2]);
     ret[0] = dx;
     ret[1] = dx;
-    return ret;
+    return once(std::move(ret));
   }
 };
 
 // One block on x + pending (both [T, d]; pending may be missing).  p: norm1, q, k, v, o, norm2, gate, up, down.  Returns two
 // tensors whose sum is the block's output, or None where the kernels do not cover the case.
 py::object block(const Tensor& x, const OptTensor& pending, const std::vector<Tensor>& p, int64_t b, int64_t s, int64_t heads, double theta,
-                 double eps, int64_t sink) {
-  if (p.size() != 9 || x.dim() != 2 || !usable(x, p) || (pending && !plainBf16(*pending, x))) return py::none();
-  const int64_t d = x.size(1);
-  if (d % heads || (d / heads) % 16) return py::none();
+                 double eps, bool sink) {
+  if (p.size() != 9 || x.dim() != 2 || !usable(x, p) || !attentionOnce()) return py::none();
+  const int64_t d = x.size(1), f = p[6].size(0);
+  if (heads <= 0 || d % heads || (d / heads) % 16 || x.size(0) != b * s) return py::none();
+  if (pending && (!plainBf16(*pending, x) || !shaped(*pending, x.sizes()))) return py::none();
+  if (!shaped(p[0], {d}) || !shaped(p[5], {d}) || !shaped(p[6], {f, d}) || !shaped(p[7], {f, d}) || !shaped(p[8], {d, f})) return py::none();
+  for (int i = 1; i < 5; ++i) if (!shaped(p[i], {d, d})) return py::none();
   c10::cuda::CUDAGuard guard(x.device());
   variable_list in = LlamaInFn::apply(x, pending, p[0], p[1], p[2], p[3], b, s, heads, theta, eps, sink);
   Tensor a = at::scaled_dot_product_attention(in[1], in[2], in[3], {}, 0.0, true);
@@ -177,8 +181,8 @@ py::object block(const Tensor& x, const OptTensor& pending, const std::vector<Te
   return py::make_tuple(out[0], out[1]);
 }
 
-py::object finalRms(const Tensor& x, const Tensor& pending, const Tensor& w, double eps, int64_t sink) {
-  if (!usable(x, {pending, w})) return py::none();
+py::object finalRms(const Tensor& x, const Tensor& pending, const Tensor& w, double eps, bool sink) {
+  if (!usable(x, {pending, w}) || x.dim() != 2 || !shaped(pending, x.sizes()) || !shaped(w, {x.size(1)})) return py::none();
   c10::cuda::CUDAGuard guard(x.device());
   return py::cast(FinalRmsFn::apply(x, pending, w, eps, sink));
 }

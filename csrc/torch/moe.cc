@@ -49,12 +49,12 @@ struct RouteFn : torch::autograd::Function<RouteFn> {
                                dl.data_ptr(), nullptr, (int)l.size(0), (int)l.size(1), (int)ctx->saved_data["capacity"].toInt(), 0,
                                streamOf(l)), "mcclMoeTokenBackward");
     counters().moe++;
-    return {dl, Tensor()};
+    return once({dl, Tensor()});
   }
 };
 
 bool routable(const Tensor& logits, int64_t capacity) {
-  return bf16Cuda(logits) && logits.dim() == 2 && logits.size(0) > 0 && logits.size(0) < (1 << 30) && logits.size(1) > 0 &&
+  return !recorded() && ordinary(logits) && bf16Cuda(logits) && logits.dim() == 2 && logits.size(0) > 0 && logits.size(0) < (1 << 30) && logits.size(1) > 0 &&
          logits.size(1) <= mcclMoeRouteMaxExperts() && capacity > 0 && logits.size(1) * capacity <= INT32_MAX;
 }
 
@@ -70,7 +70,7 @@ constexpr int64_t kFusedRouterExperts = 64;
 
 struct MoeFn : torch::autograd::Function<MoeFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& xIn, const Tensor& router, const Tensor& wIn, const Tensor& wOut, int64_t capacity) {
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(xIn.device());
     Tensor x = xIn.contiguous();
     if (!aligned16(x)) x = x.clone();
@@ -96,7 +96,20 @@ struct MoeFn : torch::autograd::Function<MoeFn> {
     auto v = ctx->get_saved_variables();
     const Tensor &x = v[0], &router = v[1], &wIn = v[2], &wOut = v[3], &logits = v[4], &gate = v[5], &lse = v[6], &flat = v[7],
                  &inverse = v[8], &kept = v[9], &slots = v[10], &pre = v[11], &h = v[12], &out = v[13];
-    at::AutoDispatchBelowADInplaceOrView below;
+    if (at::GradMode::is_enabled()) {                                // to be differentiated again: from the inputs, by operators
+      const int64_t E = router.size(0), C = ctx->saved_data["capacity"].toInt(), d = x.size(1);
+      Tensor rows = (flat >= 0).nonzero().squeeze(1), slot = flat.index({rows}).to(at::kLong);
+      Tensor p = at::softmax(at::linear(x, router).to(at::kFloat), -1), top = std::get<0>(p.max(-1)).to(x.scalar_type());
+      Tensor in = at::zeros({E * C, d}, x.options()).index_put({slot}, x.index({rows})).view({E, C, d});
+      Tensor o = at::bmm(at::silu(at::bmm(in, wIn.transpose(1, 2))), wOut.transpose(1, 2)).view({E * C, d});
+      Tensor y = at::zeros_like(x).index_put({rows}, o.index({slot}) * top.index({rows}).unsqueeze(1));
+      variable_list of, ret(5);
+      for (int i = 0; i < 4; ++i) if (ctx->needs_input_grad(i)) of.push_back(v[i]);
+      variable_list dv = torch::autograd::grad({y}, of, {g[0]}, std::nullopt, true);
+      for (int i = 0, k = 0; i < 4; ++i) if (ctx->needs_input_grad(i)) ret[i] = dv[k++];
+      return ret;
+    }
+    Below below;
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t T = x.size(0), d = x.size(1), E = router.size(0), C = ctx->saved_data["capacity"].toInt();
     mcclStream_t s = streamOf(x);
@@ -125,10 +138,12 @@ struct MoeFn : torch::autograd::Function<MoeFn> {
 
 // The layer's output, or None where the kernels do not cover the case.
 py::object moeLayer(const Tensor& x, const Tensor& router, const Tensor& wIn, const Tensor& wOut, int64_t capacity) {
-  if (!bf16Cuda(x) || x.dim() != 2 || x.size(0) == 0 || x.size(0) >= (1 << 30) || x.size(1) % 8 || router.dim() != 2 || router.size(1) != x.size(1) ||
+  if (recorded() || !ordinary(x) || !bf16Cuda(x) || x.dim() != 2 || x.size(0) == 0 || x.size(0) >= (1 << 30) || x.size(1) % 8 || router.dim() != 2 || router.size(1) != x.size(1) ||
       router.size(0) > mcclMoeRouteMaxExperts() || capacity <= 0 || router.size(0) * capacity > INT32_MAX) return py::none();
   for (const Tensor* w : {&router, &wIn, &wOut})
-    if (!bf16Cuda(*w) || !w->is_contiguous() || !aligned16(*w)) return py::none();
+    if (!ordinary(*w) || !bf16Cuda(*w) || !w->is_contiguous() || !aligned16(*w)) return py::none();
+  if (wIn.dim() != 3 || wIn.size(0) != router.size(0) || wIn.size(2) != x.size(1) || wOut.dim() != 3 || wOut.size(0) != router.size(0) ||
+      wOut.size(1) != x.size(1) || wOut.size(2) != wIn.size(1)) return py::none();
   return py::cast(MoeFn::apply(x, router, wIn, wOut, capacity));
 }
 

@@ -7,7 +7,7 @@ namespace {
 // ---- LayerNorm ------------------------------------------------------------------------------------------------------
 bool normSupported(const Tensor& x, const Tensor& w, const Tensor& b) {
   const int64_t d = x.dim() > 0 ? x.size(-1) : 0;
-  return bf16Cuda(x) && w.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && w.is_cuda() && b.is_cuda() && d > 0 &&
+  return !recorded() && ordinary(x) && ordinary(w) && ordinary(b) && bf16Cuda(x) && bf16Cuda(w) && bf16Cuda(b) && d > 0 &&
          d % 8 == 0 && d <= 4096 && w.numel() == d && b.numel() == d && w.is_contiguous() && b.is_contiguous() && aligned16(w) && aligned16(b);
 }
 
@@ -23,13 +23,19 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
     check(mcclLayerNormForward(xc.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean, mean + rows, rows, (int)d, (float)eps,
                                streamOf(xc)), "mcclLayerNormForward");
     counters().norm++;
-    ctx->save_for_backward({xc, w, stats});
+    ctx->save_for_backward({xc, w, stats, b});
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
     const Tensor &x = saved[0], &w = saved[1], &stats = saved[2];
     const int64_t d = x.size(-1), rows = x.numel() / d;
+    if (at::GradMode::is_enabled()) {                                // to be differentiated again: from the inputs, by operators
+      Tensor xs = x.reshape({rows, d}), dy = g[0].reshape({rows, d});
+      auto r = at::native_layer_norm_backward(dy, xs, {d}, stats.select(0, 0).unsqueeze(1), stats.select(0, 1).unsqueeze(1), w, saved[3],
+                                              {true, true, true});
+      return {std::get<0>(r).view(x.sizes()), std::get<1>(r), std::get<2>(r), Tensor()};
+    }
     Tensor dx = at::empty(x.sizes(), x.options()), dw = at::empty({d}, w.options()), db = at::empty({d}, w.options());
     if (rows == 0) { dw.zero_(); db.zero_(); return {dx, dw, db, Tensor()}; }
     Tensor dy = g[0].contiguous();
@@ -148,7 +154,7 @@ py::object gemm(const Tensor& x, const Tensor& w, const std::optional<Tensor>& o
 // and one elementwise pass; without gradients they are not kept.
 struct MlpFn : torch::autograd::Function<MlpFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& xIn, const Tensor& wUp, const Tensor& wDown, bool keep) {
-    at::AutoDispatchBelowADInplaceOrView below;
+    Below below;
     c10::cuda::CUDAGuard guard(xIn.device());
     Tensor x = xIn.contiguous();
     const int T = (int)x.size(0), h = (int)x.size(1), f = (int)wUp.size(0);
@@ -163,7 +169,15 @@ struct MlpFn : torch::autograd::Function<MlpFn> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto v = ctx->get_saved_variables();
     const Tensor &x = v[0], &wUp = v[1], &wDown = v[2], &act = v[3], &pre = v[4];
-    at::AutoDispatchBelowADInplaceOrView below;
+    if (at::GradMode::is_enabled()) {                                // to be differentiated again: from the inputs, by operators
+      variable_list in;
+      for (int i = 0; i < 3; ++i) if (ctx->needs_input_grad(i)) in.push_back(v[i]);
+      Tensor y = at::linear(at::silu(at::linear(x, wUp)), wDown);
+      variable_list d = torch::autograd::grad({y}, in, {g[0]}, std::nullopt, true), ret(4);
+      for (int i = 0, k = 0; i < 3; ++i) if (ctx->needs_input_grad(i)) ret[i] = d[k++];
+      return ret;
+    }
+    Below below;
     c10::cuda::CUDAGuard guard(x.device());
     Tensor dy = g[0].contiguous();
     variable_list ret(4);
@@ -178,8 +192,9 @@ struct MlpFn : torch::autograd::Function<MlpFn> {
 
 // None where the kernels do not cover the case.
 py::object mlp(const Tensor& x, const Tensor& wUp, const Tensor& wDown) {
+  if (recorded()) return py::none();
   for (const Tensor* t : {&x, &wUp, &wDown})
-    if (!bf16Cuda(*t) || t->dim() != 2 || !aligned16(*t)) return py::none();
+    if (!ordinary(*t) || !bf16Cuda(*t) || t->dim() != 2 || !aligned16(*t)) return py::none();
   const int64_t T = x.size(0), h = x.size(1), f = wUp.size(0);
   if (!wUp.is_contiguous() || !wDown.is_contiguous() || wUp.size(1) != h || wDown.size(0) != h || wDown.size(1) != f || T <= 0 || T % 128 || h % 64 ||
       f % 64) return py::none();

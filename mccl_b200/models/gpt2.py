@@ -20,6 +20,7 @@ import torch.nn.functional as F
 
 from .. import _ext
 from ..ops.norm import FusedLayerNorm
+from ..utils.fuse import as_made, may_fuse
 
 
 @dataclass
@@ -54,7 +55,7 @@ def _added(x: torch.Tensor, pending, pending_bias) -> torch.Tensor:
 
 
 class Block(nn.Module):
-    grad_sink = 0          # set by a data-parallel wrapper: how the fused nodes hand over weight gradients (csrc/torch/gradsink.h)
+    grad_sink = False      # set by a data-parallel wrapper: fused nodes add weight gradients to .grad (csrc/torch/gradsink.h)
 
     def __init__(self, cfg: GPT2Config, fused: bool = True):
         super().__init__()
@@ -75,17 +76,31 @@ class Block(nn.Module):
         self.ln2 = norm(cfg.d_model)
         self.fc = nn.Linear(cfg.d_model, cfg.d_ff)
         self.out = nn.Linear(cfg.d_ff, cfg.d_model)
-        # Where the parameters live, in the order the fused nodes take them (a look-up per parameter and call otherwise).
-        self._slots = [(m._parameters, n) for m in (self.ln1, self.q, self.k, self.v, self.proj, self.ln2, self.fc, self.out)
-                       for n in ("weight", "bias")] if fused else None
+
+    _PARTS = (("ln1", FusedLayerNorm), ("q", nn.Linear), ("k", nn.Linear), ("v", nn.Linear), ("proj", nn.Linear), ("ln2", FusedLayerNorm),
+              ("fc", nn.Linear), ("out", nn.Linear))
+
+    def _params(self):
+        """Weights and biases in the order the fused nodes take them; None where a part is not what this class made it."""
+        mods, out = self._modules, []
+        for name, cls in self._PARTS:
+            m = mods.get(name)
+            if m is None or not as_made(m, cls):
+                return None
+            p = m._parameters
+            if p["bias"] is None:
+                return None
+            out += (p["weight"], p["bias"])
+        return out if self.ln1.eps == self.ln2.eps else None
 
     def fused(self, x: torch.Tensor, pending, pending_bias, shape, bias_here: bool):
         """The block on x + pending ([tokens, d_model]) as two tensors still to be added, or None where it has to run as plain
         PyTorch.  `bias_here`: whether the gradient of the last bias is taken here or by whoever adds the two."""
-        if self._slots is None or not x.is_cuda or torch.is_autocast_enabled("cuda"):
+        params = self._params() if self.split_qkv and may_fuse(x) else None
+        if params is None:
             return None
         b, s = shape
-        return _ext.load().gpt2_block(x, pending, pending_bias, [d[n] for d, n in self._slots], b, s, self.n_head, bias_here,
+        return _ext.load().gpt2_block(x, pending, pending_bias, params, b, s, self.n_head, bias_here,
                                       self.ln1.eps, self.grad_sink)
 
     def forward(self, x: torch.Tensor, pending=None, pending_bias=None, shape=None):
@@ -97,7 +112,7 @@ class Block(nn.Module):
                 return pair
             x = _added(x, pending, pending_bias)
             return self._plain(x.view(*shape, -1)).view(x.shape), None
-        if self._slots is not None and x.is_cuda and x.dim() == 3 and x.is_contiguous():
+        if self.split_qkv and x.is_cuda and x.dim() == 3 and x.is_contiguous():
             pair = self.fused(x.view(-1, x.shape[-1]), None, None, x.shape[:2], True)
             if pair is not None:
                 return (pair[0] + pair[1]).view(x.shape)
@@ -120,7 +135,7 @@ class GPT2(nn.Module):
     """Decoder-only transformer with learned positions, pre-LayerNorm blocks and a tied output projection;
     forward(idx, targets) returns the mean cross-entropy, forward(idx) the logits."""
 
-    grad_sink = 0          # see Block
+    grad_sink = False      # see Block
 
     def __init__(self, cfg: GPT2Config, fused_loss: bool = True):
         super().__init__()
@@ -149,23 +164,26 @@ class GPT2(nn.Module):
         b, s = idx.shape
         w = self.wte.weight
         x = None
-        if self.fused_loss and w.is_cuda and w.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
+        if self.fused_loss and w.dtype == torch.bfloat16 and may_fuse(w) and as_made(self.wte, nn.Embedding) and as_made(self.wpe, nn.Embedding):
             x = _ext.load().decoder_embed(idx, w, self.wpe.weight, self.grad_sink)      # None where the kernels do not cover the case
         if x is not None:
             pending = bias = None
             for blk in self.blocks:
+                if not as_made(blk, Block):                  # its caller's hooks or wrapper see a block as it is called elsewhere
+                    x, pending = blk(_added(x, pending, bias).view(b, s, -1)).reshape(b * s, -1), None
+                    continue
                 x, pending = blk(x, pending, bias, (b, s))
                 # a block that ran as plain PyTorch has added everything and taken its bias gradient itself
                 bias = blk.out.bias if pending is not None else None
-            x = self._final_norm(x, pending, bias)
+            x = self._final_norm(x, pending, bias if pending is not None else None)
         else:
             pos = torch.arange(s, device=idx.device)
             x = self.wte(idx) + self.wpe(pos)
             for blk in self.blocks:
                 x = blk(x)
             x = self.ln_f(x)
-        if targets is not None and self.fused_loss and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_autocast_enabled("cuda"):
-            loss = _ext.load().decoder_head_loss(x.view(b * s, -1), w, targets, self.cfg.vocab_size, True, False, self.grad_sink)
+        if targets is not None and self.fused_loss and x.dtype == torch.bfloat16 and may_fuse(x):
+            loss = _ext.load().decoder_head_loss(x.view(b * s, -1), w, targets, self.cfg.vocab_size, False, self.grad_sink)
             if loss is not None:
                 return loss
         logits = F.linear(x, w).view(b, s, -1)           # tied output projection, padded vocab
@@ -181,5 +199,7 @@ class GPT2(nn.Module):
         n = self.ln_f
         if pending is None:
             return n(x)
-        h = _ext.load().gpt2_final_norm(x, pending, bias, n.weight, n.bias, n.eps, self.grad_sink)
+        h = None
+        if as_made(n, FusedLayerNorm):
+            h = _ext.load().gpt2_final_norm(x, pending, bias, n.weight, n.bias, n.eps, self.grad_sink)
         return h if h is not None else n(_added(x, pending, bias))

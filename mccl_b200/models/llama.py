@@ -27,6 +27,7 @@ from .. import _ext
 from ..comm import Communicator
 from ..parallel import functional as PF
 from ..parallel.layers import ColumnParallelLinear, RowParallelLinear
+from ..utils.fuse import as_made, may_fuse
 
 
 @dataclass
@@ -73,7 +74,7 @@ class Block(nn.Module):
     """Pre-norm attention + SwiGLU block holding 1/n of every projection.  With one rank, on CUDA in bf16, it runs as two fused
     autograd nodes around attention (csrc/torch/llama.cc)."""
 
-    grad_sink = 0          # set by a data-parallel wrapper: how the fused nodes hand over weight gradients (csrc/torch/gradsink.h)
+    grad_sink = False      # set by a data-parallel wrapper: fused nodes add weight gradients to .grad (csrc/torch/gradsink.h)
 
     def __init__(self, cfg: LlamaConfig, comm: Communicator, sp: bool):
         super().__init__()
@@ -92,8 +93,19 @@ class Block(nn.Module):
         self.gate = ColumnParallelLinear(comm, d, f, bias=False, sequence_parallel=sp)
         self.up = ColumnParallelLinear(comm, d, f, bias=False)
         self.down = RowParallelLinear(comm, f, d, bias=False, sequence_parallel=sp)
-        self._slots = [m._parameters for m in (self.norm1, self.q, self.k, self.v, self.o, self.norm2, self.gate, self.up, self.down)] \
-            if n == 1 else None
+
+    _PARTS = (("norm1", RMSNorm), ("q", ColumnParallelLinear), ("k", ColumnParallelLinear), ("v", ColumnParallelLinear), ("o", RowParallelLinear),
+              ("norm2", RMSNorm), ("gate", ColumnParallelLinear), ("up", ColumnParallelLinear), ("down", RowParallelLinear))
+
+    def _params(self):
+        """The weights in the order the fused nodes take them; None where a part is not what this class made it."""
+        mods, out = self._modules, []
+        for name, cls in self._PARTS:
+            m = mods.get(name)
+            if m is None or not as_made(m, cls) or m._parameters.get("bias") is not None:
+                return None
+            out.append(m._parameters["weight"])
+        return out if self.norm1.eps == self.norm2.eps == self.cfg.eps else None
 
     def _enter(self, x: torch.Tensor) -> torch.Tensor:
         """[batch*seq (/ n), d] -> the full token set every rank's weight shards are applied to."""
@@ -101,9 +113,10 @@ class Block(nn.Module):
 
     def fused(self, x: torch.Tensor, pending, batch: int, seq: int):
         """The block on x + pending as two tensors still to be added, or None where it has to run as separate operations."""
-        if self._slots is None or not x.is_cuda or torch.is_autocast_enabled("cuda"):
+        params = self._params() if self.comm.size == 1 and may_fuse(x) else None
+        if params is None:
             return None
-        return _ext.load().llama_block(x, pending, [d["weight"] for d in self._slots], batch, seq, self.heads_local, self.cfg.rope_theta,
+        return _ext.load().llama_block(x, pending, params, batch, seq, self.heads_local, self.cfg.rope_theta,
                                        self.cfg.eps, self.grad_sink)
 
     def forward(self, x: torch.Tensor, batch: int, seq: int, pending=None, pair: bool = False):
@@ -129,7 +142,7 @@ class Llama(nn.Module):
     """Tensor-parallel Llama-style decoder on `comm`; forward(idx, targets) returns the mean cross-entropy over all
     tokens (the same value on every rank), forward(idx) the logits of this rank's tokens."""
 
-    grad_sink = 0          # see Block
+    grad_sink = False      # see Block
 
     def __init__(self, cfg: LlamaConfig, comm: Communicator, sequence_parallel: bool = False):
         super().__init__()
@@ -142,7 +155,7 @@ class Llama(nn.Module):
     def forward(self, idx: torch.Tensor, targets: Optional[torch.Tensor] = None) -> torch.Tensor:
         b, s = idx.shape
         n, r = self.comm.size, self.comm.rank
-        if n == 1 and idx.is_cuda and not torch.is_autocast_enabled("cuda"):
+        if n == 1 and may_fuse(idx):
             return self._forward_one_rank(idx, targets)
         x = self.embed(idx).view(b * s, -1)
         if self.sp:                                       # this rank's rows of the flattened (batch, seq) tokens
@@ -163,17 +176,22 @@ class Llama(nn.Module):
     def _forward_one_rank(self, idx: torch.Tensor, targets: Optional[torch.Tensor]) -> torch.Tensor:
         """Every piece in a fused node where the kernels cover it (they answer None elsewhere) and as separate operations where not."""
         ext, (b, s) = _ext.load(), idx.shape
-        x = ext.decoder_embed(idx, self.embed.weight, None, self.grad_sink)
+        x = ext.decoder_embed(idx, self.embed.weight, None, self.grad_sink) if as_made(self.embed, nn.Embedding) else None
         if x is None:
             x = self.embed(idx).view(b * s, -1)
         pending = None
         for blk in self.blocks:
+            if not as_made(blk, Block):                     # its caller's hooks or wrapper see a block as it is called elsewhere
+                x, pending = blk(x if pending is None else x + pending, b, s), None
+                continue
             x, pending = blk(x, b, s, pending, True)
-        h = ext.llama_final_norm(x, pending, self.norm.weight, self.norm.eps, self.grad_sink) if pending is not None else None
+        h = None
+        if pending is not None and as_made(self.norm, RMSNorm):
+            h = ext.llama_final_norm(x, pending, self.norm.weight, self.norm.eps, self.grad_sink)
         if h is None:
             h = self.norm(x if pending is None else x + pending)
-        if targets is not None:
-            loss = ext.decoder_head_loss(h, self.head.weight, targets, self.head.weight.shape[0], False, True, self.grad_sink)
+        if targets is not None and as_made(self.head, nn.Linear) and self.head.bias is None:
+            loss = ext.decoder_head_loss(h, self.head.weight, targets, self.head.weight.shape[0], True, self.grad_sink)
             if loss is not None:
                 return loss
         logits = self.head(h)

@@ -23,7 +23,6 @@ docs/perf-scaling.png, README.md:55-57); the wrapper itself has no counterpart t
 from __future__ import annotations
 
 import os
-import weakref
 from contextlib import contextmanager
 from typing import List, Optional
 
@@ -127,25 +126,13 @@ class DistributedDataParallel(nn.Module):
 
     # ---- construction helpers
     def _attach_sink(self, module: nn.Module) -> None:
-        """Modules with fused nodes (an attribute `grad_sink`) add their weight gradients to the bucket views themselves and,
-        with several ranks, report every finished parameter as the gradient hooks do."""
-        if self.device.type != "cuda":
+        """On one rank, modules with fused nodes (an attribute `grad_sink`) add their weight gradients to the bucket views
+        themselves.  With several ranks the hooks have to see every finished gradient, so autograd delivers them."""
+        if self.device.type != "cuda" or self.world > 1:
             return
-        sink = -1
-        if self.world > 1:
-            from .. import _ext
-            me = weakref.ref(self)
-
-            def finished(p):
-                ddp = me()
-                if ddp is not None:
-                    ddp._on_grad(p)
-
-            sink = _ext.load().register_sink(finished)
-            weakref.finalize(self, _ext.load().drop_sink, sink)
         for m in module.modules():
             if hasattr(m, "grad_sink"):
-                m.grad_sink = sink
+                m.grad_sink = True
 
     def _sync_initial_state(self, module: nn.Module) -> None:
         """Every replica starts from rank 0's parameters and buffers, whatever each rank was seeded with (only

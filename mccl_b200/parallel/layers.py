@@ -24,6 +24,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..comm import Communicator
+from ..utils.fuse import as_made, may_fuse
 from . import functional as PF
 
 
@@ -179,14 +180,17 @@ class ExpertParallelMoE(nn.Module):
         if self.fused and x.is_cuda:
             from .. import _ext
             from ..ops import moe as M
-            if n == 1:                                                         # nothing to exchange: the whole layer is one node
+            # The kernels route as `route` here does with the router made above.
+            stock = (type(self).route is ExpertParallelMoE.route and "route" not in self.__dict__ and as_made(self.router, nn.Linear)
+                     and self.router.bias is None and may_fuse(x))
+            if n == 1 and stock:                                              # nothing to exchange: the whole layer is one node
                 y = _ext.load().moe_layer(x, self.router.weight, self.w_in, self.w_out, c)
                 if y is not None:
                     return y
             if self._buf is None:                                              # collective allocations, first call
                 self._buf = M.ExchangeBuffer(self.comm, e, c, d, x.dtype)
                 self._grad_buf = M.ExchangeBuffer(self.comm, e, c, d, x.dtype)
-            routed = _ext.load().moe_route(self.router(x), c)                  # None where the kernels do not cover the case
+            routed = _ext.load().moe_route(self.router(x), c) if stock else None     # None where the kernels do not cover the case
             if routed is not None:
                 gate, flat32 = routed
             else:

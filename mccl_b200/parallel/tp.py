@@ -18,6 +18,7 @@ from .. import _ext
 from .. import _lib as L
 from ..comm import Communicator
 from ..ops import gemm as G
+from ..utils.fuse import may_fuse
 from . import functional as PF
 
 
@@ -94,7 +95,13 @@ class _FusedMLPFunction(torch.autograd.Function):
         x_full, w_up, w_down = ctx.saved_tensors
         comm = ctx.layer.comm
         dy_full = PF._ag(comm, dy.contiguous())                    # [tokens, hidden]
-        h, du = _ext.load().silu_both(x_full @ w_up.t(), dy_full @ w_down)
+        u, dh = x_full @ w_up.t(), dy_full @ w_down
+        if u.is_cuda:
+            h, du = _ext.load().silu_both(u, dh)
+        else:
+            h = torch.nn.functional.silu(u.float()).to(u.dtype)
+            sig = torch.sigmoid(u.float())
+            du = (dh.float() * (sig * (1.0 + u.float() * (1.0 - sig)))).to(u.dtype)
         d_w_down = dy_full.t() @ h
         d_w_up = du.t() @ x_full
         dx = PF._rs(comm, du @ w_up)                               # this rank's rows of the input gradient
@@ -115,7 +122,7 @@ class FusedTensorParallelMLP(torch.nn.Module):
         self.layer = TensorParallelFFN(comm, tokens, hidden, ffn, self.w_up.data, self.w_down.data)
 
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
-        if self.layer.comm.size == 1:                             # nothing to gather or scatter: the two products are one node
+        if self.layer.comm.size == 1 and may_fuse(x_shard) and x_shard.shape == self.layer.x_shard.shape:     # nothing to gather or scatter: one node
             y = _ext.load().mlp(x_shard, self.w_up, self.w_down)
             if y is not None:
                 return y

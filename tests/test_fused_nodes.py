@@ -1,0 +1,262 @@
+"""When the decoders' fused nodes stand for their modules, and that they do nothing else there than the modules would: GPU tests
+compare the fused route with the plain one of the same model (a hook on a part sends a block down the plain one)."""
+import pytest
+import torch
+import torch.nn as nn
+
+from mccl_b200.models.gpt2 import GPT2, GPT2Config
+from mccl_b200.models.llama import Llama, LlamaConfig
+from mccl_b200.utils.fuse import as_made
+
+gpu = pytest.mark.gpu
+
+
+def test_as_made_sees_replacements_and_hooks():
+    m = nn.Linear(4, 4)
+    assert as_made(m, nn.Linear)
+
+    class Mine(nn.Linear):
+        pass
+
+    assert not as_made(Mine(4, 4), nn.Linear)
+    h = m.register_forward_pre_hook(lambda mod, args: None)
+    assert not as_made(m, nn.Linear)
+    h.remove()
+    m.forward = lambda x: x
+    assert not as_made(m, nn.Linear)
+    w = nn.utils.parametrizations.weight_norm(nn.Linear(4, 4))
+    assert not as_made(w, nn.Linear)
+
+
+def _comm():
+    import mccl_b200 as mccl
+    return mccl.Communicator(1, mccl.get_unique_id(), 0, transport="cuda")
+
+
+def _gpt2(d=128, layers=2, vocab=300, seq=40):
+    torch.manual_seed(0)
+    cfg = GPT2Config(n_layer=layers, d_model=d, n_head=d // 32, d_ff=4 * d, vocab_size=vocab, seq_len=seq)
+    model = GPT2(cfg).to(device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if n.endswith("bias"):
+                p.normal_(std=0.05)
+    return model
+
+
+def _llama(d=128, layers=2, vocab=300, seq=40, heads=None):
+    torch.manual_seed(0)
+    cfg = LlamaConfig(n_layer=layers, d_model=d, n_head=heads or d // 32, d_ff=3 * d, vocab_size=vocab, seq_len=seq)
+    return Llama(cfg, _comm()).to(device="cuda", dtype=torch.bfloat16)
+
+
+def _batch(vocab=300, b=3, s=37):
+    t = torch.randint(0, vocab, (b, s + 1), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    return t[:, :-1].contiguous(), t[:, 1:].contiguous()
+
+
+def _grads(model, idx, tgt):
+    loss = model(idx, tgt)
+    return [loss.detach()] + list(torch.autograd.grad(loss, list(model.parameters())))
+
+
+def _plain(model):
+    """The same model with a hook that does nothing on every part: the fused nodes stand aside."""
+    for m in model.modules():
+        if m is not model:
+            m.register_forward_pre_hook(lambda mod, args: None)
+    return model
+
+
+def _reference(model, idx, tgt):
+    """Loss and gradients of the same weights in 64 bits (no kernels take it)."""
+    model = _plain(model).double()
+    loss = model(idx, tgt)
+    return [loss.detach()] + list(torch.autograd.grad(loss, list(model.parameters())))
+
+
+@gpu
+@pytest.mark.parametrize("make,kw", [(_gpt2, {"d": 128}), (_gpt2, {"d": 384}), (_gpt2, {"d": 1056}), (_llama, {"d": 128}), (_llama, {"d": 64, "heads": 4}),
+                                     (_llama, {"d": 1152, "heads": 9})])
+def test_fused_route_is_as_close_to_64_bits_as_the_plain_one(make, kw):
+    idx, tgt = _batch()
+    fused = _grads(make(**kw), idx, tgt)
+    plain = _grads(_plain(make(**kw)), idx, tgt)
+    want = _reference(make(**kw), idx, tgt)
+    for f, p, w in zip(fused, plain, want):
+        scale = w.norm().clamp_min(1e-30)
+        ef, ep = (f.double() - w).norm() / scale, (p.double() - w).norm() / scale
+        # Two routes of the same roundings in another order: their errors are draws of one distribution.  1.5 x and half a
+        # bf16 step (2^-9) cover the spread of the smallest tensors (a bias of 128 values).
+        assert ef <= 1.5 * ep + 2.0 ** -9, (tuple(w.shape), ef.item(), ep.item())
+
+
+@gpu
+@pytest.mark.parametrize("make", [_gpt2, _llama])
+def test_hooks_and_replaced_parts_are_called(make):
+    idx, tgt = _batch()
+    model, seen = make(), []
+    getattr(model.blocks[0], "fc" if make is _gpt2 else "o").register_forward_hook(lambda mod, args, out: seen.append("part"))
+    model.blocks[1].register_forward_hook(lambda mod, args, out: seen.append(out if isinstance(out, tuple) else out.shape))
+    model(idx, tgt).backward()
+    assert seen[0] == "part" and isinstance(seen[1], torch.Size) and seen[1][-1] == 128
+
+    class Twice(nn.Module):                      # a part put in the place of another
+        def __init__(self, inner):
+            super().__init__()
+            self.inner, self.weight = inner, inner.weight
+
+        def forward(self, x):
+            return 2 * self.inner(x)
+
+    a, b = make(), make()
+    name = "fc" if make is _gpt2 else "o"
+    setattr(a.blocks[0], name, Twice(getattr(a.blocks[0], name)))
+    with torch.no_grad():
+        for p in getattr(b.blocks[0], name).parameters():
+            p.mul_(2)
+    la, lb = a(idx, tgt), b(idx, tgt)
+    assert abs(la.item() - lb.item()) <= 2.0 ** -8 * abs(lb.item()) and abs(la.item() - make()(idx, tgt).item()) > 0
+
+
+@gpu
+def test_input_changed_in_place_is_noticed():
+    blk = _gpt2().blocks[0]
+    x = torch.randn(2, 8, 128, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    h = x * 1
+    y = blk(h)
+    with torch.no_grad():
+        h.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
+
+
+@gpu
+@pytest.mark.parametrize("make", [_gpt2, _llama])
+def test_frozen_weights_get_no_gradient(make):
+    idx, tgt = _batch()
+    model = make()
+    for blk in model.blocks:
+        blk.q.weight.requires_grad_(False)
+    model(idx, tgt).backward()
+    for n, p in model.named_parameters():
+        assert (p.grad is None) == (not p.requires_grad), n
+
+
+@gpu
+def test_gradients_reach_buckets_hooks_and_other_streams():
+    from mccl_b200.parallel.ddp import DistributedDataParallel
+    idx, tgt = _batch()
+    want = [g.clone() for g in _grads(_gpt2(), idx, tgt)[1:]]
+    model = _gpt2()
+    ddp = DistributedDataParallel(model, None)
+    # twice into the buckets: each the sum of two equal gradients, one rounding later
+    for _ in range(2):
+        ddp(idx, tgt).backward()
+    for p, w in zip(model.parameters(), want):
+        assert (p.grad.float() - 2 * w.float()).norm() <= 2.0 ** -7 * (2 * w.float()).norm()
+        p.grad.zero_()
+    # a hook of the user's sees the gradient of its parameter
+    seen = []
+    model.blocks[0].fc.weight.register_post_accumulate_grad_hook(lambda p: seen.append(p.grad.clone()))
+    ddp(idx, tgt).backward()
+    fc = [n for n, _ in model.named_parameters()].index("blocks.0.fc.weight")
+    assert len(seen) == 1 and torch.equal(seen[0], model.blocks[0].fc.weight.grad)
+    assert (seen[0].float() - want[fc].float()).norm() <= 2.0 ** -7 * want[fc].float().norm()
+    for p in model.parameters():
+        p.grad.zero_()
+    torch.cuda.synchronize()
+    # forward on another stream: what the caller's stream reads after backward() is complete
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        loss = ddp(idx, tgt)
+    loss.backward()
+    got = [p.grad.clone() for p in model.parameters()]
+    for g, w in zip(got, want):
+        assert (g.float() - w.float()).norm() <= 2.0 ** -7 * w.float().norm()
+
+
+@gpu
+@pytest.mark.parametrize("make", [_gpt2, _llama])
+def test_second_derivatives_are_not_constants(make):
+    """The nodes' gradients raise when differentiated; with attention by products the plain operations answer."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    idx, tgt = _batch(b=1, s=16)
+    model = make()
+    w = model.blocks[0].v.weight
+    g, = torch.autograd.grad(model(idx, tgt), [w], create_graph=True)
+    with pytest.raises(RuntimeError):
+        g.float().pow(2).sum().backward()
+    if make is _llama:
+        with sdpa_kernel(SDPBackend.MATH):
+            x = torch.randn(16, 128, device="cuda").to(torch.bfloat16).requires_grad_(True)
+            g, = torch.autograd.grad(model.blocks[0](x, 1, 16).float().sum(), [x], create_graph=True)
+            assert torch.autograd.grad(g.float().pow(2).sum(), [x])[0].abs().sum() > 0
+
+
+@gpu
+def test_layers_differentiated_twice_match_plain_operations():
+    from mccl_b200.ops.norm import FusedLayerNorm
+    from mccl_b200.parallel.layers import ExpertParallelMoE
+    from mccl_b200.parallel.tp import FusedTensorParallelMLP
+    torch.manual_seed(0)
+
+    def twice(f, x):
+        g, = torch.autograd.grad(f(x).float().pow(2).sum(), [x], create_graph=True)
+        return torch.autograd.grad(g.float().pow(2).sum(), [x])[0].double()
+
+    x = torch.randn(128, 64, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    x64 = x.detach().double().requires_grad_(True)
+
+    def twice64(f):
+        g, = torch.autograd.grad(f(x64).pow(2).sum(), [x64], create_graph=True)
+        return torch.autograd.grad(g.pow(2).sum(), [x64])[0]
+
+    ln = FusedLayerNorm(64).to(device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        ln.weight.normal_(1.0, 0.3)
+    mlp = FusedTensorParallelMLP(_comm(), 128, 64, 128)
+    wu, wd = mlp.w_up.detach().double(), mlp.w_down.detach().double()
+    silu = nn.functional.silu
+    moe = ExpertParallelMoE(_comm(), 64, 64, 1, 128, device="cuda", dtype=torch.bfloat16, fused=True)      # one expert: its gate is 1
+    wi, wo = moe.w_in.detach().double()[0], moe.w_out.detach().double()[0]
+    for f, f64 in ((ln, lambda t: nn.functional.layer_norm(t, (64,), ln.weight.detach().double(), ln.bias.detach().double(), ln.eps)),
+                   (mlp, lambda t: silu(t @ wu.t()) @ wd.t()), (moe, lambda t: silu(t @ wi.t()) @ wo.t())):
+        want = twice64(f64)
+        assert (twice(f, x) - want).norm() <= 0.05 * want.norm()      # about a dozen bf16 roundings of 2^-8 each
+
+
+@gpu
+def test_torch_func_and_tracing_take_the_plain_route():
+    idx, tgt = _batch(b=1, s=16)
+    model = _llama()
+    params = {n: p.detach() for n, p in model.named_parameters()}
+    g = torch.func.grad(lambda ps: torch.func.functional_call(model, ps, (idx, tgt)))(params)
+    want = _grads(model, idx, tgt)[1:]
+    for (n, a), b in zip(g.items(), want):
+        assert (a.float() - b.float()).norm() <= 0.05 * b.float().norm(), n      # the two routes round in another order
+    model.requires_grad_(False)
+    traced = torch.jit.trace(lambda t: model(t), (idx,), check_trace=False)
+    other, _ = _batch(b=1, s=16)
+    other = (other + 7) % 300
+    with torch.no_grad():
+        a, b = traced(other), model(other)
+    assert (a.float() - b.float()).norm() <= 0.05 * b.float().norm()
+
+
+@gpu
+def test_moe_subclass_routes_its_own_way():
+    from mccl_b200.parallel.layers import ExpertParallelMoE
+
+    class First(ExpertParallelMoE):
+        def route(self, x):
+            z = torch.zeros(x.shape[0], dtype=torch.int64, device=x.device)
+            slot = torch.arange(x.shape[0], device=x.device)
+            return z, torch.ones(x.shape[0], dtype=x.dtype, device=x.device), slot, slot < self.capacity
+
+    torch.manual_seed(0)
+    layer = First(_comm(), 64, 64, 4, 64, device="cuda", dtype=torch.bfloat16, fused=True)
+    x = torch.randn(64, 64, device="cuda").to(torch.bfloat16)
+    want = nn.functional.silu(x.double() @ layer.w_in[0].double().t()) @ layer.w_out[0].double().t()
+    assert (layer(x).double() - want).norm() <= 4 * 2.0 ** -8 * want.norm()
