@@ -34,20 +34,41 @@ __device__ __forceinline__ uint4 pack(const float* f) {
 __device__ __forceinline__ float rounded(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
-// tanh by its exponential form, for the gradient: absolute error of a few 2^-22, far below the bf16 rounding of the result.
-__device__ __forceinline__ float tanhOf(float x) {
-  const float e = __expf(-2.f * fabsf(x));
-  return copysignf(__fdividef(1.f - e, 1.f + e), x);
-}
+// The tanh-GELU is x * s with s = (1 + tanh(z)) / 2 = 1 / (1 + exp(-2 z)), z = c (x + a x^3): one exponential and one
+// reciprocal, absolute error of s a few 2^-23, and its gradient is s + 2 z' x s (1 - s).
 constexpr float kGeluC = 0.7978845608028654f;      // sqrt(2 / pi)
 constexpr float kGeluA = 0.044715f;
-__device__ __forceinline__ float gelu(float x) {
+constexpr float kGeluE = -2.f * kGeluC * 1.4426950408889634f;      // exp(-2 z) = 2^(kGeluE (x + a x^3))
+__device__ __forceinline__ float geluGate(float x, float x2) {
+  float e, s;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * fmaf(kGeluE * kGeluA, x2, kGeluE)));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.f + e));
+  return s;
+}
+__device__ __forceinline__ float geluGrad(float x) {
+  const float x2 = x * x, s = geluGate(x, x2);
+  return fmaf(fmaf(-s, s, s), x * fmaf(6.f * kGeluC * kGeluA, x2, 2.f * kGeluC), s);
+}
+
+// Forward, to the last bit what 0.5 x (1 + tanhf(z)) rounds to (scores compare with recorded ones only so): the short form
+// and the long one differ by less than `w` (both within 3e-7 of 1 + tanh, products within 2^-22), so where the ends of that
+// interval round to the same bf16 number it is the result; elsewhere, about one value in a thousand, the long form decides.
+__device__ __noinline__ float geluLong(float x) {
   const float cube = x * x * x;
   return 0.5f * x * (1.f + tanhf(kGeluC * (x + kGeluA * cube)));
 }
-__device__ __forceinline__ float geluGrad(float x) {
-  const float t = tanhOf(kGeluC * (x + kGeluA * x * x * x));
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * kGeluC * (1.f + 3.f * kGeluA * x * x);
+__device__ __forceinline__ uint32_t gelu2(float x0, float x1) {
+  const float g0 = x0 * geluGate(x0, x0 * x0), g1 = x1 * geluGate(x1, x1 * x1);
+  const float w0 = fmaf(fabsf(g0), 5e-7f, fabsf(x0) * 5e-7f), w1 = fmaf(fabsf(g1), 5e-7f, fabsf(x1) * 5e-7f);
+  __nv_bfloat162 lo = __floats2bfloat162_rn(g0 - w0, g1 - w1), hi = __floats2bfloat162_rn(g0 + w0, g1 + w1);
+  uint32_t a = *reinterpret_cast<uint32_t*>(&lo);
+  const uint32_t b = *reinterpret_cast<uint32_t*>(&hi);
+  if (a != b) {
+    if ((a ^ b) & 0xffffu) lo.x = __float2bfloat16_rn(geluLong(x0));
+    if ((a ^ b) >> 16) lo.y = __float2bfloat16_rn(geluLong(x1));
+    a = *reinterpret_cast<uint32_t*>(&lo);
+  }
+  return a;
 }
 
 // An operation maps IN input values to OUT output values.
@@ -77,7 +98,6 @@ struct SwigluBwd {                                 // (gate, up, gradient) -> pr
     o[2] = i[2] * act;
   }
 };
-struct GeluFwd { static constexpr int IN = 1, OUT = 1; __device__ static void f(const float* i, float* o) { o[0] = gelu(i[0]); } };
 
 template <class Op> struct ActArgs { const uint4* in[Op::IN]; uint4* out[Op::OUT]; int64_t n; };
 
@@ -121,6 +141,26 @@ __global__ void __launch_bounds__(kActThreads) actKernel(const __grid_constant__
   }
 }
 
+// GELU: four 16-byte pieces per thread as above; bound by memory with the short form (8192 x 4096: TIMES).
+__global__ void __launch_bounds__(kActThreads) geluKernel(const uint4* x, uint4* y, int64_t n) {
+  constexpr int U = 4;
+  const int64_t vecs = n / 8, i0 = (int64_t)blockIdx.x * (kActThreads * U) + threadIdx.x;
+  uint4 q[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) if (i0 + u * kActThreads < vecs) q[u] = x[i0 + u * kActThreads];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (i0 + u * kActThreads >= vecs) continue;
+    float f[8];
+    unpack(q[u], f);
+    y[i0 + u * kActThreads] = make_uint4(gelu2(f[0], f[1]), gelu2(f[2], f[3]), gelu2(f[4], f[5]), gelu2(f[6], f[7]));
+  }
+  if (blockIdx.x == 0 && threadIdx.x < (unsigned)(n % 8)) {          // the last few elements
+    const int64_t i = vecs * 8 + threadIdx.x;
+    reinterpret_cast<__nv_bfloat16*>(y)[i] = __float2bfloat16_rn(geluLong(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i])));
+  }
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 template <class Op>
@@ -142,21 +182,26 @@ mcclResult_t act(std::initializer_list<const void*> in, std::initializer_list<vo
 // ---- column sums ------------------------------------------------------------------------------------------------------
 // A CTA takes a strip of 64 x 8 columns (one vector per lane of two warps' width) and walks rows; four groups of 64 threads
 // take every fourth row.  Up to three matrices of the same shape in one launch (blockIdx.z).  With GELU the matrix is the
-// gradient of the activation, replaced by the gradient of the pre-activation on the way.
+// gradient of the activation, replaced by the gradient of the pre-activation on the way.  With PACK the matrices are also
+// written side by side into one [rows, segments x D] matrix, so that the products behind take them as one operand: three
+// products of 1024 x 1024 x 8192 (77 us: 128 tiles of 128 x 64, which one product of 3072 x 1024 does not need) and three
+// that share an output become two, for a write of the matrices.
+enum ColMode { COL_SUM, COL_GELU, COL_PACK };
 constexpr int kStripVecs = 64, kStripCols = kStripVecs * 8, kRowGroups = kActThreads / kStripVecs;
 
 struct ColArgs {
   const uint4* x[colred::kMaxSegments];       // [rows, D] each, row stride `ld` vectors
   const uint4* pre;                           // GELU: pre-activation
-  uint4* dx;                                  // GELU: where the gradient goes
+  uint4* dx;                                  // GELU: where the gradient goes; PACK: the matrix of all
   float* partial;                             // [gridDim.y][segments * D]
-  int64_t rows, ld;
+  int64_t rows, ld, ldx;                      // ldx: row stride of dx
   int D;
   colred::Out out;
 };
 
-template <bool GELU>
+template <int MODE>
 __global__ void __launch_bounds__(kActThreads, 3) colSumKernel(const __grid_constant__ ColArgs a) {
+  constexpr bool GELU = MODE == COL_GELU;
   __shared__ float red[kRowGroups][kStripCols];
   const int tv = threadIdx.x % kStripVecs, g = threadIdx.x / kStripVecs, vecs = a.D / 8;
   const int v = blockIdx.x * kStripVecs + tv, seg = blockIdx.z;
@@ -178,13 +223,14 @@ __global__ void __launch_bounds__(kActThreads, 3) colSumKernel(const __grid_cons
         if (r >= a.rows) continue;
         float f[8];
         unpack(q[u], f);
+        if (MODE == COL_PACK) a.dx[r * a.ldx + (int64_t)seg * vecs + v] = q[u];
         if (GELU) {
           float z[8];
           unpack(p[u], z);
 #pragma unroll
           for (int k = 0; k < 8; ++k) f[k] *= geluGrad(z[k]);
           const uint4 o = pack(f);
-          a.dx[r * a.ld + v] = o;
+          a.dx[r * a.ldx + v] = o;
           unpack(o, f);
         }
 #pragma unroll
@@ -216,10 +262,10 @@ int colSlices(int64_t rows, int D, int segments) {
   return s < 1 ? 1 : (int)s;
 }
 
-template <bool GELU>
+template <int MODE>
 mcclResult_t colSums(const ColArgs& a, cudaStream_t s) {
   const int strips = (a.D / 8 + kStripVecs - 1) / kStripVecs, slices = colSlices(a.rows, a.D, a.out.segments);
-  colSumKernel<GELU><<<dim3(strips, slices, a.out.segments), kActThreads, 0, s>>>(a);
+  colSumKernel<MODE><<<dim3(strips, slices, a.out.segments), kActThreads, 0, s>>>(a);
   if (cudaGetLastError() != cudaSuccess) return mcclSystemError;
   return colred::addPartials(a.partial, slices, 1, a.out.segments * a.D, a.out, s) == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
@@ -235,7 +281,14 @@ extern "C" mcclResult_t mcclSwigluForward(const void* gate, const void* up, void
 extern "C" mcclResult_t mcclSwigluBackward(const void* gate, const void* up, const void* dy, void* y, void* dgate, void* dup, int64_t n, mcclStream_t s) {
   return act<SwigluBwd>({gate, up, dy}, {y, dgate, dup}, n, s);
 }
-extern "C" mcclResult_t mcclGeluForward(const void* x, void* y, int64_t n, mcclStream_t s) { return act<GeluFwd>({x}, {y}, n, s); }
+extern "C" mcclResult_t mcclGeluForward(const void* x, void* y, int64_t n, mcclStream_t stream) {
+  if (!x || !y || !aligned16(x) || !aligned16(y) || n < 0) return mcclInvalidArgument;
+  if (n == 0) return mcclSuccess;
+  const int64_t per = kActThreads * 4, blocks = (n / 8 + per - 1) / per;
+  geluKernel<<<(unsigned)(blocks < 1 ? 1 : blocks), kActThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(x), static_cast<uint4*>(y), n);
+  return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
+}
 
 // Floats of work memory the two functions below need.
 extern "C" int64_t mcclColumnSumScratch(int64_t rows, int D, int segments) {
@@ -248,9 +301,9 @@ extern "C" mcclResult_t mcclGeluBackward(const void* x, const void* dy, void* dx
   if (!x || !dy || !dx || !scratch || rows <= 0 || D <= 0 || D % 8 || !aligned16(x) || !aligned16(dy) || !aligned16(dx)) return mcclInvalidArgument;
   ColArgs a = {};
   a.x[0] = static_cast<const uint4*>(dy); a.pre = static_cast<const uint4*>(x); a.dx = static_cast<uint4*>(dx);
-  a.partial = scratch; a.rows = rows; a.ld = D / 8; a.D = D;
+  a.partial = scratch; a.rows = rows; a.ld = a.ldx = D / 8; a.D = D;
   a.out.seg[0] = static_cast<__nv_bfloat16*>(dbias); a.out.segments = 1; a.out.width = D; a.out.accumulate = accumulate;
-  return colSums<true>(a, reinterpret_cast<cudaStream_t>(stream));
+  return colSums<COL_GELU>(a, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // out[i] = [+] column sums of x[i], up to three [rows, D] matrices with rows `ld` elements apart.
@@ -265,5 +318,22 @@ extern "C" mcclResult_t mcclColumnSums(const void* const* x, void* const* out, i
   }
   a.partial = scratch; a.rows = rows; a.ld = ld / 8; a.D = D;
   a.out.segments = n; a.out.width = D; a.out.accumulate = accumulate;
-  return colSums<false>(a, reinterpret_cast<cudaStream_t>(stream));
+  return colSums<COL_SUM>(a, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// The same for contiguous matrices, which are also written side by side: packed[r][i * D + c] = x[i][r][c].
+extern "C" mcclResult_t mcclPackColumnSums(const void* const* x, void* packed, void* const* out, int n, int accumulate, float* scratch,
+                                           int64_t rows, int D, mcclStream_t stream) {
+  if (!x || !packed || !out || !scratch || n < 1 || n > colred::kMaxSegments || rows <= 0 || D <= 0 || D % 8 || !aligned16(packed))
+    return mcclInvalidArgument;
+  ColArgs a = {};
+  for (int i = 0; i < n; ++i) {
+    if (!x[i] || !out[i] || !aligned16(x[i])) return mcclInvalidArgument;
+    a.x[i] = static_cast<const uint4*>(x[i]);
+    a.out.seg[i] = static_cast<__nv_bfloat16*>(out[i]);
+  }
+  a.dx = static_cast<uint4*>(packed);
+  a.partial = scratch; a.rows = rows; a.ld = D / 8; a.ldx = (int64_t)n * (D / 8); a.D = D;
+  a.out.segments = n; a.out.width = D; a.out.accumulate = accumulate;
+  return colSums<COL_PACK>(a, reinterpret_cast<cudaStream_t>(stream));
 }

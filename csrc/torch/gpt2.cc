@@ -91,18 +91,35 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     auto zeros = [&] { return at::zeros({T, d}, h.options()); };
     Tensor dq = g[1].defined() ? fromHeads(g[1], T, d) : zeros(), dk = g[2].defined() ? fromHeads(g[2], T, d) : zeros(),
            dv = g[3].defined() ? fromHeads(g[3], T, d) : zeros();
-    Tensor dwq, dwk, dwv;
-    VectorGrads db(sink, {&bq, &bk, &bv});
-    {
-      Tensor scratch = columnScratch(h, T, d, 3);
-      const void* in[3] = {dq.data_ptr(), dk.data_ptr(), dv.data_ptr()};
-      void* out[3] = {db.t[0].data_ptr(), db.t[1].data_ptr(), db.t[2].data_ptr()};
+    Tensor dwq, dwk, dwv, dhv, dhk, dhq;
+    VectorGrads db(sink, {&bv, &bk, &bq});
+    Tensor scratch = columnScratch(h, T, d, 3);
+    const void* in[3] = {dv.data_ptr(), dk.data_ptr(), dq.data_ptr()};
+    void* out[3] = {db.t[0].data_ptr(), db.t[1].data_ptr(), db.t[2].data_ptr()};
+    Tensor w3 = adjacent(wv, wk, wq);
+    if (w3.defined()) {
+      // The weights as one matrix: the gradients are laid side by side on the pass that sums their columns, and one product
+      // gives the norm's gradient, another the three weight gradients where those are one matrix too.
+      Tensor d3 = at::empty({T, 3 * d}, h.options());
+      check(mcclPackColumnSums(in, d3.data_ptr(), out, 3, db.direct, scratch.data_ptr<float>(), T, (int)d, s), "mcclPackColumnSums");
+      dhv = at::mm(d3, w3);
+      Tensor gv = sink.buffer(wv), gk = sink.buffer(wk), gq = sink.buffer(wq);
+      Tensor g3 = gv.defined() && gk.defined() && gq.defined() ? adjacent(gv, gk, gq) : Tensor();
+      if (g3.defined()) {
+        at::addmm_out(g3, g3, d3.t(), h);
+      } else {
+        weightGrad(sink, wv, dv, h, &dwv);
+        weightGrad(sink, wk, dk, h, &dwk);
+        weightGrad(sink, wq, dq, h, &dwq);
+      }
+    } else {
       check(mcclColumnSums(in, out, 3, db.direct, scratch.data_ptr<float>(), T, (int)d, d, s), "mcclColumnSums");
+      dhv = at::mm(dv, wv); dhk = at::mm(dk, wk); dhq = at::mm(dq, wq);      // the norm's backward kernel adds them up
+      weightGrad(sink, wv, dv, h, &dwv);
+      weightGrad(sink, wk, dk, h, &dwk);
+      weightGrad(sink, wq, dq, h, &dwq);
     }
-    Tensor dhv = at::mm(dv, wv), dhk = at::mm(dk, wk), dhq = at::mm(dq, wq);      // the norm's backward kernel adds them up
-    weightGrad(sink, wv, dv, h, &dwv);
-    weightGrad(sink, wk, dk, h, &dwk);
-    weightGrad(sink, wq, dq, h, &dwq);
+    const void *part2 = dhk.defined() ? dhk.data_ptr() : nullptr, *part3 = dhq.defined() ? dhq.data_ptr() : nullptr;
     Tensor dx = at::empty({T, d}, h.options());
     Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * 3 * d}, stats.options());
     const float* mean = stats.data_ptr<float>();
@@ -111,13 +128,13 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
       Tensor dres = rows2d(g[0], T, d);
       if (pb.defined()) {
         VectorGrads dn(sink, {&lw, &lb, &pb});
-        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), dhk.data_ptr(), dhq.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
+        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), part2, part3, dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
                                        dn.t[0].data_ptr(), dn.t[1].data_ptr(), dn.t[2].data_ptr(), dn.direct, partial.data_ptr<float>(), T,
                                        (int)d, s), "mcclAddLayerNormBackward");
         ret[3] = dn.ret(0); ret[4] = dn.ret(1); ret[2] = dn.ret(2);
       } else {
         VectorGrads dn(sink, {&lw, &lb});
-        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), dhk.data_ptr(), dhq.data_ptr(), dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
+        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), part2, part3, dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
                                        dn.t[0].data_ptr(), dn.t[1].data_ptr(), nullptr, dn.direct, partial.data_ptr<float>(), T, (int)d, s),
               "mcclAddLayerNormBackward");
         ret[3] = dn.ret(0); ret[4] = dn.ret(1);
@@ -125,7 +142,7 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     } else {                                       // nobody uses the residual: the plain norm, and the bias on its own
       ret[3] = at::empty(lw.sizes(), lw.options());
       ret[4] = at::empty(lb.sizes(), lb.options());
-      Tensor dh = dhv.add_(dhk).add_(dhq);
+      Tensor dh = part2 ? dhv.add_(dhk).add_(dhq) : dhv;
       check(mcclLayerNormBackward(sum.data_ptr(), dh.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(), ret[3].data_ptr(),
                                   ret[4].data_ptr(), partial.data_ptr<float>(), T, (int)d, s), "mcclLayerNormBackward");
       if (pb.defined()) ret[2] = dx.sum(0);
@@ -133,7 +150,7 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     counters().norm += 2;
     ret[0] = dx;
     if (pending) ret[1] = dx;
-    ret[5] = dwq; ret[6] = db.ret(0); ret[7] = dwk; ret[8] = db.ret(1); ret[9] = dwv; ret[10] = db.ret(2);
+    ret[5] = dwq; ret[6] = db.ret(2); ret[7] = dwk; ret[8] = db.ret(1); ret[9] = dwv; ret[10] = db.ret(0);
     return once(std::move(ret));
   }
 };

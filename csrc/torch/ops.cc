@@ -210,6 +210,22 @@ std::pair<Tensor, Tensor> siluBoth(const Tensor& u, const Tensor& dh) {
   return {h, du};
 }
 
+// Tanh-GELU and, with a gradient, the gradient of x and its column sums.
+Tensor geluForward(const Tensor& x) {
+  TORCH_CHECK(bf16Cuda(x) && x.is_contiguous(), "gelu: a contiguous bf16 cuda tensor");
+  Tensor y = at::empty_like(x);
+  check(mcclGeluForward(x.data_ptr(), y.data_ptr(), x.numel(), streamOf(x)), "mcclGeluForward");
+  return y;
+}
+std::pair<Tensor, Tensor> geluBackward(const Tensor& x, const Tensor& dy) {
+  TORCH_CHECK(bf16Cuda(x) && bf16Cuda(dy) && x.dim() == 2 && x.is_contiguous() && dy.is_contiguous() && x.sizes() == dy.sizes(), "gelu: bf16 cuda matrices");
+  Tensor dx = at::empty_like(x), db = at::empty({x.size(1)}, x.options());
+  Tensor scratch = at::empty({mcclColumnSumScratch(x.size(0), (int)x.size(1), 1)}, x.options().dtype(at::kFloat));
+  check(mcclGeluBackward(x.data_ptr(), dy.data_ptr(), dx.data_ptr(), db.data_ptr(), 0, scratch.data_ptr<float>(), x.size(0), (int)x.size(1),
+                         streamOf(x)), "mcclGeluBackward");
+  return {dx, db};
+}
+
 }  // namespace
 
 void bindOps(py::module_& m) {
@@ -220,6 +236,8 @@ void bindOps(py::module_& m) {
   m.def("gemm", &gemm);
   m.def("mlp", &mlp);
   m.def("silu_both", &siluBoth);
+  m.def("gelu_forward", &geluForward);
+  m.def("gelu_backward", &geluBackward);
   m.def("launches", [](const std::string& what) -> int64_t {
     Counters& c = counters();
     if (what == "norm") return c.norm;

@@ -130,6 +130,8 @@ mcclResult_t mcclLayerNormBackward(const void* x, const void* dy, const void* ga
  * dres; dcol (nullable, needs dres) = column sums of dx; accumulate: dgamma, dbeta and dcol are added to what is there. */
 mcclResult_t mcclAddLayerNormForward(const void* x, const void* delta, const void* gamma, const void* beta, void* sum, void* y, float* mean,
                                      float* rstd, int64_t rows, int D, float eps, mcclStream_t stream);
+mcclResult_t mcclPackColumnSums(const void* const* x, void* packed, void* const* out, int n, int accumulate, float* scratch, int64_t rows,
+                                int D, mcclStream_t stream);
 mcclResult_t mcclAddLayerNormBackward(const void* x, const void* dy, const void* dy2, const void* dy3, const void* dres, const void* gamma,
                                       const float* mean, const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate, float* partial,
                                       int64_t rows, int D, mcclStream_t stream);

@@ -69,6 +69,27 @@ def test_silu_both(n):
     _close(du, torch.autograd.grad(want, ur, dh.double())[0])
 
 
+def test_gelu_of_every_value_is_what_the_tensor_library_rounds_to():
+    from mccl_b200 import _ext
+    x = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    y, want = _ext.load().gelu_forward(x), F.gelu(x, approximate="tanh")
+    ok = (y.view(torch.int16) == want.view(torch.int16)) | (y.isnan() & want.isnan())
+    assert ok.all(), x[~ok]
+    for n in (1, 7, 8, 1021, 8193):                    # a remainder that no 16-byte piece holds
+        assert torch.equal(_ext.load().gelu_forward(x[16256:16256 + n].clone()), F.gelu(x[16256:16256 + n], approximate="tanh"))
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (5, 520), (129, 1032), (2000, 4096)])
+def test_gelu_gradient_and_its_column_sums(rows, d):
+    from mccl_b200 import _ext
+    x, dy = _bf(rows, d, std=2.0), _bf(rows, d)
+    dx, db = _ext.load().gelu_backward(x, dy)
+    xr = x.double().requires_grad_(True)
+    want = torch.autograd.grad(F.gelu(xr, approximate="tanh"), xr, dy.double())[0]
+    _close(dx, want)
+    _close(db, dx.double().sum(0))
+
+
 @pytest.mark.parametrize("vocab,d,tokens", [(5, 8, (1, 1)), (3, 64, (2, 300)), (1000, 1024, (4, 129)), (50, 2056, (1, 65)), (70, 4096, (3, 130))])
 @pytest.mark.parametrize("with_pos", [True, False])
 def test_embedding_adds_repeated_tokens(vocab, d, tokens, with_pos):

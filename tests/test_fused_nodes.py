@@ -92,6 +92,32 @@ def test_fused_route_is_as_close_to_64_bits_as_the_plain_one(make, kw):
 
 
 @gpu
+@pytest.mark.parametrize("frozen", [(), ("k.weight",), ("q.bias", "v.weight")])
+@pytest.mark.parametrize("d", [128, 1056])
+def test_adjacent_projections_are_one_product(d, frozen):
+    """In a bucket the three projections' weights lie next to each other; the gradients are those of the separate parameters."""
+    from mccl_b200.parallel.ddp import DistributedDataParallel
+    idx, tgt = _batch()
+
+    def make():
+        m = _gpt2(d)
+        for n, p in m.named_parameters():
+            p.requires_grad_(not n.endswith(frozen) if frozen else True)
+        return m
+
+    apart, packed = make(), make()
+    apart(idx, tgt).backward()
+    DistributedDataParallel(packed, None)(idx, tgt).backward()
+    want = _plain(make()).double()
+    want(idx, tgt).backward()
+    for (n, a), b, w in zip(apart.named_parameters(), packed.parameters(), want.parameters()):
+        assert (b.grad is None) == (not a.requires_grad), n
+        if a.requires_grad and not n.endswith("k.bias"):        # the gradient of a key's bias is zero but for rounding
+            ea, eb = ((t.grad.double() - w.grad).norm() / w.grad.norm() for t in (a, b))
+            assert eb <= 1.5 * ea + 2.0 ** -9, (n, ea.item(), eb.item())
+
+
+@gpu
 @pytest.mark.parametrize("make", [_gpt2, _llama])
 def test_hooks_and_replaced_parts_are_called(make):
     idx, tgt = _batch()
