@@ -17,7 +17,10 @@ namespace {
 
 using namespace mccl;
 
-constexpr int kCeThreads = 512;
+// Small CTAs: eight of them share an SM, so that the ends of rows (a last turn of the walk that few threads take, the fold of
+// the CTA's sums) lie beside other rows' loads.  512 threads / 256, rows x columns: 8192 x 50257 forward 172 / 151 us, backward
+// 285 / 258 us (6.4 TB/s); 16384 x 1000 forward 96 / 47 us, backward 94 / 41 us.
+constexpr int kCeThreads = 256;
 constexpr int kCeUnroll = 4;                   // 16-byte pieces in flight per thread: with one, the row's loads wait for each other
 constexpr int64_t kIgnored = -100;             // the target value torch's cross-entropy leaves out
 constexpr float kLog2e = 1.4426950408889634f;
@@ -36,7 +39,7 @@ __device__ __forceinline__ void unpack(const uint4& q, float* f) {
 }
 // Eight values at once: one comparison with the running maximum and, in the common case that it stands, eight fused
 // multiply-adds and exponentials with no branch between them.  (One value at a time, every value waits for a branch: the
-// forward pass took 217 us on 8192 x 50257, 3.8 TB/s; this form takes 163 us, 5.0 TB/s.)
+// forward pass took 217 us on 8192 x 50257, 3.8 TB/s; this form took 163 us.)
 __device__ __forceinline__ void push8(MaxSum& a, const uint4& q) {
   float f[8];
   unpack(q, f);
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, co
   if (inverse != nullptr) *inverse = 1.f / rows;
 }
 
-// Reads and writes every logit once: 301 us on 8192 x 50304 with one piece in flight, 288 us (5.7 TB/s) with four.
+// Reads and writes every logit once: 301 us on 8192 x 50304 with one piece in flight, 288 us with four (CTAs of 512).
 // blockIdx.y: which slice of the row (one unless there are few rows).  The last rows come first: they are what the forward
 // pass, or the projection, left in L2.
 __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* logits, int64_t ld, int vocab, int width,
@@ -200,10 +203,11 @@ __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* lo
   }
 }
 
-// CTAs per row: with fewer rows than SMs a row is shared by up to eight, as long as each keeps a tile of it.
+// CTAs per row: few rows are shared by up to eight CTAs each, as long as there are no more than six CTAs an SM and each keeps
+// 4096 elements (two turns of its loads).
 int ceSplit(int64_t rows, int n) {
   int r = 1;
-  while (r < 8 && rows * r * 2 <= 148 && n / (r * 2) >= kCeThreads * 8) r *= 2;
+  while (r < 8 && rows * r * 2 <= 148 * 6 && n / (r * 2) >= 4096) r *= 2;
   return r;
 }
 
