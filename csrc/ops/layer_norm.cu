@@ -158,14 +158,37 @@ struct LnBwdArgs {
   colred::Out out;                             // dgamma, dbeta, column sums of dx
 };
 
-// Rows are walked by a fixed number of CTAs (two per SM) so that a lane can keep its columns' sums in registers; the
-// vectors of the next row are loaded before the current one is worked on.  Two vectors per lane bound the registers: 16
+// Sums of (a0, b0) and of (a1, b1) over the W warps of a group: four values through six exchanges, because every exchange
+// also halves what a lane still carries, and one barrier.  `slot` as above, four floats a warp.
+template <int W>
+__device__ __forceinline__ float4 groupSum2(float a0, float b0, float a1, float b1, float4* slot, int group, int warpInGroup) {
+  const int lane = threadIdx.x & 31;
+  const bool second = lane & 16, isB = lane & 8;
+  float a = (second ? a1 : a0) + __shfl_xor_sync(0xffffffffu, second ? a0 : a1, 16);
+  float b = (second ? b1 : b0) + __shfl_xor_sync(0xffffffffu, second ? b0 : b1, 16);
+  float v = (isB ? b : a) + __shfl_xor_sync(0xffffffffu, isB ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((lane & 7) == 0) reinterpret_cast<float*>(slot + group * W + warpInGroup)[lane >> 3] = v;
+  asm volatile("bar.sync %0, %1;" :: "r"(1 + group), "n"(W * 32) : "memory");
+  float4 t = slot[group * W];
+#pragma unroll
+  for (int w = 1; w < W; ++w) { const float4 u = slot[group * W + w]; t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+  return t;
+}
+
+// Rows are walked by a fixed number of CTAs (two or three per SM) so that a lane can keep its columns' sums in registers; the
+// vectors of the next rows are loaded before the current ones are worked on.  Two vectors per lane bound the registers: 16
 // columns x (three sums + gamma) + two rows of x, dy and dres.
-template <int W, int VPL, bool RMS, bool RES, int PARTS>
-__global__ void __launch_bounds__(kLnThreads, VPL == 1 && PARTS == 1 ? 3 : 2) lnBackwardKernel(const __grid_constant__ LnBwdArgs a) {
+// R rows at a time.  What bounds the kernel is the chain of a row (the reductions' exchanges and the barrier between two
+// passes over registers), so where a row is spread over warps and the registers suffice a group takes two rows and goes
+// through the chain once for both (8192 x 1024 with dres: 21.4 us one row at a time, 18.4 us, 3.6 TB/s).  (A pipeline of four rows in shared memory by cp.async did not help: 25.9 us.)
+template <int W, int VPL, bool RMS, bool RES, int PARTS, int R>
+__global__ void __launch_bounds__(kLnThreads, VPL == 1 && PARTS == 1 && R == 1 ? 3 : 2) lnBackwardKernel(const __grid_constant__ LnBwdArgs a) {
+  static_assert(R == 1 || (R == 2 && W > 1), "two rows at a time need a group of warps");
   constexpr int G = kLnWarps / W, T = W * 32;
   extern __shared__ float cols[];
-  __shared__ float2 slots[2][kLnWarps];
+  __shared__ float4 slots[2][kLnWarps];
   const int group = threadIdx.x / T, t = threadIdx.x % T, vecs = a.D / 8;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   const bool third = RES && !RMS && a.out.segments == 3;
@@ -177,69 +200,97 @@ __global__ void __launch_bounds__(kLnThreads, VPL == 1 && PARTS == 1 ? 3 : 2) ln
     for (int k = 0; k < 8; ++k) dg[8 * j + k] = db[8 * j + k] = dc[8 * j + k] = 0.f;
   }
   const float invD = 1.0f / (float)a.D;
-  const int64_t step = (int64_t)gridDim.x * G;
-  int64_t row = (int64_t)blockIdx.x * G + group;
-  uint4 xq[VPL], dq[VPL], rq[VPL], d2[VPL], d3[VPL];
-  float mu = 0.f, rs = 0.f;
-  auto load = [&](int64_t r) {
+  const int64_t step = (int64_t)gridDim.x * (G * R);
+  int64_t row = ((int64_t)blockIdx.x * G + group) * R;
+  uint4 xq[R][VPL], dq[R][VPL], rq[R][VPL], d2[R][VPL], d3[R][VPL];
+  float mu[R] = {}, rs[R] = {};
+  auto load = [&](int64_t first) {
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-      const int i = t + T * j;
-      const bool in = r < a.rows && i < vecs;
-      xq[j] = in ? a.x[r * vecs + i] : zero;
-      dq[j] = in ? a.dy[r * vecs + i] : zero;
-      if (RES) rq[j] = in ? a.dres[r * vecs + i] : zero;
-      if (PARTS == 3) {
-        d2[j] = in && a.dy2 != nullptr ? a.dy2[r * vecs + i] : zero;
-        d3[j] = in && a.dy3 != nullptr ? a.dy3[r * vecs + i] : zero;
+    for (int q = 0; q < R; ++q) {
+      const int64_t r = first + q;
+#pragma unroll
+      for (int j = 0; j < VPL; ++j) {
+        const int i = t + T * j;
+        const bool in = r < a.rows && i < vecs;
+        xq[q][j] = in ? a.x[r * vecs + i] : zero;
+        dq[q][j] = in ? a.dy[r * vecs + i] : zero;
+        if (RES) rq[q][j] = in ? a.dres[r * vecs + i] : zero;
+        if (PARTS == 3) {
+          d2[q][j] = in && a.dy2 != nullptr ? a.dy2[r * vecs + i] : zero;
+          d3[q][j] = in && a.dy3 != nullptr ? a.dy3[r * vecs + i] : zero;
+        }
       }
+      const bool live = R == 1 || r < a.rows;                          // past the end everything is zero
+      if (r < a.rows) { if (!RMS) mu[q] = a.mean[r]; rs[q] = a.rstd[r]; }
+      if (!live) mu[q] = rs[q] = 0.f;
     }
-    if (r < a.rows) { if (!RMS) mu = a.mean[r]; rs = a.rstd[r]; }
   };
   load(row);
   for (int par = 0; row < a.rows; row += step, par ^= 1) {
-    uint4 xc[VPL], dc4[VPL], rc[VPL];
+    uint4 xc[R][VPL], dc4[R][VPL], rc[R][VPL];
+    float m[R], r[R], s1[R], s2[R];
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) { xc[j] = xq[j]; dc4[j] = PARTS == 3 ? add8(add8(dq[j], d2[j]), d3[j]) : dq[j]; if (RES) rc[j] = rq[j]; }
-    const float m = mu, r = rs;
+    for (int q = 0; q < R; ++q) {
+#pragma unroll
+      for (int j = 0; j < VPL; ++j) {
+        xc[q][j] = xq[q][j];
+        dc4[q][j] = PARTS == 3 ? add8(add8(dq[q][j], d2[q][j]), d3[q][j]) : dq[q][j];
+        if (RES) rc[q][j] = rq[q][j];
+      }
+      m[q] = mu[q];
+      r[q] = rs[q];
+    }
     load(row + step);
-    float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-      float xf[8], df[8];
-      unpack(xc[j], xf);
-      unpack(dc4[j], df);
+    for (int q = 0; q < R; ++q) {
+      s1[q] = s2[q] = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float xh = (xf[k] - m) * r, gd = df[k] * g[8 * j + k];
-        s1 += gd; s2 += gd * xh;
-        dg[8 * j + k] += df[k] * (RMS ? __bfloat162float(__float2bfloat16_rn(xh)) : xh);
-        if (!RMS) db[8 * j + k] += df[k];
+      for (int j = 0; j < VPL; ++j) {
+        float xf[8], df[8];
+        unpack(xc[q][j], xf);
+        unpack(dc4[q][j], df);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float xh = (xf[k] - m[q]) * r[q], gd = df[k] * g[8 * j + k];
+          s1[q] += gd; s2[q] += gd * xh;
+          dg[8 * j + k] += df[k] * (RMS ? __bfloat162float(__float2bfloat16_rn(xh)) : xh);       // rows past the end: df is zero
+          if (!RMS) db[8 * j + k] += df[k];
+        }
       }
     }
-    float2 sums = groupSum<W>(s1, s2, slots[par], group, t >> 5);
-    s1 = RMS ? 0.f : sums.x * invD;
-    s2 = sums.y * invD;
+    if (R == 2) {
+      const float4 sums = groupSum2<W>(s1[0], s2[0], s1[R - 1], s2[R - 1], slots[par], group, t >> 5);
+      s1[0] = sums.x; s2[0] = sums.y; s1[R - 1] = sums.z; s2[R - 1] = sums.w;
+    } else {
+      const float2 sums = groupSum<W>(s1[0], s2[0], reinterpret_cast<float2*>(slots[par]), group, t >> 5);
+      s1[0] = sums.x; s2[0] = sums.y;
+    }
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-      if (t + T * j >= vecs) continue;
-      float xf[8], df[8], o[8];
-      unpack(xc[j], xf);
-      unpack(dc4[j], df);
-      if (RES) unpack(rc[j], o);
+    for (int q = 0; q < R; ++q) {
+      if (R > 1 && row + q >= a.rows) continue;
+      s1[q] = RMS ? 0.f : s1[q] * invD;
+      s2[q] *= invD;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float xh = (xf[k] - m) * r, gd = df[k] * g[8 * j + k];
-        const float dn = r * (gd - s1 - xh * s2);
-        o[k] = RES ? __bfloat162float(__float2bfloat16_rn(dn)) + o[k] : dn;
+      for (int j = 0; j < VPL; ++j) {
+        if (t + T * j >= vecs) continue;
+        float xf[8], df[8], o[8];
+        unpack(xc[q][j], xf);
+        unpack(dc4[q][j], df);
+        if (RES) unpack(rc[q][j], o);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float xh = (xf[k] - m[q]) * r[q], gd = df[k] * g[8 * j + k];
+          const float dn = r[q] * (gd - s1[q] - xh * s2[q]);
+          o[k] = RES ? __bfloat162float(__float2bfloat16_rn(dn)) + o[k] : dn;
+        }
+        const uint4 out = pack(o);
+        if (third) {
+          unpack(out, o);                      // the sum over what is stored, as a separate reduction would read it
+#pragma unroll
+          for (int k = 0; k < 8; ++k) dc[8 * j + k] += o[k];
+        }
+        a.dx[(row + q) * vecs + t + T * j] = out;
       }
-      const uint4 q = pack(o);
-      if (third) {
-        unpack(q, o);                          // the sum over what is stored, as a separate reduction would read it
-#pragma unroll
-        for (int k = 0; k < 8; ++k) dc[8 * j + k] += o[k];
-      }
-      a.dx[row * vecs + t + T * j] = q;
     }
   }
   const int C = a.out.segments * a.D;
@@ -278,21 +329,21 @@ cudaError_t fwdAny(const LnFwdArgs& a, cudaStream_t s) {
   return fwd<4, 4, RMS>(a, s);
 }
 
-template <int W, int VPL, bool RMS, bool RES, int PARTS = 1>
+template <int W, int VPL, bool RMS, bool RES, int PARTS = 1, int R = 1>
 cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
   constexpr int G = kLnWarps / W;
   static bool opted[64] = {false};             // 48 KB of column sums and the row slots: past the default limit
   int dev = 0;
   cudaGetDevice(&dev);
   if (!opted[dev & 63]) {
-    const cudaError_t e = cudaFuncSetAttribute(lnBackwardKernel<W, VPL, RMS, RES, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
+    const cudaError_t e = cudaFuncSetAttribute(lnBackwardKernel<W, VPL, RMS, RES, PARTS, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
     if (e != cudaSuccess) return e;
     opted[dev & 63] = true;
   }
   int cluster;
-  const int grid = colred::grid((a.rows + G * 4 - 1) / (G * 4), VPL == 1 && PARTS == 1 ? 3 : 2, &cluster);      // four rows per group before more CTAs pay
+  const int grid = colred::grid((a.rows + G * R * 4 - 1) / (G * R * 4), VPL == 1 && PARTS == 1 && R == 1 ? 3 : 2, &cluster);      // four rows per group before more CTAs pay
   const int C = a.out.segments * a.D;
-  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES, PARTS>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
+  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES, PARTS, R>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
   return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, C, a.out, s);
 }
 
@@ -301,9 +352,10 @@ cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
 template <bool RMS, int PARTS>
 cudaError_t bwdRes(const LnBwdArgs& a, cudaStream_t s) {
   if (a.D <= 256) return bwdLaunch<1, 1, RMS, true, PARTS>(a, s);
-  if (a.D <= 512) return bwdLaunch<2, 1, RMS, true, PARTS>(a, s);
-  if (a.D <= 1024) return bwdLaunch<4, 1, RMS, true, PARTS>(a, s);
-  if (a.D <= 2048) return bwdLaunch<8, 1, RMS, true, PARTS>(a, s);
+  constexpr int R = PARTS == 1 ? 2 : 1;        // five rows of operands leave no registers for a second one
+  if (a.D <= 512) return bwdLaunch<2, 1, RMS, true, PARTS, R>(a, s);
+  if (a.D <= 1024) return bwdLaunch<4, 1, RMS, true, PARTS, R>(a, s);
+  if (a.D <= 2048) return bwdLaunch<8, 1, RMS, true, PARTS, R>(a, s);
   return bwdLaunch<8, 2, RMS, true, PARTS>(a, s);
 }
 template <bool RMS>
