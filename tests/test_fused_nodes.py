@@ -76,7 +76,7 @@ def _reference(model, idx, tgt):
 
 
 @gpu
-@pytest.mark.parametrize("make,kw", [(_gpt2, {"d": 128}), (_gpt2, {"d": 384}), (_gpt2, {"d": 1056}), (_llama, {"d": 128}), (_llama, {"d": 64, "heads": 4}),
+@pytest.mark.parametrize("make,kw", [(_gpt2, {"d": 128}), (_gpt2, {"d": 384}), (_gpt2, {"d": 768}), (_gpt2, {"d": 1056}), (_llama, {"d": 128}), (_llama, {"d": 64, "heads": 4}), (_llama, {"d": 768, "heads": 6}),
                                      (_llama, {"d": 1152, "heads": 9})])
 def test_fused_route_is_as_close_to_64_bits_as_the_plain_one(make, kw):
     idx, tgt = _batch()
