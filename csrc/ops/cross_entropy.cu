@@ -1,5 +1,5 @@
 // Fused softmax cross-entropy over bf16 logits for the language-model head.
-//   forward : one CTA per row (several when rows are few), one pass (online max / sum-of-exponentials in fp32) -> per-row loss and
+//   forward : one CTA per row, one pass (online max / sum-of-exponentials in fp32) -> per-row loss and
 //             log-sum-exp; the 8192 x 50304 logits are read once and never widened to an fp32 tensor.
 //   backward: dlogits = (exp(logit - lse) - [j == target]) * grad / rows, written in bf16 over the logits
 //             (they are not needed afterwards); padding columns beyond the vocabulary get zero.
@@ -9,7 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "col_reduce.cuh"
+#include "f32x2.cuh"
 #include "mccl.h"
 #include "mccl_ops.h"
 
@@ -17,43 +17,53 @@ namespace {
 
 using namespace mccl;
 
-// Small CTAs: eight of them share an SM, so that the ends of rows (a last turn of the walk that few threads take, the fold of
-// the CTA's sums) lie beside other rows' loads.  512 threads / 256, rows x columns: 8192 x 50257 forward 172 / 151 us, backward
-// 285 / 258 us (6.4 TB/s); 16384 x 1000 forward 96 / 47 us, backward 94 / 41 us.
+// Small CTAs: several of them share an SM, so that the ends of rows (a last turn of the walk that few threads take, the fold of
+// the CTA's sums) lie beside other rows' loads.  Backward with 512 threads / 256: 8192 x 50257 285 / 258 us (6.4 TB/s).
 constexpr int kCeThreads = 256;
-constexpr int kCeUnroll = 4;                   // 16-byte pieces in flight per thread: with one, the row's loads wait for each other
+constexpr int kCeUnroll = 4;                   // 16-byte pieces in flight per thread in long rows: with one, the row's loads wait for each other
 constexpr int64_t kIgnored = -100;             // the target value torch's cross-entropy leaves out
-constexpr float kLog2e = 1.4426950408889634f;
 
 struct MaxSum { float m, s; };                 // running maximum and sum of exp(x - m)
-__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLowest = -3.402823466e38f;    // a maximum of nothing: below every finite bf16 number, and minus itself zero
 __device__ __forceinline__ MaxSum combine(MaxSum a, MaxSum b) {
   const float m = fmaxf(a.m, b.m);
-  if (m == -INFINITY) return MaxSum{m, 0.f};
-  return MaxSum{m, a.s * ex2((a.m - m) * kLog2e) + b.s * ex2((b.m - m) * kLog2e)};
+  return MaxSum{m, a.s * __expf(a.m - m) + b.s * __expf(b.m - m)};
 }
 __device__ __forceinline__ void unpack(const uint4& q, float* f) {
   const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
   for (int k = 0; k < 4; ++k) { const float2 t = __bfloat1622float2(e[k]); f[2 * k] = t.x; f[2 * k + 1] = t.y; }
 }
-// Eight values at once: one comparison with the running maximum and, in the common case that it stands, eight fused
-// multiply-adds and exponentials with no branch between them.  (One value at a time, every value waits for a branch: the
-// forward pass took 217 us on 8192 x 50257, 3.8 TB/s; this form took 163 us.)
-__device__ __forceinline__ void push8(MaxSum& a, const uint4& q) {
-  float f[8];
-  unpack(q, f);
-  const float mx = fmaxf(fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])), fmaxf(fmaxf(f[4], f[5]), fmaxf(f[6], f[7])));
-  if (mx > a.m) { a.s *= ex2((a.m - mx) * kLog2e); a.m = mx; }
-  const float off = a.m == -INFINITY ? 0.f : -a.m * kLog2e;
-  float t[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) t[k] = ex2(fmaf(f[k], kLog2e, off));
-  a.s += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+// Values enter one after another: s = s exp(m - x) + 1 where x is a new maximum and s + exp(x - m) where not.  The maximum
+// is subtracted before anything is scaled: exp(x - m) as 2^(x log2e - m log2e) would save an instruction, but it rounds
+// m log2e (an error of |m| 2^-24 in every exponent) and overflows for logits near the type's lowest value, which masks are made
+// of.
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ void add(MaxSum& a, bool up, float e) { a.s = up ? __fmaf_rn(a.s, e, 1.f) : __fadd_rn(a.s, e); }
+__device__ __forceinline__ void push(MaxSum& a, float x) {
+  add(a, x > a.m, ex2(-fabsf((x - a.m) * kLog2e)));
+  a.m = fmaxf(a.m, x);
 }
-__device__ __forceinline__ void push1(MaxSum& a, float x) {
-  if (x > a.m) { a.s *= ex2((a.m - x) * kLog2e); a.m = x; }
-  if (x != -INFINITY) a.s += ex2((x - a.m) * kLog2e);
+// Eight of them.  Instructions bound the forward pass here, at eight values of nine slots each a turn (8192 x 50257: 201 us):
+// the eight maxima first, then differences and products two at a time, then the sums, predicated: 148 us, 5.6 TB/s.  (With a
+// branch for a new maximum, which some lane of a warp takes nearly always: 254 us.)
+__device__ __forceinline__ void push8(MaxSum& a, const uint4& q) {
+  float f[8], m[9], e[8];
+  unpack(q, f);
+  m[0] = a.m;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) m[k + 1] = fmaxf(m[k], f[k]);
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    float d0, d1;
+    split((f2(f[k], f[k + 1]) + f2(-m[k], -m[k + 1])) * f2(kLog2e), &d0, &d1);
+    e[k] = ex2(-fabsf(d0));
+    e[k + 1] = ex2(-fabsf(d1));
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) add(a, f[k] > m[k], e[k]);
+  a.m = m[8];
 }
 
 // The part of a row between its first and last 16-byte boundary: [head, head + 8 * vecs) of n elements.
@@ -64,31 +74,25 @@ __device__ __forceinline__ Span spanOf(const __nv_bfloat16* x, int n) {
   return Span{head, (n - head) / 8};
 }
 
-// A cluster of CTAs per row (one CTA each when there are enough rows to fill the GPU): CTA r takes every
-// clusterSize-th tile of the row, and the per-CTA (maximum, sum) pairs meet in CTA 0's shared memory.
-__global__ void __launch_bounds__(kCeThreads) ceForwardKernel(const __nv_bfloat16* logits, int64_t ld, int vocab,
+template <int U>
+__global__ void __launch_bounds__(kCeThreads, 6) ceForwardKernel(const __nv_bfloat16* logits, int64_t ld, int vocab,
                                                               const int64_t* targets, float* loss, float* lse) {
   __shared__ MaxSum warpAcc[kCeThreads / 32];
-  __shared__ MaxSum ctaAcc;
-  const uint32_t R = colred::clusterSize(), r = colred::clusterRank();
-  const int64_t row = blockIdx.x / R;
+  const int64_t row = blockIdx.x;
   const __nv_bfloat16* x = logits + row * ld;
-  MaxSum acc{-INFINITY, 0.f};
+  MaxSum acc{kLowest, 0.f};
   const Span sp = spanOf(x, vocab);
   const uint4* v = reinterpret_cast<const uint4*>(x + sp.head);
-  const int stride = (int)R * kCeThreads;
-  for (int i = (int)r * kCeThreads + threadIdx.x; i < sp.vecs; i += kCeUnroll * stride) {
-    uint4 q[kCeUnroll];
+  for (int i = threadIdx.x; i < sp.vecs; i += U * kCeThreads) {
+    uint4 q[U];
 #pragma unroll
-    for (int u = 0; u < kCeUnroll; ++u) if (i + u * stride < sp.vecs) q[u] = v[i + u * stride];
+    for (int u = 0; u < U; ++u) if (i + u * kCeThreads < sp.vecs) q[u] = v[i + u * kCeThreads];
 #pragma unroll
-    for (int u = 0; u < kCeUnroll; ++u) if (i + u * stride < sp.vecs) push8(acc, q[u]);
+    for (int u = 0; u < U; ++u) if (i + u * kCeThreads < sp.vecs) push8(acc, q[u]);
   }
-  if (r == 0) {
-    const int tail = sp.head + sp.vecs * 8;
-    if ((int)threadIdx.x < sp.head) push1(acc, __bfloat162float(x[threadIdx.x]));
-    if (tail + (int)threadIdx.x < vocab) push1(acc, __bfloat162float(x[tail + threadIdx.x]));
-  }
+  const int tail = sp.head + sp.vecs * 8;
+  if ((int)threadIdx.x < sp.head) push(acc, __bfloat162float(x[threadIdx.x]));
+  if (tail + (int)threadIdx.x < vocab) push(acc, __bfloat162float(x[tail + threadIdx.x]));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     MaxSum other{__shfl_xor_sync(0xffffffffu, acc.m, o), __shfl_xor_sync(0xffffffffu, acc.s, o)};
@@ -99,18 +103,11 @@ __global__ void __launch_bounds__(kCeThreads) ceForwardKernel(const __nv_bfloat1
   if (threadIdx.x == 0) {
     MaxSum t = warpAcc[0];
     for (int w = 1; w < kCeThreads / 32; ++w) t = combine(t, warpAcc[w]);
-    ctaAcc = t;
-  }
-  if (R > 1) colred::clusterSync();
-  if (r == 0 && threadIdx.x == 0) {
-    MaxSum t = ctaAcc;
-    for (uint32_t p = 1; p < R; ++p) t = combine(t, MaxSum{colred::ldPeerShared(&ctaAcc.m, p), colred::ldPeerShared(&ctaAcc.s, p)});
-    const float l = t.m + logf(t.s);
+    const float l = t.m == INFINITY ? __int_as_float(0x7fffffff) : t.m + logf(t.s);      // inf - inf in the exponent
     const int64_t tgt = targets[row];
     lse[row] = l;
     loss[row] = (tgt >= 0 && tgt < vocab) ? l - __bfloat162float(x[tgt]) : 0.f;     // out-of-range target: ignored row
   }
-  if (R > 1) colred::clusterSync();
 }
 
 // Mean over the rows' losses, in a fixed order: over all rows or, with `targets`, over those whose target is a column
@@ -152,9 +149,10 @@ __global__ void __launch_bounds__(1024) meanKernel(const float* v, int64_t n, co
   if (inverse != nullptr) *inverse = 1.f / rows;
 }
 
-// Reads and writes every logit once: 301 us on 8192 x 50304 with one piece in flight, 288 us with four (CTAs of 512).
+// Reads and writes every logit once: 8192 x 50257 307 us with one piece in flight, 259 us with four.
 // blockIdx.y: which slice of the row (one unless there are few rows).  The last rows come first: they are what the forward
 // pass, or the projection, left in L2.
+template <int U>
 __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* logits, int64_t ld, int vocab, int width,
                                                                const int64_t* targets, const float* lse, const float* gradOut,
                                                                const float* inverse, float invRows) {
@@ -165,27 +163,26 @@ __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* lo
   const bool live = tgt64 >= 0 && tgt64 < vocab;
   const int tgt = live ? (int)tgt64 : -1;
   const float scale = live ? (*gradOut) * (inverse != nullptr ? *inverse : invRows) : 0.f;
-  const float off = -l * kLog2e;
   auto one = [&](int j, float xj) -> float {
     if (j >= vocab) return 0.f;
-    return (ex2(fmaf(xj, kLog2e, off)) - (j == tgt ? 1.f : 0.f)) * scale;
+    return (__expf(xj - l) - (j == tgt ? 1.f : 0.f)) * scale;
   };
   const Span sp = spanOf(x, width);
   uint4* v = reinterpret_cast<uint4*>(x + sp.head);
   const int stride = (int)gridDim.y * kCeThreads;
-  for (int i = (int)blockIdx.y * kCeThreads + threadIdx.x; i < sp.vecs; i += kCeUnroll * stride) {
-    uint4 q[kCeUnroll];
+  for (int i = (int)blockIdx.y * kCeThreads + threadIdx.x; i < sp.vecs; i += U * stride) {
+    uint4 q[U];
 #pragma unroll
-    for (int u = 0; u < kCeUnroll; ++u) if (i + u * stride < sp.vecs) q[u] = v[i + u * stride];
+    for (int u = 0; u < U; ++u) if (i + u * stride < sp.vecs) q[u] = v[i + u * stride];
 #pragma unroll
-    for (int u = 0; u < kCeUnroll; ++u) {
+    for (int u = 0; u < U; ++u) {
       if (i + u * stride >= sp.vecs) continue;
       const int j0 = sp.head + (i + u * stride) * 8;
       float f[8];
       unpack(q[u], f);
       if (j0 + 8 <= vocab && (unsigned)(tgt - j0) >= 8u) {       // neither the target nor padding in these eight
 #pragma unroll
-        for (int k = 0; k < 8; ++k) f[k] = ex2(fmaf(f[k], kLog2e, off)) * scale;
+        for (int k = 0; k < 8; ++k) f[k] = __expf(f[k] - l) * scale;
       } else {
 #pragma unroll
         for (int k = 0; k < 8; ++k) f[k] = one(j0 + k, f[k]);
@@ -203,7 +200,11 @@ __global__ void __launch_bounds__(kCeThreads) ceBackwardKernel(__nv_bfloat16* lo
   }
 }
 
-// CTAs per row: few rows are shared by up to eight CTAs each, as long as there are no more than six CTAs an SM and each keeps
+// Rows that 256 threads walk in two turns or fewer take the form with one piece in flight: fewer registers, so more
+// rows a SM (16384 x 1000 forward 47 -> 39 us, backward 41 -> 30 us).
+bool shortRow(int n) { return n <= 2 * 8 * kCeThreads; }
+
+// CTAs per row in the backward pass: few rows are shared by up to eight CTAs each, as long as there are no more than six CTAs an SM and each keeps
 // 4096 elements (two turns of its loads).
 int ceSplit(int64_t rows, int n) {
   int r = 1;
@@ -219,9 +220,10 @@ extern "C" mcclResult_t mcclCrossEntropyForward(const void* logits, int64_t rows
   if (logits == nullptr || targets == nullptr || loss == nullptr || lse == nullptr || rows < 0 || vocab <= 0 || ld < vocab)
     return mcclInvalidArgument;
   if (rows == 0) return mcclSuccess;
-  const int split = ceSplit(rows, vocab);
-  return colred::launch(ceForwardKernel, (int)rows * split, split, kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream),
-                        static_cast<const __nv_bfloat16*>(logits), ld, vocab, targets, loss, lse) == cudaSuccess ? mcclSuccess : mcclSystemError;
+  auto* kernel = shortRow(vocab) ? ceForwardKernel<1> : ceForwardKernel<kCeUnroll>;
+  kernel<<<(unsigned)rows, kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(logits), ld, vocab,
+                                                                                   targets, loss, lse);
+  return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 
 // The same followed by the mean of the rows' losses in *mean: over all rows, or with `inverse` over the rows whose target is
@@ -243,7 +245,8 @@ extern "C" mcclResult_t mcclCrossEntropyMeanBackward(void* logits, int64_t rows,
   if (logits == nullptr || targets == nullptr || lse == nullptr || gradOut == nullptr || rows < 0 || vocab <= 0 || width < vocab ||
       ld < width) return mcclInvalidArgument;
   if (rows == 0) return mcclSuccess;
-  ceBackwardKernel<<<dim3((unsigned)rows, (unsigned)ceSplit(rows, width)), kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  auto* kernel = shortRow(width) ? ceBackwardKernel<1> : ceBackwardKernel<kCeUnroll>;
+  kernel<<<dim3((unsigned)rows, (unsigned)ceSplit(rows, width)), kCeThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       static_cast<__nv_bfloat16*>(logits), ld, vocab, width, targets, lse, gradOut, inverse, 1.0f / (float)rows);
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }

@@ -124,6 +124,31 @@ def test_cross_entropy_mean_forms(rows, vocab, width):
     _close(torch.autograd.grad(loss, logits)[0], wg)
 
 
+@pytest.mark.parametrize("fill", [torch.finfo(torch.bfloat16).min, float("-inf")])
+@pytest.mark.parametrize("rows,vocab,lo,hi", [(5, 1000, 0, 64), (3, 4096, 0, 4088), (2, 5000, 8, 4999), (700, 64, 0, 56)])
+def test_cross_entropy_of_masked_columns(rows, vocab, lo, hi, fill):
+    """Masks of the type's lowest value or of minus infinity, before, around and behind what a thread reads first."""
+    from mccl_b200.ops.loss import fused_cross_entropy
+    logits = _bf(rows, vocab, std=2.0)
+    logits[:, lo:hi] = fill
+    t = torch.randint(hi, vocab, (rows,), device="cuda")
+    lr = logits.double().requires_grad_(True)
+    want = F.cross_entropy(lr, t)
+    x = logits.clone().requires_grad_(True)
+    loss = fused_cross_entropy(x, t, vocab)
+    assert abs(loss.item() - want.item()) <= 1e-5 * max(1.0, abs(want.item()))
+    _close(torch.autograd.grad(loss, x)[0], torch.autograd.grad(want, lr)[0])
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_cross_entropy_of_a_row_without_a_maximum_is_nan(bad):
+    from mccl_b200.ops.loss import fused_cross_entropy
+    for col in (0, 7, 900):
+        logits = _bf(2, 1000)
+        logits[1, col] = bad
+        assert math.isnan(fused_cross_entropy(logits.requires_grad_(True), torch.tensor([3, 5], device="cuda")).item())
+
+
 @pytest.mark.parametrize("ignored", [0, 5, 17])
 def test_head_loss_leaves_ignored_targets_out(ignored):
     from mccl_b200 import _ext
