@@ -10,6 +10,7 @@
 #include <initializer_list>
 
 #include "col_reduce.cuh"
+#include "f32x2.cuh"
 #include "mccl.h"
 #include "mccl_ops.h"
 
@@ -35,10 +36,13 @@ __device__ __forceinline__ float rounded(float x) { return __bfloat162float(__fl
 __device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
 // The tanh-GELU is x * s with s = (1 + tanh(z)) / 2 = 1 / (1 + exp(-2 z)), z = c (x + a x^3): one exponential and one
-// reciprocal, absolute error of s a few 2^-23, and its gradient is s + 2 z' x s (1 - s).  (With tanh from an exponential and a
-// divide the gradient took twice the instructions: 8192 x 4096 with its column sums 49.4 us, now 37.1 us, 5.4 TB/s.)
+// reciprocal, absolute error of s a few 2^-23, and its gradient is s + 2 z' x s (1 - s).  Results are to the last bit what the
+// long form, with tanhf, rounds to: models are compared with runs of the separate operations, and one last bit here is a
+// percent twenty layers down.  So the short form is only a guess with a bound: where both ends of its interval round to the
+// same bf16 number that is the result, and elsewhere, about one value in a thousand, the long form decides.
 constexpr float kGeluC = 0.7978845608028654f;      // sqrt(2 / pi)
 constexpr float kGeluA = 0.044715f;
+constexpr float kGeluGradW0 = 1.6e-7f, kGeluGradW2 = 1.3e-7f;
 constexpr float kGeluE = -2.f * kGeluC * 1.4426950408889634f;      // exp(-2 z) = 2^(kGeluE (x + a x^3))
 __device__ __forceinline__ float geluGate(float x, float x2) {
   float e, s;
@@ -46,14 +50,8 @@ __device__ __forceinline__ float geluGate(float x, float x2) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.f + e));
   return s;
 }
-__device__ __forceinline__ float geluGrad(float x) {
-  const float x2 = x * x, s = geluGate(x, x2);
-  return fmaf(fmaf(-s, s, s), x * fmaf(6.f * kGeluC * kGeluA, x2, 2.f * kGeluC), s);
-}
 
-// Forward, to the last bit what 0.5 x (1 + tanhf(z)) rounds to (scores compare with recorded ones only so): the short form
-// and the long one differ by less than `w` (both within 3e-7 of 1 + tanh, products within 2^-22), so where the ends of that
-// interval round to the same bf16 number it is the result; elsewhere, about one value in a thousand, the long form decides.
+// Forward: the two forms differ by less than `w` (both within 3e-7 of 1 + tanh, products within 2^-22).
 __device__ __noinline__ float geluLong(float x) {
   const float cube = x * x * x;
   return 0.5f * x * (1.f + tanhf(kGeluC * (x + kGeluA * cube)));
@@ -70,6 +68,61 @@ __device__ __forceinline__ uint32_t gelu2(float x0, float x1) {
     a = *reinterpret_cast<uint32_t*>(&lo);
   }
   return a;
+}
+
+// Gradient of x from that of the result.  The two forms of gelu'(x) differ by less than `w` for |x| < 5.5 (at most by 2.1e-6,
+// around |x| = 5, where the long form's 1 - t^2 cancels; all bf16 numbers were compared), and beyond that the long form is 1
+// or 0.
+constexpr uint32_t kGeluFlat = 0x40b0;             // 5.5 as bf16
+__device__ __forceinline__ float geluGradLong(float x) {
+  if (!(fabsf(x) < 5.5f)) return x > 0.f ? 1.f : x < 0.f ? 0.f : x;
+  const float x2 = __fmul_rn(x, x), t = tanhf(__fmul_rn(kGeluC, __fmaf_rn(kGeluA, __fmul_rn(x2, x), x)));
+  const float dz = __fmul_rn(kGeluC, __fmaf_rn(3.f * kGeluA, x2, 1.f));
+  return __fadd_rn(__fmul_rn(0.5f, __fadd_rn(1.f, t)), __fmul_rn(__fmul_rn(__fmul_rn(0.5f, x), __fmaf_rn(-t, t, 1.f)), dz));
+}
+// The ends of the intervals of two products gelu'(x) dy, rounded.
+__device__ __forceinline__ void geluGradEnds(uint32_t xw, uint32_t dyw, uint32_t* lo, uint32_t* hi) {
+  const F2 x = f2OfBf16(xw), dy = f2OfBf16(dyw), x2 = x * x;
+  float z0, z1, s0, s1;
+  split(x * fma(f2(kGeluE * kGeluA), x2, f2(kGeluE)), &z0, &z1);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(s0) : "f"(z0));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(s1) : "f"(z1));
+  split(f2(s0, s1) + f2(1.f), &z0, &z1);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s0) : "f"(z0));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s1) : "f"(z1));
+  const F2 s = f2(s0, s1), g = fma(fma(s * f2(-1.f), s, s), x * fma(f2(6.f * kGeluC * kGeluA), x2, f2(2.f * kGeluC)), s);
+  const F2 w = fma(f2(kGeluGradW2), x2, f2(kGeluGradW0));
+  float a, b;
+  split(dy * fma(w, f2(-1.f), g), &a, &b);
+  __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
+  *lo = *reinterpret_cast<uint32_t*>(&r);
+  split(dy * (g + w), &a, &b);
+  r = __floats2bfloat162_rn(a, b);
+  *hi = *reinterpret_cast<uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t word(const uint4& q, int i) { return i & 2 ? (i & 1 ? q.w : q.z) : (i & 1 ? q.y : q.x); }
+__device__ __forceinline__ float half(uint32_t w, int odd) { return __uint_as_float(odd ? w & 0xffff0000u : w << 16); }
+// Eight gradients of x from eight of the result.
+__device__ __forceinline__ uint4 geluGrad8(const uint4& x, const uint4& dy) {
+  uint32_t o[4], open = 0;                                            // open: a bit for each that the long form decides
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t xw = word(x, j);
+    uint32_t hi;
+    geluGradEnds(xw, word(dy, j), &o[j], &hi);
+    const uint32_t diff = o[j] ^ hi, flat = (xw & 0x7fff7fffu) + (0x8000u - kGeluFlat) * 0x10001u;     // bits 15 and 31: |x| >= 5.5 or NaN
+    open |= (diff & 0xffffu ? 1u << (2 * j) : 0u) | (diff >> 16 ? 2u << (2 * j) : 0u);
+    open |= (flat >> (15 - 2 * j) & 1u << (2 * j)) | (flat >> (30 - 2 * j) & 2u << (2 * j));
+  }
+  while (open != 0) {
+    const int k = __ffs(open) - 1, j = k >> 1, odd = k & 1;
+    open &= open - 1;
+    const __nv_bfloat16 r = __float2bfloat16_rn(half(word(dy, j), odd) * geluGradLong(half(word(x, j), odd)));
+    const uint32_t bits = __bfloat16_as_ushort(r);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) if (i == j) o[i] = odd ? (o[i] & 0xffffu) | bits << 16 : (o[i] & 0xffff0000u) | bits;
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // An operation maps IN input values to OUT output values.
@@ -207,34 +260,41 @@ __global__ void __launch_bounds__(kActThreads, 3) colSumKernel(const __grid_cons
   __shared__ float red[kRowGroups][kStripCols];
   const int tv = threadIdx.x % kStripVecs, g = threadIdx.x / kStripVecs, vecs = a.D / 8;
   const int v = blockIdx.x * kStripVecs + tv, seg = blockIdx.z;
-  constexpr int U = 4;                         // rows in flight per thread
+  // Rows in flight per thread.  The GELU's arithmetic takes as long as its loads, so there the next rows are on their way
+  // meanwhile.
+  constexpr int U = GELU ? 2 : 4;
   float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (v < vecs) {
     const uint4* x = a.x[seg];
     const int64_t step = (int64_t)gridDim.y * kRowGroups;
-    for (int64_t r0 = (int64_t)blockIdx.y * kRowGroups + g; r0 < a.rows; r0 += U * step) {
-      uint4 q[U], p[U];
+    uint4 q[U], p[U], qn[U], pn[U];
+    auto load = [&](int64_t first, uint4* to, uint4* pre) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int64_t r = r0 + u * step;
-        if (r < a.rows) { q[u] = x[r * a.ld + v]; if (GELU) p[u] = a.pre[r * a.ld + v]; }
+        const int64_t r = first + u * step;
+        if (r < a.rows) { to[u] = x[r * a.ld + v]; if (GELU) pre[u] = a.pre[r * a.ld + v]; }
+      }
+    };
+    int64_t r0 = (int64_t)blockIdx.y * kRowGroups + g;
+    if (GELU) load(r0, qn, pn);
+    for (; r0 < a.rows; r0 += U * step) {
+      if (GELU) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) { q[u] = qn[u]; p[u] = pn[u]; }
+        load(r0 + U * step, qn, pn);
+      } else {
+        load(r0, q, p);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int64_t r = r0 + u * step;
         if (r >= a.rows) continue;
+        uint4 o = q[u];
+        if (GELU) o = geluGrad8(p[u], q[u]);
+        if (GELU) a.dx[r * a.ldx + v] = o;
+        if (MODE == COL_PACK) a.dx[r * a.ldx + (int64_t)seg * vecs + v] = o;
         float f[8];
-        unpack(q[u], f);
-        if (MODE == COL_PACK) a.dx[r * a.ldx + (int64_t)seg * vecs + v] = q[u];
-        if (GELU) {
-          float z[8];
-          unpack(p[u], z);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) f[k] *= geluGrad(z[k]);
-          const uint4 o = pack(f);
-          a.dx[r * a.ldx + v] = o;
-          unpack(o, f);
-        }
+        unpack(o, f);
 #pragma unroll
         for (int k = 0; k < 8; ++k) sum[k] += f[k];
       }

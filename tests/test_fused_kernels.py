@@ -90,6 +90,19 @@ def test_gelu_gradient_and_its_column_sums(rows, d):
     _close(db, dx.double().sum(0))
 
 
+def test_gelu_gradient_of_every_value_is_what_the_tensor_library_rounds_to():
+    from mccl_b200 import _ext
+    x = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    for scale in (1.0, 1e-3, 30.0):
+        dy = _bf(65536, std=scale)
+        dx, _ = _ext.load().gelu_backward(x.view(64, 1024), dy.view(64, 1024))
+        want = torch.ops.aten.gelu_backward(dy, x, approximate="tanh")
+        ok = (dx.view(-1) == want) | (dx.view(-1).isnan() & x.isnan())
+        far = x.abs() >= 2.0 ** 63                     # x^2 overflows in the tensor library's form; here the slope is 1 or 0
+        assert ok[~far].all(), x[~far & ~ok]
+        assert torch.equal(dx.view(-1)[far], torch.where(x > 0, dy, torch.copysign(torch.zeros_like(dy), dy))[far])
+
+
 @pytest.mark.parametrize("vocab,d,tokens", [(5, 8, (1, 1)), (3, 64, (2, 300)), (1000, 1024, (4, 129)), (50, 2056, (1, 65)), (70, 4096, (3, 130))])
 @pytest.mark.parametrize("with_pos", [True, False])
 def test_embedding_adds_repeated_tokens(vocab, d, tokens, with_pos):
