@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kEmbThreads) tableGradKernel(const int64_t* id
     float f[8];
     unpack(grad[id * vecs + v], f);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] += acc[j][e];
+    for (int e = 0; e < 8; ++e) f[e] += __bfloat162float(__float2bfloat16_rn(acc[j][e]));      // rounded as a gradient of its own is
     grad[id * vecs + v] = pack(f);
   }
 }

@@ -3,7 +3,8 @@
 //   forward : mean / rstd by warp shuffles, y = (x - mean) * rstd * gamma + beta, mean and rstd saved in fp32.  With
 //             `delta` the row is x + delta, rounded to bf16 and written out too: the residual add of a pre-norm block and
 //             the norm behind it in one pass over memory.
-//   backward: dx per row from two reductions; every lane also accumulates dgamma / dbeta of its columns over the rows its
+//   backward: (rows of 256, 512 and 1024 elements of a LayerNorm have a kernel of their own, lnRowsBackwardKernel)
+//             dx per row from two reductions; every lane also accumulates dgamma / dbeta of its columns over the rows its
 //             group walks (col_reduce.cuh adds them up).  With `dres` the gradient that reaches the row past the norm (the
 //             residual branch) is added (to the norm's gradient as a separate norm would have stored it), and the gradient
 //             of y may come in up to three parts (one per projection that read y), added up here.  The column sums of the total can be had as well: the bias gradient of the
@@ -67,6 +68,12 @@ __device__ __forceinline__ uint4 add8(const uint4& a, const uint4& b) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) x[k] += y[k];
   return pack(x);
+}
+
+// The arithmetic of a LayerNorm's gradient, its roundings spelled out: every form of the kernel gives the same bits.
+__device__ __forceinline__ float normalised(float x, float mean, float rstd) { return __fmul_rn(__fsub_rn(x, mean), rstd); }
+__device__ __forceinline__ float normGradient(float dy, float gamma, float xh, const float4& stats) {
+  return __fmul_rn(stats.y, __fmaf_rn(-xh, stats.w, __fsub_rn(__fmul_rn(dy, gamma), stats.z)));
 }
 
 struct LnFwdArgs {
@@ -309,6 +316,183 @@ __global__ void __launch_bounds__(kLnThreads, VPL == 1 && PARTS == 1 && R == 1 ?
   colred::finish(cols, G, C, a.partial, a.out);
 }
 
+// ---- LayerNorm backward for rows of 256, 512 and 1024 elements -----------------------------------------------------
+// A batch of eight rows at a time.  A row's two sums need one order whatever else the kernel does (models are compared with
+// runs of the separate operations, and one last bit here is a percent twenty layers down), so each warp takes one row of the
+// batch for them: 32 lanes, VPL vectors each, one butterfly.  For the column sums that split is the wrong one (3 x 8 x VPL
+// accumulators a lane), so the rows pass through shared memory and a thread then takes one vector of columns of VPL rows:
+// 24 accumulators, and the gradients leave in whole rows.  One barrier a batch, because two copies of the rows alternate.
+// 8192 x 1024 from cold caches: 23.6 us, 27.6 us with dres, 35.8 us with three parts, as long as the form below that spreads
+// a row over four warps (and 29.7 us for one warp a row without the exchange, plain).
+template <int VPL, bool RES, int PARTS>
+__global__ void __launch_bounds__(kLnThreads, 2) lnRowsBackwardKernel(const __grid_constant__ LnBwdArgs a) {
+  constexpr int VECS = VPL * 32, D = VPL * 256;
+  extern __shared__ __align__(16) float cols[];
+  uint4* sx = reinterpret_cast<uint4*>(cols);                          // [2][kLnWarps][VECS] rows of x, then as many of dy
+  uint4* sd = sx + 2 * kLnWarps * VECS;
+  __shared__ float4 stats[2][kLnWarps];                                // mean, rstd and the two sums of a row
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = threadIdx.x % VECS, slot0 = threadIdx.x / VECS * VPL;
+  const bool third = RES && a.out.segments == 3;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  constexpr bool AHEAD = VPL * PARTS < 12;                             // the next batch's rows on their way: not with 24 vectors
+  float g[8], dg[8], db[8], dc[8];
+  unpack(a.gamma[c], g);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) dg[k] = db[k] = dc[k] = 0.f;
+  uint4 xq[VPL], dq[VPL], d2[VPL], d3[VPL];
+  float mu = 0.f, rs = 0.f;
+  auto load = [&](int64_t row) {
+    const bool in = row < a.rows;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      const int64_t i = row * VECS + lane + 32 * j;
+      xq[j] = in ? a.x[i] : zero;
+      dq[j] = in ? a.dy[i] : zero;
+      if (PARTS == 3) { d2[j] = in ? a.dy2[i] : zero; d3[j] = in ? a.dy3[i] : zero; }
+    }
+    if (in) { mu = a.mean[row]; rs = a.rstd[row]; }
+  };
+  const int64_t step = (int64_t)gridDim.x * kLnWarps;
+  int64_t first = (int64_t)blockIdx.x * kLnWarps;
+  if (AHEAD) load(first + warp);
+  for (int par = 0; first < a.rows; first += step, par ^= 1) {
+    if (!AHEAD) load(first + warp);
+    float s1 = 0.f, s2 = 0.f;
+    const int at = (par * kLnWarps + warp) * VECS + lane;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      float xf[8], df[8], gf[8];
+      const uint4 dy = PARTS == 3 ? add8(add8(dq[j], d2[j]), d3[j]) : dq[j];
+      sx[at + 32 * j] = xq[j];
+      sd[at + 32 * j] = dy;
+      unpack(xq[j], xf);
+      unpack(dy, df);
+      unpack(a.gamma[lane + 32 * j], gf);                              // from L1: sixteen registers a lane otherwise
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float gd = __fmul_rn(df[k], gf[k]);
+        s1 = __fadd_rn(s1, gd);
+        s2 = __fmaf_rn(gd, normalised(xf[k], mu, rs), s2);
+      }
+    }
+    s1 = warpSum(s1) * (1.0f / D);
+    s2 = warpSum(s2) * (1.0f / D);
+    if (lane == 0) stats[par][warp] = make_float4(mu, rs, s1, s2);
+    uint4 rq[VPL];
+    if (RES) {
+#pragma unroll
+      for (int q = 0; q < VPL; ++q) rq[q] = first + slot0 + q < a.rows ? a.dres[(first + slot0 + q) * VECS + c] : zero;
+    }
+    if (AHEAD) load(first + step + warp);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < VPL; ++q) {
+      const int slot = slot0 + q;
+      if (first + slot >= a.rows) break;
+      const float4 st = stats[par][slot];
+      float xf[8], df[8], o[8];
+      unpack(sx[(par * kLnWarps + slot) * VECS + c], xf);
+      unpack(sd[(par * kLnWarps + slot) * VECS + c], df);
+      if (RES) unpack(rq[q], o);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float xh = normalised(xf[k], st.x, st.y);
+        const float dn = normGradient(df[k], g[k], xh, st);
+        dg[k] += df[k] * xh;
+        db[k] += df[k];
+        o[k] = RES ? __bfloat162float(__float2bfloat16_rn(dn)) + o[k] : dn;
+      }
+      const uint4 out = pack(o);
+      if (third) {
+        unpack(out, o);                      // the sum over what is stored, as a separate reduction would read it
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dc[k] += o[k];
+      }
+      a.dx[(first + slot) * VECS + c] = out;
+    }
+  }
+  __syncthreads();                           // the rows' memory now takes the column sums
+  float* mine = cols + threadIdx.x / VECS * (a.out.segments * D) + c * 8;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    mine[k] = dg[k];
+    mine[D + k] = db[k];
+    if (third) mine[2 * D + k] = dc[k];
+  }
+  colred::finish(cols, kLnWarps / VPL, a.out.segments * D, a.partial, a.out);
+}
+
+// ---- what is left of a LayerNorm's backward pass when the gradient through it is there (dn) -------------------------------
+// dx = dn + dres and the column sums: dgamma, dbeta and those of dx.  One pass, a strip of 64 vectors of columns per CTA, four
+// groups of 64 threads taking every fourth row, two rows in flight each.
+constexpr int kTailVecs = 64, kTailGroups = kLnThreads / kTailVecs;
+
+struct LnTailArgs {
+  const uint4 *x, *dy, *dn, *dres;             // dres: may be null
+  const float *mean, *rstd;
+  uint4* dx;                                   // written where dres is given
+  float* partial;
+  int64_t rows;
+  int D;
+  colred::Out out;                             // dgamma, dbeta, column sums of dx
+};
+
+template <bool RES>
+__global__ void __launch_bounds__(kLnThreads, 2) lnTailKernel(const __grid_constant__ LnTailArgs a) {
+  __shared__ float red[colred::kMaxSegments][kTailGroups][kTailVecs * 8];
+  const int tv = threadIdx.x % kTailVecs, group = threadIdx.x / kTailVecs, vecs = a.D / 8, v = blockIdx.x * kTailVecs + tv;
+  float sum[colred::kMaxSegments][8] = {};
+  if (v < vecs) {
+    const int64_t step = (int64_t)gridDim.y * kTailGroups;
+    for (int64_t r0 = (int64_t)blockIdx.y * kTailGroups + group; r0 < a.rows; r0 += 2 * step) {
+      uint4 xq[2], dq[2], nq[2], rq[2];
+      float mu[2], rs[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int64_t r = r0 + u * step, i = r * vecs + v;
+        if (r >= a.rows) continue;
+        xq[u] = a.x[i];
+        dq[u] = a.dy[i];
+        nq[u] = a.dn[i];
+        if (RES) rq[u] = a.dres[i];
+        mu[u] = a.mean[r];
+        rs[u] = a.rstd[r];
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int64_t r = r0 + u * step;
+        if (r >= a.rows) continue;
+        float xf[8], df[8], o[8];
+        unpack(xq[u], xf);
+        unpack(dq[u], df);
+        const uint4 dx = RES ? add8(nq[u], rq[u]) : nq[u];
+        unpack(dx, o);
+        if (RES) a.dx[r * vecs + v] = dx;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          sum[0][k] += df[k] * normalised(xf[k], mu[u], rs[u]);
+          sum[1][k] += df[k];
+          sum[2][k] += o[k];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < colred::kMaxSegments; ++s)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) red[s][group][tv + kTailVecs * k] = sum[s][k];             // transposed: no bank conflicts
+  __syncthreads();
+  for (int i = threadIdx.x; i < a.out.segments * kTailVecs * 8; i += kLnThreads) {
+    const int s = i / (kTailVecs * 8), c = i % (kTailVecs * 8), col = (blockIdx.x * kTailVecs + c % kTailVecs) * 8 + c / kTailVecs;
+    if (col >= a.D) continue;
+    float t = red[s][0][c];
+#pragma unroll
+    for (int g = 1; g < kTailGroups; ++g) t += red[s][g][c];
+    if (gridDim.y == 1) colred::put(a.out, s * a.D + col, t);
+    else a.partial[((int64_t)blockIdx.y * a.out.segments + s) * a.D + col] = t;
+  }
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 template <int W, int VPL, bool RMS>
@@ -347,6 +531,25 @@ cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
   return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, C, a.out, s);
 }
 
+template <int VPL, bool RES, int PARTS>
+cudaError_t bwdRows(const LnBwdArgs& a, cudaStream_t s) {
+  constexpr int kRowBytes = 2 * kLnWarps * VPL * 512 * 2, kSumBytes = kLnWarps * 3 * 256 * (int)sizeof(float);
+  constexpr int kSmem = kRowBytes > kSumBytes ? kRowBytes : kSumBytes;
+  if (kSmem > 48 << 10) {
+    const cudaError_t e = cudaFuncSetAttribute(lnRowsBackwardKernel<VPL, RES, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e != cudaSuccess) return e;
+  }
+  int cluster;
+  const int grid = colred::grid((a.rows + kLnWarps - 1) / kLnWarps, 2, &cluster);
+  const cudaError_t e = colred::launch(lnRowsBackwardKernel<VPL, RES, PARTS>, grid, cluster, kLnThreads, kSmem, s, a);
+  return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, a.out.segments * a.D, a.out, s);
+}
+template <int VPL>
+cudaError_t bwdRowsAny(const LnBwdArgs& a, cudaStream_t s) {
+  if (!a.dres) return bwdRows<VPL, false, 1>(a, s);
+  return a.dy2 ? bwdRows<VPL, true, 3>(a, s) : bwdRows<VPL, true, 1>(a, s);
+}
+
 // A lane's columns cost four registers each (three sums and gamma) beside two rows of x, dy and dres: two vectors a lane
 // fit 128 registers without dres and spill with it (8192 x 1024: 26 us, with one vector a lane 19 us).
 template <bool RMS, int PARTS>
@@ -360,6 +563,9 @@ cudaError_t bwdRes(const LnBwdArgs& a, cudaStream_t s) {
 }
 template <bool RMS>
 cudaError_t bwdAny(const LnBwdArgs& a, cudaStream_t s) {
+  if (!RMS && a.D == 256) return bwdRowsAny<1>(a, s);
+  if (!RMS && a.D == 512) return bwdRowsAny<2>(a, s);
+  if (!RMS && a.D == 1024) return bwdRowsAny<4>(a, s);
   if (a.dres) return a.dy2 ? bwdRes<RMS, 3>(a, s) : bwdRes<RMS, 1>(a, s);
   if (a.D <= 256) return bwdLaunch<1, 1, RMS, false>(a, s);
   if (a.D <= 512) return bwdLaunch<1, 2, RMS, false>(a, s);
@@ -443,4 +649,31 @@ extern "C" mcclResult_t mcclRmsNormForward(const void* x, const void* delta, con
 extern "C" mcclResult_t mcclRmsNormBackward(const void* x, const void* dy, const void* dy2, const void* dy3, const void* dres, const void* gamma,
                                             const float* rstd, void* dx, void* dgamma, int accumulate, float* partial, int64_t rows, int D, mcclStream_t stream) {
   return backward(x, dy, dy2, dy3, dres, gamma, nullptr, rstd, dx, dgamma, nullptr, nullptr, accumulate, partial, rows, D, true, stream);
+}
+
+// The rest of a LayerNorm's backward pass with the gradient through it, dn, given: dx = dn + dres (dres and dx may be null: dx is
+// dn), dgamma, dbeta and, when given, dcol = column sums of dx.  dy: the gradient of the norm's result.  partial as above.
+extern "C" mcclResult_t mcclLayerNormBackwardTail(const void* x, const void* dy, const void* dn, const void* dres, const float* mean,
+                                                  const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate,
+                                                  float* partial, int64_t rows, int D, mcclStream_t stream) {
+  if (!x || !dy || !dn || !mean || !rstd || !dgamma || !dbeta || !partial || rows <= 0 || D <= 0 || D % 8 || (dres && !dx)) return mcclInvalidArgument;
+  if (!aligned16(x) || !aligned16(dy) || !aligned16(dn) || !aligned16(dres) || !aligned16(dx)) return mcclInvalidArgument;
+  LnTailArgs a;
+  a.x = static_cast<const uint4*>(x); a.dy = static_cast<const uint4*>(dy);
+  a.dn = static_cast<const uint4*>(dn); a.dres = static_cast<const uint4*>(dres);
+  a.mean = mean; a.rstd = rstd; a.dx = static_cast<uint4*>(dx); a.partial = partial; a.rows = rows; a.D = D;
+  a.out = colred::Out{};
+  a.out.seg[0] = static_cast<__nv_bfloat16*>(dgamma); a.out.seg[1] = static_cast<__nv_bfloat16*>(dbeta);
+  a.out.seg[2] = static_cast<__nv_bfloat16*>(dcol);
+  a.out.segments = dcol ? 3 : 2; a.out.width = D; a.out.accumulate = accumulate;
+  // Two CTAs a SM, at least sixteen rows each.
+  const int strips = (D / 8 + kTailVecs - 1) / kTailVecs;
+  int64_t slices = 148 * 2 / strips;
+  if (slices > (rows + 15) / 16) slices = (rows + 15) / 16;
+  if (slices < 1) slices = 1;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  auto* kernel = dres ? lnTailKernel<true> : lnTailKernel<false>;
+  kernel<<<dim3(strips, (unsigned)slices), kLnThreads, 0, s>>>(a);
+  if (cudaGetLastError() != cudaSuccess) return mcclSystemError;
+  return colred::addPartials(partial, (int)slices, 1, a.out.segments * D, a.out, s) == cudaSuccess ? mcclSuccess : mcclSystemError;
 }

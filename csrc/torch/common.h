@@ -39,6 +39,9 @@ inline void check(mcclResult_t rc, const char* what) {
   TORCH_CHECK(rc == mcclSuccess || rc == mcclInProgress, "mccl: ", mcclResultStr(rc), " (code ", (int)rc, "): ", what);
 }
 inline bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+// Widths at which LayerNorm runs in the library's kernels (FusedLayerNorm and the decoder's nodes alike).  The kernels take
+// others too, in another order of their sums than the tensor library's: a model's results would depend on it.
+inline bool layerNormWidth(int64_t d) { return d == 256 || d == 512 || d == 1024; }
 inline bool bf16Cuda(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; }
 
 // Whether a kernel may be launched on t's memory in place of tensor operations: not for the wrappers of torch.func, of tensor

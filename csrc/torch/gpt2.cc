@@ -22,29 +22,95 @@ Tensor adjacent(const Tensor& a, const Tensor& b, const Tensor& c) {
   return a.dim() == 2 ? a.as_strided(sizes, {sizes[1], 1}) : a.as_strided(sizes, {1});
 }
 
-// sum = x + pending (pending may be missing: sum = x) and its norm.  `exact`: at widths this library had no kernel for, a
-// forward pass without gradients keeps the tensor library's norm, bit for bit (a last-bit difference in the first norm is a
-// difference of a percent in the logits of a 12-layer model in bf16, so scores would not compare with recorded ones).
-void addNorm(const Tensor& x, const Tensor* pending, const Tensor& lw, const Tensor& lb, double eps, bool exact, Tensor* sum, Tensor* h, Tensor* stats) {
+// The norms here give FusedLayerNorm's results: the library's kernel at the widths it has one for, the tensor library's
+// elsewhere.  A model then scores and trains with the same bits on this route and on the plain one.  (Another order of a
+// norm's sums is a last bit of some of its results; in bf16, twelve layers on, that is a percent of the logits, and over 24
+// layers and two steps of training up to 0.03 of the moments, more than two runs of one route lie apart.)
+struct Norm { Tensor sum, h, mean, rstd; };        // own kernels: both statistics in `mean`, rstd undefined
+
+Norm addNorm(const Tensor& x, const Tensor* pending, const Tensor& lw, const Tensor& lb, double eps) {
   const int64_t T = x.size(0), d = x.size(1);
-  if (exact && d != 256 && d != 512 && d != 1024) {
-    *sum = pending ? at::add(x, *pending) : at::alias(x);
-    *h = std::get<0>(at::native_layer_norm(*sum, {d}, lw, lb, eps));
-    return;
+  Norm n;
+  if (!layerNormWidth(d)) {
+    n.sum = pending ? at::add(x, *pending) : at::alias(x);
+    std::tie(n.h, n.mean, n.rstd) = at::native_layer_norm(n.sum, {d}, lw, lb, eps);
+    return n;
   }
-  Norm n = normStats(x, T);
-  *stats = n.stats;
-  *h = at::empty({T, d}, x.options());
+  n.mean = at::empty({2, T}, x.options().dtype(at::kFloat));
+  float* mean = n.mean.data_ptr<float>();
+  n.h = at::empty({T, d}, x.options());
   if (pending) {
-    *sum = at::empty({T, d}, x.options());
-    check(mcclAddLayerNormForward(x.data_ptr(), pending->data_ptr(), lw.data_ptr(), lb.data_ptr(), sum->data_ptr(), h->data_ptr(), n.mean(),
-                                  n.rstd(T), T, (int)d, (float)eps, streamOf(x)), "mcclAddLayerNormForward");
+    n.sum = at::empty({T, d}, x.options());
+    check(mcclAddLayerNormForward(x.data_ptr(), pending->data_ptr(), lw.data_ptr(), lb.data_ptr(), n.sum.data_ptr(), n.h.data_ptr(), mean,
+                                  mean + T, T, (int)d, (float)eps, streamOf(x)), "mcclAddLayerNormForward");
   } else {
-    *sum = at::alias(x);
-    check(mcclLayerNormForward(x.data_ptr(), lw.data_ptr(), lb.data_ptr(), h->data_ptr(), n.mean(), n.rstd(T), T, (int)d, (float)eps,
-                               streamOf(x)), "mcclLayerNormForward");
+    n.sum = at::alias(x);
+    check(mcclLayerNormForward(x.data_ptr(), lw.data_ptr(), lb.data_ptr(), n.h.data_ptr(), mean, mean + T, T, (int)d, (float)eps, streamOf(x)),
+          "mcclLayerNormForward");
   }
   counters().norm++;
+  return n;
+}
+
+// out = [+] column sums of up to three [T, d] matrices, a gradient each.
+void columnSums(GradSink& sink, std::initializer_list<Tensor> x, const VectorGrads& out) {
+  const Tensor& first = *x.begin();
+  const int64_t T = first.size(0), d = first.size(1);
+  const void* in[3];
+  void* to[3];
+  int n = 0;
+  for (const Tensor& t : x) { in[n] = t.data_ptr(); to[n] = out.t[n].data_ptr(); ++n; }
+  Tensor scratch = columnScratch(first, T, d, n);
+  check(mcclColumnSums(in, to, n, out.direct, scratch.data_ptr<float>(), T, (int)d, d, streamOf(first)), "mcclColumnSums");
+}
+
+// Gradient of a norm's sum from those of its result (the sum of `parts`, added up in their order with a rounding each) and, where
+// defined, of the residual stream; *dw, *db and, with `bias`, *dbias (column sums of the whole) as they are to be returned.
+Tensor normBackward(GradSink& sink, const Tensor& sum, std::initializer_list<Tensor> parts, const Tensor& dres, const Tensor& lw, const Tensor& lb,
+                    const Tensor& mean, const Tensor& rstd, const Tensor& bias, Tensor* dw, Tensor* db, Tensor* dbias) {
+  const int64_t T = sum.size(0), d = sum.size(1);
+  const bool own = !rstd.defined();
+  Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * 3 * d}, mean.options()), dx, dn;
+  const float *m = mean.data_ptr<float>(), *r = own ? m + T : rstd.data_ptr<float>();
+  const void* dh[3] = {};
+  int n = 0;
+  for (const Tensor& p : parts) dh[n++] = p.data_ptr();
+  if (own) {
+    dx = at::empty({T, d}, sum.options());
+  } else {
+    Tensor dy = *parts.begin();
+    for (const Tensor& p : parts) if (!p.is_same(dy)) dy.add_(p);
+    dn = std::get<0>(at::native_layer_norm_backward(dy, sum, {d}, mean, rstd, lw, lb, {true, false, false}));
+    dx = dres.defined() ? at::empty({T, d}, sum.options()) : dn;
+  }
+  void* res = dres.defined() ? dres.data_ptr() : nullptr;
+  auto run = [&](const VectorGrads& g, void* dcol) {
+    if (own) {
+      check(mcclAddLayerNormBackward(sum.data_ptr(), dh[0], dh[1], dh[2], res, lw.data_ptr(), m, r, dx.data_ptr(), g.t[0].data_ptr(),
+                                     g.t[1].data_ptr(), dcol, g.direct, partial.data_ptr<float>(), T, (int)d, streamOf(sum)),
+            "mcclAddLayerNormBackward");
+    } else {
+      check(mcclLayerNormBackwardTail(sum.data_ptr(), dh[0], dn.data_ptr(), res, m, r, dx.data_ptr(), g.t[0].data_ptr(), g.t[1].data_ptr(), dcol,
+                                      g.direct, partial.data_ptr<float>(), T, (int)d, streamOf(sum)), "mcclLayerNormBackwardTail");
+    }
+    *dw = g.ret(0);
+    *db = g.ret(1);
+  };
+  if (bias.defined() && dres.defined()) {
+    VectorGrads g(sink, {&lw, &lb, &bias});
+    run(g, g.t[2].data_ptr());
+    *dbias = g.ret(2);
+  } else {
+    VectorGrads g(sink, {&lw, &lb});
+    run(g, nullptr);
+    if (bias.defined()) {
+      VectorGrads b(sink, {&bias});
+      columnSums(sink, {dx}, b);
+      *dbias = b.ret(0);
+    }
+  }
+  counters().norm += 2;
+  return dx;
 }
 
 // ---- first half: (residual, pending) -> residual sum, norm, q, k, v -----------------------------------------------------
@@ -52,11 +118,11 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
   // Outputs: residual [T, d], q, k, v [b, h, s, hd].
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& pending, const OptTensor& pendingBias, const Tensor& lw,
                                const Tensor& lb, const Tensor& wq, const Tensor& bq, const Tensor& wk, const Tensor& bk, const Tensor& wv,
-                               const Tensor& bv, int64_t b, int64_t s, int64_t heads, double eps, bool sink, bool exact) {
+                               const Tensor& bv, int64_t b, int64_t s, int64_t heads, double eps, bool sink) {
     Below below;
-    const int64_t T = x.size(0), d = x.size(1), hd = d / heads;
-    Tensor sum, h, stats;
-    addNorm(x, pending ? &*pending : nullptr, lw, lb, eps, exact, &sum, &h, &stats);
+    const int64_t d = x.size(1), hd = d / heads;
+    const Norm n = addNorm(x, pending ? &*pending : nullptr, lw, lb, eps);
+    const Tensor& h = n.h;
     auto split = [&](const Tensor& t, int64_t rowStride, int64_t offset) {
       return t.as_strided({b, heads, s, hd}, {s * rowStride, hd, rowStride, 1}, t.storage_offset() + offset);
     };
@@ -73,84 +139,44 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
       v = split(at::linear(h, wv, bv), d, 0);
     }
     // Without a pending term the sum is the input: saved as such, so that a change made to it in place is noticed.
-    ctx->save_for_backward({pending ? sum : x, h, stats, lw, lb, wq, bq, wk, bk, wv, bv, pendingBias ? *pendingBias : Tensor()});
+    ctx->save_for_backward({pending ? n.sum : x, h, n.mean, n.rstd, lw, lb, wq, bq, wk, bk, wv, bv, pendingBias ? *pendingBias : Tensor()});
     ctx->saved_data["sink"] = sink;
     ctx->saved_data["pending"] = pending.has_value();
-    return {sum, q, k, v};
+    return {n.sum, q, k, v};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
-    const Tensor &sum = saved[0], &h = saved[1], &stats = saved[2], &lw = saved[3], &lb = saved[4], &wq = saved[5], &bq = saved[6],
-                 &wk = saved[7], &bk = saved[8], &wv = saved[9], &bv = saved[10], &pb = saved[11];
+    const Tensor &sum = saved[0], &h = saved[1], &mean = saved[2], &rstd = saved[3], &lw = saved[4], &lb = saved[5], &wq = saved[6],
+                 &bq = saved[7], &wk = saved[8], &bk = saved[9], &wv = saved[10], &bv = saved[11], &pb = saved[12];
     Below below;
     c10::cuda::CUDAGuard guard(h.device());
     GradSink sink(ctx->saved_data["sink"].toBool());
-    const bool pending = ctx->saved_data["pending"].toBool();
     const int64_t T = h.size(0), d = h.size(1);
-    mcclStream_t s = streamOf(h);
-    auto zeros = [&] { return at::zeros({T, d}, h.options()); };
-    Tensor dq = g[1].defined() ? fromHeads(g[1], T, d) : zeros(), dk = g[2].defined() ? fromHeads(g[2], T, d) : zeros(),
-           dv = g[3].defined() ? fromHeads(g[3], T, d) : zeros();
-    Tensor dwq, dwk, dwv, dhv, dhk, dhq;
-    VectorGrads db(sink, {&bv, &bk, &bq});
-    Tensor scratch = columnScratch(h, T, d, 3);
-    const void* in[3] = {dv.data_ptr(), dk.data_ptr(), dq.data_ptr()};
-    void* out[3] = {db.t[0].data_ptr(), db.t[1].data_ptr(), db.t[2].data_ptr()};
-    Tensor w3 = adjacent(wv, wk, wq);
-    if (w3.defined()) {
-      // The weights as one matrix: the gradients are laid side by side on the pass that sums their columns, and one product
-      // gives the norm's gradient, another the three weight gradients where those are one matrix too.
-      Tensor d3 = at::empty({T, 3 * d}, h.options());
-      check(mcclPackColumnSums(in, d3.data_ptr(), out, 3, db.direct, scratch.data_ptr<float>(), T, (int)d, s), "mcclPackColumnSums");
-      dhv = at::mm(d3, w3);
-      Tensor gv = sink.buffer(wv), gk = sink.buffer(wk), gq = sink.buffer(wq);
-      Tensor g3 = gv.defined() && gk.defined() && gq.defined() ? adjacent(gv, gk, gq) : Tensor();
-      if (g3.defined()) {
-        at::addmm_out(g3, g3, d3.t(), h);
-      } else {
-        weightGrad(sink, wv, dv, h, &dwv);
-        weightGrad(sink, wk, dk, h, &dwk);
-        weightGrad(sink, wq, dq, h, &dwq);
-      }
-    } else {
-      check(mcclColumnSums(in, out, 3, db.direct, scratch.data_ptr<float>(), T, (int)d, d, s), "mcclColumnSums");
-      dhv = at::mm(dv, wv); dhk = at::mm(dk, wk); dhq = at::mm(dq, wq);      // the norm's backward kernel adds them up
-      weightGrad(sink, wv, dv, h, &dwv);
-      weightGrad(sink, wk, dk, h, &dwk);
-      weightGrad(sink, wq, dq, h, &dwq);
-    }
-    const void *part2 = dhk.defined() ? dhk.data_ptr() : nullptr, *part3 = dhq.defined() ? dhq.data_ptr() : nullptr;
-    Tensor dx = at::empty({T, d}, h.options());
-    Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * 3 * d}, stats.options());
-    const float* mean = stats.data_ptr<float>();
+    const Tensor dq = fromHeads(g[1], T, d), dk = fromHeads(g[2], T, d), dv = fromHeads(g[3], T, d);
     variable_list ret(17);
-    if (g[0].defined()) {
-      Tensor dres = rows2d(g[0], T, d);
-      if (pb.defined()) {
-        VectorGrads dn(sink, {&lw, &lb, &pb});
-        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), part2, part3, dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
-                                       dn.t[0].data_ptr(), dn.t[1].data_ptr(), dn.t[2].data_ptr(), dn.direct, partial.data_ptr<float>(), T,
-                                       (int)d, s), "mcclAddLayerNormBackward");
-        ret[3] = dn.ret(0); ret[4] = dn.ret(1); ret[2] = dn.ret(2);
-      } else {
-        VectorGrads dn(sink, {&lw, &lb});
-        check(mcclAddLayerNormBackward(sum.data_ptr(), dhv.data_ptr(), part2, part3, dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
-                                       dn.t[0].data_ptr(), dn.t[1].data_ptr(), nullptr, dn.direct, partial.data_ptr<float>(), T, (int)d, s),
-              "mcclAddLayerNormBackward");
-        ret[3] = dn.ret(0); ret[4] = dn.ret(1);
-      }
-    } else {                                       // nobody uses the residual: the plain norm, and the bias on its own
-      ret[3] = at::empty(lw.sizes(), lw.options());
-      ret[4] = at::empty(lb.sizes(), lb.options());
-      Tensor dh = part2 ? dhv.add_(dhk).add_(dhq) : dhv;
-      check(mcclLayerNormBackward(sum.data_ptr(), dh.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(), ret[3].data_ptr(),
-                                  ret[4].data_ptr(), partial.data_ptr<float>(), T, (int)d, s), "mcclLayerNormBackward");
-      if (pb.defined()) ret[2] = dx.sum(0);
+    VectorGrads db(sink, {&bv, &bk, &bq});
+    // Weight gradients: where their buffers lie next to each other the three gradients are laid side by side on the pass that sums
+    // their columns, and one product fills all of them (the same sums: a product's columns do not meet).
+    const Tensor gv = sink.buffer(wv), gk = sink.buffer(wk), gq = sink.buffer(wq);
+    Tensor g3 = gv.defined() && gk.defined() && gq.defined() ? adjacent(gv, gk, gq) : Tensor();
+    if (g3.defined()) {
+      Tensor d3 = at::empty({T, 3 * d}, h.options()), scratch = columnScratch(h, T, d, 3);
+      const void* in[3] = {dv.data_ptr(), dk.data_ptr(), dq.data_ptr()};
+      void* out[3] = {db.t[0].data_ptr(), db.t[1].data_ptr(), db.t[2].data_ptr()};
+      check(mcclPackColumnSums(in, d3.data_ptr(), out, 3, db.direct, scratch.data_ptr<float>(), T, (int)d, streamOf(h)), "mcclPackColumnSums");
+      at::addmm_out(g3, g3, d3.t(), h);
+    } else {
+      columnSums(sink, {dv, dk, dq}, db);
+      weightGrad(sink, wv, dv, h, &ret[9]);
+      weightGrad(sink, wk, dk, h, &ret[7]);
+      weightGrad(sink, wq, dq, h, &ret[5]);
     }
-    counters().norm += 2;
-    ret[0] = dx;
-    if (pending) ret[1] = dx;
-    ret[5] = dwq; ret[6] = db.ret(2); ret[7] = dwk; ret[8] = db.ret(1); ret[9] = dwv; ret[10] = db.ret(0);
+    ret[6] = db.ret(2); ret[8] = db.ret(1); ret[10] = db.ret(0);
+    // The norm's gradient stays three products, each rounded: as one product of three times the depth it is faster (34 us for
+    // 3 x 15 at 8192 x 1024) but rounds once, and every number behind it differs from the separate operations'.
+    ret[0] = normBackward(sink, sum, {at::mm(dv, wv), at::mm(dk, wk), at::mm(dq, wq)}, rows2d(g[0], T, d), lw, lb, mean, rstd, pb, &ret[3], &ret[4],
+                          &ret[2]);
+    if (ctx->saved_data["pending"].toBool()) ret[1] = ret[0];
     return once(std::move(ret));
   }
 };
@@ -161,43 +187,37 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
   // projection is taken by this node and not by the one that adds its output.
   static variable_list forward(AutogradContext* ctx, const Tensor& a, const Tensor& res, const Tensor& wo, const Tensor& bo, const Tensor& lw,
                                const Tensor& lb, const Tensor& wf, const Tensor& bf, const Tensor& wd, const Tensor& bd, bool outBiasHere,
-                               double eps, bool sink, bool exact) {
+                               double eps, bool sink) {
     Below below;
     const int64_t T = res.size(0), d = res.size(1);
     mcclStream_t s = streamOf(res);
     Tensor a2 = fromHeads(a, T, d);
     Tensor p = at::linear(a2, wo, bo);
-    Tensor x1, h, stats;
-    addNorm(res, &p, lw, lb, eps, exact, &x1, &h, &stats);
-    Tensor u = at::linear(h, wf, bf);
+    const Norm n = addNorm(res, &p, lw, lb, eps);
+    Tensor u = at::linear(n.h, wf, bf);
     Tensor act = at::empty(u.sizes(), u.options());
     check(mcclGeluForward(u.data_ptr(), act.data_ptr(), u.numel(), s), "mcclGeluForward");
     Tensor y = at::linear(act, wd, bd);
-    ctx->save_for_backward({a2, x1, h, stats, u, act, wo, bo, lw, lb, wf, bf, wd, bd});
+    ctx->save_for_backward({a2, n.sum, n.h, n.mean, n.rstd, u, act, wo, bo, lw, lb, wf, bf, wd, bd});
     ctx->saved_data["sink"] = sink;
     ctx->saved_data["bias"] = outBiasHere;
     ctx->saved_data["b"] = a.size(0);
     ctx->saved_data["h"] = a.size(1);
-    return {x1, y};
+    return {n.sum, y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
-    const Tensor &a2 = saved[0], &x1 = saved[1], &h = saved[2], &stats = saved[3], &u = saved[4], &act = saved[5], &wo = saved[6],
-                 &bo = saved[7], &lw = saved[8], &lb = saved[9], &wf = saved[10], &bf = saved[11], &wd = saved[12], &bd = saved[13];
+    const Tensor &a2 = saved[0], &x1 = saved[1], &h = saved[2], &mean = saved[3], &rstd = saved[4], &u = saved[5], &act = saved[6], &wo = saved[7],
+                 &bo = saved[8], &lw = saved[9], &lb = saved[10], &wf = saved[11], &bf = saved[12], &wd = saved[13], &bd = saved[14];
     Below below;
     c10::cuda::CUDAGuard guard(h.device());
     GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0), d = h.size(1), f = u.size(1), b = ctx->saved_data["b"].toInt(), heads = ctx->saved_data["h"].toInt();
-    mcclStream_t s = streamOf(h);
     variable_list ret(14);
-    Tensor dy = g[1].defined() ? rows2d(g[1], T, d) : at::zeros({T, d}, h.options());
-    Tensor dres = g[0].defined() ? rows2d(g[0], T, d) : at::zeros({T, d}, h.options());
+    const Tensor dy = rows2d(g[1], T, d), dres = rows2d(g[0], T, d);
     if (ctx->saved_data["bias"].toBool()) {
       VectorGrads db(sink, {&bd});
-      Tensor scratch = columnScratch(h, T, d, 1);
-      const void* in[1] = {dy.data_ptr()};
-      void* out[1] = {db.t[0].data_ptr()};
-      check(mcclColumnSums(in, out, 1, db.direct, scratch.data_ptr<float>(), T, (int)d, d, s), "mcclColumnSums");
+      columnSums(sink, {dy}, db);
       ret[9] = db.ret(0);
     }
     Tensor du = at::mm(dy, wd);
@@ -205,23 +225,13 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     {
       VectorGrads db(sink, {&bf});
       Tensor scratch = columnScratch(h, T, f, 1);
-      check(mcclGeluBackward(u.data_ptr(), du.data_ptr(), du.data_ptr(), db.t[0].data_ptr(), db.direct, scratch.data_ptr<float>(), T, (int)f, s),
-            "mcclGeluBackward");
+      check(mcclGeluBackward(u.data_ptr(), du.data_ptr(), du.data_ptr(), db.t[0].data_ptr(), db.direct, scratch.data_ptr<float>(), T, (int)f,
+                             streamOf(h)), "mcclGeluBackward");
       ret[7] = db.ret(0);
     }
     Tensor dh = at::mm(du, wf);
     weightGrad(sink, wf, du, h, &ret[6]);
-    Tensor dx = at::empty({T, d}, h.options());
-    {
-      VectorGrads dn(sink, {&lw, &lb, &bo});
-      Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * 3 * d}, stats.options());
-      const float* mean = stats.data_ptr<float>();
-      check(mcclAddLayerNormBackward(x1.data_ptr(), dh.data_ptr(), nullptr, nullptr, dres.data_ptr(), lw.data_ptr(), mean, mean + T, dx.data_ptr(),
-                                     dn.t[0].data_ptr(), dn.t[1].data_ptr(), dn.t[2].data_ptr(), dn.direct, partial.data_ptr<float>(), T, (int)d,
-                                     s), "mcclAddLayerNormBackward");
-      counters().norm += 2;
-      ret[4] = dn.ret(0); ret[5] = dn.ret(1); ret[3] = dn.ret(2);
-    }
+    const Tensor dx = normBackward(sink, x1, {dh}, dres, lw, lb, mean, rstd, bo, &ret[4], &ret[5], &ret[3]);
     Tensor da = at::mm(dx, wo);
     weightGrad(sink, wo, dx, a2, &ret[2]);
     ret[0] = da.view({b, T / b, heads, d / heads}).transpose(1, 2);
@@ -233,41 +243,23 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
 // ---- final norm of (residual, pending) --------------------------------------------------------------------------------
 struct FinalNormFn : torch::autograd::Function<FinalNormFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& pending, const OptTensor& pendingBias, const Tensor& lw,
-                        const Tensor& lb, double eps, bool sink, bool exact) {
+                        const Tensor& lb, double eps, bool sink) {
     Below below;
-    Tensor sum, h, stats;
-    addNorm(x, &pending, lw, lb, eps, exact, &sum, &h, &stats);
-    ctx->save_for_backward({sum, stats, lw, lb, pendingBias ? *pendingBias : Tensor()});
+    const Norm n = addNorm(x, &pending, lw, lb, eps);
+    ctx->save_for_backward({n.sum, n.mean, n.rstd, lw, lb, pendingBias ? *pendingBias : Tensor()});
     ctx->saved_data["sink"] = sink;
-    return h;
+    return n.h;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
-    const Tensor &sum = saved[0], &stats = saved[1], &lw = saved[2], &lb = saved[3], &pb = saved[4];
+    const Tensor &sum = saved[0];
     Below below;
     c10::cuda::CUDAGuard guard(sum.device());
     GradSink sink(ctx->saved_data["sink"].toBool());
-    const int64_t T = sum.size(0), d = sum.size(1);
-    mcclStream_t s = streamOf(sum);
-    Tensor dh = rows2d(g[0], T, d), dx = at::empty({T, d}, sum.options());
-    Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(T) * 2 * d}, stats.options());
-    const float* mean = stats.data_ptr<float>();
     variable_list ret(8);
-    VectorGrads dn(sink, {&lw, &lb});
-    check(mcclAddLayerNormBackward(sum.data_ptr(), dh.data_ptr(), nullptr, nullptr, nullptr, lw.data_ptr(), mean, mean + T, dx.data_ptr(), dn.t[0].data_ptr(),
-                                   dn.t[1].data_ptr(), nullptr, dn.direct, partial.data_ptr<float>(), T, (int)d, s), "mcclAddLayerNormBackward");
-    counters().norm += 2;
-    ret[3] = dn.ret(0); ret[4] = dn.ret(1);
-    if (pb.defined()) {
-      VectorGrads db(sink, {&pb});
-      Tensor scratch = columnScratch(sum, T, d, 1);
-      const void* in[1] = {dx.data_ptr()};
-      void* out[1] = {db.t[0].data_ptr()};
-      check(mcclColumnSums(in, out, 1, db.direct, scratch.data_ptr<float>(), T, (int)d, d, s), "mcclColumnSums");
-      ret[2] = db.ret(0);
-    }
-    ret[0] = dx;
-    ret[1] = dx;
+    ret[0] = normBackward(sink, sum, {rows2d(g[0], sum.size(0), sum.size(1))}, Tensor(), saved[3], saved[4], saved[1], saved[2], saved[5], &ret[3], &ret[4],
+                          &ret[2]);
+    ret[1] = ret[0];
     return once(std::move(ret));
   }
 };
@@ -375,10 +367,9 @@ py::object block(const Tensor& x, const OptTensor& pending, const OptTensor& pen
   for (int i : {2, 4, 6, 8}) if (!shaped(p[i], {d, d})) return py::none();
   if (!shaped(p[12], {f, d}) || !shaped(p[13], {f}) || !shaped(p[14], {d, f})) return py::none();
   c10::cuda::CUDAGuard guard(x.device());
-  const bool exact = !at::GradMode::is_enabled();
-  variable_list in = BlockInFn::apply(x, pending, pendingBias, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], b, s, heads, eps, sink, exact);
+  variable_list in = BlockInFn::apply(x, pending, pendingBias, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], b, s, heads, eps, sink);
   Tensor a = at::scaled_dot_product_attention(in[1], in[2], in[3], {}, 0.0, true);
-  variable_list out = BlockOutFn::apply(a, in[0], p[8], p[9], p[10], p[11], p[12], p[13], p[14], p[15], outBiasHere, eps, sink, exact);
+  variable_list out = BlockOutFn::apply(a, in[0], p[8], p[9], p[10], p[11], p[12], p[13], p[14], p[15], outBiasHere, eps, sink);
   return py::make_tuple(out[0], out[1]);
 }
 
@@ -396,7 +387,7 @@ py::object finalNorm(const Tensor& x, const Tensor& pending, const OptTensor& pe
     return py::none();
   if (pendingBias && (!plainBf16(*pendingBias, x) || !shaped(*pendingBias, {x.size(1)}))) return py::none();
   c10::cuda::CUDAGuard guard(x.device());
-  return py::cast(FinalNormFn::apply(x, pending, pendingBias, w, b, eps, sink, !at::GradMode::is_enabled()));
+  return py::cast(FinalNormFn::apply(x, pending, pendingBias, w, b, eps, sink));
 }
 
 // Mean cross-entropy of h w^T: over all rows, or over those whose target is a column (`meanOfUsed`).

@@ -7,10 +7,6 @@ namespace mccl_torch {
 
 using OptTensor = std::optional<Tensor>;
 
-struct Norm { Tensor stats; float* mean() const { return stats.data_ptr<float>(); } float* rstd(int64_t rows) const { return mean() + rows; } };
-
-inline Norm normStats(const Tensor& x, int64_t rows) { return Norm{at::empty({2, rows}, x.options().dtype(at::kFloat))}; }
-
 inline Tensor columnScratch(const Tensor& like, int64_t rows, int64_t d, int n) {
   return at::empty({mcclColumnSumScratch(rows, (int)d, n)}, like.options().dtype(at::kFloat));
 }

@@ -7,8 +7,8 @@ namespace {
 // ---- LayerNorm ------------------------------------------------------------------------------------------------------
 bool normSupported(const Tensor& x, const Tensor& w, const Tensor& b) {
   const int64_t d = x.dim() > 0 ? x.size(-1) : 0;
-  return !recorded() && ordinary(x) && ordinary(w) && ordinary(b) && bf16Cuda(x) && bf16Cuda(w) && bf16Cuda(b) && d > 0 &&
-         d % 8 == 0 && d <= 4096 && w.numel() == d && b.numel() == d && w.is_contiguous() && b.is_contiguous() && aligned16(w) && aligned16(b);
+  return !recorded() && ordinary(x) && ordinary(w) && ordinary(b) && bf16Cuda(x) && bf16Cuda(w) && bf16Cuda(b) &&
+         layerNormWidth(d) && w.numel() == d && b.numel() == d && w.is_contiguous() && b.is_contiguous() && aligned16(w) && aligned16(b);
 }
 
 struct LayerNormFn : torch::autograd::Function<LayerNormFn> {

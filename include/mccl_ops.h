@@ -135,6 +135,11 @@ mcclResult_t mcclPackColumnSums(const void* const* x, void* packed, void* const*
 mcclResult_t mcclAddLayerNormBackward(const void* x, const void* dy, const void* dy2, const void* dy3, const void* dres, const void* gamma,
                                       const float* mean, const float* rstd, void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate, float* partial,
                                       int64_t rows, int D, mcclStream_t stream);
+/* What is left of the backward pass when dn, the gradient through the norm, is there: dx = dn + dres (both nullable: dx is dn),
+ * dgamma, dbeta and dcol (nullable).  partial as in the Add form. */
+mcclResult_t mcclLayerNormBackwardTail(const void* x, const void* dy, const void* dn, const void* dres, const float* mean, const float* rstd,
+                                       void* dx, void* dgamma, void* dbeta, void* dcol, int accumulate, float* partial, int64_t rows, int D,
+                                       mcclStream_t stream);
 /* RMSNorm, y = bf16(x * rstd) * gamma; delta and sum (nullable) as above; dres nullable. */
 mcclResult_t mcclRmsNormForward(const void* x, const void* delta, const void* gamma, void* sum, void* y, float* rstd, int64_t rows, int D,
                                 float eps, mcclStream_t stream);

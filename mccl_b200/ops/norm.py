@@ -1,5 +1,5 @@
-"""LayerNorm with the library's fused forward / backward kernels (csrc/ops/layer_norm.cu) for bf16 rows of up to 4096
-elements (a multiple of 8) on CUDA; anything else goes through torch.nn.functional.layer_norm."""
+"""LayerNorm with the library's fused forward / backward kernels (csrc/ops/layer_norm.cu) for bf16 rows of 256, 512 or
+1024 elements on CUDA; anything else goes through torch.nn.functional.layer_norm."""
 from __future__ import annotations
 
 import torch
@@ -13,9 +13,12 @@ def launches() -> int:
     return _ext.load().launches("norm")
 
 
+_WIDTHS = (256, 512, 1024)
+
+
 def fused_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0
-            and 0 < x.shape[-1] <= 4096 and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
+    return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[-1] in _WIDTHS
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
 
 
 class FusedLayerNorm(nn.Module):

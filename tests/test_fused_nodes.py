@@ -92,6 +92,35 @@ def test_fused_route_is_as_close_to_64_bits_as_the_plain_one(make, kw):
 
 
 @gpu
+@pytest.mark.parametrize("bucket", [False, True])
+@pytest.mark.parametrize("d", [128, 256, 384, 512, 768, 1024])
+def test_fused_gradients_are_the_plain_routes(d, bucket):
+    """Whatever a number of the backward pass flows into is the same number on both routes, so models compare with runs of the
+    separate operations: the gradients of the matrices are equal.  Sums over tokens (biases, norms, repeated tokens) are taken in another order: a rounding apart."""
+    from mccl_b200.parallel.ddp import DistributedDataParallel
+    idx, tgt = _batch()
+
+    def grads(model):
+        if bucket:
+            DistributedDataParallel(model, None)(idx, tgt).backward()
+            return [p.grad for p in model.parameters()]
+        return _grads(model, idx, tgt)[1:]
+
+    was = torch.backends.cuda.cudnn_sdp_enabled()
+    torch.backends.cuda.enable_cudnn_sdp(False)        # the other kernel adds in one order for as few tokens as these
+    try:
+        fused, again, plain = grads(_gpt2(d)), grads(_gpt2(d)), grads(_plain(_gpt2(d)))
+    finally:
+        torch.backends.cuda.enable_cudnn_sdp(was)
+    for (n, p), f, a, w in zip(_gpt2(d).named_parameters(), fused, again, plain):
+        assert torch.equal(f, a), n
+        if p.dim() == 2 and n != "wte.weight":
+            assert torch.equal(f, w), n
+        elif not n.endswith("k.bias"):                 # zero but for rounding
+            assert (f.float() - w.float()).norm() <= 2.0 ** -8 * w.float().norm(), n
+
+
+@gpu
 @pytest.mark.parametrize("frozen", [(), ("k.weight",), ("q.bias", "v.weight")])
 @pytest.mark.parametrize("d", [128, 1056])
 def test_adjacent_projections_are_one_product(d, frozen):
