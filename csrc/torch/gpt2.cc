@@ -333,9 +333,11 @@ struct HeadLossFn : torch::autograd::Function<HeadLossFn> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto saved = ctx->get_saved_variables();
     const Tensor &h = saved[0], &w = saved[1], &t = saved[2], &perRow = saved[4];
-    Tensor logits = saved[3];
     Below below;
     c10::cuda::CUDAGuard guard(h.device());
+    // Their gradient is written over the logits; a second pass over a retained graph works them out again.
+    Tensor logits = ctx->saved_data.count("spent") ? at::linear(h, w) : saved[3];
+    ctx->saved_data["spent"] = true;
     GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0);
     Tensor go = g[0].scalar_type() == at::kFloat ? g[0] : g[0].to(at::kFloat);

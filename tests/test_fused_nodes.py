@@ -240,6 +240,20 @@ def test_gradients_reach_buckets_hooks_and_other_streams():
 
 @gpu
 @pytest.mark.parametrize("make", [_gpt2, _llama])
+def test_a_retained_graph_is_differentiated_again(make):
+    idx, tgt = _batch()
+    model = make()
+    params = list(model.parameters())
+    loss = model(idx, tgt)
+    first = torch.autograd.grad(loss, params, retain_graph=True)
+    second = torch.autograd.grad(loss, params, retain_graph=True)
+    for (n, _), a, b in zip(model.named_parameters(), first, second):      # attention's gradient may add in another order
+        if not n.endswith("k.bias"):
+            assert (a.float() - b.float()).norm() <= 2.0 ** -6 * a.float().norm(), n
+
+
+@gpu
+@pytest.mark.parametrize("make", [_gpt2, _llama])
 def test_second_derivatives_are_not_constants(make):
     """The nodes' gradients raise when differentiated; with attention by products the plain operations answer."""
     from torch.nn.attention import SDPBackend, sdpa_kernel
