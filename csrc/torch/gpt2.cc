@@ -364,7 +364,7 @@ py::object block(const Tensor& x, const OptTensor& pending, const OptTensor& pen
   const int64_t d = x.size(1), f = p[12].size(0);
   if (heads <= 0 || d % heads || (d / heads) % 8 || f % 8 || x.size(0) != b * s) return py::none();
   if (pending && (!plainBf16(*pending, x) || !shaped(*pending, x.sizes()))) return py::none();
-  if (pendingBias && (!plainBf16(*pendingBias, x) || !shaped(*pendingBias, {d}))) return py::none();
+  if (pendingBias && (!pending || !plainBf16(*pendingBias, x) || !shaped(*pendingBias, {d}))) return py::none();
   for (int i : {0, 1, 3, 5, 7, 9, 10, 11, 15}) if (!shaped(p[i], {d})) return py::none();
   for (int i : {2, 4, 6, 8}) if (!shaped(p[i], {d, d})) return py::none();
   if (!shaped(p[12], {f, d}) || !shaped(p[13], {f}) || !shaped(p[14], {d, f})) return py::none();

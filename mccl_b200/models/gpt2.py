@@ -170,7 +170,8 @@ class GPT2(nn.Module):
             pending = bias = None
             for blk in self.blocks:
                 if not as_made(blk, Block):                  # its caller's hooks or wrapper see a block as it is called elsewhere
-                    x, pending = blk(_added(x, pending, bias).view(b, s, -1)).reshape(b * s, -1), None
+                    x = blk(_added(x, pending, bias).view(b, s, -1)).reshape(b * s, -1)
+                    pending = bias = None                    # it has added everything
                     continue
                 x, pending = blk(x, pending, bias, (b, s))
                 # a block that ran as plain PyTorch has added everything and taken its bias gradient itself

@@ -175,6 +175,21 @@ def test_hooks_and_replaced_parts_are_called(make):
 
 
 @gpu
+@pytest.mark.parametrize("hooked", [(1,), (0, 2), (1, 2), (3,)])
+def test_blocks_with_hooks_between_fused_ones(hooked):
+    """Every gradient, the last bias of each block among them, as without the hooks."""
+    idx, tgt = _batch()
+    want, model, ref = _grads(_gpt2(layers=4), idx, tgt), _gpt2(layers=4), _reference(_gpt2(layers=4), idx, tgt)
+    for i in hooked:
+        model.blocks[i].register_forward_hook(lambda mod, args, out: None)
+    names = ["loss"] + [n for n, _ in model.named_parameters()]
+    for n, a, b, r in zip(names, _grads(model, idx, tgt), want, ref):
+        if not n.endswith("k.bias"):                   # zero but for rounding
+            ea, eb = ((t.double() - r).norm() / r.norm() for t in (a, b))
+            assert ea <= 1.5 * eb + 2.0 ** -9, (n, ea.item(), eb.item())
+
+
+@gpu
 def test_input_changed_in_place_is_noticed():
     blk = _gpt2().blocks[0]
     x = torch.randn(2, 8, 128, device="cuda").to(torch.bfloat16).requires_grad_(True)
