@@ -6,7 +6,7 @@ import torch.nn as nn
 
 from mccl_b200.models.gpt2 import GPT2, GPT2Config
 from mccl_b200.models.llama import Llama, LlamaConfig
-from mccl_b200.utils.fuse import as_made
+from mccl_b200.utils.fuse import as_made, undisturbed
 
 gpu = pytest.mark.gpu
 
@@ -26,6 +26,38 @@ def test_as_made_sees_replacements_and_hooks():
     assert not as_made(m, nn.Linear)
     w = nn.utils.parametrizations.weight_norm(nn.Linear(4, 4))
     assert not as_made(w, nn.Linear)
+
+
+def test_as_made_sees_an_embeddings_options_and_weights_of_another_class():
+    assert as_made(nn.Embedding(4, 4), nn.Embedding)
+    for option in ({"padding_idx": 0}, {"max_norm": 1.0}, {"scale_grad_by_freq": True}, {"sparse": True}):
+        assert not as_made(nn.Embedding(4, 4, **option), nn.Embedding)
+
+    class Mine(torch.Tensor):
+        pass
+
+    m = nn.Linear(4, 4)
+    m._parameters["weight"] = m.weight.detach().as_subclass(Mine)
+    assert not as_made(m, nn.Linear)
+
+
+def test_modes_and_replaced_functions_are_seen(monkeypatch):
+    from torch.overrides import TorchFunctionMode
+
+    class Watch(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    assert undisturbed()
+    with Watch():
+        assert not undisturbed()
+    with torch.device("cpu"):                    # where new tensors go is all that this mode says
+        assert undisturbed()
+    h = nn.modules.module.register_module_forward_hook(lambda mod, args, out: None)
+    assert not undisturbed()
+    h.remove()
+    monkeypatch.setattr(nn.functional, "scaled_dot_product_attention", lambda *a, **k: None)
+    assert not undisturbed()
 
 
 def _comm():
@@ -187,6 +219,28 @@ def test_blocks_with_hooks_between_fused_ones(hooked):
         if not n.endswith("k.bias"):                   # zero but for rounding
             ea, eb = ((t.double() - r).norm() / r.norm() for t in (a, b))
             assert ea <= 1.5 * eb + 2.0 ** -9, (n, ea.item(), eb.item())
+
+
+@gpu
+@pytest.mark.parametrize("make", [_gpt2, _llama])
+def test_an_embedding_with_a_padding_row(make):
+    idx, tgt = _batch()
+    model = make()
+    name = "wte" if make is _gpt2 else "embed"
+    emb = nn.Embedding(*getattr(model, name).weight.shape, padding_idx=int(idx[0, 0])).to(device="cuda", dtype=torch.bfloat16)
+    setattr(model, name, emb)
+    model(idx, tgt).backward()
+    if make is _llama:
+        assert emb.weight.grad[idx[0, 0]].abs().sum() == 0 and emb.weight.grad.abs().sum() > 0
+        return
+    row, got = int(idx[0, 0]), emb.weight.grad.clone()         # GPT-2's weight has the tied projection's gradient as well
+    emb.padding_idx = None
+    model.zero_grad(set_to_none=True)
+    model(idx, tgt).backward()
+    other = torch.ones(len(got), dtype=torch.bool, device="cuda")
+    other[row] = False
+    assert not torch.equal(got[row], emb.weight.grad[row])
+    assert (got[other].float() - emb.weight.grad[other].float()).norm() <= 2.0 ** -6 * got.float().norm()
 
 
 @gpu
