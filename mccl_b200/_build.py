@@ -1,12 +1,13 @@
 """In-tree build of libmccl.so (host C++ with g++, device code with nvcc for sm_100a) and of the torch binding.
 
 `python -m mccl_b200._build` compiles every file under csrc/ that changed since its object was made, or whose headers did, and links
-mccl_b200/lib/libmccl.so, and mccl_torch.so from csrc/torch.  Objects live in build/ (ignored by git); the shared libraries stay inside the
-package so that they travel with the source tree.
+mccl_b200/lib/libmccl.so, and from csrc/torch the torch binding, one file per torch version (its C++ interface is no other's).  Objects
+live in build/ (ignored by git); the shared libraries stay inside the package so that they travel with the source tree.
 """
 from __future__ import annotations
 
 import concurrent.futures as cf
+import fcntl
 import os
 import shutil
 import subprocess
@@ -18,7 +19,6 @@ CSRC = ROOT / "csrc"
 OBJ = ROOT / "build" / "obj"
 TORCH_SRC = CSRC / "torch"                       # the torch binding: a library of its own, so that libmccl needs no torch
 LIB = ROOT / "mccl_b200" / "lib" / "libmccl.so"
-EXT = LIB.with_name("mccl_torch.so")
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 
@@ -57,12 +57,24 @@ def _compile(src: Path, obj: Path, extra: list[str]) -> tuple[Path, str]:
     return src, log
 
 
+def _torch_tag(version: str) -> str:
+    return "".join(c if c.isalnum() or c in ".-" else "_" for c in version)
+
+
+def ext_path(version: str) -> Path:
+    """The binding's file for this version of torch."""
+    return LIB.with_name(f"mccl_torch-{_torch_tag(version)}.so")
+
+
 def _torch_flags() -> tuple[list[str], list[str]] | None:
-    """Compile and link flags of the torch binding; None where torch is not installed (the tcp transport works without)."""
+    """Compile and link flags of the torch binding; None where torch is not installed or has no CUDA (the tcp transport and
+    numpy arrays work without)."""
     import sysconfig
     try:
         import torch
     except ImportError:
+        return None
+    if torch.version.cuda is None:
         return None
     inc = Path(torch.__file__).parent / "include"
     lib = Path(torch.__file__).parent / "lib"
@@ -88,14 +100,26 @@ def _link(cmd: list[str], target: Path) -> None:
 def build(verbose: bool = False, force: bool = False) -> Path:
     if shutil.which(NVCC) is None and not Path(NVCC).exists():
         raise RuntimeError(f"nvcc not found at {NVCC}")
+    OBJ.mkdir(parents=True, exist_ok=True)
+    with open(OBJ.parent / "lock", "w") as lock:         # ranks that find a library missing build it once
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        return _build_locked(verbose, force)
+
+
+def _build_locked(verbose: bool, force: bool) -> Path:
     srcs = sorted(list(CSRC.rglob("*.cc")) + list(CSRC.rglob("*.cu")))
     torch_flags = _torch_flags()
+    if torch_flags is not None:
+        import torch
+        ext = ext_path(torch.__version__)
     jobs, objs, ext_objs = [], [], []
     for s in srcs:
         in_ext = TORCH_SRC in s.parents
         if in_ext and torch_flags is None:
             continue
         o = OBJ / s.relative_to(CSRC).with_suffix(s.suffix + ".o")
+        if in_ext:
+            o = OBJ / ext.stem / o.name
         (ext_objs if in_ext else objs).append(o)
         if force or _stale(s, o):
             jobs.append((s, o, torch_flags[0] if in_ext else []))
@@ -111,10 +135,10 @@ def build(verbose: bool = False, force: bool = False) -> Path:
                "-Xlinker", "--no-undefined", "-lpthread", "-ldl", "-lrt"], LIB)
         if verbose:
             print(f"[mccl build] linked {LIB.relative_to(ROOT)}")
-    if ext_objs and (jobs or not EXT.exists()):
-        _link(["g++", "-shared", *map(str, ext_objs), *torch_flags[1]], EXT)
+    if ext_objs and (jobs or not ext.exists()):
+        _link(["g++", "-shared", *map(str, ext_objs), *torch_flags[1]], ext)
         if verbose:
-            print(f"[mccl build] linked {EXT.relative_to(ROOT)}")
+            print(f"[mccl build] linked {ext.relative_to(ROOT)}")
     return LIB
 
 

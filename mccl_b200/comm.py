@@ -81,10 +81,12 @@ def _stream_of(buf, stream):
 
 
 def _fast_calls():
+    """The collectives on torch tensors in C++; None without torch or where the binding has not been built: every call has the
+    general path, so a communicator needs nothing but libmccl."""
     if torch is None:
         return None
     from . import _ext
-    return _ext.load()
+    return _ext.load_if_built()
 
 
 def _fast_stream(stream) -> Optional[int]:
@@ -162,7 +164,7 @@ class Communicator:
             L.check(self._lib.mcclCommInitRankConfig(C.byref(self._h), n_ranks, uid, rank, C.byref(cfg)),
                     "mcclCommInitRankConfig")
         self._sym = {}
-        # The calls on torch tensors in C++ (None without torch); they answer -1 for whatever needs the general path here.
+        # They answer -1 for whatever needs the general path here.
         self._fast = _fast_calls()
         _live.add(self)
 

@@ -255,6 +255,31 @@ def test_single_rank_tcp_comm():
     comm.finalize(); comm.destroy()
 
 
+def test_communicator_without_the_torch_binding(monkeypatch, tmp_path):
+    """No binding for this torch, or one that does not load: the general path answers, and nothing is built."""
+    import torch
+    import mccl_b200 as mccl
+    from mccl_b200 import _build, _ext
+    monkeypatch.setattr(_ext, "_mod", None)
+    monkeypatch.setattr(_build, "build", lambda *a, **k: pytest.fail("a communicator started a build"))
+    broken = tmp_path / "broken.so"
+    broken.write_bytes(b"no library")
+    for path in (tmp_path / "missing.so", broken):
+        monkeypatch.setattr(_build, "ext_path", lambda version, path=path: path)
+        comm = mccl.Communicator(1, mccl.get_unique_id(), 0, transport="tcp")
+        x, y = torch.arange(5.0), torch.empty(5)
+        comm.all_reduce(x, y)
+        comm.all_gather(x, y)
+        assert torch.equal(x, y)
+        comm.destroy()
+
+
+def test_torch_binding_is_one_file_per_version():
+    from mccl_b200 import _build
+    a, b = _build.ext_path("2.11.0+cu128"), _build.ext_path("2.12.0+cu128")
+    assert a != b and a.parent == b.parent == _build.LIB.parent and "+" not in a.name
+
+
 def test_unknown_transport_is_refused():
     with pytest.raises(mccl.MCCLError) as e:
         mccl.Communicator(1, mccl.get_unique_id(), 0, transport="carrier-pigeon")
