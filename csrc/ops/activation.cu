@@ -33,7 +33,9 @@ __device__ __forceinline__ uint4 pack(const float* f) {
   return q;
 }
 __device__ __forceinline__ float rounded(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+// To fp32 precision, as the tensor library's: the passes are bound by memory all the same.
+__device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return x / (1.f + expf(-x)); }
 
 // The tanh-GELU is x * s with s = (1 + tanh(z)) / 2 = 1 / (1 + exp(-2 z)), z = c (x + a x^3): one exponential and one
 // reciprocal, absolute error of s a few 2^-23, and its gradient is s + 2 z' x s (1 - s).  Results are to the last bit what the
@@ -126,7 +128,7 @@ __device__ __forceinline__ uint4 geluGrad8(const uint4& x, const uint4& dy) {
 }
 
 // An operation maps IN input values to OUT output values.
-struct SiluFwd { static constexpr int IN = 1, OUT = 1; __device__ static void f(const float* i, float* o) { o[0] = i[0] * sigmoid(i[0]); } };
+struct SiluFwd { static constexpr int IN = 1, OUT = 1; __device__ static void f(const float* i, float* o) { o[0] = silu(i[0]); } };
 struct SiluBwd {                                   // (pre-activation, gradient) -> gradient of the pre-activation
   static constexpr int IN = 2, OUT = 1;
   __device__ static void f(const float* i, float* o) { const float s = sigmoid(i[0]); o[0] = i[1] * (s * (1.f + i[0] * (1.f - s))); }
@@ -141,7 +143,7 @@ struct SiluBoth {                                  // (pre-activation, gradient)
 };
 struct SwigluFwd {                                 // (gate, up) -> silu(gate) * up, the activation rounded before the product
   static constexpr int IN = 2, OUT = 1;
-  __device__ static void f(const float* i, float* o) { o[0] = rounded(i[0] * sigmoid(i[0])) * i[1]; }
+  __device__ static void f(const float* i, float* o) { o[0] = rounded(silu(i[0])) * i[1]; }
 };
 struct SwigluBwd {                                 // (gate, up, gradient) -> product (for the weight gradient behind), d gate, d up
   static constexpr int IN = 3, OUT = 3;

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kChunk) routeCountKernel(const __nv_bfloat16* 
     best = 0;
     for (int e = 0; e < E; ++e) { const float v = __bfloat162float(x[e]); if (v > m) { m = v; best = e; } }
     float s = 0.f;
-    for (int e = 0; e < E; ++e) s += __expf(__bfloat162float(x[e]) - m);
+    for (int e = 0; e < E; ++e) s += expf(__bfloat162float(x[e]) - m);
     gate[t] = rounded(1.f / s);
     lse[t] = m + logf(s);
   }
@@ -209,9 +209,9 @@ __global__ void __launch_bounds__(kRowThreads) tokenBackwardKernel(const uint4* 
     const __nv_bfloat16* x = logits + (int64_t)(t0 + i) * E;
     const int best = f[i] < 0 ? 0 : f[i] / capacity;
     const float l = lse[t0 + i], dg = f[i] < 0 ? 0.f : rounded(dgate[t0 + i]);
-    const float pb = __expf(__bfloat162float(x[best]) - l);
+    const float pb = expf(__bfloat162float(x[best]) - l);
     for (int e = lane; e < E; e += 32) {
-      const float p = __expf(__bfloat162float(x[e]) - l);
+      const float p = expf(__bfloat162float(x[e]) - l);
       const float d = rounded(p * ((e == best ? dg : 0.f) - pb * dg));
       dl[e * kTok + i] = d;
       dlogits[(int64_t)(t0 + i) * E + e] = __float2bfloat16_rn(d);

@@ -69,6 +69,20 @@ def test_silu_both(n):
     _close(du, torch.autograd.grad(want, ur, dh.double())[0])
 
 
+def test_silu_is_worked_out_in_full_fp32():
+    """With a relative error of e before it is rounded, a result rounds apart from the exact one with a probability of 2 e / 2^-8 at
+    most.  Arguments where an exponential of the product with log2(e) alone has an error of 2^-19."""
+    from mccl_b200 import _ext
+    n = 1 << 22
+    u, dh = (-80 + 40 * torch.rand(n, device="cuda")).to(torch.bfloat16), _bf(n)
+    h, du = _ext.load().silu_both(u, dh)
+    ur = u.double().requires_grad_(True)
+    want = F.silu(ur)
+    g = torch.autograd.grad(want, ur, dh.double())[0]
+    for got, exact, e in ((h, want, 2.0 ** -22), (du, g, 2.0 ** -21)):
+        assert (got != exact.to(torch.bfloat16)).float().mean().item() <= 2 * e / U
+
+
 def test_gelu_of_every_value_is_what_the_tensor_library_rounds_to():
     from mccl_b200 import _ext
     x = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
