@@ -233,8 +233,7 @@ extern "C" mcclResult_t mcclCrossEntropyMean(const void* logits, int64_t rows, i
   if (mean == nullptr) return mcclInvalidArgument;
   const mcclResult_t rc = mcclCrossEntropyForward(logits, rows, ld, vocab, targets, loss, lse, stream);
   if (rc != mcclSuccess) return rc;
-  meanKernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(loss, rows, inverse != nullptr ? targets : nullptr, vocab,
-                                                                         mean, inverse);     // no rows: 0 / 0, as a mean over none
+  meanKernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(loss, rows, inverse != nullptr ? targets : nullptr, vocab, mean, inverse);
   return cudaGetLastError() == cudaSuccess ? mcclSuccess : mcclSystemError;
 }
 

@@ -7,7 +7,7 @@ namespace {
 // ---- LayerNorm ------------------------------------------------------------------------------------------------------
 bool normSupported(const Tensor& x, const Tensor& w, const Tensor& b) {
   const int64_t d = x.dim() > 0 ? x.size(-1) : 0;
-  return !recorded() && ordinary(x) && ordinary(w) && ordinary(b) && bf16Cuda(x) && bf16Cuda(w) && bf16Cuda(b) &&
+  return x.numel() > 0 && !recorded() && ordinary(x) && ordinary(w) && ordinary(b) && bf16Cuda(x) && bf16Cuda(w) && bf16Cuda(b) &&
          layerNormWidth(d) && w.numel() == d && b.numel() == d && w.is_contiguous() && b.is_contiguous() && aligned16(w) && aligned16(b);
 }
 
@@ -37,7 +37,6 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
       return {std::get<0>(r).view(x.sizes()), std::get<1>(r), std::get<2>(r), Tensor()};
     }
     Tensor dx = at::empty(x.sizes(), x.options()), dw = at::empty({d}, w.options()), db = at::empty({d}, w.options());
-    if (rows == 0) { dw.zero_(); db.zero_(); return {dx, dw, db, Tensor()}; }
     Tensor dy = g[0].contiguous();
     if (!aligned16(dy)) dy = dy.clone();
     Tensor partial = at::empty({(int64_t)mcclLayerNormPartials(rows) * 2 * d}, stats.options());

@@ -58,6 +58,23 @@ def test_layer_norm_widths(rows, d):
         _close(g, r)
 
 
+@pytest.mark.parametrize("d", [128, 256, 768, 1024])
+def test_layer_norm_of_no_rows(d):
+    from mccl_b200.ops.norm import FusedLayerNorm
+    layer = FusedLayerNorm(d).to(device="cuda", dtype=torch.bfloat16)
+    x = torch.empty(0, d, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    y = layer(x)
+    assert y.shape == x.shape
+    dx, dw, db = torch.autograd.grad(y, [x, layer.weight, layer.bias], torch.empty_like(y))
+    assert dx.shape == x.shape and dw.abs().sum() == 0 and db.abs().sum() == 0
+
+
+def test_cross_entropy_of_no_rows_is_refused():
+    from mccl_b200.ops.loss import fused_cross_entropy
+    with pytest.raises(RuntimeError):
+        fused_cross_entropy(torch.empty(0, 64, device="cuda", dtype=torch.bfloat16), torch.empty(0, device="cuda", dtype=torch.int64))
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 4095, 8192, 8200 * 3 + 5])
 def test_silu_both(n):
     from mccl_b200 import _ext
