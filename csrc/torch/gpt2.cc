@@ -295,8 +295,11 @@ struct EmbedFn : torch::autograd::Function<EmbedFn> {
         ret[1] = dt = at::zeros(table.sizes(), table.options());
         if (withPos) ret[2] = dp = at::zeros(pos.sizes(), pos.options());
       } else {
-        // Too many tokens for the kernel's scan: the sorting form of the tensor library.
-        ret[1] = at::embedding_dense_backward(dy, idx.view({T}), V, -1, false);
+        // Too many tokens for the kernel's scan: the sorting form of the tensor library, which does not look whether an index is
+        // in the table; those that are not (their rows were NaN) go to a row behind it.
+        Tensor i = idx.view({T});
+        i = at::where(at::logical_and(i.ge(0), i.lt(V)), i, V);
+        ret[1] = at::embedding_dense_backward(dy, i, V + 1, -1, false).narrow(0, 0, V);
         if (withPos) {
           ret[2] = at::zeros(pos.sizes(), pos.options());
           ret[2].narrow(0, 0, seq).copy_(dy.view({T / seq, seq, d}).sum(0));

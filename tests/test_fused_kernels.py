@@ -154,6 +154,22 @@ def test_embedding_adds_repeated_tokens(vocab, d, tokens, with_pos):
         _close(g, r)
 
 
+@pytest.mark.parametrize("tokens", [300, 16384, 16400])
+def test_embedding_indices_outside_the_table(tokens):
+    """A NaN row forward, no gradient backward: with the kernel and beyond its number of tokens."""
+    from mccl_b200 import _ext
+    vocab, d = 40, 64
+    idx = torch.randint(0, vocab, (tokens,), device="cuda")
+    idx[0], idx[7] = vocab, -3
+    table = _bf(vocab, d).requires_grad_(True)
+    y = _ext.load().decoder_embed(idx, table, None, False)
+    assert y[[0, 7]].isnan().all() and not y[1:7].isnan().any()
+    dy = _bf(tokens, d)
+    ok = (idx >= 0) & (idx < vocab)
+    want = torch.zeros(vocab, d, device="cuda", dtype=torch.float64).index_add_(0, idx[ok], dy[ok].double())
+    _close(torch.autograd.grad(y, table, dy)[0], want)
+
+
 @pytest.mark.parametrize("rows,vocab,width", [(1, 50257, 50304), (2, 8, 8), (5, 257, 257), (37, 4096, 4096), (74, 33000, 33001), (300, 1000, 1024), (444, 8192, 8192), (445, 8193, 8193)])
 def test_cross_entropy_mean_forms(rows, vocab, width):
     """Few rows are shared by several CTAs; an odd width leaves rows unaligned; targets left out."""
