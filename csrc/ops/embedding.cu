@@ -11,7 +11,7 @@
 namespace {
 
 constexpr int kEmbThreads = 128;
-constexpr int kMaxTokens = 16384;             // of the backward pass: a token that occurs again scans all of them
+constexpr int kMaxTokens = 16384;             // of the backward pass: every token that occurs in two chunks is looked for in all of them
 constexpr int kMaxVecs = 4 * kEmbThreads;     // 16-byte pieces of a row: D <= 4096
 
 __device__ __forceinline__ void unpack(const uint4& q, float* f) {
@@ -53,14 +53,57 @@ __global__ void countTokensKernel(const int64_t* idx, int n, int64_t vocab, int*
   if (t < n && idx[t] >= 0 && idx[t] < vocab) atomicAdd(&count[idx[t]], 1);
 }
 
-// One CTA per token.  A token that occurs once adds its row.  Of one that occurs again, the first occurrence adds the sum of
-// all rows in token order (a fixed order, in fp32), which it finds by scanning the indices; the others leave as soon as the
-// scan shows them an earlier one.
+constexpr int kChunk = kEmbThreads;           // tokens that one CTA adds up
+constexpr int kMaxChunks = kMaxTokens / kChunk;
+constexpr int kScan = 8;                      // chunks looked through at once
+
+// acc += row r of a [*, vecs] matrix for every r of `list` in its order, four rows in flight; fp32 rows (two pieces) or bf16.
+template <int VPT, bool F32>
+__device__ __forceinline__ void addRows(float (*acc)[8], const uint4* rows, const int* list, int from, int n, int vecs) {
+  constexpr int P = F32 ? 2 : 1;
+  for (int k = from; k < n; k += 4) {
+    uint4 q[4][VPT][P];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) {
+        const int v = threadIdx.x + j * kEmbThreads;
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+          q[u][j][p] = k + u < n && v < vecs ? __ldcg(rows + ((int64_t)list[k + u] * vecs + v) * P + p) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) {
+        float f[8];
+        if (F32) {
+#pragma unroll
+          for (int p = 0; p < P; ++p) {
+            f[4 * p] = __uint_as_float(q[u][j][p].x); f[4 * p + 1] = __uint_as_float(q[u][j][p].y);
+            f[4 * p + 2] = __uint_as_float(q[u][j][p].z); f[4 * p + 3] = __uint_as_float(q[u][j][p].w);
+          }
+        } else {
+          unpack(q[u][j][0], f);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[j][e] += f[e];
+      }
+  }
+}
+
+// One CTA per token.  A token that occurs once adds its row.  Of one that occurs again, the first of a chunk of 128 tokens adds up the
+// rows in the chunk; if there are others elsewhere the sum stays in fp32 at its place in `partial`, and the CTA that finds all
+// of the token's rows done adds the chunks' sums, in token order whoever it is, so the result does not depend on the order of
+// arrival.  Bound by the rows' memory (2 bytes an element) and, for a token that fills the batch, by 32 turns of a chunk and
+// 32 of the chunks' sums; with one CTA for all rows of a token 16384 equal ones were 4096 turns.
 template <int VPT>
-__global__ void __launch_bounds__(kEmbThreads) tableGradKernel(const int64_t* idx, const uint4* dy, const int* count, int n, int64_t vocab,
-                                                               int vecs, uint4* grad) {
-  __shared__ int found[kEmbThreads];
-  __shared__ int warpFound[kEmbThreads / 32];
+__global__ void __launch_bounds__(kEmbThreads) tableGradKernel(const int64_t* idx, const uint4* dy, const int* count, int* done, uint4* partial,
+                                                               int n, int64_t vocab, int vecs, uint4* grad) {
+  constexpr int W = kEmbThreads / 32;
+  __shared__ int found[kMaxChunks > kChunk ? kMaxChunks : kChunk];
+  __shared__ unsigned hits[kScan][W];
+  __shared__ int arrived;
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t id = idx[t];
   if (id < 0 || id >= vocab) return;
@@ -72,39 +115,56 @@ __global__ void __launch_bounds__(kEmbThreads) tableGradKernel(const int64_t* id
   }
   const int all = count[id];
   if (all > 1) {
-    int seen = 0;
-    for (int base = 0; base < n && seen < all; base += kEmbThreads) {
-      const bool hit = base + tid < n && idx[base + tid] == id;
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) warpFound[warp] = __popc(m);
-      __syncthreads();
-      int before = 0, total = 0;
+    const int base = t / kChunk * kChunk;
+    const bool hit = base + tid < n && idx[base + tid] == id;
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) hits[0][warp] = m;
+    __syncthreads();
+    int before = 0, here = 0;
 #pragma unroll
-      for (int w = 0; w < kEmbThreads / 32; ++w) { if (w < warp) before += warpFound[w]; total += warpFound[w]; }
-      if (hit) found[before + __popc(m & ((1u << lane) - 1u))] = base + tid;
-      __syncthreads();
-      if (total > 0 && seen == 0 && found[0] != t) return;       // an earlier occurrence does the work
-      for (int k = seen == 0 ? 1 : 0; k < total; k += 4) {
-        uint4 q[4][VPT];
+    for (int w = 0; w < W; ++w) { const int c = __popc(hits[0][w]); if (w < warp) before += c; here += c; }
+    if (hit) found[before + __popc(m & ((1u << lane) - 1u))] = base + tid;
+    __syncthreads();
+    if (found[0] != t) return;                                       // an earlier one of the chunk does the work
+    addRows<VPT, false>(acc, dy, found, 1, here, vecs);
+    if (here < all) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int j = 0; j < VPT; ++j) {
-            const int v = tid + j * kEmbThreads;
-            q[u][j] = k + u < total && v < vecs ? dy[(int64_t)found[k + u] * vecs + v] : make_uint4(0, 0, 0, 0);
-          }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int j = 0; j < VPT; ++j) {
-            float f[8];
-            unpack(q[u][j], f);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc[j][e] += f[e];
-          }
+      for (int j = 0; j < VPT; ++j) {
+        const int v = tid + j * kEmbThreads;
+        if (v >= vecs) continue;
+        float4* to = reinterpret_cast<float4*>(partial + ((int64_t)t * vecs + v) * 2);
+        to[0] = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+        to[1] = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
       }
-      seen += total;
+      __threadfence();
       __syncthreads();
+      if (tid == 0) arrived = atomicAdd(&done[id], here) + here;
+      __syncthreads();
+      if (arrived < all) return;                                     // whoever completes the count adds up
+      __threadfence();
+      int firsts = 0;                                                // the first token of this kind in every chunk
+      for (int c0 = 0; c0 * kChunk < n; c0 += kScan) {
+#pragma unroll
+        for (int u = 0; u < kScan; ++u) {
+          const int i = (c0 + u) * kChunk + tid;
+          const unsigned b = __ballot_sync(0xffffffffu, i < n && idx[i] == id);
+          if (lane == 0) hits[u][warp] = b;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kScan; ++u) {
+          int first = -1;
+#pragma unroll
+          for (int w = W - 1; w >= 0; --w) if (hits[u][w]) first = w * 32 + __ffs(hits[u][w]) - 1;
+          if (first >= 0) { if (tid == 0) found[firsts] = (c0 + u) * kChunk + first; ++firsts; }
+        }
+        __syncthreads();
+      }
+#pragma unroll
+      for (int j = 0; j < VPT; ++j)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[j][e] = 0.f;
+      addRows<VPT, true>(acc, partial, found, 0, firsts, vecs);
     }
   }
 #pragma unroll
@@ -161,23 +221,42 @@ mcclResult_t mcclEmbeddingForward(const int64_t* idx, const void* table, const v
 
 int mcclEmbeddingMaxTokens(void) { return kMaxTokens; }
 
-// tableGrad rows += the rows of dy with their index; posGrad (may be null) += dy summed over the batch.  count: vocab ints of work memory.
-mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, int32_t* count, int64_t tokens, int seq,
-                                   int64_t vocab, int D, mcclStream_t stream) {
-  if (!idx || !dy || !tableGrad || !count || tokens <= 0 || tokens > kMaxTokens || seq <= 0 || tokens % seq || D <= 0 || D % 8 ||
-      D / 8 > kMaxVecs || !aligned16(dy) || !aligned16(tableGrad) || !aligned16(posGrad)) return mcclInvalidArgument;
+// Bytes of work memory of the function below.
+int64_t mcclEmbeddingWork(int64_t tokens, int64_t vocab, int D) {
+  return (2 * vocab * (int64_t)sizeof(int32_t) + 15) / 16 * 16 + tokens * D * (int64_t)sizeof(float);
+}
+
+// tableGrad rows += the rows of dy with their index; posGrad (may be null) += dy summed over the batch.  work: 16-byte aligned.
+mcclResult_t mcclEmbeddingBackwardWork(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, void* work, int64_t tokens, int seq,
+                                       int64_t vocab, int D, mcclStream_t stream) {
+  if (!idx || !dy || !tableGrad || !work || tokens <= 0 || tokens > kMaxTokens || seq <= 0 || tokens % seq || D <= 0 || D % 8 || vocab <= 0 ||
+      D / 8 > kMaxVecs || !aligned16(dy) || !aligned16(tableGrad) || !aligned16(posGrad) || !aligned16(work)) return mcclInvalidArgument;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int n = (int)tokens, vecs = D / 8;
   const uint4* g = static_cast<const uint4*>(dy);
   uint4* tg = static_cast<uint4*>(tableGrad);
-  if (cudaMemsetAsync(count, 0, vocab * sizeof(int32_t), s) != cudaSuccess) return mcclSystemError;
+  int* count = static_cast<int*>(work);
+  int* done = count + vocab;
+  uint4* partial = reinterpret_cast<uint4*>(static_cast<char*>(work) + (2 * vocab * (int64_t)sizeof(int32_t) + 15) / 16 * 16);
+  if (cudaMemsetAsync(count, 0, 2 * vocab * sizeof(int32_t), s) != cudaSuccess) return mcclSystemError;
   countTokensKernel<<<(n + 255) / 256, 256, 0, s>>>(idx, n, vocab, count);
-  if (vecs <= kEmbThreads) tableGradKernel<1><<<n, kEmbThreads, 0, s>>>(idx, g, count, n, vocab, vecs, tg);
-  else if (vecs <= 2 * kEmbThreads) tableGradKernel<2><<<n, kEmbThreads, 0, s>>>(idx, g, count, n, vocab, vecs, tg);
-  else tableGradKernel<4><<<n, kEmbThreads, 0, s>>>(idx, g, count, n, vocab, vecs, tg);
+  if (vecs <= kEmbThreads) tableGradKernel<1><<<n, kEmbThreads, 0, s>>>(idx, g, count, done, partial, n, vocab, vecs, tg);
+  else if (vecs <= 2 * kEmbThreads) tableGradKernel<2><<<n, kEmbThreads, 0, s>>>(idx, g, count, done, partial, n, vocab, vecs, tg);
+  else tableGradKernel<4><<<n, kEmbThreads, 0, s>>>(idx, g, count, done, partial, n, vocab, vecs, tg);
   const int64_t perSeq = (int64_t)seq * vecs;
   if (posGrad != nullptr) posGradKernel<<<(unsigned)((perSeq + 255) / 256), 256, 0, s>>>(g, n / seq, perSeq, static_cast<uint4*>(posGrad));
   return launchedOk();
+}
+
+// The same with work memory of its own, allocated and freed in the stream's order; count: not used.
+mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, int32_t* count, int64_t tokens, int seq,
+                                   int64_t vocab, int D, mcclStream_t stream) {
+  if (!count || tokens <= 0 || tokens > kMaxTokens || vocab <= 0 || D <= 0 || D / 8 > kMaxVecs) return mcclInvalidArgument;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  void* work = nullptr;
+  if (cudaMallocAsync(&work, mcclEmbeddingWork(tokens, vocab, D), s) != cudaSuccess) { cudaGetLastError(); return mcclSystemError; }
+  const mcclResult_t rc = mcclEmbeddingBackwardWork(idx, dy, tableGrad, posGrad, work, tokens, seq, vocab, D, stream);
+  return cudaFreeAsync(work, s) == cudaSuccess ? rc : mcclSystemError;
 }
 
 }  // extern "C"

@@ -307,9 +307,9 @@ struct EmbedFn : torch::autograd::Function<EmbedFn> {
         return once(std::move(ret));
       }
     }
-    Tensor count = at::empty({V}, idx.options().dtype(at::kInt));
-    check(mcclEmbeddingBackward(idx.data_ptr<int64_t>(), dy.data_ptr(), dt.data_ptr(), withPos ? dp.data_ptr() : nullptr, count.data_ptr<int32_t>(), T, (int)seq, V,
-                                (int)d, streamOf(dy)), "mcclEmbeddingBackward");
+    Tensor work = at::empty({mcclEmbeddingWork(T, V, (int)d)}, dy.options().dtype(at::kByte));
+    check(mcclEmbeddingBackwardWork(idx.data_ptr<int64_t>(), dy.data_ptr(), dt.data_ptr(), withPos ? dp.data_ptr() : nullptr, work.data_ptr(), T,
+                                    (int)seq, V, (int)d, streamOf(dy)), "mcclEmbeddingBackwardWork");
     return once(std::move(ret));
   }
 };

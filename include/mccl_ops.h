@@ -83,8 +83,12 @@ mcclResult_t mcclColumnSums(const void* const* x, void* const* out, int n, int a
 /* ---- embedding: out[t] = table[idx[t]] + pos[t % seq] (pos nullable); the backward pass adds into the gradients ---------- */
 mcclResult_t mcclEmbeddingForward(const int64_t* idx, const void* table, const void* pos, void* out, int64_t tokens, int seq, int64_t vocab,
                                   int D, mcclStream_t stream);
-/* tokens <= mcclEmbeddingMaxTokens(), D <= 4096; count: vocab ints of work memory. */
+/* tokens <= mcclEmbeddingMaxTokens(), D <= 4096; work: mcclEmbeddingWork() bytes, 16-byte aligned. */
 int          mcclEmbeddingMaxTokens(void);
+int64_t      mcclEmbeddingWork(int64_t tokens, int64_t vocab, int D);
+mcclResult_t mcclEmbeddingBackwardWork(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, void* work, int64_t tokens, int seq,
+                                       int64_t vocab, int D, mcclStream_t stream);
+/* The same with work memory of its own, in the stream's order (count: vocab ints, not used). */
 mcclResult_t mcclEmbeddingBackward(const int64_t* idx, const void* dy, void* tableGrad, void* posGrad, int32_t* count, int64_t tokens, int seq,
                                    int64_t vocab, int D, mcclStream_t stream);
 

@@ -154,6 +154,21 @@ def test_embedding_adds_repeated_tokens(vocab, d, tokens, with_pos):
         _close(g, r)
 
 
+@pytest.mark.parametrize("tokens,common", [(127, 127), (129, 129), (257, 200), (1024, 512), (4097, 4000), (16384, 16384), (16384, 9000)])
+@pytest.mark.parametrize("d", [8, 1024, 2056])
+def test_embedding_gradient_of_a_token_that_fills_the_batch(tokens, common, d):
+    """Chunks of 128 tokens add up by themselves and meet in token order: the same bits from run to run."""
+    from mccl_b200 import _ext
+    vocab = 700
+    idx = torch.randint(0, vocab, (tokens,), device="cuda")
+    idx[torch.randperm(tokens, device="cuda")[:common]] = 11
+    table, dy = _bf(vocab, d).requires_grad_(True), _bf(tokens, d)
+    runs = [torch.autograd.grad(_ext.load().decoder_embed(idx, table, None, False), table, dy)[0] for _ in range(3)]
+    assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
+    want = torch.zeros(vocab, d, device="cuda", dtype=torch.float64).index_add_(0, idx, dy.double())
+    _close(runs[0], want)
+
+
 @pytest.mark.parametrize("tokens", [300, 16384, 16400])
 def test_embedding_indices_outside_the_table(tokens):
     """A NaN row forward, no gradient backward: with the kernel and beyond its number of tokens."""
