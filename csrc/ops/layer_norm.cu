@@ -525,7 +525,9 @@ cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
     opted[dev & 63] = true;
   }
   int cluster;
-  const int grid = colred::grid((a.rows + G * R * 4 - 1) / (G * R * 4), VPL == 1 && PARTS == 1 && R == 1 ? 3 : 2, &cluster);      // four rows per group before more CTAs pay
+  // Four rows a group, two turns where it takes two at a time: with four turns 512 x 1024 takes 15.4 us for 13.3, and more rows
+  // the same.
+  const int grid = colred::grid((a.rows + G * 4 - 1) / (G * 4), VPL == 1 && PARTS == 1 && R == 1 ? 3 : 2, &cluster);
   const int C = a.out.segments * a.D;
   const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES, PARTS, R>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
   return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, C, a.out, s);
