@@ -32,7 +32,7 @@ class FusedLayerNorm(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         w, b = self.weight, self.bias
-        if x.is_cuda:
+        if x.is_cuda and x.shape[-1] in _WIDTHS:
             y = _ext.load().layer_norm(x, w, b, self.eps)       # None where the kernels do not cover the case
             if y is not None:
                 return y

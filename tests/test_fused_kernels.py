@@ -58,6 +58,17 @@ def test_layer_norm_widths(rows, d):
         _close(g, r)
 
 
+def test_layer_norm_of_other_widths_is_torchs_own():
+    """Traced without a break and, under autocast, in fp32."""
+    from mccl_b200.ops.norm import FusedLayerNorm
+    layer, x = FusedLayerNorm(768).to(device="cuda", dtype=torch.bfloat16), _bf(4, 768)
+    want = F.layer_norm(x, (768,), layer.weight, layer.bias, layer.eps)
+    assert torch.equal(layer(x), want)
+    assert torch.equal(torch.compile(layer, backend="eager", fullgraph=True)(x), want)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert layer(x).dtype == torch.float32
+
+
 @pytest.mark.parametrize("d", [128, 256, 768, 1024])
 def test_layer_norm_of_no_rows(d):
     from mccl_b200.ops.norm import FusedLayerNorm
