@@ -24,9 +24,11 @@ from . import functional as PF
 
 class TensorParallelFFN:
     """Forward-only SiLU FFN on the two fused kernels (all-gather -> GEMM -> SiLU, GEMM -> reduce-scatter); owns the
-    symmetric buffers for one fixed (tokens, hidden, ffn) shape."""
+    symmetric buffers for one fixed (tokens, hidden, ffn) shape.  With `when_used`, on one rank (where an allocation needs
+    nobody else), they are made when one of them is asked for."""
 
-    def __init__(self, comm: Communicator, tokens: int, hidden: int, ffn: int, w_up: torch.Tensor, w_down: torch.Tensor):
+    def __init__(self, comm: Communicator, tokens: int, hidden: int, ffn: int, w_up: torch.Tensor, w_down: torch.Tensor,
+                 when_used: bool = False):
         n = comm.size
         if not G.supported(tokens, ffn // n, hidden, n) or not G.supported(tokens, hidden, ffn // n, n):
             raise ValueError("shapes must satisfy tokens % (128 n) == 0 and hidden, ffn/n % 64 == 0")
@@ -34,7 +36,18 @@ class TensorParallelFFN:
         assert w_up.dtype == w_down.dtype == torch.bfloat16 and w_up.is_contiguous() and w_down.is_contiguous()
         self.comm, self.n, self.tokens, self.hidden, self.ffn = comm, n, tokens, hidden, ffn
         self.w_up, self.w_down = w_up, w_down
-        dev = w_up.device
+        self.calls = 0
+        if not when_used or n > 1:
+            self._allocate()
+
+    def __getattr__(self, name: str):
+        if name not in ("x_shard", "partial", "flags", "ag_flags", "x_full", "h", "out", "accum") or name in self.__dict__:
+            raise AttributeError(name)
+        self._allocate()
+        return self.__dict__[name]
+
+    def _allocate(self) -> None:
+        comm, n, tokens, hidden, ffn, dev = self.comm, self.n, self.tokens, self.hidden, self.ffn, self.w_up.device
         # symmetric buffers (collective allocations, same order on every rank)
         self.x_shard = comm.empty((tokens // n, hidden), torch.bfloat16)
         self.partial = comm.empty((tokens, hidden), torch.bfloat16)
@@ -46,7 +59,6 @@ class TensorParallelFFN:
         self.h = torch.empty(tokens, ffn // n, device=dev, dtype=torch.bfloat16)
         self.out = torch.empty(tokens // n, hidden, device=dev, dtype=torch.bfloat16)
         self.accum = torch.empty(tokens // n, hidden, device=dev, dtype=torch.float32)
-        self.calls = 0
         torch.cuda.synchronize(dev)
         comm.host_barrier()
 
@@ -119,10 +131,12 @@ class FusedTensorParallelMLP(torch.nn.Module):
         dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
         self.w_up = torch.nn.Parameter(torch.randn(ffn // n, hidden, device=dev).mul_(hidden ** -0.5).to(torch.bfloat16))
         self.w_down = torch.nn.Parameter(torch.randn(hidden, ffn // n, device=dev).mul_(ffn ** -0.5).to(torch.bfloat16))
-        self.layer = TensorParallelFFN(comm, tokens, hidden, ffn, self.w_up.data, self.w_down.data)
+        # On one rank the node below keeps the pre-activation and the activation for the backward pass, and the pair of kernels with
+        # its buffers is only the way round it.
+        self.layer = TensorParallelFFN(comm, tokens, hidden, ffn, self.w_up.data, self.w_down.data, when_used=True)
 
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
-        if self.layer.comm.size == 1 and may_fuse(x_shard) and x_shard.shape == self.layer.x_shard.shape:     # nothing to gather or scatter: one node
+        if self.layer.comm.size == 1 and may_fuse(x_shard) and x_shard.shape == (self.layer.tokens, self.layer.hidden):     # nothing to gather or scatter: one node
             y = _ext.load().mlp(x_shard, self.w_up, self.w_down)
             if y is not None:
                 return y

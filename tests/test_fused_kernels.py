@@ -305,6 +305,20 @@ def test_mlp_keeps_the_sums(tokens, hidden, ffn):
         assert (g.double() - r).norm() <= 4 * U * r.norm()                # pre-activation, activation, its gradient, result
 
 
+def test_mlp_on_one_rank_takes_no_memory_that_it_does_not_use():
+    from mccl_b200.parallel.tp import FusedTensorParallelMLP
+    comm = _comm()
+    before = torch.cuda.memory_allocated()
+    layer = FusedTensorParallelMLP(comm, 1024, 512, 2048)
+    weights = 2 * 2 * 512 * 2048
+    assert torch.cuda.memory_allocated() - before <= weights + 4096
+    x = _bf(1024, 512)
+    y = layer(x)
+    with torch.autocast("cuda", dtype=torch.bfloat16):       # the pair of fused kernels, with its buffers
+        z = layer(x)
+    assert layer.layer.h.shape == (1024, 2048) and (y.float() - z.float()).norm() <= 4 * U * y.float().norm()
+
+
 @pytest.mark.parametrize("n", [1, 7, 16383, 16384, 16385, 4096 * 16384 + 9])
 def test_sum_of_squares_tile_edges(n):
     from mccl_b200.ops.optim import scratch_floats, sum_squares_
