@@ -19,8 +19,8 @@ void addRms(const Tensor& x, const Tensor* pending, const Tensor& w, double eps,
   counters().norm++;
 }
 
-// Gradient of the sum from those of h and, where defined, of the residual stream.
-// dh: up to three parts, added up on the way.
+// Gradient of the sum from those of h (up to three parts, added up on the way where there is a residual stream) and, where
+// defined, of the residual stream.
 Tensor addRmsBackward(const Tensor& sum, std::initializer_list<Tensor> parts, const Tensor& dres, const Tensor& w, const Tensor& rstd, GradSink& sink, Tensor* dw) {
   const int64_t T = sum.size(0), d = sum.size(1);
   Tensor dx = at::empty({T, d}, sum.options());
@@ -28,10 +28,7 @@ Tensor addRmsBackward(const Tensor& sum, std::initializer_list<Tensor> parts, co
   Tensor res = dres.defined() ? rows2d(dres, T, d) : Tensor();
   const void* dh[3] = {};
   int n = 0;
-  for (const Tensor& p : parts) {
-    if (n > 0 && !res.defined()) parts.begin()->add_(p);          // nobody uses the residual: the plain norm
-    else dh[n++] = p.data_ptr();
-  }
+  for (const Tensor& p : parts) dh[n++] = p.data_ptr();
   VectorGrads g(sink, {&w});
   check(mcclRmsNormBackward(sum.data_ptr(), dh[0], dh[1], dh[2], res.defined() ? res.data_ptr() : nullptr, w.data_ptr(), rstd.data_ptr<float>(),
                             dx.data_ptr(), g.t[0].data_ptr(), g.direct, partial.data_ptr<float>(), T, (int)d, streamOf(sum)), "mcclRmsNormBackward");
@@ -81,7 +78,6 @@ struct LlamaInFn : torch::autograd::Function<LlamaInFn> {
     c10::cuda::CUDAGuard guard(h.device());
     GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0), d = h.size(1);
-    TORCH_CHECK(g[1].defined() && g[2].defined() && g[3].defined(), "attention returns all three gradients");
     variable_list ret(12);
     Tensor dq, dk, dv = fromHeads(g[3], T, d);
     unrotate(g[1], g[2], T, d, ctx->saved_data["theta"].toDouble(), &dq, &dk);
@@ -122,7 +118,7 @@ struct LlamaOutFn : torch::autograd::Function<LlamaOutFn> {
     GradSink sink(ctx->saved_data["sink"].toBool());
     const int64_t T = h.size(0), d = h.size(1), b = ctx->saved_data["b"].toInt(), heads = ctx->saved_data["h"].toInt();
     variable_list ret(9);
-    Tensor dy = g[1].defined() ? rows2d(g[1], T, d) : at::zeros({T, d}, h.options());
+    Tensor dy = rows2d(g[1], T, d);
     Tensor dact = at::mm(dy, wd);
     // The product is worked out again from gate and up: the pass reads both anyway, and it need not be kept.
     Tensor act = at::empty(gate.sizes(), gate.options()), dgate = at::empty(gate.sizes(), gate.options());
