@@ -516,20 +516,16 @@ cudaError_t fwdAny(const LnFwdArgs& a, cudaStream_t s) {
 template <int W, int VPL, bool RMS, bool RES, int PARTS = 1, int R = 1>
 cudaError_t bwdLaunch(const LnBwdArgs& a, cudaStream_t s) {
   constexpr int G = kLnWarps / W;
-  static bool opted[64] = {false};             // 48 KB of column sums and the row slots: past the default limit
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!opted[dev & 63]) {
+  const int C = a.out.segments * a.D, smem = G * C * (int)sizeof(float);
+  if (smem > 40 << 10) {                       // with the row slots past the default limit; the same value from every thread and for every width
     const cudaError_t e = cudaFuncSetAttribute(lnBackwardKernel<W, VPL, RMS, RES, PARTS, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
     if (e != cudaSuccess) return e;
-    opted[dev & 63] = true;
   }
   int cluster;
   // Four rows a group, two turns where it takes two at a time: with four turns 512 x 1024 takes 15.4 us for 13.3, and more rows
   // the same.
   const int grid = colred::grid((a.rows + G * 4 - 1) / (G * 4), VPL == 1 && PARTS == 1 && R == 1 ? 3 : 2, &cluster);
-  const int C = a.out.segments * a.D;
-  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES, PARTS, R>, grid, cluster, kLnThreads, G * C * (int)sizeof(float), s, a);
+  const cudaError_t e = colred::launch(lnBackwardKernel<W, VPL, RMS, RES, PARTS, R>, grid, cluster, kLnThreads, smem, s, a);
   return e != cudaSuccess ? e : colred::addPartials(a.partial, grid, cluster, C, a.out, s);
 }
 

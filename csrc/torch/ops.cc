@@ -89,7 +89,7 @@ struct CrossEntropyFn : torch::autograd::Function<CrossEntropyFn> {
 // None where an argument is not what the kernels take (the caller says which).
 py::object crossEntropy(const Tensor& logits, const Tensor& targets, std::optional<int64_t> vocab) {
   if (!bf16Cuda(logits) || logits.dim() != 2 || logits.stride(1) != 1 || targets.scalar_type() != at::kLong || !targets.is_contiguous() ||
-      targets.numel() != logits.size(0)) return py::none();
+      targets.numel() != logits.size(0) || (!targets.is_cuda() && !targets.is_pinned())) return py::none();
   return py::cast(CrossEntropyFn::apply(logits, targets, vocab ? *vocab : logits.size(1)));
 }
 

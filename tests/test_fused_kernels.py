@@ -86,6 +86,12 @@ def test_cross_entropy_of_no_rows_is_refused():
         fused_cross_entropy(torch.empty(0, 64, device="cuda", dtype=torch.bfloat16), torch.empty(0, device="cuda", dtype=torch.int64))
 
 
+def test_cross_entropy_of_targets_on_the_host_is_refused():
+    from mccl_b200.ops.loss import fused_cross_entropy
+    with pytest.raises(ValueError):
+        fused_cross_entropy(_bf(3, 64), torch.zeros(3, dtype=torch.int64))
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 4095, 8192, 8200 * 3 + 5])
 def test_silu_both(n):
     from mccl_b200 import _ext
