@@ -117,6 +117,24 @@ def test_silu_is_worked_out_in_full_fp32():
         assert (got != exact.to(torch.bfloat16)).float().mean().item() <= 2 * e / U
 
 
+def test_silu_of_every_value_is_rounded_exactly():
+    import ctypes as C
+    from mccl_b200 import _lib
+    x = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    up = torch.randn(65536, device="cuda").to(torch.bfloat16)
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    lib, s = _lib.load(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    assert lib.mcclSiluForward(p(x), p(y), C.c_int64(65536), s) == 0
+    assert lib.mcclSwigluForward(p(x), p(up), p(z), C.c_int64(65536), s) == 0
+    want = F.silu(x.double()).to(torch.bfloat16)
+    library = F.silu(x)                            # beyond 88 the exponential overflows in fp32 and the result is zero
+    assert ((y == want) | (y == library) | (y.isnan() & want.isnan())).all()
+    assert (y == want)[x.abs() < 80].all()
+    ok = torch.isfinite(y)
+    assert torch.equal(z[ok], (y * up)[ok])
+
+
 def test_gelu_of_every_value_is_what_the_tensor_library_rounds_to():
     from mccl_b200 import _ext
     x = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
