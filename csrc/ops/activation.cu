@@ -244,10 +244,11 @@ mcclResult_t act(std::initializer_list<const void*> in, std::initializer_list<vo
 // ---- column sums ------------------------------------------------------------------------------------------------------
 // A CTA takes a strip of 64 x 8 columns (one vector per lane of two warps' width) and walks rows; four groups of 64 threads
 // take every fourth row.  Up to three matrices of the same shape in one launch (blockIdx.z).  With GELU the matrix is the
-// gradient of the activation, replaced by the gradient of the pre-activation on the way.  With PACK the matrices are also
-// written side by side into one [rows, segments x D] matrix, so that the products behind take them as one operand: for
-// 8192 tokens and width 1024 three weight gradients of 1024 x 1024 (77 us, too small to fill the GPU with large tiles) become
-// one product (34 us), three products that share an output become one, and this pass goes from 9.5 to 13.9 us.
+// gradient of the activation, replaced by the gradient of the pre-activation on the way (8192 x 4096: 44.9 us, 4.5 TB/s, of
+// which the last bits of the long form are 6 us).  With PACK the matrices are also written side by side into one
+// [rows, segments x D] matrix, so that the product behind takes them as one operand: for 8192 tokens and width 1024 three weight
+// gradients of 1024 x 1024 (77 us, too small to fill the GPU with large tiles) become one product (35 us), and this pass goes
+// from 9.5 to 14.0 us.
 enum ColMode { COL_SUM, COL_GELU, COL_PACK };
 constexpr int kStripVecs = 64, kStripCols = kStripVecs * 8, kRowGroups = kActThreads / kStripVecs;
 

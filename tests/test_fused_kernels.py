@@ -222,7 +222,7 @@ def test_embedding_indices_outside_the_table(tokens):
 
 @pytest.mark.parametrize("rows,vocab,width", [(1, 50257, 50304), (2, 8, 8), (5, 257, 257), (37, 4096, 4096), (74, 33000, 33001), (300, 1000, 1024), (444, 8192, 8192), (445, 8193, 8193)])
 def test_cross_entropy_mean_forms(rows, vocab, width):
-    """Few rows are shared by several CTAs; an odd width leaves rows unaligned; targets left out."""
+    """In the backward pass few rows are shared by several CTAs; an odd width leaves rows unaligned; targets left out."""
     from mccl_b200.ops.loss import fused_cross_entropy
     logits = _bf(rows, width, std=2.0).requires_grad_(True)
     t = torch.randint(0, vocab, (rows,), device="cuda")

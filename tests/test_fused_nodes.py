@@ -274,7 +274,7 @@ def test_gradients_reach_buckets_hooks_and_other_streams():
     want = [g.clone() for g in _grads(_gpt2(), idx, tgt)[1:]]
     model = _gpt2()
     ddp = DistributedDataParallel(model, None)
-    # In a bucket some sums are one product and not three: a few roundings of 2^-9 apart, so 2^-6 in all.  The gradient of a
+    # Attention's gradient may add in another order from run to run: a few roundings of 2^-9, so 2^-6 in all.  The gradient of a
     # key's bias is zero but for rounding and is left out.
     keep = [not n.endswith("k.bias") for n, _ in model.named_parameters()]
 
