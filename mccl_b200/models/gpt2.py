@@ -164,7 +164,7 @@ class GPT2(nn.Module):
         b, s = idx.shape
         w = self.wte.weight
         x = None
-        if self.fused_loss and w.dtype == torch.bfloat16 and may_fuse(w) and as_made(self.wte, nn.Embedding) and as_made(self.wpe, nn.Embedding):
+        if self.fused_loss and w.dtype == torch.bfloat16 and may_fuse(w, idx) and as_made(self.wte, nn.Embedding) and as_made(self.wpe, nn.Embedding):
             x = _ext.load().decoder_embed(idx, w, self.wpe.weight, self.grad_sink)      # None where the kernels do not cover the case
         if x is not None:
             pending = bias = None
@@ -183,7 +183,7 @@ class GPT2(nn.Module):
             for blk in self.blocks:
                 x = blk(x)
             x = self.ln_f(x)
-        if targets is not None and self.fused_loss and x.dtype == torch.bfloat16 and may_fuse(x):
+        if targets is not None and self.fused_loss and x.dtype == torch.bfloat16 and may_fuse(x, w, targets):
             loss = _ext.load().decoder_head_loss(x.view(b * s, -1), w, targets, self.cfg.vocab_size, False, self.grad_sink)
             if loss is not None:
                 return loss

@@ -190,7 +190,7 @@ class Llama(nn.Module):
             h = ext.llama_final_norm(x, pending, self.norm.weight, self.norm.eps, self.grad_sink)
         if h is None:
             h = self.norm(x if pending is None else x + pending)
-        if targets is not None and as_made(self.head, nn.Linear) and self.head.bias is None:
+        if targets is not None and as_made(self.head, nn.Linear) and self.head.bias is None and may_fuse(h, targets):
             loss = ext.decoder_head_loss(h, self.head.weight, targets, self.head.weight.shape[0], True, self.grad_sink)
             if loss is not None:
                 return loss

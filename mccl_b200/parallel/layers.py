@@ -182,7 +182,7 @@ class ExpertParallelMoE(nn.Module):
             from ..ops import moe as M
             # The kernels route as `route` here does with the router made above.
             stock = (type(self).route is ExpertParallelMoE.route and "route" not in self.__dict__ and as_made(self.router, nn.Linear)
-                     and self.router.bias is None and may_fuse(x))
+                     and self.router.bias is None and may_fuse(x, self.w_in, self.w_out))
             if n == 1 and stock:                                              # nothing to exchange: the whole layer is one node
                 y = _ext.load().moe_layer(x, self.router.weight, self.w_in, self.w_out, c)
                 if y is not None:

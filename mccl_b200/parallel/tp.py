@@ -136,7 +136,7 @@ class FusedTensorParallelMLP(torch.nn.Module):
         self.layer = TensorParallelFFN(comm, tokens, hidden, ffn, self.w_up.data, self.w_down.data, when_used=True)
 
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
-        if self.layer.comm.size == 1 and may_fuse(x_shard) and x_shard.shape == (self.layer.tokens, self.layer.hidden):     # nothing to gather or scatter: one node
+        if self.layer.comm.size == 1 and may_fuse(x_shard, self.w_up, self.w_down) and x_shard.shape == (self.layer.tokens, self.layer.hidden):     # nothing to gather or scatter: one node
             y = _ext.load().mlp(x_shard, self.w_up, self.w_down)
             if y is not None:
                 return y

@@ -16,6 +16,7 @@ try:                                      # `with torch.device(...)` and torch.s
     from torch.utils._device import DeviceContext as _DeviceContext
 except ImportError:
     _modes = None
+_mode_count = getattr(torch._C, "_len_torch_function_stack", lambda: 1)
 
 _FUNCTIONS = ("linear", "embedding", "layer_norm", "gelu", "silu", "softmax", "scaled_dot_product_attention", "cross_entropy")
 _STOCK = tuple(getattr(F, n) for n in _FUNCTIONS)
@@ -27,14 +28,14 @@ def undisturbed() -> bool:
     module, or __torch_function__ mode."""
     if torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or _has_any_global_hook():
         return False
-    if torch._C._len_torch_function_stack() and (_modes is None or any(type(m) is not _DeviceContext for m in _modes())):
+    if _mode_count() and (_modes is None or any(type(m) is not _DeviceContext for m in _modes())):
         return False
     return (F.linear, F.embedding, F.layer_norm, F.gelu, F.silu, F.softmax, F.scaled_dot_product_attention, F.cross_entropy) == _STOCK
 
 
-def may_fuse(x: torch.Tensor) -> bool:
-    """Whether the kernels' nodes may take x here."""
-    return x.is_cuda and type(x) in _PLAIN and undisturbed()
+def may_fuse(x: torch.Tensor, *others: torch.Tensor) -> bool:
+    """Whether the kernels' nodes may take x, with these others, here."""
+    return x.is_cuda and type(x) in _PLAIN and all(type(t) in _PLAIN for t in others) and undisturbed()
 
 
 def as_made(m: nn.Module, cls: type) -> bool:

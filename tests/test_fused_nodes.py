@@ -390,6 +390,30 @@ def test_torch_func_and_tracing_take_the_plain_route():
 
 
 @gpu
+def test_weights_of_another_class_are_asked():
+    from mccl_b200.parallel.layers import ExpertParallelMoE
+    seen = []
+
+    class Mine(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(func)
+            with torch._C.DisableTorchFunctionSubclass():
+                return func(*args, **(kwargs or {}))
+
+    idx, tgt = _batch()
+    layer = ExpertParallelMoE(_comm(), 64, 64, 2, 64, device="cuda", dtype=torch.bfloat16, fused=True)
+    layer._parameters["w_in"] = layer.w_in.detach().as_subclass(Mine)
+    layer(torch.randn(64, 64, device="cuda").to(torch.bfloat16))
+    assert seen
+    model = _gpt2()
+    model.wte._parameters["weight"] = model.wte.weight.detach().as_subclass(Mine)
+    seen.clear()
+    model(idx, tgt)
+    assert any(getattr(f, "__name__", "") == "linear" for f in seen)       # the tied projection
+
+
+@gpu
 def test_moe_subclass_routes_its_own_way():
     from mccl_b200.parallel.layers import ExpertParallelMoE
 
